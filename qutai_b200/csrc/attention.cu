@@ -5,11 +5,13 @@
 // src/qutai/backends/cuda/lm.cu:91-285 (wmma), CPU statement src/qutai/backends/cpu_lm.py:141-201.  Like those kernels
 // this never writes the time x time scores: keys and values stream through shared memory in blocks of 128 positions.
 //
-// One CTA per (sequence, head, block of 128 query positions); 6 warps: warp 0 asks TMA for the tiles (3-D tensor maps
-// [batch][time][heads * 64], so positions past the end of a sequence arrive as zeros and no tile reaches into the next
-// sequence), warp 1 issues the MMAs (one thread), warps 2-5 own one query row per thread (the TMEM lane of that row).
-//   forward, per key block:  S = Q K^T (TMEM) -> rows: max, exp2, sum; P (bf16) into shared memory in the K-major
-//   operand layout -> O_j = P V (TMEM) -> rows: O = O * alpha + O_j in registers.
+// Warp 0 of a CTA asks TMA for the tiles (3-D tensor maps [batch][time][heads * 64], so positions past the end of a sequence
+// arrive as zeros and no tile reaches into the next sequence), warp 1 issues the MMAs (one elected thread), the row warps
+// own one TMEM lane per thread.
+//   forward, per (sequence, head, block of 128 queries) and key block:  S = Q K^T -> rows: max, exp2, sum, P -> O += P V,
+//   accumulated in tensor memory and rescaled only when a maximum has risen by more than 2^8.  P never passes through shared
+//   memory: the rows read the scores out of tensor memory and put P, rounded to bf16, back there, where the next product
+//   takes it as its A operand; the next block's scores are formed meanwhile.
 //   backward for dq, per key block:  S = Q K^T and dP = dO V^T (TMEM) -> rows: P = exp(S / 8 - lse),
 //   dS = P (dP - delta) / 8 (bf16, shared memory) -> dQ += dS K (TMEM, accumulated over the key blocks).
 //   backward for dk, dv, one CTA per (sequence, key/value head, key block), over the query heads of the group and
@@ -25,8 +27,8 @@ namespace {
 constexpr int D = 64;                 // head width
 constexpr int BLOCK = 128;            // query rows of a CTA = key positions of a block
 constexpr int TILE_BYTES = BLOCK * D * 2;          // 16 KiB: 128 rows x 128 bytes
-constexpr int SLAB_BYTES = BLOCK * 128;            // one 64-column half of a 128 x 128 bf16 operand tile
 constexpr int THREADS = 192;              // forward: TMA warp, MMA warp, four row warps
+constexpr int SLAB_BYTES = BLOCK * 128;            // one 64-column half of a 128 x 128 bf16 operand tile
 // The backward kernels have no reduction along a row (lse and delta are known), so the columns of a block are split
 // between several warps per 32 rows: one warp per scheduler cannot hide its own arithmetic latency (measured: 4900 of
 // the 7300 cycles of a dk/dv iteration were the four row warps' work).
@@ -59,8 +61,14 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 }
 __device__ __forceinline__ float exp2_fast(float x) {
     float y;
-    asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+// 32 accumulator columns of one row, scaled, as 64 bytes of bf16
+__device__ __forceinline__ void store_row32(uint4* dst, const uint32_t* r, float scale) {
+    auto two = [&](int c) { return pack2(__uint_as_float(r[c]) * scale, __uint_as_float(r[c + 1]) * scale); };
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) dst[c / 8] = make_uint4(two(c), two(c + 2), two(c + 4), two(c + 6));
 }
 // 32 consecutive values of this thread's row (columns [32 c, 32 c + 32) of a 128-column bf16 operand tile made of two
 // 64-column slabs) into shared memory in the K-major layout the MMA reads: 128-byte rows, 16-byte piece j of row r at
@@ -84,6 +92,8 @@ struct Wait {   // bounded waits of one thread; the first that runs out marks th
         if (!*abort_flag) { *abort_flag = 1; atomicExch(status, STATUS_ATTENTION_WAIT); }
         return false;
     }
+    // the same for a whole warp: all lanes go on, or none does
+    __device__ __forceinline__ bool all(uint32_t bar, uint32_t parity) const { return __all_sync(0xffffffffu, (*this)(bar, parity)); }
 };
 
 // a CTA that gave up leaves its copies and MMAs in flight a bounded time to land before its shared memory and TMEM go away
@@ -96,32 +106,33 @@ __device__ __forceinline__ void linger_after_abort(const volatile int* abort_fla
 // ------------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 attention_forward_kernel(const __grid_constant__ AttentionParams p) {
-    // No static shared memory and a 1 KiB-aligned dynamic block: 112 KiB of tiles + the barriers and two words fit
-    // twice into an SM, and the second resident CTA is what overlaps one CTA's row work with another's MMAs.
+    // No static shared memory and a 1 KiB-aligned dynamic block: 80 KiB of tiles and half of the tensor memory per CTA,
+    // so two are resident per SM and one's exponentials run beside the other's waits.
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int blocks = (p.time + BLOCK - 1) / BLOCK;
     // heaviest query blocks first: the last block of a sequence has the most key blocks to walk
-    const int i = blocks - 1 - (int)(blockIdx.x % blocks);
-    const int h = (int)(blockIdx.x / blocks) % p.heads, b = (int)(blockIdx.x / blocks) / p.heads;
+    const int heads_all = p.heads * p.batch;
+    const int i = blocks - 1 - (int)(blockIdx.x / heads_all);
+    const int h = (int)(blockIdx.x % heads_all) % p.heads, b = (int)(blockIdx.x % heads_all) / p.heads;
     const int g = h / (p.heads / p.kv_heads);
     const int n = i + 1;                       // key blocks 0 .. i
     const uint32_t base = smem_u32(smem_raw);
-    const uint32_t q_tile = base, k_tile = base + TILE_BYTES, v_tile = k_tile + 2 * TILE_BYTES, p_tile = v_tile + 2 * TILE_BYTES;
-    const uint32_t bars = p_tile + 2 * SLAB_BYTES;
-    enum { Q_FULL = 0, KV_FULL = 1, KV_EMPTY = 3, S_FULL = 5, P_FULL = 6, O_FULL = 7, O_TAKEN = 8, BARS = 9 };
+    const uint32_t q_tile = base, k_tile = base + TILE_BYTES, v_tile = k_tile + 2 * TILE_BYTES;
+    const uint32_t bars = v_tile + 2 * TILE_BYTES;
+    enum { Q_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, S_FULL = 9, S_TAKEN = 10, P_FULL = 11, O_DONE = 12, BARS = 13 };
     auto bar = [&](int which) { return bars + 8u * which; };
-    uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + 5 * TILE_BYTES + 2 * SLAB_BYTES + 8 * BARS);
-    volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + 5 * TILE_BYTES + 2 * SLAB_BYTES + 8 * BARS + 4);
+    uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + 5 * TILE_BYTES + 8 * BARS);
+    volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + 5 * TILE_BYTES + 8 * BARS + 4);
     if (base & 1023u) {   // the operand tiles need the alignment the declaration asks for
         if (threadIdx.x == 0) atomicExch(p.status, STATUS_ATTENTION_WAIT + 1);
         return;
     }
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int w = 0; w < BARS; ++w) mbar_init(bar(w), (w == P_FULL || w == O_TAKEN) ? 4 : 1);
+        for (int w = 0; w < BARS; ++w) mbar_init(bar(w), (w == S_TAKEN || w == P_FULL) ? 4 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         prefetch_map(&p.map_q); prefetch_map(&p.map_k); prefetch_map(&p.map_v);
     }
@@ -133,7 +144,7 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem_base;
-    const uint32_t tmem_s = tmem, tmem_o = tmem + 128;
+    const uint32_t tmem_s = tmem, tmem_o = tmem + 128, tmem_p = tmem + 192;    // 128 + 64 + 64 (bf16 pairs) columns
     const Wait wait{&s_abort, p.status};
 
     if (warp == 0) {
@@ -142,114 +153,153 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
             tma_load_3d(&p.map_q, q_tile, bar(Q_FULL), h * D, i * BLOCK, b);
             for (int j = 0; j < n && !s_abort; ++j) {
                 const int st = j & 1;
-                if (!wait(bar(KV_EMPTY + st), ((uint32_t)(j >> 1) & 1u) ^ 1u)) break;
-                mbar_expect_tx(bar(KV_FULL + st), 2 * TILE_BYTES);
-                tma_load_3d(&p.map_k, k_tile + st * TILE_BYTES, bar(KV_FULL + st), g * D, j * BLOCK, b);
-                tma_load_3d(&p.map_v, v_tile + st * TILE_BYTES, bar(KV_FULL + st), g * D, j * BLOCK, b);
+                const uint32_t parity = ((uint32_t)(j >> 1) & 1u) ^ 1u;
+                if (!wait(bar(K_EMPTY + st), parity)) break;
+                mbar_expect_tx(bar(K_FULL + st), TILE_BYTES);
+                tma_load_3d(&p.map_k, k_tile + st * TILE_BYTES, bar(K_FULL + st), g * D, j * BLOCK, b);
+                if (!wait(bar(V_EMPTY + st), parity)) break;
+                mbar_expect_tx(bar(V_FULL + st), TILE_BYTES);
+                tma_load_3d(&p.map_v, v_tile + st * TILE_BYTES, bar(V_FULL + st), g * D, j * BLOCK, b);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc<false, false, 128>(128), idesc_o = make_idesc<false, true, 128>(D);
-            bool ok = wait(bar(Q_FULL), 0);
-            for (int j = 0; ok && j < n; ++j) {
-                const int st = j & 1;
-                ok = wait(bar(KV_FULL + st), (uint32_t)(j >> 1) & 1u);
-                if (!ok) break;
-                tc_fence_after();
-                // S = Q K^T: both K-major, contraction over the 64 columns (the rows that read S of the block
-                // before have all arrived on P_FULL, which was waited for before that block's P V)
+        constexpr uint32_t idesc_s = make_idesc<false, false, 128>(128), idesc_o = make_idesc<false, true, 128>(D);
+        // S = Q K^T of key block j: both K-major, contraction over the 64 columns
+        auto scores = [&](int j) {
+            const int st = j & 1;
+            if (!wait.all(bar(K_FULL + st), (uint32_t)(j >> 1) & 1u)) return false;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk)
                     umma_bf16(tmem_s, make_desc(q_tile + kk * 32, 16, 1024), make_desc(k_tile + st * TILE_BYTES + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
                 umma_commit(bar(S_FULL));
-                ok = wait(bar(P_FULL), (uint32_t)j & 1u);
-                if (ok && j > 0) ok = wait(bar(O_TAKEN), (uint32_t)(j - 1) & 1u);
-                if (!ok) break;
-                tc_fence_after();
-                // O_j = P V: P K-major (two 64-column slabs), V as it lies in memory (rows = key positions) is the
-                // MN-major operand: 16 positions every 2 KiB
+                umma_commit(bar(K_EMPTY + st));
+            }
+            __syncwarp();
+            return true;
+        };
+        bool ok = wait.all(bar(Q_FULL), 0) && scores(0);
+        for (int j = 0; ok && j < n; ++j) {
+            const int st = j & 1;
+            // the scores of the next block as soon as the rows hold this block's in registers
+            if (j + 1 < n) ok = wait.all(bar(S_TAKEN), (uint32_t)j & 1u) && scores(j + 1);
+            if (ok) ok = wait.all(bar(V_FULL + st), (uint32_t)(j >> 1) & 1u);
+            if (ok) ok = wait.all(bar(P_FULL), (uint32_t)j & 1u);
+            if (!ok) break;
+            tc_fence_after();
+            // O += P V: P from tensor memory, V as it lies in memory (rows = key positions) is the MN-major operand:
+            // 16 positions every 2 KiB
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < BLOCK / 16; ++kk)
-                    umma_bf16(tmem_o, make_desc(p_tile + (kk >> 2) * SLAB_BYTES + (kk & 3) * 32, 16, 1024),
-                              make_desc(v_tile + st * TILE_BYTES + kk * 2048, 8192, 1024), idesc_o, kk ? 1u : 0u);
-                umma_commit(bar(O_FULL));
-                umma_commit(bar(KV_EMPTY + st));
+                    umma_bf16_ts(tmem_o, tmem_p + kk * 8, make_desc(v_tile + st * TILE_BYTES + kk * 2048, 8192, 1024), idesc_o, (j | kk) ? 1u : 0u);
+                umma_commit(bar(O_DONE));
+                umma_commit(bar(V_EMPTY + st));
             }
-            // the last commit has arrived before this CTA's shared memory can go to another one
-            if (ok) wait(bar(KV_EMPTY + ((n - 1) & 1)), (uint32_t)((n - 1) >> 1) & 1u);
+            __syncwarp();
         }
+        // the last commit has arrived before this CTA's shared memory can go to another one
+        if (ok) wait.all(bar(V_EMPTY + ((n - 1) & 1)), (uint32_t)((n - 1) >> 1) & 1u);
     } else {
         const int quad = warp & 3, row = quad * 32 + lane;
         const int tq = i * BLOCK + row;                      // this thread's query position
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         const float scale2 = 0.125f * LOG2E;                 // 1 / sqrt(64), in the exponent of 2
-        float m = -INFINITY, l = 0.f, o[D];
-#pragma unroll
-        for (int c = 0; c < D; ++c) o[c] = 0.f;
+        const uint64_t scale_pair = pair2(scale2, scale2);
+        float m = -INFINITY, base2 = 0.f, l = 0.f;           // base2 = m * scale2, rounded
         bool ok = true;
         for (int j = 0; ok && j < n; ++j) {
-            ok = wait(bar(S_FULL), (uint32_t)j & 1u);
+            ok = wait.all(bar(S_FULL), (uint32_t)j & 1u);
             if (!ok) break;
             tc_fence_after();
-            const bool diagonal = j == i;
-            float peak = m;
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                uint32_t r[32];
-                tmem_ld32(tmem_s + lane_base + c * 32, r);
-                tmem_ld_wait();
+            uint32_t s[BLOCK];
 #pragma unroll
-                for (int e = 0; e < 32; ++e)
-                    if (!diagonal || c * 32 + e <= row) peak = fmaxf(peak, __uint_as_float(r[e]));
+            for (int c = 0; c < 4; ++c) tmem_ld32(tmem_s + lane_base + c * 32, s + c * 32);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(S_TAKEN));
+            if (j == i) {
+#pragma unroll
+                for (int c = 0; c < BLOCK; ++c)
+                    if (c > row) s[c] = 0xff800000u;         // -inf
             }
-            const float alpha = exp2_fast((m - peak) * scale2);   // 0 in the first block (m = -inf, peak finite: column 0 is never masked)
-            float total = 0.f;
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                uint32_t r[32], packed[16];
-                tmem_ld32(tmem_s + lane_base + c * 32, r);
-                tmem_ld_wait();
+            float peak4[4] = {__uint_as_float(s[0]), __uint_as_float(s[1]), __uint_as_float(s[2]), __uint_as_float(s[3])};
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    float p0 = exp2_fast((__uint_as_float(r[e]) - peak) * scale2), p1 = exp2_fast((__uint_as_float(r[e + 1]) - peak) * scale2);
-                    if (diagonal && c * 32 + e > row) p0 = 0.f;
-                    if (diagonal && c * 32 + e + 1 > row) p1 = 0.f;
-                    total += p0 + p1;
-                    packed[e >> 1] = pack2(p0, p1);
+            for (int c = 4; c < BLOCK; ++c) peak4[c & 3] = fmaxf(peak4[c & 3], __uint_as_float(s[c]));
+            const float peak = fmaxf(fmaxf(peak4[0], peak4[1]), fmaxf(peak4[2], peak4[3]));
+            // The base of the exponentials is the maximum so far.  (Letting it lag behind by up to 2^8 would leave O alone in
+            // most blocks, but then the largest probability of a row is no longer an exact 1 in bf16: 2.05e-3 instead of
+            // 1.74e-3 from the exact result for scores of standard deviation 4.)
+            if (j == 0) {
+                m = peak;
+                base2 = m * scale2;
+            } else {
+                if (__any_sync(0xffffffffu, peak > m)) {
+                    const float m_new = fmaxf(m, peak), alpha = exp2_fast((m - m_new) * scale2);
+                    m = m_new;
+                    base2 = m * scale2;
+                    l *= alpha;
+                    ok = wait.all(bar(O_DONE), (uint32_t)(j - 1) & 1u);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t o[16];
+                        tmem_ld16(tmem_o + lane_base + c * 16, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+                        tmem_st16(tmem_o + lane_base + c * 16, o);
+                    }
                 }
-                store_row32(p_tile, row, c, packed);
             }
-            l = l * alpha + total;
-            m = peak;
-            fence_async_shared();
+            const uint64_t base_pair = pair2(-base2, -base2);
+            uint64_t total2[2] = {0, 0};
+            uint32_t packed[BLOCK / 2];
+#pragma unroll
+            for (int c = 0; c < BLOCK; c += 2) {
+                float x0, x1;
+                unpair2(fma2(pair2(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale_pair, base_pair), x0, x1);
+                const float p0 = exp2_fast(x0), p1 = exp2_fast(x1);
+                total2[(c >> 1) & 1] = add2(total2[(c >> 1) & 1], pair2(p0, p1));
+                packed[c >> 1] = pack2(p0, p1);
+            }
+            if (j > 0) {   // the product that reads the P of the block before is done
+                ok = wait.all(bar(O_DONE), (uint32_t)(j - 1) & 1u);
+                if (!ok) break;
+                tc_fence_after();
+            }
+            tmem_st32(tmem_p + lane_base, packed);
+            tmem_st32(tmem_p + lane_base + 32, packed + 32);
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(P_FULL));
-            ok = wait(bar(O_FULL), (uint32_t)j & 1u);
-            if (!ok) break;
-            tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint32_t r[32];
-                tmem_ld32(tmem_o + lane_base + c * 32, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int e = 0; e < 32; ++e) o[c * 32 + e] = o[c * 32 + e] * alpha + __uint_as_float(r[e]);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(O_TAKEN));
+            float t0, t1;
+            unpair2(add2(total2[0], total2[1]), t0, t1);
+            l += t0 + t1;
         }
-        if (ok && tq < p.time) {
-            const float inverse = 1.f / l;
-            const long long at = ((long long)b * p.time + tq) * p.heads + h;
-            uint4* dst = reinterpret_cast<uint4*>(p.out + at * D);
+        if (ok) ok = wait.all(bar(O_DONE), (uint32_t)(n - 1) & 1u);
+        if (ok) {
+            tc_fence_after();
+            uint32_t o[D];
+            tmem_ld32(tmem_o + lane_base, o);
+            tmem_ld32(tmem_o + lane_base + 32, o + 32);
+            tmem_ld_wait();
+            if (tq < p.time) {
+                const float inverse = 1.f / l;
+                const long long at = ((long long)b * p.time + tq) * p.heads + h;
+                uint4* dst = reinterpret_cast<uint4*>(p.out + at * D);
+                auto value = [&](int c) { return __uint_as_float(o[c]) * inverse; };
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c)
-                dst[c] = make_uint4(pack2(o[8 * c] * inverse, o[8 * c + 1] * inverse), pack2(o[8 * c + 2] * inverse, o[8 * c + 3] * inverse),
-                                    pack2(o[8 * c + 4] * inverse, o[8 * c + 5] * inverse), pack2(o[8 * c + 6] * inverse, o[8 * c + 7] * inverse));
-            p.lse[at] = m * 0.125f + __logf(l);
+                for (int c = 0; c < D; c += 8)
+                    dst[c / 8] = make_uint4(pack2(value(c), value(c + 1)), pack2(value(c + 2), value(c + 3)),
+                                            pack2(value(c + 4), value(c + 5)), pack2(value(c + 6), value(c + 7)));
+                // log sum exp = ln2 (base2 + log2 l); base2 is m * scale2 rounded, the fma gives back what the rounding took
+                p.lse[at] = m * 0.125f + (__logf(l) - fmaf(m, scale2, -base2) * 0.69314718056f);
+            }
         }
     }
     linger_after_abort(&s_abort);
@@ -601,7 +651,7 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
     }
 }
 
-constexpr int FORWARD_SMEM = 5 * TILE_BYTES + 2 * SLAB_BYTES + 128;
+constexpr int FORWARD_SMEM = 5 * TILE_BYTES + 128;
 constexpr int DQ_KV = 64;
 constexpr int DQ_SMEM = 2 * TILE_BYTES + 4 * DQ_KV * 128 + (DQ_KV / 64) * SLAB_BYTES + 128;
 constexpr int DKV_SMEM = 1024 + 6 * TILE_BYTES + 4 * SLAB_BYTES + 128;

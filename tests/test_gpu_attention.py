@@ -100,3 +100,17 @@ def test_attention_rejects_what_it_does_not_cover():
     kv2 = Tensor(to_device(np.zeros((1, 4, 128)), "bfloat16"), (1, 4, 128))
     with pytest.raises(ValueError):
         attention(q3, kv2, kv2, 3, 2)                   # heads not a multiple of kv_heads
+
+
+@pytest.mark.parametrize("batch,time,heads,kv_heads,scale", [(1, 2, 2, 1, 1.0), (2, 63, 2, 2, 1.0), (1, 65, 3, 1, 1.0), (1, 127, 2, 1, 1.0),
+                                                             (1, 255, 4, 2, 1.0), (2, 257, 2, 1, 1.0), (1, 640, 4, 4, 3.0)])
+def test_attention_at_the_edges_of_blocks_and_with_growing_scores(batch, time, heads, kv_heads, scale):
+    """Lengths one off the 64- and 128-position blocks, and scores that grow along the sequence, so that the maximum of a
+    row rises by more than 2^8 between its key blocks and the accumulated output has to be rescaled."""
+    q, k, v, grad = attention_inputs(batch, time, heads, kv_heads, seed=time * 5 + heads, scale=scale)
+    k = oracle.round_bf16(k * (1.0 + 3.0 * np.arange(time)[None, :, None] / time))
+    out, lse = oracle.attention_forward(q, k, v, heads, kv_heads)
+    dq, dk, dv = oracle.attention_backward(grad, q, k, v, out, lse, heads, kv_heads)
+    # with scores of scale^2 the softmax is nearly one-hot and dS = P (dP - delta) cancels: the element bar is that of the
+    # 2048-position test there
+    check(run_attention(q, k, v, grad, heads, kv_heads), dict(out=out, dq=dq, dk=dk, dv=dv), element_tol=0.2 if scale > 1 else BF16_ELEMENT_TOL)
