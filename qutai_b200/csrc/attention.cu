@@ -7,16 +7,19 @@
 //
 // Warp 0 of a CTA asks TMA for the tiles (3-D tensor maps [batch][time][heads * 64], so positions past the end of a sequence
 // arrive as zeros and no tile reaches into the next sequence), warp 1 issues the MMAs (one elected thread), the row warps
-// own one TMEM lane per thread.
-//   forward, per (sequence, head, block of 128 queries) and key block:  S = Q K^T -> rows: max, exp2, sum, P -> O += P V,
-//   accumulated in tensor memory and rescaled only when a maximum has risen by more than 2^8.  P never passes through shared
-//   memory: the rows read the scores out of tensor memory and put P, rounded to bf16, back there, where the next product
-//   takes it as its A operand; the next block's scores are formed meanwhile.
-//   backward for dq, per key block:  S = Q K^T and dP = dO V^T (TMEM) -> rows: P = exp(S / 8 - lse),
-//   dS = P (dP - delta) / 8 (bf16, shared memory) -> dQ += dS K (TMEM, accumulated over the key blocks).
-//   backward for dk, dv, one CTA per (sequence, key/value head, key block), over the query heads of the group and
-//   the query blocks at or after it:  S, dP as above -> P and dS (shared memory) -> dV += P^T dO, dK += dS^T Q
-//   (TMEM; the K-major tile of P read as an MN-major operand is P^T, no transposed copy).
+// own one TMEM lane per thread.  Probabilities never pass through shared memory: the rows read the scores out of tensor
+// memory and put P (dS), rounded to bf16, back there, where the next product takes it as its A operand.
+//   forward, per item (sequence, head, block of 128 queries) and key block:  S = Q K^T -> rows: max, exp2, sum, P -> O += P V,
+//   accumulated in tensor memory and rescaled there when a row's maximum has risen.
+//   backward for dq, per item and key block as well:  S = Q K^T, dP = dO V^T -> rows: P = exp(S / 8 - lse), dS = P (dP - delta) -> dQ += dS K.
+//   backward for dk, dv, per (sequence, key/value head, key block), over the query heads of the group and the query blocks
+//   at or after it, everything transposed (lanes = key positions):  S^T = K Q^T, dP^T = V dO^T -> rows: P^T, dS^T ->
+//   dV += P^T dO, dK += dS^T Q.
+// The products of the next block are issued before the rows have finished with this one (S has a second buffer in the
+// backward and is taken into registers at once in the forward), so the row warps rarely wait for the tensor cores; what
+// bounds them is the exponential unit, 1024 cycles per 128 x 128 block and SM, and the latency of their own chain beside it.
+// 4 sequences x 2048 positions, 16 heads in 4 groups (L2 flushed): forward 144 -> 75 us, backward 472 -> 191 against the form
+// with P and dS in shared memory and one block in flight.
 // Every wait is bounded; on expiry the CTA records a code in the library's status word and leaves.
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -28,11 +31,8 @@ constexpr int D = 64;                 // head width
 constexpr int BLOCK = 128;            // query rows of a CTA = key positions of a block
 constexpr int TILE_BYTES = BLOCK * D * 2;          // 16 KiB: 128 rows x 128 bytes
 constexpr int THREADS = 192;              // forward: TMA warp, MMA warp, four row warps
-constexpr int SLAB_BYTES = BLOCK * 128;            // one 64-column half of a 128 x 128 bf16 operand tile
-// The backward kernels have no reduction along a row (lse and delta are known), so the columns of a block are split
-// between several warps per 32 rows: one warp per scheduler cannot hide its own arithmetic latency (measured: 4900 of
-// the 7300 cycles of a dk/dv iteration were the four row warps' work).
-constexpr int DQ_PARTS = 2, DKV_PARTS = 4;
+// Row warps per 32 rows of the backward kernels, which share the columns of a block between them
+constexpr int DQ_PARTS = 1, DKV_PARTS = 2;
 constexpr int DQ_THREADS = 64 + 128 * DQ_PARTS, DKV_THREADS = 64 + 128 * DKV_PARTS;
 constexpr float LOG2E = 1.4426950408889634f;
 enum { STATUS_ATTENTION_WAIT = 301 };
@@ -48,6 +48,7 @@ struct alignas(64) AttentionParams {
     float* delta;                 // [batch * time * heads]  sum_j grad_out * out of every row
     int* status;
     int batch, time, heads, kv_heads;
+    int split;                    // backward for dk, dv: CTAs per key block (cluster size)
 };
 
 __device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint32_t dst, uint32_t bar, int c0, int c1, int c2) {
@@ -70,19 +71,15 @@ __device__ __forceinline__ void store_row32(uint4* dst, const uint32_t* r, float
 #pragma unroll
     for (int c = 0; c < 32; c += 8) dst[c / 8] = make_uint4(two(c), two(c + 2), two(c + 4), two(c + 6));
 }
-// 32 consecutive values of this thread's row (columns [32 c, 32 c + 32) of a 128-column bf16 operand tile made of two
-// 64-column slabs) into shared memory in the K-major layout the MMA reads: 128-byte rows, 16-byte piece j of row r at
-// j ^ (r & 7)
-__device__ __forceinline__ void store_row32(uint32_t tile, int row, int c, const uint32_t* packed16) {
-    const uint32_t slab = tile + (uint32_t)(c >> 1) * SLAB_BYTES + (uint32_t)row * 128u;
-    const uint32_t twist = (uint32_t)row & 7u;
-#pragma unroll
-    for (int piece = 0; piece < 4; ++piece) {
-        const uint32_t at = (((uint32_t)(c & 1) * 4u + (uint32_t)piece) ^ twist) * 16u;
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(slab + at), "r"(packed16[4 * piece]), "r"(packed16[4 * piece + 1]),
-                     "r"(packed16[4 * piece + 2]), "r"(packed16[4 * piece + 3]) : "memory");
-    }
+__device__ __forceinline__ void load_shared4(uint32_t at, float* v) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
 }
+__device__ __forceinline__ void load_cluster4(uint32_t at, float* v) {
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
+}
+// Where the 16 contraction elements [16 kk, 16 kk + 16) of a bf16 operand start that the rows wrote over the scores they had
+// read: a thread keeps to its own COLS columns, P (or the only operand) in their first half, dS in their second
+template <int COLS> __device__ __forceinline__ constexpr uint32_t p_column(int kk) { return (uint32_t)(kk * 16 / COLS * COLS + kk * 16 % COLS / 2); }
 
 struct Wait {   // bounded waits of one thread; the first that runs out marks the CTA
     volatile int* abort_flag;
@@ -313,50 +310,50 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
 
 
 // ------------------------------------------------------------------------------------------------
-// backward, part 1: dq (and delta), one CTA per (sequence, head, query block); key blocks of KV positions.  With
-// KV = 64 a CTA needs 192 TMEM columns and 80 KiB, so two are resident per SM and overlap each other's chains.
+// backward, part 1: dq (and delta), one CTA per (sequence, head, query block); key blocks of 64 positions.  A CTA needs
+// 256 TMEM columns (two S, one dP, dQ) and 80 KiB, so two are resident per SM.
 // ------------------------------------------------------------------------------------------------
-template <int KV>
-__global__ void __launch_bounds__(DQ_THREADS)
+constexpr int DQ_KV = 64, DQ_TILE = DQ_KV * 128, DQ_STAGES = 3;
+constexpr int DQ_TILES = 2 * TILE_BYTES + 2 * DQ_STAGES * DQ_TILE;
+constexpr int DQ_SMEM = DQ_TILES + 128;
+
+__global__ void __launch_bounds__(DQ_THREADS, 2)
 attention_dq_kernel(const __grid_constant__ AttentionParams p) {
-    constexpr int KV_TILE = KV * 128, SLABS = KV / 64, TMEM_COLUMNS = KV == 64 ? 256 : 512;
-    constexpr int TILES = 2 * TILE_BYTES + 4 * KV_TILE + SLABS * SLAB_BYTES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int blocks = (p.time + BLOCK - 1) / BLOCK;
-    const int i = blocks - 1 - (int)(blockIdx.x % blocks);
-    const int h = (int)(blockIdx.x / blocks) % p.heads, b = (int)(blockIdx.x / blocks) / p.heads;
+    const int heads_all = p.heads * p.batch;
+    const int i = blocks - 1 - (int)(blockIdx.x / heads_all);
+    const int h = (int)(blockIdx.x % heads_all) % p.heads, b = (int)(blockIdx.x % heads_all) / p.heads;
     const int g = h / (p.heads / p.kv_heads);
-    const int n = (i + 1) * (BLOCK / KV);      // key blocks that hold a position <= the last query of this block
+    const int n = (i + 1) * (BLOCK / DQ_KV);   // key blocks that hold a position <= the last query of this block
     const uint32_t base = smem_u32(smem_raw);
-    const uint32_t q_tile = base, do_tile = base + TILE_BYTES, k_tile = do_tile + TILE_BYTES, v_tile = k_tile + 2 * KV_TILE,
-                   ds_tile = v_tile + 2 * KV_TILE;
-    const uint32_t bars = ds_tile + SLABS * SLAB_BYTES;
-    enum { Q_FULL = 0, KV_FULL = 1, KV_EMPTY = 3, SP_FULL = 5, DS_FULL = 6, DQ_DONE = 7, BARS = 8 };
+    const uint32_t q_tile = base, do_tile = base + TILE_BYTES, k_tile = do_tile + TILE_BYTES, v_tile = k_tile + DQ_STAGES * DQ_TILE;
+    const uint32_t bars = base + DQ_TILES;
+    enum { Q_FULL = 0, KV_FULL = 1, KV_EMPTY = KV_FULL + DQ_STAGES, S_FULL = KV_EMPTY + DQ_STAGES, DP_FULL = S_FULL + 2, DS_FULL, DQ_DONE, BARS };
     auto bar = [&](int which) { return bars + 8u * which; };
-    uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + TILES + 8 * BARS);
-    volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + TILES + 8 * BARS + 4);
+    uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + DQ_TILES + 8 * BARS);
+    volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + DQ_TILES + 8 * BARS + 4);
     if (base & 1023u) {
         if (threadIdx.x == 0) atomicExch(p.status, STATUS_ATTENTION_WAIT + 1);
         return;
     }
-    const CUtensorMap* map_k = KV == 64 ? &p.map_k2 : &p.map_k;
-    const CUtensorMap* map_v = KV == 64 ? &p.map_v2 : &p.map_v;
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int w = 0; w < BARS; ++w) mbar_init(bar(w), w == DS_FULL ? 4 * DQ_PARTS : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        prefetch_map(&p.map_q); prefetch_map(map_k); prefetch_map(map_v); prefetch_map(&p.map_do);
+        prefetch_map(&p.map_q); prefetch_map(&p.map_k2); prefetch_map(&p.map_v2); prefetch_map(&p.map_do);
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(TMEM_COLUMNS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(256) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem_base;
-    const uint32_t tmem_s = tmem, tmem_dp = tmem + KV, tmem_dq = tmem + 2 * KV;
+    // S of block j in columns 64 (j & 1) ..; the rows put dS (bf16 pairs) back over the columns they read
+    const uint32_t tmem_dp = tmem + 2 * DQ_KV, tmem_dq = tmem + 3 * DQ_KV;
     const Wait wait{&s_abort, p.status};
 
     if (warp == 0) {
@@ -364,48 +361,69 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
             mbar_expect_tx(bar(Q_FULL), 2 * TILE_BYTES);
             tma_load_3d(&p.map_q, q_tile, bar(Q_FULL), h * D, i * BLOCK, b);
             tma_load_3d(&p.map_do, do_tile, bar(Q_FULL), h * D, i * BLOCK, b);
+            int st = 0;
+            uint32_t parity = 1;
             for (int j = 0; j < n && !s_abort; ++j) {
-                const int st = j & 1;
-                if (!wait(bar(KV_EMPTY + st), ((uint32_t)(j >> 1) & 1u) ^ 1u)) break;
-                mbar_expect_tx(bar(KV_FULL + st), 2 * KV_TILE);
-                tma_load_3d(map_k, k_tile + st * KV_TILE, bar(KV_FULL + st), g * D, j * KV, b);
-                tma_load_3d(map_v, v_tile + st * KV_TILE, bar(KV_FULL + st), g * D, j * KV, b);
+                if (!wait(bar(KV_EMPTY + st), parity)) break;
+                mbar_expect_tx(bar(KV_FULL + st), 2 * DQ_TILE);
+                tma_load_3d(&p.map_k2, k_tile + st * DQ_TILE, bar(KV_FULL + st), g * D, j * DQ_KV, b);
+                tma_load_3d(&p.map_v2, v_tile + st * DQ_TILE, bar(KV_FULL + st), g * D, j * DQ_KV, b);
+                if (++st == DQ_STAGES) { st = 0; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc<false, false, 128>(KV), idesc_dq = make_idesc<false, true, 128>(D);
-            bool ok = wait(bar(Q_FULL), 0);
-            for (int j = 0; ok && j < n; ++j) {
-                const int st = j & 1;
-                ok = wait(bar(KV_FULL + st), (uint32_t)(j >> 1) & 1u);
-                if (!ok) break;
-                tc_fence_after();
-                // S = Q K^T and dP = dO V^T (the rows that read both of the block before have arrived on DS_FULL)
+        constexpr uint32_t idesc_s = make_idesc<false, false, 128>(DQ_KV), idesc_dq = make_idesc<false, true, 128>(D);
+        // S = Q K^T of block j into its buffer
+        auto scores = [&](int j) {
+            const int st = j % DQ_STAGES;
+            if (!wait.all(bar(KV_FULL + st), (uint32_t)(j / DQ_STAGES) & 1u)) return false;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk)
-                    umma_bf16(tmem_s, make_desc(q_tile + kk * 32, 16, 1024), make_desc(k_tile + st * KV_TILE + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
-#pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk)
-                    umma_bf16(tmem_dp, make_desc(do_tile + kk * 32, 16, 1024), make_desc(v_tile + st * KV_TILE + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
-                umma_commit(bar(SP_FULL));
-                ok = wait(bar(DS_FULL), (uint32_t)j & 1u);
-                if (!ok) break;
-                tc_fence_after();
-                // dQ += dS K: dS K-major (slabs of 64 key positions), the K tile read as the MN-major operand (rows = key positions)
-#pragma unroll
-                for (int kk = 0; kk < KV / 16; ++kk)
-                    umma_bf16(tmem_dq, make_desc(ds_tile + (kk >> 2) * SLAB_BYTES + (kk & 3) * 32, 16, 1024),
-                              make_desc(k_tile + st * KV_TILE + kk * 2048, 8192, 1024), idesc_dq, (j | kk) ? 1u : 0u);
-                umma_commit(bar(DQ_DONE));          // dS may be overwritten, and after the last block dQ is complete
-                umma_commit(bar(KV_EMPTY + st));
+                    umma_bf16(tmem + (uint32_t)(j & 1) * DQ_KV, make_desc(q_tile + kk * 32, 16, 1024),
+                              make_desc(k_tile + st * DQ_TILE + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
+                umma_commit(bar(S_FULL + (j & 1)));
             }
-            if (ok) wait(bar(KV_EMPTY + ((n - 1) & 1)), (uint32_t)((n - 1) >> 1) & 1u);   // the last commit has arrived
+            __syncwarp();
+            return true;
+        };
+        auto d_probabilities = [&](int j) {    // dP = dO V^T of block j
+            const int st = j % DQ_STAGES;
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk)
+                    umma_bf16(tmem_dp, make_desc(do_tile + kk * 32, 16, 1024), make_desc(v_tile + st * DQ_TILE + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
+                umma_commit(bar(DP_FULL));
+            }
+            __syncwarp();
+        };
+        bool ok = wait.all(bar(Q_FULL), 0) && scores(0);
+        if (ok) d_probabilities(0);
+        for (int j = 0; ok && j < n; ++j) {
+            // the scores of the next block into the other buffer, once the product that reads the dS of block j - 1 there is done
+            if (j > 0) ok = wait.all(bar(KV_EMPTY + (j - 1) % DQ_STAGES), (uint32_t)((j - 1) / DQ_STAGES) & 1u);
+            if (ok && j + 1 < n) ok = scores(j + 1);
+            if (ok) ok = wait.all(bar(DS_FULL), (uint32_t)j & 1u);
+            if (!ok) break;
+            tc_fence_after();
+            if (j + 1 < n) d_probabilities(j + 1);       // the rows have read this block's dP
+            const int st = j % DQ_STAGES;
+            // dQ += dS K: dS from tensor memory, the K tile read as the MN-major operand (rows = key positions)
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < DQ_KV / 16; ++kk)
+                    umma_bf16_ts(tmem_dq, tmem + (uint32_t)(j & 1) * DQ_KV + p_column<DQ_KV / DQ_PARTS>(kk),
+                                 make_desc(k_tile + st * DQ_TILE + kk * 2048, 8192, 1024), idesc_dq, (j | kk) ? 1u : 0u);
+                umma_commit(bar(KV_EMPTY + st));
+                if (j == n - 1) umma_commit(bar(DQ_DONE));
+            }
+            __syncwarp();
         }
+        if (ok) wait.all(bar(DQ_DONE), 0);         // the last commit has arrived
     } else {
-        const int quad = warp & 3, row = quad * 32 + lane, part = (warp - 2) >> 2;     // part: which columns of a block
-        constexpr int CHUNKS = KV / 32 / DQ_PARTS;
-        static_assert(CHUNKS >= 1, "a key block has fewer 32-column chunks than there are row warps per 32 rows");
+        constexpr int COLS = DQ_KV / DQ_PARTS;     // columns of a block per thread
+        const int quad = warp & 3, row = quad * 32 + lane, part = (warp - 2) >> 2;
         const int tq = i * BLOCK + row;
         const bool live = tq < p.time;
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
@@ -428,37 +446,52 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
             lse2 = p.lse[at] * LOG2E;
         }
         const float scale2 = 0.125f * LOG2E;
+        const uint64_t scale_pair = pair2(scale2, scale2), lse_pair = pair2(-lse2, -lse2), delta_pair = pair2(-delta, -delta);
         bool ok = true;
         for (int j = 0; ok && j < n; ++j) {
-            ok = wait(bar(SP_FULL), (uint32_t)j & 1u);
-            if (ok && j > 0) ok = wait(bar(DQ_DONE), (uint32_t)(j - 1) & 1u);     // the MMAs that read dS of the block before are done
+            const uint32_t tmem_s = tmem + (uint32_t)(j & 1) * DQ_KV + lane_base + part * COLS;
+            const int first = j * DQ_KV + part * COLS - i * BLOCK;       // first key position of this thread, from the CTA's first query
+            const bool masked = first + COLS - 1 > quad * 32;            // some row of this warp may not see some of these columns
+            uint32_t s[COLS], dp[COLS], packed[COLS / 2];
+            ok = wait.all(bar(S_FULL + (j & 1)), (uint32_t)(j >> 1) & 1u);
             if (!ok) break;
             tc_fence_after();
-            const int first = j * KV;                              // key position of this block's column 0
-            const bool masked = first + KV - 1 > i * BLOCK;        // the block reaches past the first query of this CTA
-#pragma unroll 1
-            for (int c = part * CHUNKS; c < (part + 1) * CHUNKS; ++c) {
-                uint32_t rs[32], rp[32], packed[16];
-                tmem_ld32(tmem_s + lane_base + c * 32, rs);
-                tmem_ld32(tmem_dp + lane_base + c * 32, rp);
-                tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    float d0 = 0.f, d1 = 0.f;
-                    if (live && !(masked && first + c * 32 + e > tq))
-                        d0 = exp2_fast(__uint_as_float(rs[e]) * scale2 - lse2) * (__uint_as_float(rp[e]) - delta) * 0.125f;
-                    if (live && !(masked && first + c * 32 + e + 1 > tq))
-                        d1 = exp2_fast(__uint_as_float(rs[e + 1]) * scale2 - lse2) * (__uint_as_float(rp[e + 1]) - delta) * 0.125f;
-                    packed[e >> 1] = pack2(d0, d1);
-                }
-                store_row32(ds_tile, row, c, packed);
+            for (int c = 0; c < COLS; c += 32) tmem_ld32(tmem_s + c, s + c);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < COLS; c += 2) {
+                float x0, x1;
+                unpair2(fma2(pair2(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), scale_pair, lse_pair), x0, x1);
+                s[c] = __float_as_uint(exp2_fast(x0));
+                s[c + 1] = __float_as_uint(exp2_fast(x1));
             }
-            fence_async_shared();
+            ok = wait.all(bar(DP_FULL), (uint32_t)j & 1u);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < COLS; c += 32) tmem_ld32(tmem_dp + lane_base + part * COLS + c, dp + c);
+            tmem_ld_wait();
+            // dS without the 1/8 of the scores, which the last step applies to dQ (a power of two: the same bits)
+#pragma unroll
+            for (int c = 0; c < COLS; c += 2) {
+                float d0, d1;
+                unpair2(mul2(pair2(__uint_as_float(s[c]), __uint_as_float(s[c + 1])),
+                             add2(pair2(__uint_as_float(dp[c]), __uint_as_float(dp[c + 1])), delta_pair)), d0, d1);
+                if (masked) {
+                    if (first + c > row) d0 = 0.f;
+                    if (first + c + 1 > row) d1 = 0.f;
+                }
+                packed[c >> 1] = pack2(d0, d1);
+            }
+            if (COLS == 64) tmem_st32(tmem_s, packed);
+            else tmem_st16(tmem_s, packed);
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(DS_FULL));
         }
-        if (ok) ok = wait(bar(DQ_DONE), (uint32_t)(n - 1) & 1u);
+        if (ok) ok = wait.all(bar(DQ_DONE), 0);
         if (ok) {
             tc_fence_after();
             uint4* dst = reinterpret_cast<uint4*>(p.out + at * D);
@@ -467,14 +500,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
                 uint32_t r[32];
                 tmem_ld32(tmem_dq + lane_base + c * 32, r);
                 tmem_ld_wait();
-                if (live) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        dst[c * 4 + e] = make_uint4(pack2(__uint_as_float(r[8 * e]), __uint_as_float(r[8 * e + 1])),
-                                                    pack2(__uint_as_float(r[8 * e + 2]), __uint_as_float(r[8 * e + 3])),
-                                                    pack2(__uint_as_float(r[8 * e + 4]), __uint_as_float(r[8 * e + 5])),
-                                                    pack2(__uint_as_float(r[8 * e + 6]), __uint_as_float(r[8 * e + 7])));
-                }
+                if (live) store_row32(dst + c * 4, r, 0.125f);
             }
         }
     }
@@ -483,34 +509,53 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLUMNS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
     }
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward, part 2: dk and dv, one CTA per (sequence, key/value head, key block)
+// backward, part 2: dk and dv, one CTA per (sequence, key/value head, key block) and, where those are too few to fill the
+// machine, a cluster of `p.split` CTAs that share its (query head, query block) list and add their dk, dv through
+// distributed shared memory in a fixed order.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(DKV_THREADS)
+constexpr int DKV_STAGES = 3;
+constexpr int DKV_ROW_BYTES = 2 * BLOCK * 4;          // -lse * log2 e and -delta of a query block
+constexpr int DKV_TILES = (2 + 2 * DKV_STAGES) * TILE_BYTES;
+constexpr int DKV_SUM_PITCH = 128 * 4 + 16;            // one row of dv and dk sums; 16 more bytes spread the rows over the banks
+static_assert(BLOCK * DKV_SUM_PITCH <= 2 * DKV_STAGES * TILE_BYTES, "the sums fit where the query tiles were");
+constexpr int DKV_SMEM = DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 128;
+
+__global__ void __launch_bounds__(DKV_THREADS, 1)
 attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ uint32_t s_tmem_base;
-    __shared__ int s_abort;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int blocks = (p.time + BLOCK - 1) / BLOCK;
-    const int j = (int)(blockIdx.x % blocks);                  // the first key block has the most query blocks to walk
-    const int g = (int)(blockIdx.x / blocks) % p.kv_heads, b = (int)(blockIdx.x / blocks) / p.kv_heads;
+    const int heads_all = p.kv_heads * p.batch, job = (int)blockIdx.x / p.split, share = (int)blockIdx.x % p.split;
+    const int j = job / heads_all;                             // the first key block has the most query blocks to walk
+    const int g = job % heads_all % p.kv_heads, b = job % heads_all / p.kv_heads;
     const int group = p.heads / p.kv_heads;
     const int per_head = blocks - j;                           // query blocks j .. blocks - 1
-    const int n = group * per_head;                            // iterations: head of the group (outer), query block (inner)
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t k_tile = base, v_tile = base + TILE_BYTES, q_tile = v_tile + TILE_BYTES, do_tile = q_tile + 2 * TILE_BYTES,
-                   p_tile = do_tile + 2 * TILE_BYTES, ds_tile = p_tile + 2 * SLAB_BYTES;
-    const uint32_t bars = ds_tile + 2 * SLAB_BYTES;
-    enum { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = 3, SP_FULL = 5, PDS_FULL = 6, ACC_DONE = 7, BARS = 8 };
+    const int all = group * per_head;                          // iterations: head of the group (outer), query block (inner)
+    const int begin = all * share / p.split, n = all * (share + 1) / p.split - begin;      // this CTA's (none, when there are fewer than CTAs)
+    const int first_head = begin / per_head, first_i = j + begin % per_head;
+    const uint32_t base = smem_u32(smem_raw);
+    const uint32_t k_tile = base, v_tile = base + TILE_BYTES, q_tile = v_tile + TILE_BYTES, do_tile = q_tile + DKV_STAGES * TILE_BYTES;
+    const uint32_t rows_at = base + DKV_TILES, bars = rows_at + DKV_STAGES * DKV_ROW_BYTES;
+    enum { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = Q_FULL + DKV_STAGES, S_FULL = Q_EMPTY + DKV_STAGES, DP_FULL = S_FULL + 2, P_FULL, DS_FULL, ACC_DONE, BARS };
     auto bar = [&](int which) { return bars + 8u * which; };
+    uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 8 * BARS);
+    volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 8 * BARS + 4);
+    if (base & 1023u) {
+        if (threadIdx.x == 0) atomicExch(p.status, STATUS_ATTENTION_WAIT + 1);
+        return;
+    }
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int w = 0; w < BARS; ++w) mbar_init(bar(w), w == PDS_FULL ? 4 * DKV_PARTS : 1);
+        // a stage is full when its bytes have landed and the lanes of the loading warp have written its row values
+        for (int w = 0; w < BARS; ++w) {
+            const bool rows = w == P_FULL || w == DS_FULL, full = w >= Q_FULL && w < Q_EMPTY;
+            mbar_init(bar(w), rows ? 4 * DKV_PARTS : full ? 2 : 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         prefetch_map(&p.map_q); prefetch_map(&p.map_k); prefetch_map(&p.map_v); prefetch_map(&p.map_do);
     }
@@ -522,128 +567,238 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem_base;
-    const uint32_t tmem_s = tmem, tmem_dp = tmem + 128, tmem_dv = tmem + 256, tmem_dk = tmem + 320;
+    // everything with key positions as rows (lanes) and query positions as columns: S^T of iteration it in columns
+    // 128 (it & 1) .., over which the rows put back P^T and dS^T (bf16 pairs); one dP^T
+    const uint32_t tmem_dp = tmem + 256, tmem_dv = tmem + 384, tmem_dk = tmem + 448;
     const Wait wait{&s_abort, p.status};
 
-    if (warp == 0) {
+    if (n == 0) {
+        // nothing to do before the sum
+    } else if (warp == 0) {
         if (lane == 0) {
             mbar_expect_tx(bar(KV_FULL), 2 * TILE_BYTES);
             tma_load_3d(&p.map_k, k_tile, bar(KV_FULL), g * D, j * BLOCK, b);
             tma_load_3d(&p.map_v, v_tile, bar(KV_FULL), g * D, j * BLOCK, b);
-            for (int it = 0; it < n && !s_abort; ++it) {
-                const int st = it & 1, h = g * group + it / per_head, i = j + it % per_head;
-                if (!wait(bar(Q_EMPTY + st), ((uint32_t)(it >> 1) & 1u) ^ 1u)) break;
+        }
+        int st = 0, head = first_head, i = first_i;
+        uint32_t parity = 1;
+        bool ok = true;
+        for (int it = 0; ok && it < n; ++it) {
+            const int h = g * group + head;
+            // the row values travel through registers while the stage is still in use
+            float lse2[BLOCK / 32], delta[BLOCK / 32];
+#pragma unroll
+            for (int r = 0; r < BLOCK / 32; ++r) {
+                const int tq = i * BLOCK + r * 32 + lane;
+                const long long at = ((long long)b * p.time + tq) * p.heads + h;
+                const bool live = tq < p.time;                       // past the end: a probability of zero
+                lse2[r] = live ? -p.lse[at] * LOG2E : -INFINITY;
+                delta[r] = live ? -p.delta[at] : 0.f;
+            }
+            ok = wait.all(bar(Q_EMPTY + st), parity);
+            if (!ok) break;
+            if (lane == 0) {
                 mbar_expect_tx(bar(Q_FULL + st), 2 * TILE_BYTES);
                 tma_load_3d(&p.map_q, q_tile + st * TILE_BYTES, bar(Q_FULL + st), h * D, i * BLOCK, b);
                 tma_load_3d(&p.map_do, do_tile + st * TILE_BYTES, bar(Q_FULL + st), h * D, i * BLOCK, b);
             }
+            float* rows = reinterpret_cast<float*>(smem_raw + DKV_TILES + st * DKV_ROW_BYTES);
+#pragma unroll
+            for (int r = 0; r < BLOCK / 32; ++r) {
+                rows[r * 32 + lane] = lse2[r];
+                rows[BLOCK + r * 32 + lane] = delta[r];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(Q_FULL + st));
+            if (++st == DKV_STAGES) { st = 0; parity ^= 1u; }
+            if (++i == blocks) { i = j; ++head; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc<false, false, 128>(128), idesc_t = make_idesc<true, true, 128>(D);
-            bool ok = wait(bar(KV_FULL), 0);
-            for (int it = 0; ok && it < n; ++it) {
-                const int st = it & 1;
-                ok = wait(bar(Q_FULL + st), (uint32_t)(it >> 1) & 1u);
-                if (!ok) break;
-                tc_fence_after();
-                // S = Q K^T and dP = dO V^T, rows = query positions
+        constexpr uint32_t idesc_s = make_idesc<false, false, 128>(128), idesc_t = make_idesc<false, true, 128>(D);
+        auto scores = [&](int it) {      // S^T = K Q^T
+            const int st = it % DKV_STAGES;
+            if (!wait.all(bar(Q_FULL + st), (uint32_t)(it / DKV_STAGES) & 1u)) return false;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk)
-                    umma_bf16(tmem_s, make_desc(q_tile + st * TILE_BYTES + kk * 32, 16, 1024), make_desc(k_tile + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
-#pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk)
-                    umma_bf16(tmem_dp, make_desc(do_tile + st * TILE_BYTES + kk * 32, 16, 1024), make_desc(v_tile + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
-                umma_commit(bar(SP_FULL));
-                ok = wait(bar(PDS_FULL), (uint32_t)it & 1u);
-                if (!ok) break;
-                tc_fence_after();
-                // dV += P^T dO and dK += dS^T Q: the K-major tiles of P and dS (rows = query positions, two slabs of 64 key
-                // positions) read as MN-major operands are their transposes; dO and Q read as MN-major operands
-                // (rows = query positions = the contraction)
-#pragma unroll
-                for (int kk = 0; kk < BLOCK / 16; ++kk)
-                    umma_bf16(tmem_dv, make_desc(p_tile + kk * 2048, SLAB_BYTES, 1024), make_desc(do_tile + st * TILE_BYTES + kk * 2048, 8192, 1024),
-                              idesc_t, (it | kk) ? 1u : 0u);
-#pragma unroll
-                for (int kk = 0; kk < BLOCK / 16; ++kk)
-                    umma_bf16(tmem_dk, make_desc(ds_tile + kk * 2048, SLAB_BYTES, 1024), make_desc(q_tile + st * TILE_BYTES + kk * 2048, 8192, 1024),
-                              idesc_t, (it | kk) ? 1u : 0u);
-                umma_commit(bar(ACC_DONE));        // P and dS may be overwritten; after the last iteration dV and dK are complete
-                umma_commit(bar(Q_EMPTY + st));
+                    umma_bf16(tmem + (uint32_t)(it & 1) * 128, make_desc(k_tile + kk * 32, 16, 1024),
+                              make_desc(q_tile + st * TILE_BYTES + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
+                umma_commit(bar(S_FULL + (it & 1)));
             }
-            if (ok) wait(bar(Q_EMPTY + ((n - 1) & 1)), (uint32_t)((n - 1) >> 1) & 1u);    // the last commit has arrived
-        }
-    } else {
-        const int quad = warp & 3, row = quad * 32 + lane, part = (warp - 2) >> 2;     // part: which 32 columns of a block
-        static_assert(DKV_PARTS == 4, "one 32-column chunk of S and dP, and one of the four chunks of dV and dK, per row warp");
-        const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-        const float scale2 = 0.125f * LOG2E;
-        bool ok = true;
+            __syncwarp();
+            return true;
+        };
+        auto d_probabilities = [&](int it) {    // dP^T = V dO^T
+            const int st = it % DKV_STAGES;
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk)
+                    umma_bf16(tmem_dp, make_desc(v_tile + kk * 32, 16, 1024), make_desc(do_tile + st * TILE_BYTES + kk * 32, 16, 1024), idesc_s, kk ? 1u : 0u);
+                umma_commit(bar(DP_FULL));
+            }
+            __syncwarp();
+        };
+        bool ok = wait.all(bar(KV_FULL), 0) && scores(0);
+        if (ok) d_probabilities(0);
         for (int it = 0; ok && it < n; ++it) {
-            const int h = g * group + it / per_head, i = j + it % per_head;
-            const int tq = i * BLOCK + row;
-            const bool live = tq < p.time;
-            float delta = 0.f, lse2 = 0.f;
-            if (live) {
-                const long long at = ((long long)b * p.time + tq) * p.heads + h;
-                delta = p.delta[at];
-                lse2 = p.lse[at] * LOG2E;
-            }
-            ok = wait(bar(SP_FULL), (uint32_t)it & 1u);
-            if (ok && it > 0) ok = wait(bar(ACC_DONE), (uint32_t)(it - 1) & 1u);
+            const int st = it % DKV_STAGES;
+            const uint32_t buffer = tmem + (uint32_t)(it & 1) * 128;
+            // the next scores into the other buffer, once the products that read the P and dS of iteration it - 1 there are done
+            if (it > 0) ok = wait.all(bar(Q_EMPTY + (it - 1) % DKV_STAGES), (uint32_t)((it - 1) / DKV_STAGES) & 1u);
+            if (ok && it + 1 < n) ok = scores(it + 1);
+            if (ok) ok = wait.all(bar(P_FULL), (uint32_t)it & 1u);
             if (!ok) break;
             tc_fence_after();
-            const bool diagonal = i == j;
-            {
-                const int c = part;
-                uint32_t rs[32], rp[32], pp[16], pd[16];
-                tmem_ld32(tmem_s + lane_base + c * 32, rs);
-                tmem_ld32(tmem_dp + lane_base + c * 32, rp);
-                tmem_ld_wait();
+            // dV += P^T dO and dK += dS^T Q: P^T and dS^T from tensor memory, dO and Q as they lie in memory (rows = query
+            // positions = the contraction) are MN-major operands
+            if (elect_one()) {
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    float p0 = 0.f, p1 = 0.f;
-                    if (live && !(diagonal && c * 32 + e > row)) p0 = exp2_fast(__uint_as_float(rs[e]) * scale2 - lse2);
-                    if (live && !(diagonal && c * 32 + e + 1 > row)) p1 = exp2_fast(__uint_as_float(rs[e + 1]) * scale2 - lse2);
-                    pp[e >> 1] = pack2(p0, p1);
-                    pd[e >> 1] = pack2(p0 * (__uint_as_float(rp[e]) - delta) * 0.125f, p1 * (__uint_as_float(rp[e + 1]) - delta) * 0.125f);
-                }
-                store_row32(p_tile, row, c, pp);
-                store_row32(ds_tile, row, c, pd);
+                for (int kk = 0; kk < BLOCK / 16; ++kk)
+                    umma_bf16_ts(tmem_dv, buffer + p_column<BLOCK / DKV_PARTS>(kk), make_desc(do_tile + st * TILE_BYTES + kk * 2048, 8192, 1024),
+                                 idesc_t, (it | kk) ? 1u : 0u);
             }
-            fence_async_shared();
+            __syncwarp();
+            ok = wait.all(bar(DS_FULL), (uint32_t)it & 1u);
+            if (!ok) break;
+            tc_fence_after();
+            if (it + 1 < n) d_probabilities(it + 1);     // the rows have read this iteration's dP
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < BLOCK / 16; ++kk)
+                    umma_bf16_ts(tmem_dk, buffer + p_column<BLOCK / DKV_PARTS>(kk) + BLOCK / DKV_PARTS / 2,
+                                 make_desc(q_tile + st * TILE_BYTES + kk * 2048, 8192, 1024), idesc_t, (it | kk) ? 1u : 0u);
+                umma_commit(bar(Q_EMPTY + st));
+                if (it == n - 1) umma_commit(bar(ACC_DONE));
+            }
+            __syncwarp();
+        }
+        if (ok) wait.all(bar(ACC_DONE), 0);        // the last commit has arrived
+    } else {
+        constexpr int COLS = BLOCK / DKV_PARTS;    // columns (query positions) of a block per thread
+        const int quad = warp & 3, row = quad * 32 + lane, part = (warp - 2) >> 2;
+        const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
+        const float scale2 = 0.125f * LOG2E;
+        const uint64_t scale_pair = pair2(scale2, scale2);
+        int st = 0, i = first_i;
+        bool ok = true;
+        for (int it = 0; ok && it < n; ++it) {
+            const uint32_t tmem_s = tmem + (uint32_t)(it & 1) * 128 + lane_base + part * COLS;
+            const uint32_t row_values = rows_at + st * DKV_ROW_BYTES + part * COLS * 4;
+            const bool masked = i == j && part * COLS < quad * 32 + 31;  // some row of this warp is not seen by some of these columns
+            uint32_t s[COLS], dp[COLS], packed[COLS / 2];
+            // the row values of this stage (the scores of this iteration were formed from the same stage, but the barrier that
+            // publishes the loading warp's plain stores is the stage's own)
+            ok = wait.all(bar(Q_FULL + st), (uint32_t)(it / DKV_STAGES) & 1u);
+            if (ok) ok = wait.all(bar(S_FULL + (it & 1)), (uint32_t)(it >> 1) & 1u);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < COLS; c += 32) tmem_ld32(tmem_s + c, s + c);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < COLS; c += 4) {
+                float l[4], x[4];
+                load_shared4(row_values + c * 4, l);
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    unpair2(fma2(pair2(__uint_as_float(s[c + e]), __uint_as_float(s[c + e + 1])), scale_pair, pair2(l[e], l[e + 1])), x[e], x[e + 1]);
+                    x[e] = exp2_fast(x[e]);
+                    x[e + 1] = exp2_fast(x[e + 1]);
+                    if (masked) {
+                        if (part * COLS + c + e < row) x[e] = 0.f;
+                        if (part * COLS + c + e + 1 < row) x[e + 1] = 0.f;
+                    }
+                    s[c + e] = __float_as_uint(x[e]);
+                    s[c + e + 1] = __float_as_uint(x[e + 1]);
+                    packed[(c + e) >> 1] = pack2(x[e], x[e + 1]);
+                }
+            }
+            if (COLS == 64) tmem_st32(tmem_s, packed);
+            else tmem_st16(tmem_s, packed);
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(PDS_FULL));
+            if (lane == 0) mbar_arrive(bar(P_FULL));
+            ok = wait.all(bar(DP_FULL), (uint32_t)it & 1u);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < COLS; c += 32) tmem_ld32(tmem_dp + lane_base + part * COLS + c, dp + c);
+            tmem_ld_wait();
+            // dS without the 1/8 of the scores, which the last step applies to dK (a power of two: the same bits)
+#pragma unroll
+            for (int c = 0; c < COLS; c += 4) {
+                float d[4];
+                load_shared4(row_values + BLOCK * 4 + c * 4, d);
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    float d0, d1;
+                    unpair2(mul2(pair2(__uint_as_float(s[c + e]), __uint_as_float(s[c + e + 1])),
+                                 add2(pair2(__uint_as_float(dp[c + e]), __uint_as_float(dp[c + e + 1])), pair2(d[e], d[e + 1]))), d0, d1);
+                    if (masked) {
+                        if (part * COLS + c + e < row) d0 = 0.f;
+                        if (part * COLS + c + e + 1 < row) d1 = 0.f;
+                    }
+                    packed[(c + e) >> 1] = pack2(d0, d1);
+                }
+            }
+            if (COLS == 64) tmem_st32(tmem_s + COLS / 2, packed);
+            else tmem_st16(tmem_s + COLS / 2, packed);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(DS_FULL));
+            if (++st == DKV_STAGES) st = 0;
+            if (++i == blocks) i = j;
         }
-        if (ok) ok = wait(bar(ACC_DONE), (uint32_t)(n - 1) & 1u);
+        if (ok) ok = wait.all(bar(ACC_DONE), 0);
         if (ok) {
             tc_fence_after();
             const int tk = j * BLOCK + row;                     // this thread's key position
             const long long at = ((long long)b * p.time + (tk < p.time ? tk : 0)) * p.kv_heads + g;
-            {
-                const int which = part >> 1;                                                  // parts 0, 1: dv; parts 2, 3: dk
-                uint4* dst = reinterpret_cast<uint4*>((which ? p.out : p.out2) + at * D);
-                {
-                    const int c = part & 1;
-                    uint32_t r[32];
-                    tmem_ld32((which ? tmem_dk : tmem_dv) + lane_base + c * 32, r);
-                    tmem_ld_wait();
-                    if (tk < p.time) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            dst[c * 4 + e] = make_uint4(pack2(__uint_as_float(r[8 * e]), __uint_as_float(r[8 * e + 1])),
-                                                        pack2(__uint_as_float(r[8 * e + 2]), __uint_as_float(r[8 * e + 3])),
-                                                        pack2(__uint_as_float(r[8 * e + 4]), __uint_as_float(r[8 * e + 5])),
-                                                        pack2(__uint_as_float(r[8 * e + 6]), __uint_as_float(r[8 * e + 7])));
-                    }
+            for (int c = part; c < 4; c += DKV_PARTS) {         // 32-column chunks 0, 1: dv; 2, 3: dk
+                uint32_t r[32];
+                tmem_ld32(tmem_dv + lane_base + c * 32, r);
+                tmem_ld_wait();
+                if (p.split > 1) {      // the tiles of this CTA are spent: its sums take their place
+                    float4* sums = reinterpret_cast<float4*>(smem_raw + 2 * TILE_BYTES + row * DKV_SUM_PITCH + c * 128);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        sums[e] = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3]));
+                } else if (tk < p.time) {
+                    store_row32(reinterpret_cast<uint4*>((c >> 1 ? p.out : p.out2) + at * D) + (c & 1) * 4, r, c >> 1 ? 0.125f : 1.f);
                 }
             }
         }
     }
     linger_after_abort(&s_abort);
     tc_fence_before();
+    if (p.split > 1) {
+        cluster_sync();
+        // every CTA adds the sums of all for its share of the 128 rows: 16 pieces of 8 columns (0-7: dv, 8-15: dk) per row
+        const int row0 = BLOCK * share / p.split, rows = BLOCK * (share + 1) / p.split - row0;
+        for (int at = threadIdx.x; at < rows * 16; at += DKV_THREADS) {
+            const int row = row0 + at / 16, piece = at % 16, tk = j * BLOCK + row;
+            float total[8] = {};
+            for (int other = 0; other < p.split; ++other) {
+                if (all * (other + 1) / p.split == all * other / p.split) continue;        // had no iterations
+                const uint32_t from = map_to_cta(q_tile + row * DKV_SUM_PITCH + piece * 32, other);
+                float v[8];
+                load_cluster4(from, v);
+                load_cluster4(from + 16, v + 4);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) total[e] += v[e];
+            }
+            const float scale = piece >> 3 ? 0.125f : 1.f;
+            if (tk < p.time)
+                reinterpret_cast<uint4*>((piece >> 3 ? p.out : p.out2) + (((long long)b * p.time + tk) * p.kv_heads + g) * D)[piece & 7] =
+                    make_uint4(pack2(total[0] * scale, total[1] * scale), pack2(total[2] * scale, total[3] * scale),
+                               pack2(total[4] * scale, total[5] * scale), pack2(total[6] * scale, total[7] * scale));
+        }
+        cluster_sync();        // nobody leaves while its sums are being read
+    }
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
@@ -652,11 +807,18 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
 }
 
 constexpr int FORWARD_SMEM = 5 * TILE_BYTES + 128;
-constexpr int DQ_KV = 64;
-constexpr int DQ_SMEM = 2 * TILE_BYTES + 4 * DQ_KV * 128 + (DQ_KV / 64) * SLAB_BYTES + 128;
-constexpr int DKV_SMEM = 1024 + 6 * TILE_BYTES + 4 * SLAB_BYTES + 128;
 
 }  // namespace
+
+// CTAs per key block of the dk, dv kernel: one while the longest list (the first key block's: every query block of every
+// head of the group) is within a quarter of the SMs' average share, else as many, up to 8 and a power of two, as bring it there.
+int dkv_split(const qmoe_attention_t* a, int blocks) {
+    const long long group = a->heads / a->kv_heads, longest = group * blocks;
+    const long long total = (long long)a->batch * a->kv_heads * group * blocks * (blocks + 1) / 2, share = total / sm_count();
+    int split = 1;
+    while (split < 8 && longest * 4 > (share * 5 + 4) * split && longest > 2 * split) split *= 2;
+    return split;
+}
 
 int attention_check(const qmoe_attention_t* a, bool backward) {
     if (!a) return fail_arg("attention is null");
@@ -710,14 +872,28 @@ extern "C" int qmoe_attention_backward(const qmoe_attention_t* a, uint64_t strea
     const int blocks = (a->time + BLOCK - 1) / BLOCK;
     if (int rc = make_map_3d(&p.map_k2, a->k, narrow, (uint64_t)a->time, (uint64_t)a->batch, DQ_KV)) return rc;
     if (int rc = make_map_3d(&p.map_v2, a->v, narrow, (uint64_t)a->time, (uint64_t)a->batch, DQ_KV)) return rc;
-    QMOE_CUDA(cudaFuncSetAttribute(attention_dq_kernel<DQ_KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
+    QMOE_CUDA(cudaFuncSetAttribute(attention_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
     QMOE_CUDA(cudaFuncSetAttribute(attention_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DKV_SMEM));
     p.out = (__nv_bfloat16*)a->dq; p.out2 = nullptr;
-    attention_dq_kernel<DQ_KV><<<(unsigned)(blocks * a->heads * a->batch), DQ_THREADS, DQ_SMEM, stream>>>(p);
+    attention_dq_kernel<<<(unsigned)(blocks * a->heads * a->batch), DQ_THREADS, DQ_SMEM, stream>>>(p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("attention_dq_kernel");
     p.out = (__nv_bfloat16*)a->dk; p.out2 = (__nv_bfloat16*)a->dv;
-    attention_dkv_kernel<<<(unsigned)(blocks * a->kv_heads * a->batch), DKV_THREADS, DKV_SMEM, stream>>>(p);
+    p.split = dkv_split(a, blocks);
+    cudaLaunchConfig_t config = {};
+    cudaLaunchAttribute cluster[1];
+    config.gridDim = dim3((unsigned)(blocks * a->kv_heads * a->batch * p.split));
+    config.blockDim = dim3(DKV_THREADS);
+    config.dynamicSmemBytes = DKV_SMEM;
+    config.stream = stream;
+    if (p.split > 1) {
+        cluster[0].id = cudaLaunchAttributeClusterDimension;
+        cluster[0].val.clusterDim.x = (unsigned)p.split;
+        cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+        config.attrs = cluster;
+        config.numAttrs = 1;
+    }
+    QMOE_CUDA(cudaLaunchKernelEx(&config, attention_dkv_kernel, p));
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("attention_dkv_kernel");
     return 0;
