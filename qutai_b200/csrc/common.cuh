@@ -152,9 +152,9 @@ struct TcScatter {
     unsigned long long base[16];    // destination buffer of every rank
 };
 int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, cudaStream_t stream,
-               const TcScatter* scatter = nullptr);
+               const TcScatter* scatter = nullptr, long long rows = 0);
 int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c, long long K,
-               long long N, cudaStream_t stream, const TcScatter* scatter = nullptr);
+               long long N, cudaStream_t stream, const TcScatter* scatter = nullptr, long long rows = 0);
 int tc_dswiglu(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t w_down, uint64_t g, uint64_t u, uint64_t dg,
                uint64_t du, long long d, long long h, cudaStream_t stream);
 int tc_wgrad3(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t h_act, uint64_t x, uint64_t dg, uint64_t du,

@@ -99,7 +99,7 @@ struct alignas(64) GemmParams {
     const int* scatter_ret;              // [rows] return addresses, or null for a plain store
     unsigned long long scatter_base[16]; // every rank's destination buffer (own entry: local address)
     int scatter_wide;     // scatter in 256-byte row pieces (0: 64-byte pieces)
-    int plain_rows;       // > 0: one group of this many rows instead of the expert groups of `offsets`
+    int plain_rows;       // > 0: one group of this many rows (any number) instead of the expert groups of `offsets` and `counts`
     int transpose_out;    // WGRAD: bit i set = problem i stores the [M, N] product of each expert as [N, M]
     int problems;         // WGRAD: 1, or 3 products of the same shape (outputs out0, out1, out2) sharing the tile queue
     int group_stride;     // ROUTER: accumulator columns [0,S), [S,2S), [2S,3S) hold the three bf16 terms of the weights
@@ -147,7 +147,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         tile.expert = e;
         tile.row0 = (rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
         tile.n0 = (rem / p.m_tiles) * BN;
-        const int count = p.counts[e];
+        const int count = p.plain_rows > 0 ? p.plain_rows : p.counts[e];
         tile.kblocks = (count + BK - 1) / BK;
         tile.krow0 = s_start[e] * kRowPad;
         tile.valid = count > 0;
@@ -217,8 +217,9 @@ constexpr int EPI_STAGE_BYTES = 32 * STAGE_PITCH;
 
 // Thread `lane` holds 32 consecutive bf16 (16 packed words) of row `lane`.  Write the 32 x 32 block to
 // global memory (dst = first element of the block, row pitch ldc elements) so that every store
-// instruction covers 8 rows x 64 contiguous bytes.
-__device__ __forceinline__ void store_block32(uint32_t stage, int lane, const uint32_t* w, __nv_bfloat16* dst, long long ldc) {
+// instruction covers 8 rows x 64 contiguous bytes; rows >= rows_left are skipped.
+__device__ __forceinline__ void store_block32(uint32_t stage, int lane, const uint32_t* w, __nv_bfloat16* dst, long long ldc,
+                                              int rows_left = 32) {
     const uint32_t mine = stage + lane * STAGE_PITCH;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -231,7 +232,7 @@ __device__ __forceinline__ void store_block32(uint32_t stage, int lane, const ui
         uint4 v;
         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                      : "r"(stage + row * STAGE_PITCH + 16 * piece) : "memory");
-        *reinterpret_cast<uint4*>(dst + (long long)row * ldc + piece * 8) = v;
+        if (row < rows_left) *reinterpret_cast<uint4*>(dst + (long long)row * ldc + piece * 8) = v;
     }
     __syncwarp();
 }
@@ -353,7 +354,9 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     if (MODE == MODE_WGRAD) {
         // Tiles of large experts cost more (longer contraction).  Walking the experts from large to
         // small and dealing tiles round-robin gives every CTA the same mix of long and short tiles.
-        for (int i = threadIdx.x; i < p.experts; i += NUM_THREADS) {
+        if (p.plain_rows > 0) {
+            if (threadIdx.x == 0) s_order[0] = 0;
+        } else for (int i = threadIdx.x; i < p.experts; i += NUM_THREADS) {
             const int mine = p.counts[i];
             int rank = 0;
             for (int j = 0; j < p.experts; ++j) {
@@ -742,6 +745,8 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                         remote = (__nv_bfloat16*)p.scatter_base[address >> 26] + (long long)(address & ((1 << 26) - 1)) * p.ldc + tile.n0;
                     }
                 }
+                // a plain product may end inside a tile; the dispatched layout is padded to whole tiles
+                const int rows_left = p.plain_rows > 0 ? (int)min(32ll, (long long)p.plain_rows - row0w) : 32;
                 const bool wide = p.scatter_ret && p.scatter_wide && c_end - c_begin == 4 && p.N - (tile.n0 + c_begin * 32) >= 128;
                 if (wide) {  // this warp's 128 columns are all there: scatter them as 256-byte row pieces
                     uint32_t w[64];
@@ -767,13 +772,14 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) w[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
                         if (p.scatter_ret) scatter_block32(stage, lane, w, remote ? remote + c * 32 : nullptr);
-                        else store_block32(stage, lane, w, C + c * 32, p.ldc);
+                        else store_block32(stage, lane, w, C + c * 32, p.ldc, rows_left);
                     } else if (valid > 0) {
                         float v[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-                        if (!p.scatter_ret) store_row32_bf16(C + lane * p.ldc + c * 32, v, valid);
-                        else if (remote) store_row32_bf16(remote + c * 32, v, valid);
+                        if (!p.scatter_ret) {
+                            if (lane < rows_left) store_row32_bf16(C + lane * p.ldc + c * 32, v, valid);
+                        } else if (remote) store_row32_bf16(remote + c * 32, v, valid);
                     }
                 }
             } else if (MODE == MODE_ROUTER) {
@@ -1017,7 +1023,7 @@ int tc_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t 
     return launch<MODE_SWIGLU, false, false>(p, stream);
 }
 
-// C [rows, N] = A [rows, K] . B_e^T with B stacked [E*N, K]
+// C [rows, N] = A [rows, K] . B_e^T with B stacked [E*N, K]; `rows` > 0: one group whose last tile may be ragged
 void set_scatter(GemmParams& p, const TcScatter* scatter) {
     if (!scatter) return;
     p.scatter_ret = scatter->ret;
@@ -1026,9 +1032,10 @@ void set_scatter(GemmParams& p, const TcScatter* scatter) {
 }
 
 int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N,
-               cudaStream_t stream, const TcScatter* scatter) {
+               cudaStream_t stream, const TcScatter* scatter, long long rows) {
     GemmParams p = {};
     set_scatter(p, scatter);
+    p.plain_rows = (int)rows;
     if (int rc = make_map(&p.map_a, a, (uint64_t)K, (uint64_t)r->rows_bound, BM)) return rc;
     const int ctas = gemm_ctas();
     if (int rc = make_map(&p.map_b, b, (uint64_t)K, (uint64_t)experts * N, BN / ctas)) return rc;
@@ -1042,9 +1049,10 @@ int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
 
 // C [rows, N] = A [rows, K] . B_e (+ A2 . B2_e) with B stacked [E*K, N]
 int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c,
-               long long K, long long N, cudaStream_t stream, const TcScatter* scatter) {
+               long long K, long long N, cudaStream_t stream, const TcScatter* scatter, long long rows) {
     GemmParams p = {};
     set_scatter(p, scatter);
+    p.plain_rows = (int)rows;
     if (int rc = make_map(&p.map_a, a, (uint64_t)K, (uint64_t)r->rows_bound, BM)) return rc;
     if (int rc = make_map(&p.map_b, b, (uint64_t)N, (uint64_t)experts * K, 64)) return rc;
     p.map_a2 = p.map_a; p.map_b2 = p.map_b;
@@ -1170,11 +1178,12 @@ int tc_wgrad3(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t h_act, u
 
 // out [M, N] (fp32) = A^T . B over the rows of ONE group (counts[0] rows from row offsets[0]): A [rows, M], B [rows, N].
 // The weight gradient of a plain linear map (the language-model head), on CTA pairs.  With `groups` > 1 the rows are cut
-// into that many ranges (offsets[g], counts[g]; every offset a multiple of 128) and range g leaves its own product in
+// into that many ranges (offsets[g], counts[g]; every offset a multiple of 128; without tables: one group of all rows) and range g leaves its own product in
 // out + g * slab: a short, wide product then fills the machine, and the caller adds the slabs in a fixed order.
 int tc_wgrad1(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t out, long long M, long long N, cudaStream_t stream,
               int groups, long long slab) {
     GemmParams p = {};
+    if (!r->offsets) p.plain_rows = (int)r->rows_bound;
     if (out & 15u || (N * 4) % 16) return fail_arg("weight-gradient output must be 16-byte aligned with a 16-byte row pitch");
     const int ctas = gemm_ctas();
     const uint64_t rows = (uint64_t)r->rows_bound;

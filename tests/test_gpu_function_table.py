@@ -234,3 +234,40 @@ def test_split_weight_gradient_of_a_linear_layer(rows, cols_out, cols_in):
     assert lib.load().qmoe_gemm_wgrad_partials(32000, 8192, 1024) == 0
     with pytest.raises(ValueError):
         lib.call("qmoe_gemm_wgrad_split", gs.ptr, xs.ptr, out.ptr, scratch.ptr, 32000, 8192, 1024, 0)
+
+
+@pytest.mark.parametrize("rows,inner,cols", [(129, 64, 72), (200, 264, 512), (602, 512, 128), (1001, 1024, 264)])
+def test_gemm_takes_ragged_row_counts_to_the_tensor_cores(rows, inner, cols, kernel_variant):
+    """Row counts that fill no whole tile: the three products of a linear layer give what the CUDA-core kernel gives, and
+    what lies behind the last row of a result keeps its bits."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(rows)
+    x, w = oracle.round_bf16(rng.standard_normal((rows, inner))), oracle.round_bf16(rng.standard_normal((cols, inner)) * 0.1)
+    g = oracle.round_bf16(rng.standard_normal((rows, cols)))
+    xs, ws, gs = to_device(x, "bfloat16"), to_device(w, "bfloat16"), to_device(g, "bfloat16")
+    bf16, f32 = lib.QMOE_BF16, lib.QMOE_F32
+    count = lib.load().qmoe_tensor_core_launch_count
+
+    def product(a, b, m, k, n, ta, tb, dtype, code):
+        out = DeviceStorage((m + 3) * n, dtype)
+        lib.call("qmoe_memset", out.ptr, 0x3C, out.nbytes, 0)
+        lib.call("qmoe_gemm", a.ptr, bf16, b.ptr, bf16, out.ptr, code, m, k, n, ta, tb, 0, 0)
+        raw = np.frombuffer(out.tobytes(), dtype=np.uint8)
+        assert np.all(raw[m * n * (2 if code == bf16 else 4):] == 0x3C)
+        return to_host(out, (m + 3, n))[:m]
+
+    def products():
+        return (product(xs, ws, rows, inner, cols, 0, 1, "bfloat16", bf16), product(gs, ws, rows, cols, inner, 0, 0, "bfloat16", bf16),
+                product(gs, xs, cols, rows, inner, 1, 0, "float32", f32))
+
+    before = count()
+    fast = products()
+    assert count() - before == 3
+    kernel_variant(lib.VARIANT_PLAIN_GEMM_ON_CUDA_CORES)
+    for got, slow, exact in zip(fast, products(), (x @ w.T, g @ w, g.T @ x)):
+        assert oracle.max_rel_err(got, exact) <= 1e-2
+        assert oracle.max_rel_err(got, slow) <= 8e-3
+    assert lib.device_status() == 0
