@@ -7,6 +7,7 @@
 // One generic kernel: arbitrary element strides for both operands, optional second (A2, B2) segment
 // accumulated into the same tile, and three ways of grouping by expert.
 #include "common.cuh"
+#include "tc_ptx.cuh"
 
 namespace qmoe {
 
@@ -109,6 +110,166 @@ simt_gemm_kernel(SimtGemmArgs g) {
     }
 }
 
+// ---- fp32 operands, many rows: 128 x 128 tiles ------------------------------------------------------
+// The same sums in the same order (one fp32 FMA chain per output, k ascending) as the kernel above, bit for bit; what
+// differs is how the operands reach the FMAs.  That kernel fetches two shared-memory words for every four FMAs and
+// stalls on each tile's loads (19 .. 25 TFLOP/s from 128 tiles on); here (30 .. 46) a thread owns 8 x 8 outputs (two 4-row and two 4-column pieces, so that
+// the reads of a warp are whole 16-byte broadcasts), multiplies pairs of columns with one fma.rn.f32x2, and the next
+// 16-deep tile travels from global memory through registers into the other shared buffer meanwhile.
+// A_KFAST / B_KFAST: the operand is contiguous along k (rows of 4 k per load, transposed on the way into shared memory),
+// else along its own rows / columns.
+constexpr int TILE = 128, TILE_K = 16, TILE_PITCH = TILE + 4;
+
+template <bool KFAST>
+struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice of one operand
+    const float* base;       // element (row 0 of the tile, k = 0)
+    long long pitch;         // elements between rows (KFAST) or between k (not KFAST)
+    int rows_left;           // rows of the tile inside the matrix
+    float v[8];
+    __device__ __forceinline__ void fetch(long long k0, long long k_end) {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const int i = threadIdx.x + l * 256;
+            const int row = KFAST ? i / 4 : i % (TILE / 4) * 4, k = KFAST ? i % 4 * 4 : i / (TILE / 4);
+            float* dst = v + 4 * l;
+            const float* src = base + (KFAST ? row * pitch + (k0 + k) : (k0 + k) * pitch + row);
+            const int along = KFAST ? (int)(k_end - (k0 + k) < 4 ? k_end - (k0 + k) : 4) : rows_left - row;   // values of the 4 that exist
+            const bool across = KFAST ? row < rows_left : k0 + k < k_end;
+            if (across && along >= 4) {
+                const float4 w = *reinterpret_cast<const float4*>(src);
+                dst[0] = w.x; dst[1] = w.y; dst[2] = w.z; dst[3] = w.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dst[e] = across && e < along ? src[e] : 0.f;
+            }
+        }
+    }
+    __device__ __forceinline__ void store(float (*tile)[TILE_PITCH]) const {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const int i = threadIdx.x + l * 256;
+            if (KFAST) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) tile[i % 4 * 4 + e][i / 4] = v[4 * l + e];
+            } else {
+                *reinterpret_cast<float4*>(&tile[i / (TILE / 4)][i % (TILE / 4) * 4]) = make_float4(v[4 * l], v[4 * l + 1], v[4 * l + 2], v[4 * l + 3]);
+            }
+        }
+    }
+};
+
+template <bool A_KFAST, bool B_KFAST>
+__global__ void __launch_bounds__(256, 2)
+simt_tile_kernel(SimtGemmArgs g) {
+    __shared__ __align__(16) float As[2][TILE_K][TILE_PITCH];
+    __shared__ __align__(16) float Bs[2][TILE_K][TILE_PITCH];
+    const long long m0 = (long long)blockIdx.y * TILE, n0 = (long long)blockIdx.x * TILE;
+    long long M = g.M, k_begin = 0, k_end = g.K, b_offset = 0;
+    float* C = (float*)g.C;
+    if (g.mode == SG_ROWS) {
+        M = g.meta[0];
+        if (m0 >= M) return;
+        b_offset = (long long)g.tile_expert[m0 / kRowPad] * g.b_slab;
+    } else if (g.mode == SG_K) {
+        const int e = blockIdx.z;
+        if (g.counts[e] == 0) return;  // expert received nothing: its slab is left untouched
+        k_begin = g.offsets[e];
+        k_end = k_begin + g.counts[e];
+        C += (long long)e * g.c_slab;
+    }
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    uint64_t acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    for (int seg = 0; seg < 2; ++seg) {
+        const float* Ap = (const float*)(seg ? g.A2 : g.A);
+        if (!Ap) break;
+        const float* Bp = (const float*)(seg ? g.B2 : g.B) + b_offset;
+        TileLoader<A_KFAST> a{Ap + m0 * g.a_rs, A_KFAST ? g.a_rs : g.a_cs, (int)(M - m0 < TILE ? M - m0 : TILE)};
+        TileLoader<B_KFAST> b{Bp + n0 * g.b_cs, B_KFAST ? g.b_cs : g.b_rs, (int)(g.N - n0 < TILE ? g.N - n0 : TILE)};
+        a.fetch(k_begin, k_end);
+        b.fetch(k_begin, k_end);
+        __syncthreads();               // the segment before has been read out of the buffers
+        a.store(As[0]);
+        b.store(Bs[0]);
+        __syncthreads();
+        int buffer = 0;
+        for (long long k0 = k_begin; k0 < k_end; k0 += TILE_K, buffer ^= 1) {
+            const bool more = k0 + TILE_K < k_end;
+            if (more) {
+                a.fetch(k0 + TILE_K, k_end);
+                b.fetch(k0 + TILE_K, k_end);
+            }
+#pragma unroll
+            for (int kk = 0; kk < TILE_K; ++kk) {
+                const float4 a0 = *reinterpret_cast<const float4*>(&As[buffer][kk][ty * 4]), a1 = *reinterpret_cast<const float4*>(&As[buffer][kk][64 + ty * 4]);
+                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[buffer][kk][tx * 4]), b1 = *reinterpret_cast<const ulonglong2*>(&Bs[buffer][kk][64 + tx * 4]);
+                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                const uint64_t bv[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint64_t twice = pair2(av[i], av[i]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fma2(twice, bv[j], acc[i][j]);
+                }
+            }
+            if (more) {
+                a.store(As[buffer ^ 1]);
+                b.store(Bs[buffer ^ 1]);
+                __syncthreads();       // the one barrier of a tile: the other buffer is complete, and nobody reads this one any more
+            }
+        }
+    }
+    const bool vec = g.ldc % 4 == 0 && ((uintptr_t)C & 15u) == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const long long m = m0 + (i / 4) * 64 + ty * 4 + i % 4;
+        if (m >= M) continue;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const long long n = n0 + half * 64 + tx * 4;
+            float v[4];
+            unpair2(acc[i][2 * half], v[0], v[1]);
+            unpair2(acc[i][2 * half + 1], v[2], v[3]);
+            float* dst = C + m * g.ldc + n;
+            if (vec && n + 4 <= g.N) {
+                *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < g.N) dst[e] = v[e];
+            }
+        }
+    }
+}
+
+// What the 128 x 128 kernel takes: fp32 operands and results, each operand contiguous along one of its axes with whole
+// 16-byte pieces, no accumulation, and a tile for every second SM (with fewer, the four times smaller tiles of the general
+// kernel spread better: 48 tiles with K = 512 take 66 us there and 66 .. 70 here, 64 tiles 66 and 59 .. 72, 128 tiles 113 and
+// 61 .. 72).
+bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
+    if (g.accumulate || (g.mode != SG_PLAIN && g.mode != SG_ROWS && g.mode != SG_K)) return false;
+    const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
+    if ((!a_kfast && g.a_rs != 1) || (!b_kfast && g.b_cs != 1)) return false;
+    const long long a_pitch = a_kfast ? g.a_rs : g.a_cs, b_pitch = b_kfast ? g.b_cs : g.b_rs;
+    if (a_pitch % 4 || b_pitch % 4 || g.b_slab % 4) return false;
+    if (((uintptr_t)g.A | (uintptr_t)g.B | (uintptr_t)g.A2 | (uintptr_t)g.B2) & 15u) return false;
+    return (long long)ceil_div(g.N, TILE) * ceil_div(m_extent, TILE) * groups * 2 >= sm_count();
+}
+
+int launch_tiles(const SimtGemmArgs& g, long long m_extent, int groups, cudaStream_t stream) {
+    const dim3 grid(ceil_div(g.N, TILE), ceil_div(m_extent, TILE), groups);
+    const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
+    if (a_kfast && b_kfast) simt_tile_kernel<true, true><<<grid, 256, 0, stream>>>(g);
+    else if (a_kfast) simt_tile_kernel<true, false><<<grid, 256, 0, stream>>>(g);
+    else if (b_kfast) simt_tile_kernel<false, true><<<grid, 256, 0, stream>>>(g);
+    else simt_tile_kernel<false, false><<<grid, 256, 0, stream>>>(g);
+    QMOE_LAUNCH_CHECK("simt_tile_kernel");
+    return 0;
+}
+
 // sum S partial [S][n] slabs in a fixed order
 __global__ void __launch_bounds__(256)
 reduce_partials_kernel(const float* __restrict__ partials, float* __restrict__ out, long long n, int splits) {
@@ -140,7 +301,9 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
     using bf = __nv_bfloat16;
     const int key = (a_dtype << 2) | (b_dtype << 1) | c_dtype;
     switch (key) {
-        case 0: return launch_typed<float, float, float>(g, m_extent, groups, stream);
+        case 0:
+            if (tile_kernel_ok(g, m_extent, groups)) return launch_tiles(g, m_extent, groups, stream);
+            return launch_typed<float, float, float>(g, m_extent, groups, stream);
         case 1: return launch_typed<float, float, bf>(g, m_extent, groups, stream);
         case 2: return launch_typed<float, bf, float>(g, m_extent, groups, stream);
         case 3: return launch_typed<float, bf, bf>(g, m_extent, groups, stream);

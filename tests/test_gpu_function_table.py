@@ -271,3 +271,22 @@ def test_gemm_takes_ragged_row_counts_to_the_tensor_cores(rows, inner, cols, ker
         assert oracle.max_rel_err(got, exact) <= 1e-2
         assert oracle.max_rel_err(got, slow) <= 8e-3
     assert lib.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n", [(128, 16, 128), (1000, 37, 900), (4097, 100, 132), (700, 260, 1028)])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_float32_gemm_in_every_orientation(m, k, n, ta, tb):
+    """float32 products on the 128 x 128 tiles (and, for pitches that are no whole 16 bytes, on the general kernel): one
+    fp32 FMA chain per output, so the error is at most k roundings of sums of |a||b|."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(m + k + n)
+    a, b = (rng.standard_normal(shape).astype(np.float32) for shape in ((k, m) if ta else (m, k), (n, k) if tb else (k, n)))
+    out, sa, sb = DeviceStorage(m * n, "float32"), to_device(a, "float32"), to_device(b, "float32")
+    lib.call("qmoe_gemm", sa.ptr, lib.QMOE_F32, sb.ptr, lib.QMOE_F32, out.ptr, lib.QMOE_F32, m, k, n, ta, tb, 0, 0)
+    got = to_host(out, (m, n))
+    a64, b64 = (a.T if ta else a).astype(np.float64), (b.T if tb else b).astype(np.float64)
+    bound = k * 2.0 ** -24 * (np.abs(a64) @ np.abs(b64)) * 1.01
+    assert np.all(np.abs(got - a64 @ b64) <= bound)
