@@ -14,13 +14,72 @@ namespace qmoe {
 
 namespace {
 
-constexpr int kWarps = 8;
-constexpr int kRowsPerWarp = kRouteRowsPerBlock / kWarps;  // 4
+// A warp per token row of a block: the ranking of a row is a serial chain (32768 rows, 64 experts, top 6: 57 us with four rows
+// per warp and ten shuffles per slot, 27 like this).
+constexpr int kWarps = 32;
+static_assert(kWarps == kRouteRowsPerBlock, "one row per warp");
+constexpr int kPackWarps = 8;
+constexpr int kRowsPerPackWarp = kRouteRowsPerBlock / kPackWarps;
+
+// Softmax and top-k of one token row by one warp; lane l holds experts l, l + 32, ... (EPL of them) of `scores`.  Lane s < k
+// returns the expert and the gate weight of slot s; `p` are the row's probabilities.  Ranking uses the raw scores: softmax
+// is strictly monotone, so this is the ranking by exact probability, without the extra ties that rounding the
+// probabilities to fp32 would create.
+template <int EPL>
+__device__ __forceinline__ void rank_row(const float* __restrict__ scores, int E, int k, float (&p)[EPL], int& expert, float& weight) {
+    const int lane = threadIdx.x & 31;
+    float v[EPL], m = -INFINITY, s = 0.f;
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        const int e = lane + 32 * j;
+        v[j] = e < E ? scores[e] : -INFINITY;
+        m = fmaxf(m, v[j]);
+    }
+    m = warp_max(m);
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        p[j] = lane + 32 * j < E ? expf(v[j] - m) : 0.f;
+        s += p[j];
+    }
+    s = warp_sum(s);
+    // top-k by (score descending, expert index ascending) over unsigned keys in the order of the scores (-0 counts as 0), so
+    // that a slot is two warp reductions of one instruction each.  A NaN score ranks as -inf; the probabilities and gate
+    // weights still carry the NaN to the output.  Key 0: no expert, or already taken.
+    unsigned key[EPL];
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        p[j] = p[j] / s;
+        const float score = v[j] != v[j] ? -INFINITY : v[j] + 0.f;
+        const unsigned bits = __float_as_uint(score);
+        key[j] = lane + 32 * j < E ? bits ^ ((unsigned)((int)bits >> 31) | 0x80000000u) : 0u;
+    }
+    float total = 0.f;
+    expert = 0;
+    weight = 0.f;
+#pragma unroll
+    for (int slot = 0; slot < kMaxTopK; ++slot) {
+        if (slot >= k) break;
+        unsigned best = key[0];
+        int at = lane;
+#pragma unroll
+        for (int j = 1; j < EPL; ++j)
+            if (key[j] > best) { best = key[j]; at = lane + 32 * j; }
+        const unsigned top = __reduce_max_sync(0xffffffffu, best);
+        const int winner = (int)__reduce_min_sync(0xffffffffu, best == top ? (unsigned)at : 0x7fffffffu);   // < E: k <= E
+        float mine = 0.f;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+            if (j == (winner >> 5)) mine = p[j];
+            if (lane + 32 * j == winner) key[j] = 0u;
+        }
+        const float pw = __shfl_sync(0xffffffffu, mine, winner & 31);
+        total += pw;  // left-to-right sum over the slots, like the upstream `sum(...)`
+        if (lane == slot) { expert = winner; weight = pw; }
+    }
+    weight = weight / total;
+}
 
 // ---- K1: softmax + top-k + per-block histogram and probability column sums --------------------
-// One warp per token row; lane l holds experts l, l+32, ... (EPL of them).  Ranking uses the raw
-// scores: softmax is strictly monotone, so this is the ranking by exact probability, without the
-// extra ties that rounding the probabilities to fp32 would create.
 template <int EPL>
 __global__ void __launch_bounds__(kWarps * 32)
 route_topk_kernel(const float* __restrict__ scores, float* __restrict__ probs,
@@ -28,99 +87,29 @@ route_topk_kernel(const float* __restrict__ scores, float* __restrict__ probs,
                   int* __restrict__ block_counts, float* __restrict__ block_colsum,
                   long long T, int E, int k) {
     __shared__ int s_cnt[kMaxExperts];
-    __shared__ float s_col[kWarps][kMaxExperts];
+    __shared__ float s_col[kWarps][32 * EPL];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < E; i += blockDim.x) s_cnt[i] = 0;
     __syncthreads();
-
-    float col[EPL];
+    const long long row = (long long)blockIdx.x * kRouteRowsPerBlock + warp;
+    float p[EPL];
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) col[j] = 0.f;
-
-    const long long row0 = (long long)blockIdx.x * kRouteRowsPerBlock + warp * kRowsPerWarp;
-    for (int r = 0; r < kRowsPerWarp; ++r) {
-        const long long row = row0 + r;
-        if (row >= T) break;
-        float v[EPL], p[EPL];
-        float m = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) {
-            const int e = lane + 32 * j;
-            v[j] = e < E ? scores[row * E + e] : -INFINITY;
-            m = fmaxf(m, v[j]);
+    for (int j = 0; j < EPL; ++j) p[j] = 0.f;
+    if (row < T) {
+        int expert;
+        float weight;
+        rank_row<EPL>(scores + row * E, E, k, p, expert, weight);
+        if (lane < k) {
+            expert_idx[row * k + lane] = expert;
+            gate_w[row * k + lane] = weight;
+            atomicAdd(&s_cnt[expert], 1);  // integer: order does not matter
         }
-        m = warp_max(m);
-        float s = 0.f;
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) {
-            const int e = lane + 32 * j;
-            p[j] = e < E ? expf(v[j] - m) : 0.f;
-            s += p[j];
-        }
-        s = warp_sum(s);
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) {
-            const int e = lane + 32 * j;
-            p[j] = p[j] / s;
-            if (e < E) probs[row * E + e] = p[j];
-            col[j] += p[j];
-        }
-        // top-k by (score descending, expert index ascending).  A NaN score ranks as -inf: every comparison below
-        // then has the same outcome in every lane, so the lanes agree on each winner (with NaNs left in, each lane
-        // would keep its own candidate, mark only that one as taken, and run out of candidates before slot k).
-        // The probabilities and gate weights still carry the NaN to the output.
 #pragma unroll
         for (int j = 0; j < EPL; ++j)
-            if (v[j] != v[j]) v[j] = -INFINITY;
-        unsigned taken = 0;
-        float wsel[kMaxTopK];
-        float total = 0.f;
-#pragma unroll
-        for (int slot = 0; slot < kMaxTopK; ++slot) {
-            wsel[slot] = 0.f;
-            if (slot < k) {
-                float bv = -INFINITY;
-                int be = INT_MAX;
-#pragma unroll
-                for (int j = 0; j < EPL; ++j) {
-                    const int e = lane + 32 * j;
-                    if (e < E && !((taken >> j) & 1u) && (be == INT_MAX || v[j] > bv)) {
-                        bv = v[j];
-                        be = e;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o; o >>= 1) {
-                    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                    const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-                    if (oe != INT_MAX && (be == INT_MAX || ov > bv || (ov == bv && oe < be))) {
-                        bv = ov;
-                        be = oe;
-                    }
-                }
-                float mine = 0.f;
-#pragma unroll
-                for (int j = 0; j < EPL; ++j)
-                    if (j == (be >> 5)) mine = p[j];
-                if ((be & 31) == lane) taken |= 1u << (be >> 5);
-                const float pw = __shfl_sync(0xffffffffu, mine, be & 31);
-                wsel[slot] = pw;
-                total += pw;  // left-to-right sum over the slots, like the upstream `sum(...)`
-                if (lane == 0) {   // be < E here: k <= E and the ranking is a total order
-                    expert_idx[row * k + slot] = be;
-                    atomicAdd(&s_cnt[be], 1);  // integer: order does not matter
-                }
-            }
-        }
-#pragma unroll
-        for (int slot = 0; slot < kMaxTopK; ++slot)
-            if (slot < k && lane == slot) gate_w[row * k + slot] = wsel[slot] / total;
+            if (lane + 32 * j < E) probs[row * E + lane + 32 * j] = p[j];
     }
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) {
-        const int e = lane + 32 * j;
-        if (e < E) s_col[warp][e] = col[j];
-    }
+    for (int j = 0; j < EPL; ++j) s_col[warp][lane + 32 * j] = p[j];
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         float t = 0.f;
@@ -128,6 +117,46 @@ route_topk_kernel(const float* __restrict__ scores, float* __restrict__ probs,
         for (int w = 0; w < kWarps; ++w) t += s_col[w][e];  // fixed order
         block_colsum[(long long)blockIdx.x * E + e] = t;
         block_counts[(long long)blockIdx.x * E + e] = s_cnt[e];
+    }
+}
+
+// ---- what follows from the counts and the probability sums of all experts -----------------------
+// Two warps: the first forms the padded offsets (s_off) and writes meta, the second the auxiliary loss.  Fixed order.
+__device__ __forceinline__ void publish_totals(const int* s_cnt, const double* s_cs, int* s_off, int* __restrict__ offsets, int* __restrict__ meta,
+                                               float* __restrict__ aux, long long T, int E, int k) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        int before = 0;
+        for (int base = 0; base < E; base += 32) {
+            const int e = base + lane;
+            const int padded = e < E ? (s_cnt[e] + kRowPad - 1) / kRowPad * kRowPad : 0;
+            int sum = padded;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += up;
+            }
+            if (e < E) {
+                s_off[e] = before + sum - padded;
+                offsets[e] = before + sum - padded;
+            }
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) {
+            s_off[E] = before;
+            offsets[E] = before;
+            meta[0] = before;
+            meta[1] = before / kRowPad;
+            meta[2] = (int)(T * k);
+            meta[3] = 0;
+        }
+    } else if (warp == 1) {
+        const double A = (double)T * k;
+        double total = 0.0;
+        for (int e = lane; e < E; e += 32) total += ((double)s_cnt[e] / A) * s_cs[e] / (double)T;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        if (lane == 0) aux[0] = (float)((double)E * total);
     }
 }
 
@@ -180,28 +209,11 @@ route_scan_kernel(const int* __restrict__ block_counts, const float* __restrict_
         }
     }
     __syncthreads();
-    const double A = (double)T * k;
-    if (threadIdx.x == 0) {
-        int off = 0;
-        double total = 0.0;
-        for (int i = 0; i < E; ++i) {
-            s_off[i] = off;
-            offsets[i] = off;
-            off += (s_cnt[i] + kRowPad - 1) / kRowPad * kRowPad;
-            total += ((double)s_cnt[i] / A) * s_cs[i] / (double)T;
-        }
-        s_off[E] = off;
-        offsets[E] = off;
-        meta[0] = off;
-        meta[1] = off / kRowPad;
-        meta[2] = (int)(T * k);
-        meta[3] = 0;
-        aux[0] = (float)((double)E * total);
-    }
+    publish_totals(s_cnt, s_cs, s_off, offsets, meta, aux, T, E, k);
     __syncthreads();
     if (threadIdx.x < E) {
         const int x = threadIdx.x;
-        util[x] = (float)((double)s_cnt[x] / A);
+        util[x] = (float)((double)s_cnt[x] / ((double)T * k));
         for (int t = s_off[x] / kRowPad; t < s_off[x + 1] / kRowPad; ++t) tile_expert[t] = x;
     }
 }
@@ -209,17 +221,17 @@ route_scan_kernel(const int* __restrict__ block_counts, const float* __restrict_
 // ---- K3: stable rank of every assignment inside (block, expert) -> dispatch tables -----------
 // Same block partition as K1.  Warp w owns a contiguous slice of the block's assignments; a
 // `match_any` per 32-assignment chunk ranks equal experts by lane, so order is (token, slot).
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kPackWarps * 32)
 route_pack_kernel(const int* __restrict__ expert_idx, const int* __restrict__ block_base,
                   const int* __restrict__ offsets, int* __restrict__ dest_row,
                   int* __restrict__ row_source, long long T, int E, int k) {
-    __shared__ int s_hist[kWarps][kMaxExperts];
+    __shared__ int s_hist[kPackWarps][kMaxExperts];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < kWarps * kMaxExperts; i += blockDim.x) (&s_hist[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < kPackWarps * kMaxExperts; i += blockDim.x) (&s_hist[0][0])[i] = 0;
     __syncthreads();
     const long long A = T * k;
-    const long long begin = ((long long)blockIdx.x * kRouteRowsPerBlock + warp * kRowsPerWarp) * k;
-    long long end = begin + (long long)kRowsPerWarp * k;
+    const long long begin = ((long long)blockIdx.x * kRouteRowsPerBlock + warp * kRowsPerPackWarp) * k;
+    long long end = begin + (long long)kRowsPerPackWarp * k;
     if (end > A) end = A;
     const unsigned lt = (1u << lane) - 1u;
     for (long long base = begin; base < end; base += 32) {
@@ -233,7 +245,7 @@ route_pack_kernel(const int* __restrict__ expert_idx, const int* __restrict__ bl
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         int run = offsets[e] + block_base[(long long)blockIdx.x * E + e];
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < kPackWarps; ++w) {
             const int c = s_hist[w][e];
             s_hist[w][e] = run;
             run += c;
@@ -253,6 +265,92 @@ route_pack_kernel(const int* __restrict__ expert_idx, const int* __restrict__ bl
             dest_row[a] = dest;
             row_source[dest] = (int)a;
         }
+    }
+}
+
+// ---- few tokens (decoding): the whole routing in one block -------------------------------------------
+// At 64 tokens the three kernels above and the fill of row_source are four launches of which none has work for more than
+// one or two SMs; here the same steps meet at block barriers (64 tokens, 64 experts, top 6: 31 us in four launches with one
+// warp per four rows, 11 here; 4 tokens, 8 experts, top 2: 19 and 5.5).  What is left is the chain of a row's reductions.  A warp ranks the rows warp, warp + 32, ...; then warp w
+// holds the w-th slice of at most 32 consecutive assignments, ranked among equals by `match_any`.
+constexpr long long kSmallRouteTokens = 128;
+static_assert(kSmallRouteTokens * kMaxTopK <= kWarps * 32, "a slice of assignments is one per lane");
+template <int EPL>
+__global__ void __launch_bounds__(kWarps * 32, 1)
+route_small_kernel(const float* __restrict__ scores, float* __restrict__ probs, float* __restrict__ gate_w, int* __restrict__ expert_idx,
+                   int* __restrict__ dest_row, int* row_source, int* __restrict__ counts, int* __restrict__ offsets,
+                   int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util, float* __restrict__ aux,
+                   float* __restrict__ block_colsum, int T, int E, int k, long long rows_bound) {
+    // [warp][expert]: probability sums, then assignments; one more column, so that a warp reading one expert's 32 entries
+    // meets 32 banks
+    __shared__ union { float col[kWarps][32 * EPL + 1]; int hist[kWarps][32 * EPL + 1]; } s;
+    __shared__ int s_idx[kSmallRouteTokens * kMaxTopK];
+    __shared__ int s_cnt[32 * EPL], s_off[32 * EPL + 1];
+    __shared__ double s_cs[32 * EPL];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (long long i = threadIdx.x; i < rows_bound; i += blockDim.x) row_source[i] = -1;
+    float col[EPL];
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) col[j] = 0.f;
+    for (int row = warp; row < T; row += kWarps) {
+        float p[EPL], weight;
+        int expert;
+        rank_row<EPL>(scores + (long long)row * E, E, k, p, expert, weight);
+        if (lane < k) {
+            s_idx[row * k + lane] = expert;
+            expert_idx[row * k + lane] = expert;
+            gate_w[row * k + lane] = weight;
+        }
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+            col[j] += p[j];
+            if (lane + 32 * j < E) probs[(long long)row * E + lane + 32 * j] = p[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) s.col[warp][lane + 32 * j] = col[j];
+    __syncthreads();
+    for (int e = warp; e < E; e += kWarps) {       // a warp per expert, its lanes the 32 partial sums
+        double t = (double)s.col[lane][e];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) s_cs[e] = t;
+        // readers of the per-block sums (expert parallelism) add them over the blocks: the first holds all
+        if (lane * kRouteRowsPerBlock < T) block_colsum[(long long)lane * E + e] = lane ? 0.f : (float)t;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kWarps * (32 * EPL + 1); i += blockDim.x) (&s.hist[0][0])[i] = 0;
+    __syncthreads();
+    const int A = T * k, slice = (A + kWarps - 1) / kWarps, a = warp * slice + lane;
+    const int mine = lane < slice && a < A ? s_idx[a] : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, mine);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    if (mine >= 0 && rank == 0) s.hist[warp][mine] = __popc(peers);
+    __syncthreads();
+    for (int e = warp; e < E; e += kWarps) {       // prefix over the slices
+        const int own = s.hist[lane][e];
+        int run = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += up;
+        }
+        s.hist[lane][e] = run - own;
+        if (lane == 31) {
+            s_cnt[e] = run;
+            counts[e] = run;
+            util[e] = (float)((double)run / (double)A);
+        }
+    }
+    __syncthreads();
+    publish_totals(s_cnt, s_cs, s_off, offsets, meta, aux, T, E, k);
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x)
+        for (int t = s_off[e] / kRowPad; t < s_off[e + 1] / kRowPad; ++t) tile_expert[t] = e;
+    if (mine >= 0) {
+        const int dest = s_off[mine] + s.hist[warp][mine] + rank;
+        dest_row[a] = dest;
+        row_source[dest] = a;      // after the fill above: barriers lie between
     }
 }
 
@@ -348,7 +446,6 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
     const int nblk = (int)qmoe_route_blocks(r->tokens);
     const long long T = r->tokens;
     const int E = r->experts, k = r->top_k;
-    QMOE_CUDA(cudaMemsetAsync((void*)r->row_source, 0xff, (size_t)r->rows_bound * sizeof(int), stream));
     const float* sc = (const float*)scores;
     float* probs = (float*)r->probs;
     float* gw = (float*)r->gate_weights;
@@ -356,6 +453,18 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
     int* bc = (int*)r->block_counts;
     float* bs = (float*)r->block_colsum;
     const int epl = (E + 31) / 32;
+    if (T <= kSmallRouteTokens) {
+#define ARGS <<<1, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, (int*)r->dest_row, (int*)r->row_source, (int*)r->counts, (int*)r->offsets, \
+        (int*)r->tile_expert, (int*)r->meta, (float*)r->utilization, (float*)r->aux, bs, (int)T, E, k, (long long)r->rows_bound)
+        if (epl <= 1) route_small_kernel<1> ARGS;
+        else if (epl <= 2) route_small_kernel<2> ARGS;
+        else if (epl <= 4) route_small_kernel<4> ARGS;
+        else route_small_kernel<8> ARGS;
+#undef ARGS
+        QMOE_LAUNCH_CHECK("route_small_kernel");
+        return 0;
+    }
+    QMOE_CUDA(cudaMemsetAsync((void*)r->row_source, 0xff, (size_t)r->rows_bound * sizeof(int), stream));
     if (epl <= 1) route_topk_kernel<1><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
     else if (epl <= 2) route_topk_kernel<2><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
     else if (epl <= 4) route_topk_kernel<4><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
@@ -366,7 +475,7 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
                                                       (int*)r->meta, (float*)r->utilization,
                                                       (float*)r->aux, nblk, T, E, k);
     QMOE_LAUNCH_CHECK("route_scan_kernel");
-    route_pack_kernel<<<nblk, kWarps * 32, 0, stream>>>(eidx, (const int*)r->block_base,
+    route_pack_kernel<<<nblk, kPackWarps * 32, 0, stream>>>(eidx, (const int*)r->block_base,
                                                         (const int*)r->offsets, (int*)r->dest_row,
                                                         (int*)r->row_source, T, E, k);
     QMOE_LAUNCH_CHECK("route_pack_kernel");
