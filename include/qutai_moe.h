@@ -27,8 +27,9 @@
  * to expert 0, then expert 1, ...; inside one expert rows keep increasing (token, slot) order —
  * the order of the upstream `ids`/`slots` lists (src/qutai/backends/cpu_lm.py:204-221,
  * src/qutai/backends/cuda/lm.cu:353-383) — and each expert group starts at a multiple of
- * QMOE_ROW_PAD rows; the pad rows hold zeros.  A buffer in that layout has
- * qmoe_rows_bound(T, E, k) rows.
+ * QMOE_ROW_PAD rows; the pad rows hold zeros (in the buffers that a whole-layer or whole-block call
+ * fills for itself only those up to the next multiple of 16 rows may be relied on).  A buffer in
+ * that layout has qmoe_rows_bound(T, E, k) rows.
  */
 #ifndef QUTAI_MOE_H
 #define QUTAI_MOE_H
@@ -118,7 +119,8 @@ enum {
     QMOE_VARIANT_WGRAD_PER_PRODUCT = 1, /* one launch per weight-gradient product instead of one for all three */
     QMOE_VARIANT_NARROW_SCATTER = 2,    /* 64-byte instead of 256-byte row pieces in the peer-memory scatter epilogues */
     QMOE_VARIANT_PLAIN_GEMM_ON_CUDA_CORES = 3, /* qmoe_gemm never takes the tensor-core kernels */
-    QMOE_VARIANT_COUNT = 4
+    QMOE_VARIANT_NO_STREAM_GEMM = 4,    /* expert products of few rows on the kernel for many rows */
+    QMOE_VARIANT_COUNT = 5
 };
 int qmoe_test_select_variant(int32_t which, int32_t value);
 

@@ -110,6 +110,24 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Zero rows count .. round_up(count, pad) - 1 of every expert's group (pad divides kRowPad), a warp per row.
+template <typename T, bool VEC>
+__device__ __forceinline__ void zero_pad_rows(T* out, const int* offsets, const int* counts, int experts, int pad, long long width,
+                                              long long warp, long long nwarps) {
+    const int lane = threadIdx.x & 31;
+    for (long long i = warp; i < (long long)experts * pad; i += nwarps) {
+        const int e = (int)(i / pad), count = counts[e], row = count + (int)(i % pad);
+        if (row >= (count + pad - 1) / pad * pad) continue;
+        T* dst = out + ((long long)offsets[e] + row) * width;
+        if constexpr (VEC) {
+            constexpr int N = Vec16<T>::N;
+            for (int c = lane; c < (int)(width / N); c += 32) *reinterpret_cast<uint4*>(dst + (long long)c * N) = make_uint4(0, 0, 0, 0);
+        } else {
+            for (long long c = lane; c < width; c += 32) Act<T>::store(dst + c, 0.f);
+        }
+    }
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 int sm_count();
 
@@ -140,6 +158,10 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
                      cudaStream_t stream);
 
 // ---- cross-file entry points -----------------------------------------------------------------
+// qmoe_permute / qmoe_permute_norm with the pad rows zeroed only up to a multiple of `pad` rows per expert
+int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream);
+int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t weight, uint64_t out, int32_t dtype, int64_t width, int pad,
+                        uint64_t stream);
 int route_check(const qmoe_route_t* r);
 int launch_swiglu(const qmoe_route_t* r, uint64_t g, uint64_t u, uint64_t h, int dtype, long long hidden, cudaStream_t stream);
 int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint64_t u, uint64_t dg, uint64_t du, int dtype,
@@ -155,6 +177,14 @@ int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
                const TcScatter* scatter = nullptr, long long rows = 0);
 int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c, long long K,
                long long N, cudaStream_t stream, const TcScatter* scatter = nullptr, long long rows = 0);
+// the same two forward products for few rows per expert (gemm_stream.cu)
+// pad_rows: every pad row holds zeros afterwards; else only those up to a multiple of kStreamPad rows of each expert
+constexpr int kStreamPad = 16;
+bool stream_shape_ok(const qmoe_route_t* r, int experts);
+int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows,
+                          cudaStream_t stream);
+int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows,
+                   cudaStream_t stream);
 int tc_dswiglu(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t w_down, uint64_t g, uint64_t u, uint64_t dg,
                uint64_t du, long long d, long long h, cudaStream_t stream);
 int tc_wgrad3(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t h_act, uint64_t x, uint64_t dg, uint64_t du,

@@ -1,0 +1,294 @@
+// Expert products for few rows per expert (decoding, short prompts), where the pass over the weights is the work:
+// C[rows, N] = A[rows, K] . B_e formed as its transpose, so that the WEIGHT tile is the 128-row operand of the MMA and an
+// expert's rows are its columns (N = 16 .. 128, as many as there are).
+//
+// The kernel for many rows (gemm_tcgen05.cu) gives every expert tiles of 256 rows: an expert with six rows still costs
+// the tensor time of 256 and stages 128 rows of activations beside every 128 rows of weights.  Here both follow the
+// expert's own row count, and what bounds a product is HBM: 128 KiB of weight tiles in flight per SM.  64 rows over 64 experts,
+// top 6, 2048 x 1408: SwiGLU 144 -> 113 us (738 MB: 6.5 TB/s), down product 72 -> 60.
+//
+// One persistent CTA per SM, 6 warps: warp 0 asks TMA for the tiles, warp 1 issues the MMAs, warps 2-5 convert the
+// accumulators (lane = output column, TMEM column = row of the expert) and store them; two accumulator sets, so a
+// tile's epilogue runs beside the next tile's main loop.
+//   STREAM_SWIGLU   G, U, H from X: a stage holds 64 columns of a gate tile and of the up tile beside it
+//   STREAM_NT       C = A . B_e^T, B stacked [E * N, K]
+//   STREAM_NT2      the same with 256 output columns per tile, so that a stage of activations serves two weight tiles: for
+//                   experts of many rows, whose activations are as many bytes as a weight tile
+// Every wait is bounded (status codes 111 .. 113).
+#include "common.cuh"
+#include "tc_ptx.cuh"
+
+namespace qmoe {
+namespace {
+
+constexpr int SM_ROWS = 128, SK = 64;                  // weight rows of a tile, contraction columns of a stage
+constexpr int W_BYTES = SM_ROWS * SK * 2;              // 16 KiB
+constexpr int X_BOX = 32, X_BOX_BYTES = X_BOX * SK * 2;  // activations arrive in boxes of 32 rows
+constexpr int X_BYTES = kRowPad * SK * 2;              // at most 128 rows: 16 KiB
+constexpr int STREAM_THREADS = 192;
+constexpr uint32_t STREAM_TMEM = 512;                  // two sets of two 128-column accumulators
+
+enum { STREAM_SWIGLU = 0, STREAM_NT = 1, STREAM_NT2 = 2 };
+enum { STATUS_STREAM_PRODUCER = 111, STATUS_STREAM_MMA = 112, STATUS_STREAM_EPILOGUE = 113 };
+
+template <int MODE> struct StreamCfg {
+    static constexpr int W_TILES = MODE == STREAM_NT ? 1 : 2;
+    static constexpr int STAGE_BYTES = W_TILES * W_BYTES + X_BYTES;
+    static constexpr int STAGES = MODE == STREAM_NT ? 6 : 4;
+    static constexpr int COLUMNS = MODE == STREAM_NT2 ? 2 * SM_ROWS : SM_ROWS;    // output columns of a tile
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+};
+
+struct alignas(64) StreamParams {
+    CUtensorMap map_w, map_w2;     // weights (gate and up, or the only one)
+    CUtensorMap map_x;             // activations in the dispatched layout
+    const int* offsets;
+    const int* counts;
+    int* status;
+    __nv_bfloat16* out0;           // SWIGLU: G; NT: C
+    __nv_bfloat16* out1;           // SWIGLU: U
+    __nv_bfloat16* out2;           // SWIGLU: H
+    int experts, m_tiles, N, K;
+    int pad_rows;                  // zero every pad row; else those from `columns` on are left as they are
+};
+
+struct StreamTile { int expert, n0, row0, columns; };   // `columns`: rows of the expert in this tile, rounded up to 16
+
+// tiles of expert e: m_tiles weight tiles x its 128-row chunks, the chunks of one weight tile side by side (the second
+// finds the weights in L2)
+__device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const int* first, int t, int columns) {
+    int lo = 0, hi = p.experts;        // largest e with first[e] <= t
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= t) lo = mid; else hi = mid;
+    }
+    const int chunks = (first[lo + 1] - first[lo]) / p.m_tiles, local = t - first[lo], chunk = local % chunks;
+    StreamTile tile;
+    tile.expert = lo;
+    tile.n0 = local / chunks * columns;
+    tile.row0 = p.offsets[lo] + chunk * kRowPad;
+    const int left = p.counts[lo] - chunk * kRowPad;
+    tile.columns = left >= kRowPad ? kRowPad : (left + kStreamPad - 1) / kStreamPad * kStreamPad;
+    return tile;
+}
+
+__device__ __forceinline__ float logistic(float v) {   // 1 / (1 + 2^(-v log2 e)) as in the kernel for many rows
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * v));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return r;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(STREAM_THREADS, 1)
+stream_gemm_kernel(const __grid_constant__ StreamParams p) {
+    using Config = StreamCfg<MODE>;
+    constexpr int STAGES = Config::STAGES, STAGE_BYTES = Config::STAGE_BYTES, W_TILES = Config::W_TILES;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ int s_first[kMaxExperts + 1];     // first tile of each expert
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = base + STAGES * STAGE_BYTES;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+    auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
+    auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
+
+    for (int e = threadIdx.x; e <= p.experts; e += STREAM_THREADS) {
+        int tiles = 0;
+        for (int j = 0; j < e; ++j) tiles += (p.counts[j] + kRowPad - 1) / kRowPad;
+        s_first[e] = tiles * p.m_tiles;
+    }
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_map(&p.map_w); prefetch_map(&p.map_w2); prefetch_map(&p.map_x);
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(STREAM_TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem_base;
+    const int total = s_first[p.experts], kblocks = (p.K + SK - 1) / SK;
+    volatile int* abort_flag = &s_abort;
+    auto gave_up = [&](int code) { if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, code); } };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int t = blockIdx.x; t < total && !*abort_flag; t += gridDim.x) {
+                const StreamTile tile = stream_tile(p, s_first, t, Config::COLUMNS);
+                const int boxes = (tile.columns + X_BOX - 1) / X_BOX, w_row = tile.expert * p.N + tile.n0;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { gave_up(STATUS_STREAM_PRODUCER); break; }
+                    const uint32_t w = base + stage * STAGE_BYTES, x = w + W_TILES * W_BYTES, bar = full_bar(stage);
+                    mbar_expect_tx(bar, W_TILES * W_BYTES + boxes * X_BOX_BYTES);
+                    tma_load_2d(&p.map_w, w, bar, kb * SK, w_row);
+                    if (MODE == STREAM_SWIGLU) tma_load_2d(&p.map_w2, w + W_BYTES, bar, kb * SK, w_row);
+                    if (MODE == STREAM_NT2) tma_load_2d(&p.map_w, w + W_BYTES, bar, kb * SK, w_row + SM_ROWS);
+                    for (int j = 0; j < boxes; ++j) tma_load_2d(&p.map_x, x + j * X_BOX_BYTES, bar, kb * SK, tile.row0 + j * X_BOX);
+                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        int stage = 0, iter = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < total; t += gridDim.x, ++iter) {
+            const StreamTile tile = stream_tile(p, s_first, t, Config::COLUMNS);
+            const uint32_t idesc = make_idesc<false, false, SM_ROWS>(tile.columns), acc = tmem + (uint32_t)(iter & 1) * 256;
+            ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(iter & 1), ((uint32_t)(iter >> 1) & 1u) ^ 1u, abort_flag));
+            tc_fence_after();
+            for (int kb = 0; ok && kb < kblocks; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t w = base + stage * STAGE_BYTES, x = w + W_TILES * W_BYTES;
+                if (elect_one()) {
+#pragma unroll
+                    for (int which = 0; which < W_TILES; ++which)
+#pragma unroll
+                        for (int kk = 0; kk < SK / 16; ++kk)
+                            umma_bf16(acc + which * 128, make_desc(w + which * W_BYTES + kk * 32, 16, 1024), make_desc(x + kk * 32, 16, 1024), idesc,
+                                      (kb | kk) ? 1u : 0u);
+                    umma_commit(empty_bar(stage));
+                    if (kb == kblocks - 1) umma_commit(tfull_bar(iter & 1));
+                }
+                __syncwarp();
+                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+            }
+        }
+        if (!ok && lane == 0) gave_up(STATUS_STREAM_MMA);
+    } else {
+        const int quad = warp & 3;
+        int iter = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, ++iter) {
+            const StreamTile tile = stream_tile(p, s_first, t, Config::COLUMNS);
+            const int a = iter & 1, n = tile.n0 + quad * 32 + lane;
+            if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(a), (uint32_t)(iter >> 1) & 1u, abort_flag))) {
+                if (lane == 0) gave_up(STATUS_STREAM_EPILOGUE);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t acc = tmem + (uint32_t)a * 256 + ((uint32_t)(quad * 32) << 16);
+            const long long at = (long long)tile.row0 * p.N + n;
+#pragma unroll 1
+            for (int c = 0; c < tile.columns; c += 16) {      // a store instruction covers 32 consecutive columns of one row
+                uint32_t v0[16], v1[16];
+                tmem_ld16(acc + c, v0);
+                if (W_TILES == 2) tmem_ld16(acc + 128 + c, v1);
+                tmem_ld_wait();
+                if (n < p.N) {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        const long long to = at + (long long)(c + e) * p.N;
+                        if (MODE == STREAM_SWIGLU) {
+                            // H from the rounded G and U, which are what the backward reads
+                            const __nv_bfloat16 gb = __float2bfloat16_rn(__uint_as_float(v0[e])), ub = __float2bfloat16_rn(__uint_as_float(v1[e]));
+                            const float g = __bfloat162float(gb);
+                            p.out0[to] = gb;
+                            p.out1[to] = ub;
+                            p.out2[to] = __float2bfloat16_rn(g * logistic(g) * __bfloat162float(ub));
+                        } else {
+                            p.out0[to] = __float2bfloat16_rn(__uint_as_float(v0[e]));
+                            if (MODE == STREAM_NT2 && n + SM_ROWS < p.N) p.out0[to + SM_ROWS] = __float2bfloat16_rn(__uint_as_float(v1[e]));
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty_bar(a));
+            if (p.pad_rows && n < p.N) {
+                const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
+                for (int c = tile.columns; c < kRowPad; ++c) {
+                    const long long to = at + (long long)c * p.N;
+                    p.out0[to] = zero;
+                    if (MODE == STREAM_SWIGLU) { p.out1[to] = zero; p.out2[to] = zero; }
+                    if (MODE == STREAM_NT2 && n + SM_ROWS < p.N) p.out0[to + SM_ROWS] = zero;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (s_abort) {   // copies and MMAs in flight get a bounded time to land before shared memory and TMEM go away
+        const unsigned long long start = global_ns();
+        while (global_ns() - start < 2000000ull) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(STREAM_TMEM) : "memory");
+    }
+}
+
+template <int MODE>
+int stream_launch(const StreamParams& p, cudaStream_t stream) {
+    static bool configured[64] = {};      // per device, like the kernels of gemm_tcgen05.cu
+    int dev = 0;
+    QMOE_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail_arg("device ordinal beyond 63");
+    if (!configured[dev]) {
+        QMOE_CUDA(cudaFuncSetAttribute(stream_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamCfg<MODE>::SMEM_BYTES));
+        configured[dev] = true;
+    }
+    stream_gemm_kernel<MODE><<<sm_count(), STREAM_THREADS, StreamCfg<MODE>::SMEM_BYTES, stream>>>(p);
+    count_tensor_core_launch();
+    QMOE_LAUNCH_CHECK("stream_gemm_kernel");
+    return 0;
+}
+
+}  // namespace
+
+// Few rows per expert, on average.  SwiGLU and down product together, here against the kernel for many rows (us, L2 flushed):
+// 32 experts, 2048 x 1408: 136 / 146 at 16 rows, 143 / 145 at 96, 159 / 150 at 128; 16 experts, 1024 x 2048: 68 / 78, 71 / 78,
+// 82 / 80; 8 experts, 1024 x 2816: 60 / 68, 66 / 69, 66 / 70.
+constexpr long long kStreamRowsPerExpert = 96;
+bool stream_shape_ok(const qmoe_route_t* r, int experts) {
+    return r->tokens * r->top_k <= kStreamRowsPerExpert * experts && !kernel_variant(QMOE_VARIANT_NO_STREAM_GEMM);
+}
+
+int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows,
+                          cudaStream_t stream) {
+    StreamParams p = {};
+    const uint64_t d = (uint64_t)ex->width, hd = (uint64_t)ex->hidden, E = (uint64_t)ex->experts;
+    if (int rc = make_map_2d(&p.map_w, ex->w_gate, d, E * hd, SM_ROWS)) return rc;
+    if (int rc = make_map_2d(&p.map_w2, ex->w_up, d, E * hd, SM_ROWS)) return rc;
+    if (int rc = make_map_2d(&p.map_x, x, d, (uint64_t)r->rows_bound, X_BOX)) return rc;
+    p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
+    p.out0 = (__nv_bfloat16*)g; p.out1 = (__nv_bfloat16*)u; p.out2 = (__nv_bfloat16*)h;
+    p.experts = ex->experts; p.m_tiles = ceil_div((long long)hd, SM_ROWS); p.N = (int)hd; p.K = (int)d;
+    p.pad_rows = pad_rows;
+    return stream_launch<STREAM_SWIGLU>(p, stream);
+}
+
+int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows,
+                   cudaStream_t stream) {
+    StreamParams p = {};
+    if (int rc = make_map_2d(&p.map_w, b, (uint64_t)K, (uint64_t)experts * N, SM_ROWS)) return rc;
+    p.map_w2 = p.map_w;
+    if (int rc = make_map_2d(&p.map_x, a, (uint64_t)K, (uint64_t)r->rows_bound, X_BOX)) return rc;
+    p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
+    p.out0 = (__nv_bfloat16*)c;
+    p.experts = experts; p.N = (int)N; p.K = (int)K; p.pad_rows = pad_rows;
+    // Two weight tiles per stage where that leaves a tile for every SM and an expert's rows take more than one box of
+    // activations: 64 experts, 94 rows on average, 1408 -> 2048 columns: 81 us with one, 74 with two; but 16 experts, 96 rows,
+    // 2048 -> 1024 columns (64 tiles of 256): 27 with one, 32 with two.
+    if (r->tokens * r->top_k > (long long)X_BOX * experts && (long long)ceil_div(N, 2 * SM_ROWS) * experts >= sm_count()) {
+        p.m_tiles = ceil_div(N, 2 * SM_ROWS);
+        return stream_launch<STREAM_NT2>(p, stream);
+    }
+    p.m_tiles = ceil_div(N, SM_ROWS);
+    return stream_launch<STREAM_NT>(p, stream);
+}
+
+}  // namespace qmoe

@@ -108,6 +108,7 @@ struct alignas(64) GemmParams {
 struct Tile {
     int expert, row0, n0, kblocks, krow0;
     int problem;      // WGRAD: which of the launch's products this tile belongs to
+    int depth;        // WGRAD: rows of the contraction
     int bn;           // accumulator columns of this tile: 256, or 128 for a last tile that is at most half full (B in MN-major only)
     bool valid;       // false: nothing to do for the whole tile (all CTAs of the tile skip it)
     bool rows_valid;  // CTAS == 2: false when this CTA's 128 rows lie past the end of the expert (compute, do not store)
@@ -148,6 +149,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         tile.row0 = (rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
         tile.n0 = (rem / p.m_tiles) * BN;
         const int count = p.plain_rows > 0 ? p.plain_rows : p.counts[e];
+        tile.depth = count;
         tile.kblocks = (count + BK - 1) / BK;
         tile.krow0 = s_start[e] * kRowPad;
         tile.valid = count > 0;
@@ -529,6 +531,8 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                         // the look at the next stage's barrier goes between the MMAs, where the tensor pipe has work queued,
                         // rather than after the last one, where its latency would leave the pipe idle
                         if (kk == BK / UMMA_K - 1) ready = kb + 1 < tile.kblocks && mbar_try(full_bar(next_stage), next_phase);
+                        // WGRAD: rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten)
+                        if (MODE == MODE_WGRAD && kb * BK + kk * UMMA_K >= tile.depth) continue;
                         if (CTAS == 2) umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
                         else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
                     }
@@ -928,6 +932,8 @@ int make_map(CUtensorMap* out, uint64_t ptr, uint64_t inner, uint64_t outer, uin
 }
 
 }  // namespace
+
+int make_map_2d(CUtensorMap* out, uint64_t ptr, uint64_t inner, uint64_t outer, uint32_t box_outer) { return make_map(out, ptr, inner, outer, box_outer); }
 
 // 3-D bf16 tensor [outer][mid][inner] (dense), box {64, box_mid, 1}, 128-byte swizzle: the attention kernels' view of
 // [batch][time][heads * 64], in which a box never crosses from one sequence into the next and positions past the end

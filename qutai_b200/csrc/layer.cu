@@ -59,8 +59,9 @@ int simt_wgrad(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint
 
 using namespace qmoe;
 
-extern "C" int qmoe_expert_forward_parts(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u,
-                                         uint64_t h, uint64_t y, int32_t parts, uint64_t stream_) {
+// pad_rows: see stream_swiglu_forward (the kernels for many rows always write whole 128-row tiles)
+static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, uint64_t y,
+                          int32_t parts, bool pad_rows, uint64_t stream_) {
     int engine = 0;
     if (int rc = check_experts(r, ex, &engine)) return rc;
     if (!(parts & (QMOE_FWD_UP | QMOE_FWD_DOWN)) || (parts & ~(QMOE_FWD_UP | QMOE_FWD_DOWN)))
@@ -69,9 +70,12 @@ extern "C" int qmoe_expert_forward_parts(const qmoe_route_t* r, const qmoe_exper
         return fail_arg("expert_forward: null buffer address");
     cudaStream_t stream = (cudaStream_t)stream_;
     const long long d = ex->width, hd = ex->hidden;
-    const bool tc = engine == QMOE_ENGINE_TCGEN05;
+    const bool tc = engine == QMOE_ENGINE_TCGEN05, few_rows = tc && stream_shape_ok(r, ex->experts);
     if (parts & QMOE_FWD_UP) {
-        if (tc) {
+        if (few_rows) {
+            TimedScope timed(KC_EXPERT_GEMM, stream);
+            if (int rc = stream_swiglu_forward(r, ex, x, g, u, h, pad_rows, stream)) return rc;
+        } else if (tc) {
             TimedScope timed(KC_EXPERT_GEMM, stream);
             if (int rc = tc_swiglu_forward(r, ex, x, g, u, h, stream)) return rc;
         } else {
@@ -85,10 +89,16 @@ extern "C" int qmoe_expert_forward_parts(const qmoe_route_t* r, const qmoe_exper
     }
     if (parts & QMOE_FWD_DOWN) {
         TimedScope timed(KC_EXPERT_GEMM, stream);
+        if (few_rows) return stream_rows_nt(r, ex->experts, h, ex->w_down, y, hd, d, pad_rows, stream);
         return tc ? tc_rows_nt(r, ex->experts, h, ex->w_down, y, hd, d, stream)
                   : simt_rows(r, ex, h, ex->w_down, 0, 0, y, hd, d, true, stream);
     }
     return 0;
+}
+
+extern "C" int qmoe_expert_forward_parts(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u,
+                                         uint64_t h, uint64_t y, int32_t parts, uint64_t stream) {
+    return expert_forward(r, ex, x, g, u, h, y, parts, true, stream);
 }
 
 extern "C" int qmoe_expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u,
@@ -278,6 +288,13 @@ extern "C" int qmoe_gemm_wgrad_split(uint64_t a, uint64_t b, uint64_t c, uint64_
     return 0;
 }
 
+// Inside the layer the pad rows of few-row experts hold zeros only up to a multiple of 16 rows, which is as far as any of the
+// layer's products reaches (the weight gradients; everything else works row by row): at 64 tokens over 64 experts the
+// other pad rows of x, G, U, H and y are 135 MB of zeros beside 1.1 GB of weights.
+static int layer_pad(const qmoe_route_t* r, const qmoe_experts_t* ex, int engine) {
+    return engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex->experts) ? kStreamPad : kRowPad;
+}
+
 extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
     if (!L) return fail_arg("layer is null");
     const qmoe_route_t* r = &L->route;
@@ -295,8 +312,8 @@ extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
     }
     if (int rc = qmoe_router_forward(L->x, ex->dtype, L->w_router, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
-    if (int rc = qmoe_permute(r, L->x, L->x_dispatched, ex->dtype, d, stream)) return rc;
-    if (int rc = qmoe_expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, stream)) return rc;
+    if (int rc = launch_permute(r, L->x, L->x_dispatched, ex->dtype, d, layer_pad(r, ex, engine), stream)) return rc;
+    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, false, stream)) return rc;
     return qmoe_combine(r, L->y_dispatched, L->out, ex->dtype, d, stream);
 }
 
@@ -352,8 +369,8 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
     if (int rc = qmoe_router_forward(L->x, ex->dtype, B->w_router_folded, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
     if (int rc = qmoe_scale_f32(L->scores, L->scores, B->inverse, 0, r->tokens, E, stream)) return rc;
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
-    if (int rc = qmoe_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, stream)) return rc;
-    if (int rc = qmoe_expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, stream)) return rc;
+    if (int rc = launch_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, layer_pad(r, ex, engine), stream)) return rc;
+    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, false, stream)) return rc;
     return qmoe_combine_residual(r, L->y_dispatched, L->x, L->out, ex->dtype, d, stream);
 }
 

@@ -85,8 +85,8 @@ scale_kernel(const float* __restrict__ in, float* __restrict__ out, const float*
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, const float* __restrict__ weight,
-                    T* __restrict__ out, const int* __restrict__ dest_row, const int* __restrict__ row_source,
-                    const int* __restrict__ meta, long long tokens, int k, long long width) {
+                    T* __restrict__ out, const int* __restrict__ dest_row, const int* __restrict__ offsets,
+                    const int* __restrict__ counts, int experts, int pad, long long tokens, int k, long long width) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -117,17 +117,7 @@ permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, 
             }
         }
     }
-    const int rows_used = meta[0];
-    for (long long r = warp; r < rows_used; r += nwarps) {
-        if (row_source[r] >= 0) continue;
-        T* dst = out + r * width;
-        if constexpr (VEC) {
-            constexpr int N = Vec16<T>::N;
-            for (int c = lane; c < (int)(width / N); c += 32) st16(dst + (long long)c * N, make_uint4(0, 0, 0, 0));
-        } else {
-            for (long long c = lane; c < width; c += 32) Act<T>::store(dst + c, 0.f);
-        }
-    }
+    zero_pad_rows<T, VEC>(out, offsets, counts, experts, pad, width, warp, nwarps);
 }
 
 // out[t] = round(residual[t] + sum_s w[t, s] * y[dest_row[t, s]]): fp32 sum, one rounding
@@ -392,16 +382,21 @@ extern "C" int qmoe_scale_f32(uint64_t in, uint64_t out, uint64_t row_scale, uin
 }
 
 extern "C" int qmoe_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t norm_weight, uint64_t out,
-                                 int32_t dtype, int64_t width, uint64_t stream_) {
+                                 int32_t dtype, int64_t width, uint64_t stream) {
+    return launch_permute_norm(r, x, inverse, norm_weight, out, dtype, width, kRowPad, stream);
+}
+
+int qmoe::launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t norm_weight, uint64_t out, int32_t dtype,
+                              int64_t width, int pad, uint64_t stream_) {
     if (int rc = route_check(r)) return rc;
     if (int rc = check_dtype(dtype)) return rc;
     if (!x || !inverse || !norm_weight || !out || width <= 0) return fail_arg("permute_norm: null address or non-positive width");
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_PERMUTE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {x, out, norm_weight}) : can_vec<float>(width, {x, out, norm_weight});
-    const int grid = grid_for_rows(r->tokens > (long long)r->experts * 64 ? r->tokens : (long long)r->experts * 64, 8);
+    const int grid = grid_for_rows(r->tokens > (long long)r->experts * pad / 2 ? r->tokens : (long long)r->experts * pad / 2, 8);
 #define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (const float*)inverse, (const float*)norm_weight, (T*)out,       \
-        (const int*)r->dest_row, (const int*)r->row_source, (const int*)r->meta, (long long)r->tokens, r->top_k, (long long)width)
+        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width)
     if (dtype == QMOE_BF16) { if (vec) BY_K(permute_norm_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(permute_norm_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(permute_norm_kernel, float, true, ARGS(float)); else BY_K(permute_norm_kernel, float, false, ARGS(float)); }
 #undef ARGS

@@ -31,7 +31,7 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restrict__ dest_row,
-               const int* __restrict__ row_source, const int* __restrict__ meta, long long tokens, int k,
+               const int* __restrict__ offsets, const int* __restrict__ counts, int experts, int pad, long long tokens, int k,
                long long width) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -67,17 +67,7 @@ permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restri
             }
         }
     }
-    const int rows_used = meta[0];
-    for (long long r = warp; r < rows_used; r += nwarps) {
-        if (row_source[r] >= 0) continue;
-        T* dst = out + r * width;
-        if constexpr (VEC) {
-            constexpr int N = Vec16<T>::N;
-            for (int c = lane; c < (int)(width / N); c += 32) st16(dst + (long long)c * N, make_uint4(0, 0, 0, 0));
-        } else {
-            for (long long c = lane; c < width; c += 32) Act<T>::store(dst + c, 0.f);
-        }
-    }
+    zero_pad_rows<T, VEC>(out, offsets, counts, experts, pad, width, warp, nwarps);
 }
 
 // ---- combine: out[t] = sum_s w[t,s] * y[dest_row[t,s]] ----------------------------------------
@@ -399,17 +389,20 @@ int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint6
 
 using namespace qmoe;
 
-extern "C" int qmoe_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width,
-                            uint64_t stream_) {
+extern "C" int qmoe_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, uint64_t stream) {
+    return launch_permute(r, x, out, dtype, width, kRowPad, stream);
+}
+
+int qmoe::launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream_) {
     if (int rc = route_check(r)) return rc;
     if (int rc = check_dtype(dtype)) return rc;
     if (!x || !out || width <= 0) return fail_arg("permute: null address or non-positive width");
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_PERMUTE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {x, out}) : can_vec<float>(width, {x, out});
-    // enough warps for the tokens and for zeroing up to experts * 127 pad rows
-    const int grid = grid_for_rows(r->tokens > (long long)r->experts * 64 ? r->tokens : (long long)r->experts * 64);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->row_source, (const int*)r->meta, (long long)r->tokens, r->top_k, (long long)width)
+    // enough warps for the tokens and for zeroing up to experts * (pad - 1) pad rows
+    const int grid = grid_for_rows(r->tokens > (long long)r->experts * pad / 2 ? r->tokens : (long long)r->experts * pad / 2);
+#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width)
 #define BY_K(T, V)                                                  \
     do {                                                            \
         if (r->top_k <= 1) permute_kernel<T, V, 1> ARGS(T);         \

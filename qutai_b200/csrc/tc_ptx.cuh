@@ -204,6 +204,8 @@ __device__ __forceinline__ constexpr uint32_t make_idesc(int n) {
 }
 
 }  // namespace
+// dense row-major bf16 matrix [outer, inner] in boxes of 64 columns x box_outer rows, 128-byte swizzle
+int make_map_2d(CUtensorMap* out, uint64_t ptr, uint64_t inner, uint64_t outer, uint32_t box_outer);
 int make_map_3d(CUtensorMap* out, uint64_t ptr, uint64_t inner, uint64_t mid, uint64_t outer, uint32_t box_mid);
 
 }  // namespace qmoe

@@ -1,10 +1,62 @@
-"""Few rows per expert: the one-block routing against the oracle, at the sizes where it can go wrong.  Needs a B200: ``-m gpu``."""
+"""Few rows per expert: the weight-streaming forward products (``stream_gemm_kernel``) against the kernel for many rows, and
+the one-block routing against the oracle, at the sizes where either can go wrong.  Needs a B200: ``-m gpu``."""
 import numpy as np
 import pytest
 
 from oracle import moe_oracle as oracle
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("counts,width,hidden", [
+    ((0, 1, 15, 16, 17), 64, 128),           # around one 16-row step, an expert without rows
+    ((127, 128, 129, 0, 3), 72, 136),        # around one 128-row chunk, widths that fill no tile
+    ((300, 2, 0, 40, 33), 264, 1032),        # an expert with three chunks, several k blocks and tiles
+    ((1,), 2048, 8),                         # one row, the narrowest hidden width
+])
+def test_streamed_products_match_the_kernel_for_many_rows(counts, width, hidden, kernel_variant):
+    import ctypes
+
+    from gpu_util import RouteTables, to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    experts, tokens = len(counts), sum(counts)
+    rng = np.random.default_rng(tokens + width)
+    choice = np.repeat(np.arange(experts), counts)
+    scores = np.zeros((tokens, experts), dtype=np.float32)
+    scores[np.arange(tokens), rng.permutation(choice)] = 5.0
+    tables = RouteTables(tokens, experts, 1)
+    tables.run(to_device(scores, "float32"))
+    assert tuple(tables.host("counts").tolist()) == counts
+    rows = tables.rows_bound
+    x = to_device(rng.standard_normal((tokens, width)), "bfloat16")
+    weights = [to_device(rng.standard_normal(shape) / np.sqrt(shape[-1]), "bfloat16")
+               for shape in ((experts, hidden, width), (experts, hidden, width), (experts, width, hidden))]
+    dispatched = DeviceStorage(rows * width, "bfloat16")
+    lib.call("qmoe_permute", tables.ref, x.ptr, dispatched.ptr, lib.QMOE_BF16, width, 0)
+    ex = lib.Experts()
+    ex.experts, ex.dtype, ex.engine, ex.width, ex.hidden = experts, lib.QMOE_BF16, lib.ENGINE_TCGEN05, width, hidden
+    ex.w_gate, ex.w_up, ex.w_down = (w.ptr for w in weights)
+    used = int(tables.host("offsets")[experts])
+
+    def forward():
+        g, u, h, y = (DeviceStorage(rows * n, "bfloat16") for n in (hidden, hidden, hidden, width))
+        for buffer in (g, u, h, y):
+            lib.call("qmoe_memset", buffer.ptr, 0xFF, buffer.nbytes, 0)       # NaN: every row of a tile has to be written
+        lib.call("qmoe_expert_forward", tables.ref, ctypes.byref(ex), dispatched.ptr, g.ptr, u.ptr, h.ptr, y.ptr, 0)
+        assert lib.device_status() == 0
+        return [to_host(b, (rows, -1))[:used] for b in (g, u, h, y)]
+
+    streamed = forward()
+    kernel_variant(lib.VARIANT_NO_STREAM_GEMM)
+    for got, want in zip(streamed, forward()):
+        assert np.all(np.isfinite(got))
+        # the same fp32 sums in another order, rounded to bf16: at most one step (2^-8) of the largest value apart
+        assert oracle.max_rel_err(got, want) <= 2.0 ** -7
+    source = tables.host("row_source")[:used]
+    for got in streamed:
+        assert not np.any(got[source < 0])                                    # pad rows hold zeros
 
 
 @pytest.mark.parametrize("tokens,experts,top_k", [(1, 1, 1), (1, 256, 8), (31, 33, 4), (33, 32, 3), (128, 256, 8), (128, 64, 6), (129, 64, 6), (97, 5, 5)])
