@@ -110,6 +110,15 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Warps that share a token row in the row kernels (permute, combine): one where the tokens alone fill the machine, up to 8
+// (each with at least one 16-byte piece per lane) for a handful of tokens, where a row's serial chain of loads is the
+// kernel's time (64 rows of 2048: permute 9.2 -> 4 us, combine 9.0 -> 4 us).
+inline int parts_per_row(long long tokens, long long pieces) {
+    int parts = 1;
+    while (parts < 8 && tokens * parts < 2048 && pieces > 32ll * parts) parts *= 2;
+    return parts;
+}
+
 // Zero rows count .. round_up(count, pad) - 1 of every expert's group (pad divides kRowPad), a warp per row.
 template <typename T, bool VEC>
 __device__ __forceinline__ void zero_pad_rows(T* out, const int* offsets, const int* counts, int experts, int pad, long long width,
@@ -162,6 +171,9 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
 int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream);
 int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t weight, uint64_t out, int32_t dtype, int64_t width, int pad,
                         uint64_t stream);
+bool router_norm_ok(int64_t tokens);
+int router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
+                        int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
 int route_check(const qmoe_route_t* r);
 int launch_swiglu(const qmoe_route_t* r, uint64_t g, uint64_t u, uint64_t h, int dtype, long long hidden, cudaStream_t stream);
 int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint64_t u, uint64_t dg, uint64_t du, int dtype,

@@ -364,10 +364,15 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
         if (int rc = qmoe_cast_bf16(L->master_down, ex->w_down, E * hd * d, stream)) return rc;
     }
     // scores = rms_norm(x) . W_r^T = inverse[t] * (x . (W_r * w)^T): the product reads the raw activations
-    if (int rc = qmoe_rms_inverse(L->x, ex->dtype, B->inverse, r->tokens, d, B->norm_eps, stream)) return rc;
-    if (int rc = qmoe_scale_f32(L->w_router, B->w_router_folded, 0, B->norm_weight, E, d, stream)) return rc;
-    if (int rc = qmoe_router_forward(L->x, ex->dtype, B->w_router_folded, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
-    if (int rc = qmoe_scale_f32(L->scores, L->scores, B->inverse, 0, r->tokens, E, stream)) return rc;
+    if (router_norm_ok(r->tokens)) {
+        if (int rc = router_forward_norm(L->x, ex->dtype, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, r->tokens, d, r->experts, stream))
+            return rc;
+    } else {
+        if (int rc = qmoe_rms_inverse(L->x, ex->dtype, B->inverse, r->tokens, d, B->norm_eps, stream)) return rc;
+        if (int rc = qmoe_scale_f32(L->w_router, B->w_router_folded, 0, B->norm_weight, E, d, stream)) return rc;
+        if (int rc = qmoe_router_forward(L->x, ex->dtype, B->w_router_folded, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
+        if (int rc = qmoe_scale_f32(L->scores, L->scores, B->inverse, 0, r->tokens, E, stream)) return rc;
+    }
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
     if (int rc = launch_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, layer_pad(r, ex, engine), stream)) return rc;
     if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, false, stream)) return rc;

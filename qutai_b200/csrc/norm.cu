@@ -86,11 +86,13 @@ template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, const float* __restrict__ weight,
                     T* __restrict__ out, const int* __restrict__ dest_row, const int* __restrict__ offsets,
-                    const int* __restrict__ counts, int experts, int pad, long long tokens, int k, long long width) {
+                    const int* __restrict__ counts, int experts, int pad, long long tokens, int k, long long width, int parts) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long t = warp; t < tokens; t += nwarps) {
+    for (long long i = warp; i < tokens * parts; i += nwarps) {
+        const long long t = i / parts;
+        const int mine = lane + 32 * (int)(i - t * parts), step = 32 * parts;     // this warp's pieces of the row: mine, mine + step, ...
         long long rows[KMAX];
 #pragma unroll
         for (int s = 0; s < KMAX; ++s) rows[s] = s < k ? dest_row[t * k + s] : 0;
@@ -98,7 +100,7 @@ permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, 
         const float inv = inverse[t];
         if constexpr (VEC) {
             constexpr int N = Vec16<T>::N;
-            for (int c = lane; c < (int)(width / N); c += 32) {
+            for (int c = mine; c < (int)(width / N); c += step) {
                 float f[N], w[N];
                 Vec16<T>::unpack(ld16_stream(src + (long long)c * N), f);
                 load_f32<N>(weight + (long long)c * N, w);
@@ -110,7 +112,7 @@ permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, 
                     if (s < k) st16(out + rows[s] * width + (long long)c * N, v);
             }
         } else {
-            for (long long c = lane; c < width; c += 32) {
+            for (long long c = mine; c < width; c += step) {
                 T v;
                 Act<T>::store(&v, Act<T>::load(src + c) * inv * weight[c]);
                 for (int s = 0; s < k; ++s) out[rows[s] * width + c] = v;
@@ -124,11 +126,13 @@ permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, 
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 combine_residual_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const int* __restrict__ dest_row,
-                        const T* __restrict__ residual, T* __restrict__ out, long long tokens, int k, long long width) {
+                        const T* __restrict__ residual, T* __restrict__ out, long long tokens, int k, long long width, int parts) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long t = warp; t < tokens; t += nwarps) {
+    for (long long i = warp; i < tokens * parts; i += nwarps) {
+        const long long t = i / parts;
+        const int mine = lane + 32 * (int)(i - t * parts), step = 32 * parts;     // this warp's pieces of the row: mine, mine + step, ...
         int rows[KMAX];
         float w[KMAX];
 #pragma unroll
@@ -140,7 +144,7 @@ combine_residual_kernel(const T* __restrict__ y, const float* __restrict__ gate_
         const T* res = residual + t * width;
         if constexpr (VEC) {
             constexpr int N = Vec16<T>::N;
-            for (int c = lane; c < (int)(width / N); c += 32) {
+            for (int c = mine; c < (int)(width / N); c += step) {
                 uint4 v[KMAX];
 #pragma unroll
                 for (int s = 0; s < KMAX; ++s)
@@ -162,7 +166,7 @@ combine_residual_kernel(const T* __restrict__ y, const float* __restrict__ gate_
                 st16(dst + (long long)c * N, Vec16<T>::pack(acc));
             }
         } else {
-            for (long long c = lane; c < width; c += 32) {
+            for (long long c = mine; c < width; c += step) {
                 float acc = 0.f;
                 for (int s = 0; s < k; ++s) acc = fmaf(w[s], Act<T>::load(y + (long long)rows[s] * width + c), acc);
                 Act<T>::store(dst + c, acc + Act<T>::load(res + c));
@@ -394,9 +398,11 @@ int qmoe::launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t invers
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_PERMUTE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {x, out, norm_weight}) : can_vec<float>(width, {x, out, norm_weight});
-    const int grid = grid_for_rows(r->tokens > (long long)r->experts * pad / 2 ? r->tokens : (long long)r->experts * pad / 2, 8);
+    const int parts = parts_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
+    const long long warps = r->tokens * parts;
+    const int grid = grid_for_rows(warps > (long long)r->experts * pad / 2 ? warps : (long long)r->experts * pad / 2, 8);
 #define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (const float*)inverse, (const float*)norm_weight, (T*)out,       \
-        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width)
+        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width, parts)
     if (dtype == QMOE_BF16) { if (vec) BY_K(permute_norm_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(permute_norm_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(permute_norm_kernel, float, true, ARGS(float)); else BY_K(permute_norm_kernel, float, false, ARGS(float)); }
 #undef ARGS
@@ -412,9 +418,10 @@ extern "C" int qmoe_combine_residual(const qmoe_route_t* r, uint64_t y, uint64_t
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_COMBINE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {y, residual, out}) : can_vec<float>(width, {y, residual, out});
-    const int grid = grid_for_rows(r->tokens, 8);
+    const int parts = parts_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
+    const int grid = grid_for_rows(r->tokens * parts, 8);
 #define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row,           \
-        (const T*)residual, (T*)out, (long long)r->tokens, r->top_k, (long long)width)
+        (const T*)residual, (T*)out, (long long)r->tokens, r->top_k, (long long)width, parts)
     if (dtype == QMOE_BF16) { if (vec) BY_K(combine_residual_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(combine_residual_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(combine_residual_kernel, float, true, ARGS(float)); else BY_K(combine_residual_kernel, float, false, ARGS(float)); }
 #undef ARGS

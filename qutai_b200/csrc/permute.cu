@@ -32,11 +32,13 @@ template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restrict__ dest_row,
                const int* __restrict__ offsets, const int* __restrict__ counts, int experts, int pad, long long tokens, int k,
-               long long width) {
+               long long width, int parts) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long t = warp; t < tokens; t += nwarps) {
+    for (long long i = warp; i < tokens * parts; i += nwarps) {
+        const long long t = i / parts;
+        const int mine = lane + 32 * (int)(i - t * parts), step = 32 * parts;     // this warp's pieces of the row: mine, mine + step, ...
         long long rows[KMAX];
 #pragma unroll
         for (int s = 0; s < KMAX; ++s) rows[s] = s < k ? dest_row[t * k + s] : 0;
@@ -44,24 +46,24 @@ permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restri
         if constexpr (VEC) {
             constexpr int N = Vec16<T>::N;
             const int chunks = (int)(width / N);
-            int c = lane;
-            for (; c + 32 < chunks; c += 64) {
-                const uint4 v0 = ld16_stream(src + (long long)c * N), v1 = ld16_stream(src + (long long)(c + 32) * N);
+            int c = mine;
+            for (; c + step < chunks; c += 2 * step) {
+                const uint4 v0 = ld16_stream(src + (long long)c * N), v1 = ld16_stream(src + (long long)(c + step) * N);
 #pragma unroll
                 for (int s = 0; s < KMAX; ++s)
                     if (s < k) {
                         st16(out + rows[s] * width + (long long)c * N, v0);
-                        st16(out + rows[s] * width + (long long)(c + 32) * N, v1);
+                        st16(out + rows[s] * width + (long long)(c + step) * N, v1);
                     }
             }
-            for (; c < chunks; c += 32) {
+            for (; c < chunks; c += step) {
                 const uint4 v0 = ld16_stream(src + (long long)c * N);
 #pragma unroll
                 for (int s = 0; s < KMAX; ++s)
                     if (s < k) st16(out + rows[s] * width + (long long)c * N, v0);
             }
         } else {
-            for (long long c = lane; c < width; c += 32) {
+            for (long long c = mine; c < width; c += step) {
                 const T v = src[c];
                 for (int s = 0; s < k; ++s) out[rows[s] * width + c] = v;
             }
@@ -74,11 +76,13 @@ permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restri
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 combine_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const int* __restrict__ dest_row,
-               T* __restrict__ out, long long tokens, int k, long long width) {
+               T* __restrict__ out, long long tokens, int k, long long width, int parts) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long t = warp; t < tokens; t += nwarps) {
+    for (long long i = warp; i < tokens * parts; i += nwarps) {
+        const long long t = i / parts;
+        const int mine = lane + 32 * (int)(i - t * parts), step = 32 * parts;     // this warp's pieces of the row: mine, mine + step, ...
         int rows[KMAX];
         float w[KMAX];
 #pragma unroll
@@ -90,7 +94,7 @@ combine_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const 
         if constexpr (VEC) {
             constexpr int N = Vec16<T>::N;
             const int chunks = (int)(width / N);
-            for (int c = lane; c < chunks; c += 32) {
+            for (int c = mine; c < chunks; c += step) {
                 uint4 v[KMAX];
 #pragma unroll
                 for (int s = 0; s < KMAX; ++s)
@@ -109,7 +113,7 @@ combine_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const 
                 st16(dst + (long long)c * N, Vec16<T>::pack(acc));
             }
         } else {
-            for (long long c = lane; c < width; c += 32) {
+            for (long long c = mine; c < width; c += step) {
                 float acc = 0.f;
                 for (int s = 0; s < k; ++s) acc = fmaf(w[s], Act<T>::load(y + (long long)rows[s] * width + c), acc);
                 Act<T>::store(dst + c, acc);
@@ -401,8 +405,10 @@ int qmoe::launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_
     TimedScope timed(KC_PERMUTE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {x, out}) : can_vec<float>(width, {x, out});
     // enough warps for the tokens and for zeroing up to experts * (pad - 1) pad rows
-    const int grid = grid_for_rows(r->tokens > (long long)r->experts * pad / 2 ? r->tokens : (long long)r->experts * pad / 2);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width)
+    const int parts = parts_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
+    const long long warps = r->tokens * parts;
+    const int grid = grid_for_rows(warps > (long long)r->experts * pad / 2 ? warps : (long long)r->experts * pad / 2);
+#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width, parts)
 #define BY_K(T, V)                                                  \
     do {                                                            \
         if (r->top_k <= 1) permute_kernel<T, V, 1> ARGS(T);         \
@@ -427,8 +433,9 @@ extern "C" int qmoe_combine(const qmoe_route_t* r, uint64_t y, uint64_t out, int
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_COMBINE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {y, out}) : can_vec<float>(width, {y, out});
-    const int grid = grid_for_rows(r->tokens);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row, (T*)out, (long long)r->tokens, r->top_k, (long long)width)
+    const int parts = parts_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
+    const int grid = grid_for_rows(r->tokens * parts);
+#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row, (T*)out, (long long)r->tokens, r->top_k, (long long)width, parts)
 #define BY_K(T, V)                                                  \
     do {                                                            \
         if (r->top_k <= 1) combine_kernel<T, V, 1> ARGS(T);         \

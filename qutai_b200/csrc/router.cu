@@ -120,16 +120,19 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
 }
 // grid (tokens, ceil(E / 8)): warp w of block (t, g) computes scores[t, 8 g + w].  Four 16-byte loads of the weight
 // row and of the token row are in flight per lane and iteration, so the few round trips to L2 overlap.
-template <typename T>
+// NORM: the logits of the normalised row, inverse * (x . (w * norm weight)), with inverse = 1 / rms from the same pass over
+// the row (kept for the later kernels): four launches in one.
+template <typename T, bool NORM>
 __global__ void __launch_bounds__(256)
-router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float* __restrict__ scores, int E, long long d) {
+router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float* __restrict__ scores, int E, long long d,
+                    const float* __restrict__ norm_weight, float eps, float* __restrict__ inverse) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.y * 8 + warp;
     if (e >= E) return;
     const T* row = x + (long long)blockIdx.x * d;
     const float* we = w + (long long)e * d;
-    const bool vec = (d & 3) == 0 && (((uintptr_t)row | (uintptr_t)we) & 15u) == 0;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+    const bool vec = (d & 3) == 0 && (((uintptr_t)row | (uintptr_t)we | (NORM ? (uintptr_t)norm_weight : 0)) & 15u) == 0;
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, square = 0.f;
     if (vec) {
         for (long long j = (long long)lane * 4; j < d; j += 512) {
             float4 wv[4], xv[4];
@@ -139,6 +142,10 @@ router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float*
                 const bool in = at < d;
                 wv[u] = in ? load4(we + at) : make_float4(0.f, 0.f, 0.f, 0.f);
                 xv[u] = in ? load4(row + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (NORM && in) {
+                    const float4 nv = load4(norm_weight + at);
+                    wv[u].x *= nv.x; wv[u].y *= nv.y; wv[u].z *= nv.z; wv[u].w *= nv.w;
+                }
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {   // fixed order: the sums do not depend on timing
@@ -146,14 +153,24 @@ router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float*
                 a1 = fmaf(xv[u].y, wv[u].y, a1);
                 a2 = fmaf(xv[u].z, wv[u].z, a2);
                 a3 = fmaf(xv[u].w, wv[u].w, a3);
+                if (NORM) square = fmaf(xv[u].w, xv[u].w, fmaf(xv[u].z, xv[u].z, fmaf(xv[u].y, xv[u].y, fmaf(xv[u].x, xv[u].x, square))));
             }
         }
     } else {
-        for (long long j = lane; j < d; j += 32) a0 = fmaf(Act<T>::load(row + j), we[j], a0);
+        for (long long j = lane; j < d; j += 32) {
+            const float v = Act<T>::load(row + j);
+            a0 = fmaf(v, NORM ? we[j] * norm_weight[j] : we[j], a0);
+            if (NORM) square = fmaf(v, v, square);
+        }
     }
     float acc = (a0 + a1) + (a2 + a3);
 #pragma unroll
     for (int step = 16; step > 0; step >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, step);
+    if (NORM) {
+        const float inv = rsqrtf(warp_sum(square) / (float)d + eps);
+        acc *= inv;
+        if (lane == 0 && e == 0) inverse[blockIdx.x] = inv;
+    }
     if (lane == 0) scores[(long long)blockIdx.x * E + e] = acc;
 }
 
@@ -187,12 +204,13 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
     // fp32 rows over up to 16 experts: the tile kernel's 128 x 16 tiles take 31 us for 2048 tokens of width 512 over 8, this 5
     if (tokens <= kSmallRouterTokens || (x_dtype == QMOE_F32 && experts <= 16)) {
         TimedScope timed(KC_ROUTER_GEMM, stream);
+        const dim3 grid((unsigned)tokens, (unsigned)((experts + 7) / 8));
         if (x_dtype == QMOE_BF16)
-            router_small_kernel<__nv_bfloat16><<<dim3((unsigned)tokens, (unsigned)((experts + 7) / 8)), 256, 0, stream>>>((const __nv_bfloat16*)x, (const float*)w_router,
-                                                                                   (float*)scores, experts, width);
+            router_small_kernel<__nv_bfloat16, false><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (const float*)w_router, (float*)scores,
+                                                                                experts, width, nullptr, 0.f, nullptr);
         else
-            router_small_kernel<float><<<dim3((unsigned)tokens, (unsigned)((experts + 7) / 8)), 256, 0, stream>>>((const float*)x, (const float*)w_router,
-                                                                             (float*)scores, experts, width);
+            router_small_kernel<float, false><<<grid, 256, 0, stream>>>((const float*)x, (const float*)w_router, (float*)scores, experts, width,
+                                                                        nullptr, 0.f, nullptr);
         QMOE_LAUNCH_CHECK("router_small_kernel");
         return 0;
     }
@@ -204,6 +222,24 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
         (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, r.S, width);
     QMOE_LAUNCH_CHECK("router_split_w_kernel");
     return tc_router_forward(x, scratch + r.w3, scores, tokens, width, experts, r.S, stream);
+}
+
+bool qmoe::router_norm_ok(int64_t tokens) { return tokens <= kSmallRouterTokens; }
+
+// inverse[t] and the logits of the normalised rows in one launch (tokens within router_norm_ok)
+int qmoe::router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
+                              int64_t tokens, int64_t width, int32_t experts, uint64_t stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    TimedScope timed(KC_ROUTER_GEMM, stream);
+    const dim3 grid((unsigned)tokens, (unsigned)((experts + 7) / 8));
+    if (x_dtype == QMOE_BF16)
+        router_small_kernel<__nv_bfloat16, true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (const float*)w_router, (float*)scores, experts, width,
+                                                                           (const float*)norm_weight, (float)eps, (float*)inverse);
+    else
+        router_small_kernel<float, true><<<grid, 256, 0, stream>>>((const float*)x, (const float*)w_router, (float*)scores, experts, width,
+                                                                   (const float*)norm_weight, (float)eps, (float*)inverse);
+    QMOE_LAUNCH_CHECK("router_small_kernel");
+    return 0;
 }
 
 extern "C" int qmoe_router_logits(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t scores, int64_t tokens,
