@@ -302,11 +302,23 @@ cast_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst,
         dst[i] = __float2bfloat16_rn(src[i]);
 }
 
+// out may be a or b.  Eight bf16 (four fp32) per access: one value per thread and access moved 4 TB/s at 8192 x 1024
+// (12.7 us), these 16-byte pieces (7.4 us); the tail and unaligned buffers go value by value.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-add_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, long long n) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        Act<T>::store(out + i, Act<T>::load(a + i) + Act<T>::load(b + i));
+add_kernel(const T* a, const T* b, T* out, long long n, long long pieces) {
+    constexpr int N = Vec16<T>::N;
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = first; i < pieces; i += stride) {
+        const uint4 va = reinterpret_cast<const uint4*>(a)[i], vb = reinterpret_cast<const uint4*>(b)[i];
+        float fa[N], fb[N];
+        Vec16<T>::unpack(va, fa);
+        Vec16<T>::unpack(vb, fb);
+#pragma unroll
+        for (int e = 0; e < N; ++e) fa[e] += fb[e];
+        st16(out + i * N, Vec16<T>::pack(fa));
+    }
+    for (long long i = pieces * N + first; i < n; i += stride) Act<T>::store(out + i, Act<T>::load(a + i) + Act<T>::load(b + i));
 }
 
 // counter-based generator: a 64-bit mix of (seed, index) gives two uniforms, Box-Muller one normal
@@ -539,11 +551,13 @@ extern "C" int qmoe_add(uint64_t a, uint64_t b, uint64_t out, int32_t dtype, int
     if (n == 0) return 0;
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_ELEMENTWISE, stream);
+    const bool aligned = !((a | b | out) & 15u);
+    const long long pieces = aligned ? n / (dtype == QMOE_BF16 ? 8 : 4) : 0;
+    const int grid = grid_for_elems(aligned ? pieces + 8 : n);
     if (dtype == QMOE_BF16)
-        add_kernel<__nv_bfloat16><<<grid_for_elems(n), kThreads, 0, stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
-                                                                               (__nv_bfloat16*)out, n);
+        add_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n, pieces);
     else
-        add_kernel<float><<<grid_for_elems(n), kThreads, 0, stream>>>((const float*)a, (const float*)b, (float*)out, n);
+        add_kernel<float><<<grid, kThreads, 0, stream>>>((const float*)a, (const float*)b, (float*)out, n, pieces);
     QMOE_LAUNCH_CHECK("add_kernel");
     return 0;
 }
