@@ -414,6 +414,19 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     else if (CTAS == 2) total_tiles = s_pair[p.experts] * p.n_tiles;
     else total_tiles = (s_start[p.experts] - s_start[0]) * p.n_tiles;
     volatile int* abort_flag = &s_abort;
+    // An epilogue warp hands its accumulator back as soon as its last read of it has arrived in registers, before the stores
+    // of what it read, and without release semantics across the pair: a release at cluster scope waits until every global
+    // store of the thread has been acknowledged, which with short contractions was most of a tile's time (weight gradients
+    // over 375 rows per expert: 146 us, of which the MMAs are 35).  Nothing but tensor memory is handed over, and the reads
+    // of it are complete.
+    auto release_accumulator = [&](int acc) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            if (CTAS == 2) mbar_arrive_relaxed_cluster(map_to_cta(tempty_bar(acc), 0));
+            else mbar_arrive(tempty_bar(acc));
+        }
+    };
 
     if (warp == 0 || warp == B_PRODUCER_WARP) {
         // ------------------------------ TMA producers -----------------------------
@@ -598,6 +611,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
             }
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN + (uint32_t)side * 32u;
+            bool released = false;
 #pragma unroll 1
             for (int c = 0; c < c_end; ++c) {
                 uint32_t r[32];
@@ -621,6 +635,10 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     }
                 }
                 tmem_ld_wait();
+                if (c + 1 == c_end) {
+                    release_accumulator(acc);
+                    released = true;
+                }
                 if (!mbar_wait(load_bar(n), (n >> 1) & 1u, abort_flag)) {
                     if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, STATUS_WAIT_EPILOGUE); }
                     gave_up = true;
@@ -665,12 +683,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 }
                 ++n;
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                if (CTAS == 2 && cta_rank) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
-                else mbar_arrive(tempty_bar(acc));
-            }
+            if (!released) release_accumulator(acc);
             ++iter;
         }
         if (leader && lane == 0) bulk_wait_all();   // shared memory stays until the last store has left it
@@ -699,6 +712,13 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
             const long long row0w = (long long)tile.row0 + quad * 32;
             // 32-column chunks of this warp: its half of the tile's columns (4 of 8, or 2 of 4 in a narrow tile)
             const int c_begin = half * (tile.bn / 64), c_end = c_begin + tile.bn / 64;
+            bool released = false;
+            auto last_read = [&](bool last) {     // after a tmem_ld_wait: `last` when nothing of the accumulator is left to read
+                if (last) {
+                    release_accumulator(acc);
+                    released = true;
+                }
+            };
             if (CTAS == 2 && !tile.rows_valid) {
                 // second half of an odd pair-tile: these rows belong to nobody, nothing is stored
             } else if (MODE == MODE_SWIGLU) {
@@ -711,6 +731,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     tmem_ld32(taddr + c * 32, rg);
                     tmem_ld32(taddr + 128 + c * 32, ru);
                     tmem_ld_wait();
+                    last_read(c == 2 * half + 1);
                     const int valid = p.N - (tile.n0 + c * 32);
                     if (valid >= 32) {
                         uint32_t wg[16], wu[16], wh[16];
@@ -763,6 +784,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                         for (int j = 0; j < 16; ++j)
                             w[cc * 16 + j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
                     }
+                    last_read(true);
                     scatter_rows256(stage, lane, w, remote ? remote + c_begin * 32 : nullptr);
                 }
 #pragma unroll 1
@@ -770,6 +792,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c * 32, r);
                     tmem_ld_wait();
+                    last_read(c + 1 == c_end);
                     const int valid = p.N - (tile.n0 + c * 32);
                     if (valid >= 32) {
                         uint32_t w[16];
@@ -817,6 +840,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c * 32, r);
                     tmem_ld_wait();
+                    last_read(c + 1 == c_end);
                     const int valid = p.N - (tile.n0 + c * 32);
                     if (row_ok) {
 #pragma unroll
@@ -834,6 +858,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c * 32, r);
                     tmem_ld_wait();
+                    last_read(c + 1 == c_end);
                     const int valid = p.N - (tile.n0 + c * 32);
                     if (valid >= 32) {
                         store_block32_f32(stage, lane, r, Cw + c * 32, p.ldc, (long long)p.M - row0w);
@@ -844,12 +869,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     }
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                if (CTAS == 2 && cta_rank) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
-                else mbar_arrive(tempty_bar(acc));
-            }
+            if (!released) release_accumulator(acc);
             ++iter;
         }
         // rows stored into other GPUs' memory: one system-scope fence per thread after its last tile (the

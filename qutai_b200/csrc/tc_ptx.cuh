@@ -81,8 +81,8 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+__device__ __forceinline__ void mbar_arrive_relaxed_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // TMA load issued by one CTA of a pair: the data lands in this CTA's shared memory, the transaction
 // bytes are counted on the barrier of the pair's first CTA (same offset, CTA-rank bit cleared).
