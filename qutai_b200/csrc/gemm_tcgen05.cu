@@ -148,7 +148,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         tile.expert = e;
         tile.row0 = (rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
         tile.n0 = (rem / p.m_tiles) * BN;
-        const int count = p.plain_rows > 0 ? p.plain_rows : p.counts[e];
+        const int count = s_pair[e];      // WGRAD keeps the row counts in this table
         tile.depth = count;
         tile.kblocks = (count + BK - 1) / BK;
         tile.krow0 = s_start[e] * kRowPad;
@@ -329,7 +329,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     constexpr bool STARTS_IN_SHARED = starts_in_shared<MODE, CTAS>();
     __shared__ int s_start_table[STARTS_IN_SHARED ? kMaxExperts + 1 : 1];  // first 128-row tile of each expert
     const StartTable<STARTS_IN_SHARED> s_start{s_start_table, p.offsets};
-    __shared__ int s_pair[kMaxExperts + 1];   // CTAS == 2: first 256-row pair-tile of each expert
+    __shared__ int s_pair[kMaxExperts + 1];   // CTAS == 2: first 256-row pair-tile of each expert; WGRAD: rows of each expert
     __shared__ int s_order[kMaxExperts];      // WGRAD: experts by decreasing row count (ties by index)
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
@@ -357,9 +357,10 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         // Tiles of large experts cost more (longer contraction).  Walking the experts from large to
         // small and dealing tiles round-robin gives every CTA the same mix of long and short tiles.
         if (p.plain_rows > 0) {
-            if (threadIdx.x == 0) s_order[0] = 0;
+            if (threadIdx.x == 0) { s_order[0] = 0; s_pair[0] = p.plain_rows; }
         } else for (int i = threadIdx.x; i < p.experts; i += NUM_THREADS) {
             const int mine = p.counts[i];
+            s_pair[i] = mine;
             int rank = 0;
             for (int j = 0; j < p.experts; ++j) {
                 const int other = p.counts[j];
@@ -398,7 +399,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     __syncthreads();
     if (CTAS == 2) {
         // pair-tiles of the experts before e; an odd last 128-row tile takes a pair-tile of its own
-        for (int i = threadIdx.x; i <= p.experts; i += NUM_THREADS) {
+        if (MODE != MODE_WGRAD) for (int i = threadIdx.x; i <= p.experts; i += NUM_THREADS) {
             int sum = 0;
             for (int j = 0; j < i; ++j) sum += (s_start[j + 1] - s_start[j] + 1) >> 1;
             s_pair[i] = sum;
@@ -416,8 +417,8 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     volatile int* abort_flag = &s_abort;
     // An epilogue warp hands its accumulator back as soon as its last read of it has arrived in registers, before the stores
     // of what it read, and without release semantics across the pair: a release at cluster scope waits until every global
-    // store of the thread has been acknowledged, which with short contractions was most of a tile's time (weight gradients
-    // over 375 rows per expert: 146 us, of which the MMAs are 35).  Nothing but tensor memory is handed over, and the reads
+    // store of the thread has been acknowledged (weight gradients over 375 rows per expert, 16 x 3 x 1024 x 2048: 145 us with
+    // both, 130 without).  Nothing but tensor memory is handed over, and the reads
     // of it are complete.
     auto release_accumulator = [&](int acc) {
         tc_fence_before();
@@ -842,10 +843,17 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     tmem_ld_wait();
                     last_read(c + 1 == c_end);
                     const int valid = p.N - (tile.n0 + c * 32);
-                    if (row_ok) {
+                    float* to = C + (long long)(c * 32) * ldc;
+                    // The common case without a test per store and with one running address: over a short contraction a tile waits
+                    // for the instructions of these warps (375 rows per expert, 16 x 3 x 1024 x 2048: 130 -> 95 us, where the bytes
+                    // take 62; 32768 rows over 64 experts, 2048 x 1408: 3.31 -> 3.10 ms).
+                    if (row_ok && valid >= 32) {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (i < valid) C[(long long)(c * 32 + i) * ldc] = __uint_as_float(r[i]);
+                        for (int i = 0; i < 32; ++i, to += ldc) *to = __uint_as_float(r[i]);
+                    } else if (row_ok) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i, to += ldc)
+                            if (i < valid) *to = __uint_as_float(r[i]);
                     }
                 }
             } else {
