@@ -476,6 +476,10 @@ int qmoe_rope(uint64_t values, uint64_t out, int32_t dtype, int64_t batch, int64
 /* out[i, :] = weight[ids[i], :] (ids i64; an id outside [0, vocab) gives a zero row).  Replaces `embedding` (lm_embedding). */
 int qmoe_embedding(uint64_t weight, uint64_t ids, uint64_t out, int32_t out_dtype, int64_t count, int64_t width,
                    int64_t vocab, uint64_t stream);
+/* The tables of qmoe_embedding_backward from `count` token ids, all of them host memory (i64): the distinct tokens ascending
+ * (room for min(count, vocab)), starts[*segments + 1] (one more), positions[count].  An id outside [0, vocab) is an
+ * argument error.  As upstream builds them on the host, src/qutai/backends/cuda_lm.py:97-106. */
+int qmoe_token_tables(const void* ids, int64_t count, int64_t vocab, void* distinct, void* starts, void* positions, int64_t* segments);
 /* d_weight[tokens[s], :] += sum of gradient[p, :] over positions[starts[s] .. starts[s + 1]), in that order (i64 tables made
  * on the host as upstream makes them: distinct tokens ascending, each with its positions ascending).  d_weight f32
  * [vocab, width] is added to: zero it first for upstream's `embedding_backward` (lm_embedding_backward). */

@@ -5,6 +5,8 @@
 // here a warp owns a row and moves 16 or 32 bytes per lane per access in the norm, the norm weight's gradient is reduced in a fixed
 // order (no floating-point atomics), and the embedding's backward walks each token's positions in order, as
 // upstream's does, so every result is the same on every run.
+#include <stdlib.h>
+
 #include "common.cuh"
 
 namespace qmoe {
@@ -425,6 +427,34 @@ extern "C" int qmoe_embedding(uint64_t weight, uint64_t ids, uint64_t out, int32
     else
         embedding_kernel<<<row_grid(count), kThreads, 0, stream>>>((const float*)weight, (const long long*)ids, (float*)out, count, width, vocab);
     QMOE_LAUNCH_CHECK("embedding_kernel");
+    return 0;
+}
+
+// Host side of the embedding's backward: a counting sort over the vocabulary (interpreted, the tables of 8192 ids and their
+// uploads were 2.0 of the 5.5 ms that a four-block training step takes to issue).
+extern "C" int qmoe_token_tables(const void* ids_, int64_t count, int64_t vocab, void* distinct_, void* starts_, void* positions_, int64_t* segments) {
+    if (!ids_ || !distinct_ || !starts_ || !positions_ || !segments) return fail_arg("token_tables: null address");
+    if (count <= 0 || vocab <= 0) return fail_arg("token_tables: sizes must be positive");
+    const int64_t* ids = (const int64_t*)ids_;
+    int64_t *distinct = (int64_t*)distinct_, *starts = (int64_t*)starts_, *positions = (int64_t*)positions_;
+    for (int64_t i = 0; i < count; ++i)
+        if (ids[i] < 0 || ids[i] >= vocab) return fail_arg("token id outside the vocabulary");
+    int64_t* next = (int64_t*)calloc((size_t)vocab, sizeof(int64_t));     // occurrences, then where the next position of a token goes
+    if (!next) { set_error("token_tables: out of host memory"); return QMOE_ERR_STATE; }
+    for (int64_t i = 0; i < count; ++i) ++next[ids[i]];
+    int64_t found = 0, at = 0;
+    for (int64_t t = 0; t < vocab; ++t) {
+        const int64_t n = next[t];
+        if (!n) continue;
+        distinct[found] = t;
+        starts[found++] = at;
+        next[t] = at;
+        at += n;
+    }
+    starts[found] = at;
+    for (int64_t i = 0; i < count; ++i) positions[next[ids[i]]++] = i;
+    free(next);
+    *segments = found;
     return 0;
 }
 

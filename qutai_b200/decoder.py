@@ -16,6 +16,7 @@ renewed only when a parameter's storage changed.  Head width 64 only (``qutai_b2
 """
 from __future__ import annotations
 
+import ctypes
 from array import array
 from dataclasses import dataclass
 from math import sqrt
@@ -95,6 +96,19 @@ class Linear:
             self._gemm(dy, x, dw, self.width_out, rows, self.width_in, 1, 0, lib.QMOE_F32)
         _accumulate(self.weight, dw, self.stream)
         return dx
+
+
+def _integers(rows, room):
+    """The nested sequence ``rows`` of integers as one array of 64-bit integers with ``room`` more zeros behind it.  An entry
+    beyond 64 bits becomes -1, which is outside every vocabulary."""
+    values = array("q")
+    try:
+        for row in rows:
+            values.extend(row)
+    except (TypeError, OverflowError):     # entries that only int() turns into integers, arrays of another type
+        values = array("q", (t if -2 ** 63 <= t < 2 ** 63 else -1 for t in (int(t) for row in rows for t in row)))
+    values.extend(array("q", bytes(8 * room)))
+    return values
 
 
 def _rms_norm(x, norm, rows, width, stream):
@@ -318,28 +332,25 @@ class Decoder:
         batch, time = len(tokens), len(tokens[0])
         if time < 2 or any(len(row) != time for row in tokens):
             raise ValueError("tokens must be a non-empty rectangular batch of at least two positions")
-        flat = [int(t) for row in tokens for t in row]
-        if any(t < 0 or t >= c.vocab_size for t in flat):
-            raise ValueError("token id outside the vocabulary")
-        targets = flat if labels is None else [int(t) for row in labels for t in row]
-        if len(targets) != len(flat) or any(t != -100 and not 0 <= t < c.vocab_size for t in targets):
-            raise ValueError("labels must have the shape of the tokens and be token ids or -100")
         rows, width = batch * time, c.d_model
         # The embedding's backward wants, per distinct token, the list of its positions (upstream builds the same tables,
         # src/qutai/backends/cuda_lm.py:97-106).  They depend on the ids alone, so they are built and uploaded here,
         # next to the ids: an upload waits for the stream, and at this point of a training loop the device is just
         # finishing the previous step, while at the end of the backward the wait would leave it idle through the
-        # host's preparation of the optimizer step.
-        groups = {}
-        for position, token in enumerate(flat):
-            groups.setdefault(token, []).append(position)
-        distinct = sorted(groups)
-        starts, positions = [0], []
-        for token in distinct:
-            positions.extend(groups[token])
-            starts.append(len(positions))
-        ids = DeviceStorage.from_bytes(array("q", flat).tobytes(), "int64", stream)
-        tables = tuple(DeviceStorage.from_bytes(array("q", values).tobytes(), "int64", stream) for values in (distinct, starts, positions))
+        # host's preparation of the optimizer step.  Ids and tables lie in one host array (ids | positions | distinct
+        # tokens | starts) and go up in one copy.
+        host = _integers(tokens, 3 * rows + 1)
+        if len(host) != 4 * rows + 1:
+            raise ValueError("tokens must be a non-empty rectangular batch of at least two positions")
+        base, segments = host.buffer_info()[0], ctypes.c_int64()
+        lib.call("qmoe_token_tables", base, rows, c.vocab_size, base + 16 * rows, base + 24 * rows, base + 8 * rows, ctypes.byref(segments))
+        distinct = segments.value
+        targets = host if labels is None else [int(t) for row in labels for t in row]
+        if labels is not None and (len(targets) != rows or any(t != -100 and not 0 <= t < c.vocab_size for t in targets)):
+            raise ValueError("labels must have the shape of the tokens and be token ids or -100")
+        uploaded = DeviceStorage.from_bytes(host.tobytes(), "int64", stream)
+        ids = uploaded.view(0, rows)
+        tables = (uploaded.view(2 * rows, distinct), uploaded.view(3 * rows, distinct + 1), uploaded.view(rows, rows))
         label_ids = ids if labels is None else DeviceStorage.from_bytes(array("q", targets).tobytes(), "int64", stream)
         x = DeviceStorage(rows * width, "bfloat16")
         lib.call("qmoe_embedding", self.embedding.weight.storage.ptr, ids.ptr, x.ptr, lib.QMOE_BF16, rows, width, c.vocab_size, stream)
@@ -371,7 +382,7 @@ class Decoder:
         lib.call("qmoe_scale_f32", mean_aux.ptr, scaled.ptr, 0, self._aux_coef.ptr, 1, 1, stream)
         lib.call("qmoe_add", lm.storage.ptr, scaled.ptr, total.ptr, lib.QMOE_F32, 1, stream)
         self.last_lm_loss, self.last_auxiliary_loss = lm, Tensor(mean_aux, ())
-        self._saved = (tables, len(distinct), len(positions), batch, time, x, inverse, share)
+        self._saved = (tables, distinct, rows, batch, time, x, inverse, share)
         return Tensor(total, ())
 
     # -- backward -----------------------------------------------------------------------------------------------
