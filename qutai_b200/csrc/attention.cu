@@ -18,7 +18,7 @@
 // The products of the next block are issued before the rows have finished with this one (S has a second buffer in the
 // backward and is taken into registers at once in the forward), so the row warps rarely wait for the tensor cores; what
 // bounds them is the exponential unit, 1024 cycles per 128 x 128 block and SM, and the latency of their own chain beside it.
-// 4 sequences x 2048 positions, 16 heads in 4 groups (L2 flushed): forward 144 -> 75 us, backward 472 -> 191 against the form
+// 4 sequences x 2048 positions, 16 heads in 4 groups (L2 flushed): forward 144 -> 75 us, backward 472 -> 181 against the form
 // with P and dS in shared memory and one block in flight.
 // Every wait is bounded; on expiry the CTA records a code in the library's status word and leaves.
 #include "common.cuh"
@@ -478,12 +478,16 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
                 float d0, d1;
                 unpair2(mul2(pair2(__uint_as_float(s[c]), __uint_as_float(s[c + 1])),
                              add2(pair2(__uint_as_float(dp[c]), __uint_as_float(dp[c + 1])), delta_pair)), d0, d1);
-                if (masked) {
-                    if (first + c > row) d0 = 0.f;
-                    if (first + c + 1 > row) d1 = 0.f;
-                }
-                packed[c >> 1] = pack2(d0, d1);
+                s[c] = __float_as_uint(d0);
+                s[c + 1] = __float_as_uint(d1);
             }
+            if (masked) {      // a loop of its own: as selects in the one above the mask cost every block, not only those on the diagonal
+#pragma unroll
+                for (int c = 0; c < COLS; ++c)
+                    if (first + c > row) s[c] = 0u;
+            }
+#pragma unroll
+            for (int c = 0; c < COLS; c += 2) packed[c >> 1] = pack2(__uint_as_float(s[c]), __uint_as_float(s[c + 1]));
             if (COLS == 64) tmem_st32(tmem_s, packed);
             else tmem_st16(tmem_s, packed);
             tmem_st_wait();
@@ -686,7 +690,16 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
             const uint32_t tmem_s = tmem + (uint32_t)(it & 1) * 128 + lane_base + part * COLS;
             const uint32_t row_values = rows_at + st * DKV_ROW_BYTES + part * COLS * 4;
             const bool masked = i == j && part * COLS < quad * 32 + 31;  // some row of this warp is not seen by some of these columns
-            uint32_t s[COLS], dp[COLS], packed[COLS / 2];
+            uint32_t s[COLS], dp[COLS];
+            auto put_back = [&](uint32_t to) {         // s, rounded to bf16, 32 columns at a time (the registers of all at once spill)
+#pragma unroll
+                for (int c = 0; c < COLS; c += 32) {
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int e = 0; e < 32; e += 2) packed[e >> 1] = pack2(__uint_as_float(s[c + e]), __uint_as_float(s[c + e + 1]));
+                    tmem_st16(to + c / 2, packed);
+                }
+            };
             // the row values of this stage (the scores of this iteration were formed from the same stage, but the barrier that
             // publishes the loading warp's plain stores is the stage's own)
             ok = wait.all(bar(Q_FULL + st), (uint32_t)(it / DKV_STAGES) & 1u);
@@ -703,19 +716,16 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
 #pragma unroll
                 for (int e = 0; e < 4; e += 2) {
                     unpair2(fma2(pair2(__uint_as_float(s[c + e]), __uint_as_float(s[c + e + 1])), scale_pair, pair2(l[e], l[e + 1])), x[e], x[e + 1]);
-                    x[e] = exp2_fast(x[e]);
-                    x[e + 1] = exp2_fast(x[e + 1]);
-                    if (masked) {
-                        if (part * COLS + c + e < row) x[e] = 0.f;
-                        if (part * COLS + c + e + 1 < row) x[e + 1] = 0.f;
-                    }
-                    s[c + e] = __float_as_uint(x[e]);
-                    s[c + e + 1] = __float_as_uint(x[e + 1]);
-                    packed[(c + e) >> 1] = pack2(x[e], x[e + 1]);
+                    s[c + e] = __float_as_uint(exp2_fast(x[e]));
+                    s[c + e + 1] = __float_as_uint(exp2_fast(x[e + 1]));
                 }
             }
-            if (COLS == 64) tmem_st32(tmem_s, packed);
-            else tmem_st16(tmem_s, packed);
+            if (masked) {      // a loop of its own, as in the dq kernel (both: 191 -> 181 us at 4 x 2048 positions, 16 heads)
+#pragma unroll
+                for (int c = 0; c < COLS; ++c)
+                    if (part * COLS + c < row) s[c] = 0u;
+            }
+            put_back(tmem_s);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -736,15 +746,16 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
                     float d0, d1;
                     unpair2(mul2(pair2(__uint_as_float(s[c + e]), __uint_as_float(s[c + e + 1])),
                                  add2(pair2(__uint_as_float(dp[c + e]), __uint_as_float(dp[c + e + 1])), pair2(d[e], d[e + 1]))), d0, d1);
-                    if (masked) {
-                        if (part * COLS + c + e < row) d0 = 0.f;
-                        if (part * COLS + c + e + 1 < row) d1 = 0.f;
-                    }
-                    packed[(c + e) >> 1] = pack2(d0, d1);
+                    s[c + e] = __float_as_uint(d0);
+                    s[c + e + 1] = __float_as_uint(d1);
                 }
             }
-            if (COLS == 64) tmem_st32(tmem_s + COLS / 2, packed);
-            else tmem_st16(tmem_s + COLS / 2, packed);
+            if (masked) {
+#pragma unroll
+                for (int c = 0; c < COLS; ++c)
+                    if (part * COLS + c < row) s[c] = 0u;
+            }
+            put_back(tmem_s + COLS / 2);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
