@@ -171,9 +171,11 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
 int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream);
 int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t weight, uint64_t out, int32_t dtype, int64_t width, int pad,
                         uint64_t stream);
-bool router_norm_ok(int64_t tokens);
+bool router_norm_ok(int64_t tokens, int32_t experts, int64_t width);
 int router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
                         int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
+int router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,
+                           uint64_t d_w_router, uint64_t col_scale, uint64_t scratch, int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
 int route_check(const qmoe_route_t* r);
 int launch_swiglu(const qmoe_route_t* r, uint64_t g, uint64_t u, uint64_t h, int dtype, long long hidden, cudaStream_t stream);
 int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint64_t u, uint64_t dg, uint64_t du, int dtype,

@@ -364,7 +364,7 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
         if (int rc = qmoe_cast_bf16(L->master_down, ex->w_down, E * hd * d, stream)) return rc;
     }
     // scores = rms_norm(x) . W_r^T = inverse[t] * (x . (W_r * w)^T): the product reads the raw activations
-    if (router_norm_ok(r->tokens)) {
+    if (router_norm_ok(r->tokens, r->experts, d)) {
         if (int rc = router_forward_norm(L->x, ex->dtype, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, r->tokens, d, r->experts, stream))
             return rc;
     } else {
@@ -398,10 +398,8 @@ extern "C" int qmoe_block_backward(const qmoe_block_t* B, uint64_t stream) {
     // router: the weight gradient is d_scores^T . rms_norm(x) = ((inverse * d_scores)^T . x) * w, from the raw
     // activations; the same product call returns (inverse * d_scores) . W_r, i.e. inverse[t] times the gradient of
     // the NORMALISED input, and the kernel below takes the row scale back out
-    if (int rc = qmoe_scale_f32(L->d_scores, L->d_scores, B->inverse, 0, r->tokens, E, stream)) return rc;
-    if (int rc = qmoe_router_backward(L->d_scores, L->x, ex->dtype, L->w_router, L->dx_router, L->d_w_router, L->router_partials,
-                                      r->tokens, d, r->experts, stream)) return rc;
-    if (int rc = qmoe_scale_f32(L->d_w_router, L->d_w_router, 0, B->norm_weight, E, d, stream)) return rc;
+    if (int rc = router_backward_scaled(L->d_scores, B->inverse, L->x, ex->dtype, L->w_router, L->dx_router, L->d_w_router, B->norm_weight,
+                                        L->router_partials, r->tokens, d, r->experts, stream)) return rc;
     return qmoe_unpermute_norm_backward(r, L->dx_dispatched, L->dx_router, 1, L->x, B->inverse, B->norm_weight, L->grad_out,
                                         L->dx, B->d_norm_weight, B->norm_partials, ex->dtype, d, stream);
 }

@@ -73,10 +73,10 @@ router_split_w_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ w
     }
 }
 
-// ds [T, E] fp32 -> ds6 [T, 6S] = {hi | mid | lo | hi | mid | 0}; also the token-block tables of the split contraction
+// ds [T, E] fp32 (times row_scale[t], when given) -> ds6 [T, 6S] = {hi | mid | lo | hi | mid | 0}; also the token-block tables of the split contraction
 __global__ void __launch_bounds__(256)
-router_split_ds_kernel(const float* __restrict__ ds, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S, int* __restrict__ tables,
-                       int splits, long long rows_per_split) {
+router_split_ds_kernel(const float* __restrict__ ds, const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S,
+                       int* __restrict__ tables, int splits, long long rows_per_split) {
     if (blockIdx.x == 0 && threadIdx.x <= splits) {
         const int i = threadIdx.x;
         tables[i] = (int)(i * rows_per_split);  // offsets[splits + 1]
@@ -91,15 +91,17 @@ router_split_ds_kernel(const float* __restrict__ ds, __nv_bfloat16* __restrict__
         const long long t = i / S;
         const int e = (int)(i - t * S);
         __nv_bfloat16 hi, mid, lo;
-        split3(e < E ? ds[t * E + e] : 0.f, hi, mid, lo);
+        const float scale = row_scale ? row_scale[t] : 1.f;
+        split3(e < E ? ds[t * E + e] * scale : 0.f, hi, mid, lo);
         __nv_bfloat16* row = ds6 + t * 6 * S;
         row[e] = hi; row[S + e] = mid; row[2 * S + e] = lo; row[3 * S + e] = hi; row[4 * S + e] = mid; row[5 * S + e] = zero;
     }
 }
 
-// dW [E, d] = sum over splits and over the three term groups, in a fixed order
+// dW [E, d] = sum over splits and over the three term groups, in a fixed order (times col_scale[j], when given)
 __global__ void __launch_bounds__(256)
-router_reduce_dw_kernel(const float* __restrict__ partial, float* __restrict__ dw, int E, int S, long long d, int splits) {
+router_reduce_dw_kernel(const float* __restrict__ partial, const float* __restrict__ col_scale, float* __restrict__ dw, int E, int S, long long d,
+                        int splits) {
     const long long n = (long long)E * d;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long e = i / d, j = i - e * d;
@@ -108,14 +110,19 @@ router_reduce_dw_kernel(const float* __restrict__ partial, float* __restrict__ d
             const float* slab = partial + (long long)s * 3 * S * d;
             acc += (slab[(2 * S + e) * d + j] + slab[(S + e) * d + j]) + slab[e * d + j];
         }
-        dw[i] = acc;
+        dw[i] = col_scale ? acc * col_scale[j] : acc;
     }
 }
 
 // Few tokens (decode): one block per token, a warp per expert in turn, fp32 dot products with the lanes
 // striding over the width and a fixed shuffle tree, so the logits are run-to-run identical.  A tile kernel
 // would put the whole product on one or two SMs and walk the width serially.
-constexpr long long kSmallRouterTokens = 512;
+// The warps of a token read every weight row again, from L2: up to 512 tokens that is the shorter way whatever the sizes, and
+// beyond them while it is at most 64 MB (602 tokens, 8 experts, d 512, with the norm: 4 us in one launch, 15 in five).
+constexpr long long kSmallRouterTokens = 512, kSmallRouterProducts = 1ll << 24;
+bool small_router(long long tokens, int experts, long long width) {
+    return tokens <= kSmallRouterTokens || tokens * experts * width <= kSmallRouterProducts;
+}
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
     const uint2 v = *reinterpret_cast<const uint2*>(p);
@@ -206,7 +213,7 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
     if (x_dtype != QMOE_F32 && x_dtype != QMOE_BF16) return fail_arg("router_forward: bad dtype %d", x_dtype);
     cudaStream_t stream = (cudaStream_t)stream_;
     // fp32 rows over up to 16 experts: the tile kernel's 128 x 16 tiles take 31 us for 2048 tokens of width 512 over 8, this 5
-    if (tokens <= kSmallRouterTokens || (x_dtype == QMOE_F32 && experts <= 16)) {
+    if (small_router(tokens, experts, width) || (x_dtype == QMOE_F32 && experts <= 16)) {
         TimedScope timed(KC_ROUTER_GEMM, stream);
         const dim3 grid((unsigned)tokens, (unsigned)((experts + 7) / 8));
         if (x_dtype == QMOE_BF16)
@@ -228,7 +235,7 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
     return tc_router_forward(x, scratch + r.w3, scores, tokens, width, experts, r.S, stream);
 }
 
-bool qmoe::router_norm_ok(int64_t tokens) { return tokens <= kSmallRouterTokens; }
+bool qmoe::router_norm_ok(int64_t tokens, int32_t experts, int64_t width) { return small_router(tokens, experts, width); }
 
 // inverse[t] and the logits of the normalised rows in one launch (tokens within router_norm_ok)
 int qmoe::router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
@@ -253,13 +260,26 @@ extern "C" int qmoe_router_logits(uint64_t x, int32_t x_dtype, uint64_t w_router
 
 extern "C" int qmoe_router_backward(uint64_t d_scores, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,
                                     uint64_t d_w_router, uint64_t scratch, int64_t tokens, int64_t width, int32_t experts,
-                                    uint64_t stream_) {
+                                    uint64_t stream) {
+    return router_backward_scaled(d_scores, 0, x, x_dtype, w_router, dx_router, d_w_router, 0, scratch, tokens, width, experts, stream);
+}
+
+// The same for d_scores[t, :] * row_scale[t], with the weight gradient's columns multiplied by col_scale (0: neither).  The
+// scales ride along where the factors are split and the ranges are summed; d_scores itself may or may not hold the scaled
+// values afterwards.
+int qmoe::router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,
+                                 uint64_t d_w_router, uint64_t col_scale, uint64_t scratch, int64_t tokens, int64_t width, int32_t experts,
+                                 uint64_t stream_) {
     if (!d_scores || !x || !w_router) return fail_arg("router_backward: null address");
     if (tokens <= 0 || width <= 0 || experts <= 0) return fail_arg("router_backward: sizes must be positive");
     if (x_dtype != QMOE_F32 && x_dtype != QMOE_BF16) return fail_arg("router_backward: bad dtype %d", x_dtype);
     cudaStream_t stream = (cudaStream_t)stream_;
-    if (!tc_router_ok(x_dtype, experts, width, x, scratch))
-        return simt_router_backward(d_scores, x, x_dtype, w_router, dx_router, d_w_router, scratch, tokens, width, experts, stream);
+    if (!tc_router_ok(x_dtype, experts, width, x, scratch)) {
+        if (row_scale)
+            if (int rc = qmoe_scale_f32(d_scores, d_scores, row_scale, 0, tokens, experts, stream_)) return rc;
+        if (int rc = simt_router_backward(d_scores, x, x_dtype, w_router, dx_router, d_w_router, scratch, tokens, width, experts, stream)) return rc;
+        return col_scale && d_w_router ? qmoe_scale_f32(d_w_router, d_w_router, 0, col_scale, experts, width, stream_) : 0;
+    }
     TimedScope timed(KC_ROUTER_GEMM, stream);
     const RouterScratch r = plan_scratch(tokens, experts, width);
     const int S = r.S;
@@ -268,7 +288,7 @@ extern "C" int qmoe_router_backward(uint64_t d_scores, uint64_t x, int32_t x_dty
     router_split_w_kernel<<<elem_grid((long long)S * width), 256, 0, stream>>>(
         (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, S, width);
     QMOE_LAUNCH_CHECK("router_split_w_kernel");
-    router_split_ds_kernel<<<elem_grid(tokens * S), 256, 0, stream>>>((const float*)d_scores, (__nv_bfloat16*)(scratch + r.ds6),
+    router_split_ds_kernel<<<elem_grid(tokens * S), 256, 0, stream>>>((const float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6),
                                                                       tokens, experts, S, tables, r.splits, r.rows_per_split);
     QMOE_LAUNCH_CHECK("router_split_ds_kernel");
     if (dx_router)
@@ -277,7 +297,7 @@ extern "C" int qmoe_router_backward(uint64_t d_scores, uint64_t x, int32_t x_dty
         if (int rc = tc_split_wgrad(scratch + r.ds6, 6ll * S, x, scratch + r.partial, tables, tables + r.splits + 1, r.splits,
                                     tokens, 3ll * S, width, stream)) return rc;
         router_reduce_dw_kernel<<<elem_grid((long long)experts * width), 256, 0, stream>>>(
-            (const float*)(scratch + r.partial), (float*)d_w_router, experts, S, width, r.splits);
+            (const float*)(scratch + r.partial), (const float*)col_scale, (float*)d_w_router, experts, S, width, r.splits);
         QMOE_LAUNCH_CHECK("router_reduce_dw_kernel");
     }
     return 0;
