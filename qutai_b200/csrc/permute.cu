@@ -248,32 +248,59 @@ unpermute_kernel(const T* __restrict__ dxd, const float* __restrict__ extra, con
 // ---- SwiGLU element-wise over the dispatched rows (used by the CUDA-core GEMM path) -----------
 // Rounding points follow the upstream activations: silu(G) is stored in the activation dtype
 // before the multiply (src/qutai/lm/layers.py:311 builds it from two separate kernels).
-template <typename T>
+// WIDE: 16-byte pieces (aligned buffers; the rows are whole tiles of 128, so the values are whole pieces); value by value otherwise.  4608 x 1024 float32, forward and
+// backward: 14 and 29 us value by value, 11 and 17 in pieces.
+template <typename T, bool WIDE> struct Piece;
+template <typename T> struct Piece<T, true> {
+    static constexpr int N = Vec16<T>::N;
+    static __device__ __forceinline__ void load(const T* p, float* f) { Vec16<T>::unpack(*reinterpret_cast<const uint4*>(p), f); }
+    static __device__ __forceinline__ void store(T* p, const float* f) { st16(p, Vec16<T>::pack(f)); }
+};
+template <typename T> struct Piece<T, false> {
+    static constexpr int N = 1;
+    static __device__ __forceinline__ void load(const T* p, float* f) { f[0] = Act<T>::load(p); }
+    static __device__ __forceinline__ void store(T* p, const float* f) { Act<T>::store(p, f[0]); }
+};
+template <typename T> __device__ __forceinline__ float round_to(float v) {
+    T r;
+    Act<T>::store(&r, v);
+    return Act<T>::load(&r);
+}
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kThreads)
 swiglu_kernel(const T* __restrict__ G, const T* __restrict__ U, T* __restrict__ H,
               const int* __restrict__ meta, long long hidden) {
-    const long long n = (long long)meta[0] * hidden;
+    using P = Piece<T, WIDE>;
+    const long long n = (long long)meta[0] * hidden / P::N;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float g = Act<T>::load(G + i), u = Act<T>::load(U + i);
-        T act;
-        Act<T>::store(&act, g * sigmoid_stable(g));
-        Act<T>::store(H + i, Act<T>::load(&act) * u);
+        float g[P::N], u[P::N];
+        P::load(G + i * P::N, g);
+        P::load(U + i * P::N, u);
+#pragma unroll
+        for (int e = 0; e < P::N; ++e) g[e] = round_to<T>(g[e] * sigmoid_stable(g[e])) * u[e];
+        P::store(H + i * P::N, g);
     }
 }
 
-template <typename T>
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kThreads)
 swiglu_backward_kernel(const T* __restrict__ dH, const T* __restrict__ G, const T* __restrict__ U,
                        T* __restrict__ dG, T* __restrict__ dU, const int* __restrict__ meta, long long hidden) {
-    const long long n = (long long)meta[0] * hidden;
+    using P = Piece<T, WIDE>;
+    const long long n = (long long)meta[0] * hidden / P::N;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float dh = Act<T>::load(dH + i), g = Act<T>::load(G + i), u = Act<T>::load(U + i);
-        const float s = sigmoid_stable(g);
-        T act, ds;
-        Act<T>::store(&act, g * s);
-        Act<T>::store(dU + i, dh * Act<T>::load(&act));
-        Act<T>::store(&ds, dh * u);
-        Act<T>::store(dG + i, Act<T>::load(&ds) * s * (1.f + g * (1.f - s)));
+        float dh[P::N], g[P::N], u[P::N], dg[P::N], du[P::N];
+        P::load(dH + i * P::N, dh);
+        P::load(G + i * P::N, g);
+        P::load(U + i * P::N, u);
+#pragma unroll
+        for (int e = 0; e < P::N; ++e) {
+            const float s = sigmoid_stable(g[e]);
+            du[e] = dh[e] * round_to<T>(g[e] * s);
+            dg[e] = round_to<T>(dh[e] * u[e]) * s * (1.f + g[e] * (1.f - s));
+        }
+        P::store(dU + i * P::N, du);
+        P::store(dG + i * P::N, dg);
     }
 }
 
@@ -375,13 +402,12 @@ int check_dtype(int dtype) {
 int launch_swiglu(const qmoe_route_t* r, uint64_t g, uint64_t u, uint64_t h, int dtype, long long hidden,
                   cudaStream_t stream) {
     TimedScope timed(KC_SWIGLU, stream);
-    const int grid = grid_for_elems(r->rows_bound * hidden);
-    if (dtype == QMOE_BF16)
-        swiglu_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>((const __nv_bfloat16*)g, (const __nv_bfloat16*)u,
-                                                                     (__nv_bfloat16*)h, (const int*)r->meta, hidden);
-    else
-        swiglu_kernel<float><<<grid, kThreads, 0, stream>>>((const float*)g, (const float*)u, (float*)h,
-                                                             (const int*)r->meta, hidden);
+    const bool wide = !((g | u | h) & 15u);
+    const int grid = grid_for_elems(r->rows_bound * hidden / (wide ? (dtype == QMOE_BF16 ? 8 : 4) : 1));
+#define SWIGLU(T, W) swiglu_kernel<T, W><<<grid, kThreads, 0, stream>>>((const T*)g, (const T*)u, (T*)h, (const int*)r->meta, hidden)
+    if (dtype == QMOE_BF16) { if (wide) SWIGLU(__nv_bfloat16, true); else SWIGLU(__nv_bfloat16, false); }
+    else { if (wide) SWIGLU(float, true); else SWIGLU(float, false); }
+#undef SWIGLU
     QMOE_LAUNCH_CHECK("swiglu_kernel");
     return 0;
 }
@@ -389,14 +415,13 @@ int launch_swiglu(const qmoe_route_t* r, uint64_t g, uint64_t u, uint64_t h, int
 int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint64_t u, uint64_t dg, uint64_t du,
                            int dtype, long long hidden, cudaStream_t stream) {
     TimedScope timed(KC_SWIGLU, stream);
-    const int grid = grid_for_elems(r->rows_bound * hidden);
-    if (dtype == QMOE_BF16)
-        swiglu_backward_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>(
-            (const __nv_bfloat16*)dh, (const __nv_bfloat16*)g, (const __nv_bfloat16*)u, (__nv_bfloat16*)dg,
-            (__nv_bfloat16*)du, (const int*)r->meta, hidden);
-    else
-        swiglu_backward_kernel<float><<<grid, kThreads, 0, stream>>>((const float*)dh, (const float*)g, (const float*)u,
-                                                                      (float*)dg, (float*)du, (const int*)r->meta, hidden);
+    const bool wide = !((dh | g | u | dg | du) & 15u);
+    const int grid = grid_for_elems(r->rows_bound * hidden / (wide ? (dtype == QMOE_BF16 ? 8 : 4) : 1));
+#define SWIGLU(T, W) \
+    swiglu_backward_kernel<T, W><<<grid, kThreads, 0, stream>>>((const T*)dh, (const T*)g, (const T*)u, (T*)dg, (T*)du, (const int*)r->meta, hidden)
+    if (dtype == QMOE_BF16) { if (wide) SWIGLU(__nv_bfloat16, true); else SWIGLU(__nv_bfloat16, false); }
+    else { if (wide) SWIGLU(float, true); else SWIGLU(float, false); }
+#undef SWIGLU
     QMOE_LAUNCH_CHECK("swiglu_backward_kernel");
     return 0;
 }
