@@ -114,3 +114,23 @@ def test_attention_at_the_edges_of_blocks_and_with_growing_scores(batch, time, h
     # with scores of scale^2 the softmax is nearly one-hot and dS = P (dP - delta) cancels: the element bar is that of the
     # 2048-position test there
     check(run_attention(q, k, v, grad, heads, kv_heads), dict(out=out, dq=dq, dk=dk, dv=dv), element_tol=0.2 if scale > 1 else BF16_ELEMENT_TOL)
+
+
+def test_attention_of_one_hot_rows_returns_the_value_row():
+    """Scores of about 8e5 that grow by 2048 (256 after the scale) from one position to the next: in every row the
+    probability of the last position is 1 and all others are below exp(-256), so the output is that position's value row,
+    exactly, and the gradient of q vanishes up to rounding.  A base of the exponentials that is rounded (half an ulp of 1.5e5 is
+    2^-7) shows as a probability other than 1."""
+    batch, time, heads, kv_heads = 1, 300, 2, 1
+    at = np.arange(time)
+    q = np.full((batch, time, heads * 64), 64.0)
+    k = np.empty((batch, time, 64))
+    k[0, :, :32], k[0, :, 32:] = (128 + at % 128)[:, None], (128 + 128 * (at // 128))[:, None]      # exact in bf16
+    rng = np.random.default_rng(0)
+    v, grad = oracle.round_bf16(rng.standard_normal(k.shape)), oracle.round_bf16(rng.standard_normal(q.shape))
+    got = run_attention(q, k, v, grad, heads, kv_heads)
+    assert np.array_equal(got["out"], np.concatenate([v, v], axis=2))
+    # dS = P (dP - delta): two fp32 sums of the same 64 products in different orders, at most 64 roundings of their size apart,
+    # times keys of up to 384 over 8
+    bound = 384 / 8 * 64 * 2.0 ** -24 * np.abs(grad).max() * np.abs(v).max() * 64
+    assert np.abs(got["dq"]).max() <= bound
