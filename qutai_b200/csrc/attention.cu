@@ -546,7 +546,10 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
     const uint32_t base = smem_u32(smem_raw);
     const uint32_t k_tile = base, v_tile = base + TILE_BYTES, q_tile = v_tile + TILE_BYTES, do_tile = q_tile + DKV_STAGES * TILE_BYTES;
     const uint32_t rows_at = base + DKV_TILES, bars = rows_at + DKV_STAGES * DKV_ROW_BYTES;
-    enum { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = Q_FULL + DKV_STAGES, S_FULL = Q_EMPTY + DKV_STAGES, DP_FULL = S_FULL + 2, P_FULL, DS_FULL, ACC_DONE, BARS };
+    enum { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = Q_FULL + DKV_STAGES, S_FULL = Q_EMPTY + DKV_STAGES, DP_FULL = S_FULL + 2, P_FULL, DS_FULL = P_FULL + 2, ACC_DONE, BARS };
+    // S_FULL and P_FULL are two barriers each, by the parity of the iteration: the scores of the next iteration are formed before
+    // all rows have put back this one's P, so a fast warp may be a whole phase ahead of a slow one there, and with one barrier
+    // its second arrival would stand in for the slow warp's first.  (DS_FULL: the next dP waits for this phase.)
     auto bar = [&](int which) { return bars + 8u * which; };
     uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 8 * BARS);
     volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 8 * BARS + 4);
@@ -558,7 +561,7 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
         s_abort = 0;
         // a stage is full when its bytes have landed and the lanes of the loading warp have written its row values
         for (int w = 0; w < BARS; ++w) {
-            const bool rows = w == P_FULL || w == DS_FULL, full = w >= Q_FULL && w < Q_EMPTY;
+            const bool rows = w >= P_FULL && w <= DS_FULL, full = w >= Q_FULL && w < Q_EMPTY;
             mbar_init(bar(w), rows ? 4 * DKV_PARTS : full ? 2 : 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -652,7 +655,7 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
             // the next scores into the other buffer, once the products that read the P and dS of iteration it - 1 there are done
             if (it > 0) ok = wait.all(bar(Q_EMPTY + (it - 1) % DKV_STAGES), (uint32_t)((it - 1) / DKV_STAGES) & 1u);
             if (ok && it + 1 < n) ok = scores(it + 1);
-            if (ok) ok = wait.all(bar(P_FULL), (uint32_t)it & 1u);
+            if (ok) ok = wait.all(bar(P_FULL + (it & 1)), (uint32_t)(it >> 1) & 1u);
             if (!ok) break;
             tc_fence_after();
             // dV += P^T dO and dK += dS^T Q: P^T and dS^T from tensor memory, dO and Q as they lie in memory (rows = query
@@ -730,7 +733,7 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(P_FULL));
+            if (lane == 0) mbar_arrive(bar(P_FULL + (it & 1)));
             ok = wait.all(bar(DP_FULL), (uint32_t)it & 1u);
             if (!ok) break;
             tc_fence_after();

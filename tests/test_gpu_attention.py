@@ -134,3 +134,23 @@ def test_attention_of_one_hot_rows_returns_the_value_row():
     # times keys of up to 384 over 8
     bound = 384 / 8 * 64 * 2.0 ** -24 * np.abs(grad).max() * np.abs(v).max() * 64
     assert np.abs(got["dq"]).max() <= bound
+
+
+@pytest.mark.parametrize("batch,time,heads,kv_heads", [(2, 2048, 8, 8), (4, 1024, 16, 4), (1, 4096, 4, 1)])
+def test_attention_backward_repeats_its_bits(batch, time, heads, kv_heads):
+    """Many key blocks with a diagonal block in each, whose row warps take longer than the others': the warps that share a
+    block's probabilities drift apart, and every repetition has to give the same bits all the same."""
+    from gpu_util import to_device
+    from qutai_b200 import lib
+    from qutai_b200.attention import attention_backward, attention_forward
+    from qutai_b200.layers import Tensor
+
+    inputs = attention_inputs(batch, time, heads, kv_heads, seed=time, scale=1.0)
+    q, k, v, grad = (Tensor(to_device(a, "bfloat16"), a.shape) for a in inputs)
+    out, lse = attention_forward(q, k, v, heads, kv_heads)
+    first = None
+    for _ in range(25):
+        bits = [part.tobytes() for part in attention_backward(grad, q, k, v, out, lse, heads, kv_heads)]
+        first = first or bits
+        assert bits == first
+    assert lib.device_status() == 0
