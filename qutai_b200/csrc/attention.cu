@@ -694,6 +694,7 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
             const uint32_t tmem_s = tmem + (uint32_t)(it & 1) * 128 + lane_base + part * COLS;
             const uint32_t row_values = rows_at + st * DKV_ROW_BYTES + part * COLS * 4;
             const bool masked = i == j && part * COLS < quad * 32 + 31;  // some row of this warp is not seen by some of these columns
+            const int live = p.time - i * BLOCK - part * COLS;           // columns from here on are past the end of the sequence
             uint32_t s[COLS], dp[COLS];
             auto put_back = [&](uint32_t to) {         // s, rounded to bf16, 32 columns at a time (the registers of all at once spill)
 #pragma unroll
@@ -728,6 +729,11 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
 #pragma unroll
                 for (int c = 0; c < COLS; ++c)
                     if (part * COLS + c < row) s[c] = 0u;
+            }
+            if (live < COLS) {     // their scores are 0 * key: NaN for a key with an infinite component, although nobody sees it
+#pragma unroll
+                for (int c = 0; c < COLS; ++c)
+                    if (c >= live) s[c] = 0u;
             }
             put_back(tmem_s);
             tmem_st_wait();

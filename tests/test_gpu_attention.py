@@ -154,3 +154,21 @@ def test_attention_backward_repeats_its_bits(batch, time, heads, kv_heads):
         first = first or bits
         assert bits == first
     assert lib.device_status() == 0
+
+
+@pytest.mark.parametrize("time", [200, 256, 300])
+def test_attention_gradients_of_a_key_that_no_query_sees(time):
+    """A key with an infinite component, so that every query's score of it is -inf: its probability is zero everywhere, and its
+    gradients too, whether or not the sequence fills its last block of queries."""
+    heads, kv_heads, hidden = 2, 1, 70
+    q, k, v, grad = attention_inputs(1, time, heads, kv_heads, seed=time, scale=1.0)
+    q[:, :, 0::64] = -1.0
+    k[:, :, 0] = 0.0
+    without = k.copy()
+    k[0, hidden, 0], without[0, hidden, 0] = np.inf, 2.0 ** 100
+    got = run_attention(q, k, v, grad, heads, kv_heads)
+    out, lse = oracle.attention_forward(q, without, v, heads, kv_heads)
+    dq, dk, dv = oracle.attention_backward(grad, q, without, v, out, lse, heads, kv_heads)
+    for name in ("dk", "dv"):
+        assert np.all(np.isfinite(got[name])) and not np.any(got[name][0, hidden]), name
+    check(dict(got, dq=dq), dict(out=out, dq=dq, dk=dk, dv=dv))       # dq holds 0 * inf, as a product with that key does
