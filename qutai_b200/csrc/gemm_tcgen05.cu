@@ -102,6 +102,7 @@ struct alignas(64) GemmParams {
     int plain_rows;       // > 0: one group of this many rows (any number) instead of the expert groups of `offsets` and `counts`
     int transpose_out;    // WGRAD: bit i set = problem i stores the [M, N] product of each expert as [N, M]
     int problems;         // WGRAD: 1, or 3 products of the same shape (outputs out0, out1, out2) sharing the tile queue
+    int sum_rows;         // WGRAD: > 0 (a multiple of 64): the contraction in pieces of this many rows, their products added in fp32
     int group_stride;     // ROUTER: accumulator columns [0,S), [S,2S), [2S,3S) hold the three bf16 terms of the weights
 };
 
@@ -127,7 +128,7 @@ template <int MODE, int CTAS> constexpr bool starts_in_shared() { return !(MODE 
 // expert with an odd number of 128-row tiles gets a last pair-tile whose second half is not stored.
 template <int MODE, bool B_MN, int CTAS>
 __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTable<starts_in_shared<MODE, CTAS>()>& s_start,
-                                            const int* s_pair, const int* s_order, int t, int cta_rank) {
+                                            const int* s_pair, const int* s_order, int t, int cta_rank, int piece = 0) {
     Tile tile;
     tile.valid = true;
     tile.rows_valid = true;
@@ -148,10 +149,14 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         tile.expert = e;
         tile.row0 = (rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
         tile.n0 = (rem / p.m_tiles) * BN;
-        const int count = s_pair[e];      // WGRAD keeps the row counts in this table
+        int count = s_pair[e];            // WGRAD keeps the row counts in this table
+        tile.krow0 = s_start[e] * kRowPad;
+        if (p.sum_rows > 0) {
+            tile.krow0 += piece * p.sum_rows;
+            count = min(count - piece * p.sum_rows, p.sum_rows);
+        }
         tile.depth = count;
         tile.kblocks = (count + BK - 1) / BK;
-        tile.krow0 = s_start[e] * kRowPad;
         tile.valid = count > 0;
     } else {
         // tiles are numbered from the first group's first row (a caller may pass a sub-range of the
@@ -415,6 +420,16 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     else if (CTAS == 2) total_tiles = s_pair[p.experts] * p.n_tiles;
     else total_tiles = (s_start[p.experts] - s_start[0]) * p.n_tiles;
     volatile int* abort_flag = &s_abort;
+    // A tile's pieces (sum_rows) are worked on one after the other, all in the first accumulator; the second holds their sum,
+    // which the epilogue warps add up in registers and put back.
+    const int pieces = MODE == MODE_WGRAD && p.sum_rows > 0 ? (p.plain_rows + p.sum_rows - 1) / p.sum_rows : 1;
+    auto accumulator = [&](int iter) { return pieces > 1 ? 0 : iter & 1; };
+    auto accumulator_phase = [&](int iter) { return (uint32_t)(pieces > 1 ? iter : iter >> 1) & 1u; };
+    auto next_tile = [&](int& t, int& piece) {
+        if (MODE == MODE_WGRAD && ++piece < pieces) return;
+        piece = 0;
+        t += tile_stride;
+    };
     // An epilogue warp hands its accumulator back as soon as its last read of it has arrived in registers, before the stores
     // of what it read, and without release semantics across the pair: a release at cluster scope waits until every global
     // store of the thread has been acknowledged (weight gradients over 375 rows per expert, 16 x 3 x 1024 x 2048: 145 us with
@@ -438,8 +453,8 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
-            for (int t = first_tile; t < total_tiles && !*abort_flag; t += tile_stride) {
-                const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank);
+            for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
+                const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
                 if (!tile.valid) continue;
                 const int kb_per_seg = tile.kblocks / (MODE == MODE_WGRAD ? 1 : p.segments);
                 for (int kb = 0; kb < tile.kblocks; ++kb) {
@@ -514,11 +529,11 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 if (CTAS == 2) umma_commit_both(bar);
                 else umma_commit(bar);
             };
-            for (int t = first_tile; t < total_tiles && !*abort_flag; t += tile_stride) {
-                const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank);
+            for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
+                const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
                 if (!tile.valid) continue;
-                const int acc = iter & 1;
-                const uint32_t acc_phase = (uint32_t)(iter >> 1) & 1u;
+                const int acc = accumulator(iter);
+                const uint32_t acc_phase = accumulator_phase(iter);
                 bool ok = mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag);
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)acc * BN;
@@ -695,11 +710,11 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         const uint32_t stage = epi0 + (uint32_t)(warp - 2) * Config::EPI_WARP_BYTES;  // this warp's transpose buffer
         const int half = (warp - 2) >> 2;  // which half of the tile's columns this warp converts
         int iter = 0;
-        for (int t = first_tile; t < total_tiles && !*abort_flag; t += tile_stride) {
-            const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank);
+        for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
+            const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
             if (!tile.valid) continue;
-            const int acc = iter & 1;
-            const uint32_t acc_phase = (uint32_t)(iter >> 1) & 1u;
+            const int acc = accumulator(iter);
+            const uint32_t acc_phase = accumulator_phase(iter);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) {
                 if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, STATUS_WAIT_EPILOGUE); }
                 break;
@@ -865,8 +880,21 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 for (int c = c_begin; c < c_end; ++c) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c * 32, r);
-                    tmem_ld_wait();
+                    if (MODE == MODE_WGRAD && piece > 0) {
+                        uint32_t sum[32];
+                        tmem_ld32(taddr + BN + c * 32, sum);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(sum[i]) + __uint_as_float(r[i]));
+                    } else {
+                        tmem_ld_wait();
+                    }
                     last_read(c + 1 == c_end);
+                    if (MODE == MODE_WGRAD && piece + 1 < pieces) {
+                        tmem_st32(taddr + BN + c * 32, r);
+                        tmem_st_wait();
+                        continue;
+                    }
                     const int valid = p.N - (tile.n0 + c * 32);
                     if (valid >= 32) {
                         store_block32_f32(stage, lane, r, Cw + c * 32, p.ldc, (long long)p.M - row0w);
@@ -1214,10 +1242,11 @@ int tc_wgrad3(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t h_act, u
 // The weight gradient of a plain linear map (the language-model head), on CTA pairs.  With `groups` > 1 the rows are cut
 // into that many ranges (offsets[g], counts[g]; every offset a multiple of 128; without tables: one group of all rows) and range g leaves its own product in
 // out + g * slab: a short, wide product then fills the machine, and the caller adds the slabs in a fixed order.
+// `sum_rows`: see GemmParams (without tables only).
 int tc_wgrad1(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t out, long long M, long long N, cudaStream_t stream,
-              int groups, long long slab) {
+              int groups, long long slab, int sum_rows) {
     GemmParams p = {};
-    if (!r->offsets) p.plain_rows = (int)r->rows_bound;
+    if (!r->offsets) { p.plain_rows = (int)r->rows_bound; p.sum_rows = sum_rows; }
     if (out & 15u || (N * 4) % 16) return fail_arg("weight-gradient output must be 16-byte aligned with a 16-byte row pitch");
     const int ctas = gemm_ctas();
     const uint64_t rows = (uint64_t)r->rows_bound;

@@ -175,15 +175,26 @@ qmoe_route_t one_group_route(long long rows) {
     r.rows_bound = rows;
     return r;
 }
+
+// Weight gradients whose k is no multiple of 8 run on the CUDA cores' FMA chains where they are short, and from here on in
+// pieces on the tensor cores that are added in fp32.  Tensor memory drops the low bits of what is added to it, so the error of
+// one long product grows with k, that of an FMA chain with its root (2-norm, from the exact product: 602 rows 5.7e-7 in one
+// product, 1.8e-7 in a chain; 8191 rows 9.1e-6 and 9.6e-7); an eighth of k, between 64 and 512 rows, keeps the sum below the chain's.
+constexpr long long kRaggedContraction = 128;
+int ragged_sum_rows(long long k) {
+    const long long rows = (k / 8 + 63) / 64 * 64;
+    return (int)(rows < 64 ? 64 : rows > 512 ? 512 : rows);
+}
 }  // namespace
 }  // namespace qmoe
 
 // Plain product.  bf16 x bf16 in the three forms a linear layer needs goes to the tcgen05 kernels (A [M, K] . B[N, K]^T and
 // A [M, K] . B [K, N] with bf16 results; A [K, M]^T . B [K, N] with fp32 results: a weight gradient); everything else, and
 // every accumulating call, to the CUDA-core kernel.  The rows of the batch (M >= 128, one tile, of the first two; K of the
-// third) need be no multiple of anything: TMA fills the last tile with zeros and its rows past the end are not stored.
+// third, from kRaggedContraction on) need be no multiple of anything: TMA fills the last tile with zeros and its rows past the
+// end are not stored.
 // What must be a multiple of 8 is what a row pitch is made of (16 bytes): K and N of the first two, M and N of the third.
-// 602 rows, 512 x 512: 40 us on the CUDA cores (58 for the weight gradient), 10 .. 14 here.
+// 602 rows, 512 x 512: 40 us on the CUDA cores (74 for the weight gradient), 10 .. 14 here (21).
 extern "C" int qmoe_gemm(uint64_t a, int32_t a_dtype, uint64_t b, int32_t b_dtype, uint64_t c, int32_t c_dtype, int64_t m,
                          int64_t k, int64_t n, int32_t transpose_a, int32_t transpose_b, int32_t accumulate, uint64_t stream_) {
     if (!a || !b || !c) return fail_arg("gemm: null address");
@@ -199,10 +210,10 @@ extern "C" int qmoe_gemm(uint64_t a, int32_t a_dtype, uint64_t b, int32_t b_dtyp
             const qmoe_route_t r = one_group_route(m);
             return transpose_b ? tc_rows_nt(&r, 1, a, b, c, k, n, stream, nullptr, m) : tc_rows_nn(&r, 1, a, b, 0, 0, c, k, n, stream, nullptr, m);
         }
-        if (transpose_a && !transpose_b && c_dtype == QMOE_F32) {
+        if (transpose_a && !transpose_b && c_dtype == QMOE_F32 && (k % 8 == 0 || k >= kRaggedContraction)) {
             TimedScope timed(KC_WGRAD_GEMM, stream);
             const qmoe_route_t r = one_group_route(k);     // the contraction runs over the k rows of both operands
-            return tc_wgrad1(&r, a, b, c, m, n, stream);
+            return tc_wgrad1(&r, a, b, c, m, n, stream, 1, 0, k % 8 ? ragged_sum_rows(k) : 0);
         }
     }
     TimedScope timed(KC_OTHER, stream);

@@ -290,3 +290,46 @@ def test_float32_gemm_in_every_orientation(m, k, n, ta, tb):
     a64, b64 = (a.T if ta else a).astype(np.float64), (b.T if tb else b).astype(np.float64)
     bound = k * 2.0 ** -24 * (np.abs(a64) @ np.abs(b64)) * 1.01
     assert np.all(np.abs(got - a64 @ b64) <= bound)
+
+
+@pytest.mark.parametrize("rows,cols_out,cols_in", [(129, 64, 72), (301, 264, 512), (602, 512, 136), (1001, 1024, 264), (4503, 128, 256)])
+def test_ragged_weight_gradients_are_as_exact_as_an_fma_chain(rows, cols_out, cols_in, kernel_variant):
+    """bf16 operands, fp32 result, a row count that is no multiple of 8: the tensor cores take the rows in pieces that are added
+    in fp32, and the result is no further from the exact product than the CUDA cores' chain of fp32 FMAs.  Two pieces, pieces of
+    every length from 64 to 512 rows, and ragged last ones; with terms of both signs and of one sign."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(rows)
+    count = lib.load().qmoe_tensor_core_launch_count
+
+    def error(g, x, launches):
+        gs, xs, out, before = to_device(g, "bfloat16"), to_device(x, "bfloat16"), DeviceStorage(cols_out * cols_in, "float32"), count()
+        lib.call("qmoe_gemm", gs.ptr, lib.QMOE_BF16, xs.ptr, lib.QMOE_BF16, out.ptr, lib.QMOE_F32, cols_out, rows, cols_in, 1, 0, 0, 0)
+        exact = g.astype(np.float64).T @ x.astype(np.float64)
+        difference = np.linalg.norm(to_host(out, exact.shape) - exact) / np.linalg.norm(exact)
+        assert count() - before == launches and lib.device_status() == 0
+        return difference
+
+    operands = [oracle.round_bf16(rng.standard_normal((rows, n))) for n in (cols_out, cols_in)]
+    both_signs, one_sign = operands, [np.abs(a) for a in operands]
+    pieces = [error(*o, 1) for o in (both_signs, one_sign)]
+    kernel_variant(lib.VARIANT_PLAIN_GEMM_ON_CUDA_CORES)
+    for got, chain in zip(pieces, (error(*o, 0) for o in (both_signs, one_sign))):
+        assert got <= chain
+
+
+@pytest.mark.parametrize("rows", [1, 7, 127])
+def test_short_ragged_weight_gradients_stay_on_the_cuda_cores(rows):
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(rows)
+    g, x = (oracle.round_bf16(rng.standard_normal((rows, n))) for n in (64, 72))
+    gs, xs, out, before = to_device(g, "bfloat16"), to_device(x, "bfloat16"), DeviceStorage(64 * 72, "float32"), lib.load().qmoe_tensor_core_launch_count()
+    lib.call("qmoe_gemm", gs.ptr, lib.QMOE_BF16, xs.ptr, lib.QMOE_BF16, out.ptr, lib.QMOE_F32, 64, rows, 72, 1, 0, 0, 0)
+    assert lib.load().qmoe_tensor_core_launch_count() == before
+    g64, x64 = g.astype(np.float64), x.astype(np.float64)
+    assert np.all(np.abs(to_host(out, (64, 72)) - g64.T @ x64) <= rows * 2.0 ** -24 * (np.abs(g64).T @ np.abs(x64)) * 1.01)
