@@ -328,11 +328,11 @@ namespace {
 // The tokens of the router's weight gradient are cut into ranges that run side by side and are added in a fixed order: an
 // [experts, width] product has few tiles (8 experts of width 512: 8 of them, 251 us for 2048 tokens in one range, 18 in 16).
 constexpr long long kRouterSplitTokens = 128, kRouterMaxSplits = 32;
-long long router_split_tokens(long long tokens) {
-    long long splits = (tokens + kRouterSplitTokens - 1) / kRouterSplitTokens;
-    if (splits > kRouterMaxSplits) splits = kRouterMaxSplits;
-    return (tokens + splits - 1) / splits;
+long long router_splits(long long tokens) {    // at most this many; never fewer for more tokens
+    const long long splits = (tokens + kRouterSplitTokens - 1) / kRouterSplitTokens;
+    return splits > kRouterMaxSplits ? kRouterMaxSplits : splits;
 }
+long long router_split_tokens(long long tokens) { return (tokens + router_splits(tokens) - 1) / router_splits(tokens); }
 }
 
 int simt_router_logits(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t scores, int64_t tokens, int64_t width,
@@ -349,8 +349,7 @@ int simt_router_logits(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t 
 }
 
 long long simt_router_partials(int64_t tokens, int32_t experts, int64_t width) {
-    const int64_t per_split = router_split_tokens(tokens);
-    return (tokens + per_split - 1) / per_split * experts * width;
+    return router_splits(tokens) * experts * width;
 }
 
 int simt_router_backward(uint64_t d_scores, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,

@@ -35,14 +35,16 @@ RouterScratch plan_scratch(long long T, int E, long long d) {
     if (splits < T / 1024) splits = T / 1024;
     if (splits < 1) splits = 1;
     if (splits > 32) splits = 32;
+    const long long room = splits;     // sizes that never shrink as T grows: rounded to whole tiles, fewer ranges may be enough (3840
+                                       // tokens 15, 4095 tokens 11), and a scratch made for the most tokens serves fewer
     r.rows_per_split = ((T + splits - 1) / splits + kRowPad - 1) / kRowPad * kRowPad;
     r.splits = (int)((T + r.rows_per_split - 1) / r.rows_per_split);
     long long at = 0;
     r.w3 = at;      at = align_up(at + 3ll * r.S * d * 2);
     r.wbwd = at;    at = align_up(at + 6ll * r.S * d * 2);
     r.ds6 = at;     at = align_up(at + T * 6ll * r.S * 2);
-    r.tables = at;  at = align_up(at + (2ll * r.splits + 1) * 4);
-    r.partial = at; at = align_up(at + (long long)r.splits * 3 * r.S * d * 4);
+    r.tables = at;  at = align_up(at + (2ll * room + 1) * 4);
+    r.partial = at; at = align_up(at + room * 3 * r.S * d * 4);
     r.total = at;
     return r;
 }
@@ -197,6 +199,7 @@ int elem_grid(long long n) {
 using namespace qmoe;
 
 extern "C" int64_t qmoe_router_scratch_bytes(int64_t tokens, int32_t experts, int64_t width) {
+    if (tokens <= 0 || experts <= 0 || width <= 0) return 0;
     const long long simt = simt_router_partials(tokens, experts, width) * 4;
     const long long tc = plan_scratch(tokens, experts, width).total;
     return simt > tc ? simt : tc;

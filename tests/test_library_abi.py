@@ -45,6 +45,15 @@ def test_size_helpers_need_no_device(library_path):
     assert int(lib.load().qmoe_router_grad_partials(4096, 8, 1024)) * 4 >= scratch
 
 
+@pytest.mark.parametrize("experts,width", [(1, 64), (8, 512), (16, 1024), (64, 2048), (256, 128)])
+def test_router_scratch_never_shrinks_with_more_tokens(library_path, experts, width):
+    """A buffer made for the largest batch has to serve every smaller one."""
+    size = lib.load().qmoe_router_scratch_bytes
+    sizes = [int(size(tokens, experts, width)) for tokens in [*range(1, 6000), *range(6000, 70000, 127)]]
+    assert sizes == sorted(sizes)
+    assert size(0, experts, width) == size(-1, experts, width) == size(1, 0, width) == 0
+
+
 def test_ctypes_structures_match_the_c_layout(tmp_path):
     source = tmp_path / "layout.c"
     fields = {"qmoe_route_t": [f[0] for f in lib.Route._fields_],
