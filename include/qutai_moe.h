@@ -403,6 +403,7 @@ typedef struct qmoe_block {
     uint64_t d_norm_weight;    /* f32 [d]      backward output */
     uint64_t norm_partials;    /* f32 [qmoe_norm_backward_partials(T, d)] scratch */
     double norm_eps;
+    /* After the backward layer.d_scores holds inverse[t] * (gradient of the logits), in either dtype. */
 } qmoe_block_t;
 int qmoe_block_forward(const qmoe_block_t* block, uint64_t stream);
 int qmoe_block_backward(const qmoe_block_t* block, uint64_t stream);

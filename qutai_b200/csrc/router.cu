@@ -75,9 +75,10 @@ router_split_w_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ w
     }
 }
 
-// ds [T, E] fp32 (times row_scale[t], when given) -> ds6 [T, 6S] = {hi | mid | lo | hi | mid | 0}; also the token-block tables of the split contraction
+// ds [T, E] fp32 (first multiplied by row_scale[t] in place, when given) -> ds6 [T, 6S] = {hi | mid | lo | hi | mid | 0}; also the
+// token-block tables of the split contraction
 __global__ void __launch_bounds__(256)
-router_split_ds_kernel(const float* __restrict__ ds, const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S,
+router_split_ds_kernel(float* __restrict__ ds, const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S,
                        int* __restrict__ tables, int splits, long long rows_per_split) {
     if (blockIdx.x == 0 && threadIdx.x <= splits) {
         const int i = threadIdx.x;
@@ -93,8 +94,12 @@ router_split_ds_kernel(const float* __restrict__ ds, const float* __restrict__ r
         const long long t = i / S;
         const int e = (int)(i - t * S);
         __nv_bfloat16 hi, mid, lo;
-        const float scale = row_scale ? row_scale[t] : 1.f;
-        split3(e < E ? ds[t * E + e] * scale : 0.f, hi, mid, lo);
+        float value = e < E ? ds[t * E + e] : 0.f;
+        if (row_scale && e < E) {
+            value *= row_scale[t];
+            ds[t * E + e] = value;      // no other thread has this element
+        }
+        split3(value, hi, mid, lo);
         __nv_bfloat16* row = ds6 + t * 6 * S;
         row[e] = hi; row[S + e] = mid; row[2 * S + e] = lo; row[3 * S + e] = hi; row[4 * S + e] = mid; row[5 * S + e] = zero;
     }
@@ -267,9 +272,8 @@ extern "C" int qmoe_router_backward(uint64_t d_scores, uint64_t x, int32_t x_dty
     return router_backward_scaled(d_scores, 0, x, x_dtype, w_router, dx_router, d_w_router, 0, scratch, tokens, width, experts, stream);
 }
 
-// The same for d_scores[t, :] * row_scale[t], with the weight gradient's columns multiplied by col_scale (0: neither).  The
-// scales ride along where the factors are split and the ranges are summed; d_scores itself may or may not hold the scaled
-// values afterwards.
+// The same for d_scores[t, :] * row_scale[t], which d_scores holds afterwards, with the weight gradient's columns multiplied by
+// col_scale (0: neither).  The scales ride along where the factors are split and the ranges are summed.
 int qmoe::router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,
                                  uint64_t d_w_router, uint64_t col_scale, uint64_t scratch, int64_t tokens, int64_t width, int32_t experts,
                                  uint64_t stream_) {
@@ -291,7 +295,7 @@ int qmoe::router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t
     router_split_w_kernel<<<elem_grid((long long)S * width), 256, 0, stream>>>(
         (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, S, width);
     QMOE_LAUNCH_CHECK("router_split_w_kernel");
-    router_split_ds_kernel<<<elem_grid(tokens * S), 256, 0, stream>>>((const float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6),
+    router_split_ds_kernel<<<elem_grid(tokens * S), 256, 0, stream>>>((float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6),
                                                                       tokens, experts, S, tables, r.splits, r.rows_per_split);
     QMOE_LAUNCH_CHECK("router_split_ds_kernel");
     if (dx_router)

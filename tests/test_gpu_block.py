@@ -161,3 +161,27 @@ def test_fused_block_agrees_with_the_unfused_chain_at_full_size():
     assert rel(got["d_norm_weight"], d_weight) <= BF16_TOL
     assert rel(got["dx"][routed_alike], (grad_out.astype(np.float64) + dx_norm)[routed_alike]) <= BF16_TOL
     assert lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype,E", [("bfloat16", 8), ("bfloat16", 40), ("float32", 8)])
+def test_block_backward_leaves_the_scaled_logit_gradients(dtype, E):
+    """``d_scores`` after the backward: the gradient of the logits times the row's inverse rms, on the tensor cores' route and on
+    the CUDA cores' alike, bit for bit (one fp32 product)."""
+    import ctypes
+
+    from gpu_util import to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    T, d, k, h = 150, 128, 2, 64
+    rng = np.random.default_rng(E)
+    x, grad = (oracle.round_bf16(rng.standard_normal((T, d))) for _ in range(2))
+    gate, up = (rng.standard_normal((E, h, d)).astype(np.float32) * 0.1 for _ in range(2))
+    down = rng.standard_normal((E, d, h)).astype(np.float32) * 0.1
+    block = make_block(1.0 + 0.1 * rng.standard_normal(d), 1e-6, rng.standard_normal((E, d)).astype(np.float32) * 0.1, gate, up, down, k)
+    run_block(block, x, grad, None, dtype)
+    work = block.ffn._saved[0]
+    plain = DeviceStorage(T * E, "float32")
+    lib.call("qmoe_route_backward", ctypes.byref(work["layer"].route), work["buf"]["d_gate_weights"].ptr, 0, plain.ptr, 0)
+    inverse = to_host(block._blocks[id(work)]["extra"]["inverse"], (T, 1)).astype(np.float32)
+    assert np.array_equal(to_host(work["buf"]["d_scores"], (T, E)), to_host(plain, (T, E)).astype(np.float32) * inverse)
