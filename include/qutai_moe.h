@@ -27,9 +27,8 @@
  * to expert 0, then expert 1, ...; inside one expert rows keep increasing (token, slot) order —
  * the order of the upstream `ids`/`slots` lists (src/qutai/backends/cpu_lm.py:204-221,
  * src/qutai/backends/cuda/lm.cu:353-383) — and each expert group starts at a multiple of
- * QMOE_ROW_PAD rows; the pad rows hold zeros (in the buffers that a whole-layer or whole-block call
- * fills for itself only those up to the next multiple of 16 rows may be relied on).  A buffer in
- * that layout has qmoe_rows_bound(T, E, k) rows.
+ * QMOE_ROW_PAD rows; the pad rows hold zeros (unless QMOE_EXPERTS_SHORT_PADS is asked for).  A
+ * buffer in that layout has qmoe_rows_bound(T, E, k) rows.
  */
 #ifndef QUTAI_MOE_H
 #define QUTAI_MOE_H
@@ -233,12 +232,17 @@ int qmoe_combine_backward(const qmoe_route_t* route, uint64_t grad_out, uint64_t
 /* ---------------------------------------------------------------------------------------------
  * Expert FFN (grouped GEMMs)
  * ------------------------------------------------------------------------------------------- */
+/* experts.reserved: qmoe_layer_forward and qmoe_block_forward may leave the pad rows of x_dispatched, g, u, h and
+ * y_dispatched past an expert's next multiple of 16 rows unwritten (and the backward those of d_g, d_u, dx_dispatched with
+ * any value).  For callers that keep these buffers to themselves and read only the rows of `row_source`: with few rows
+ * per expert the other pad rows are a tenth of the bytes that a forward moves. */
+#define QMOE_EXPERTS_SHORT_PADS 0x5350
 typedef struct qmoe_experts {
     int32_t experts;   /* E */
     int32_t dtype;     /* activation dtype: QMOE_BF16 -> bf16 operands, fp32 accumulate (tcgen05);
                           QMOE_F32 -> fp32 everywhere (CUDA cores) */
     int32_t engine;    /* QMOE_ENGINE_* ; AUTO = tcgen05 whenever dtype is bf16 and d, h are multiples of 8 */
-    int32_t reserved;
+    int32_t reserved;  /* 0, or QMOE_EXPERTS_SHORT_PADS */
     int64_t width;     /* d */
     int64_t hidden;    /* h */
     /* stacked expert weights in the OPERAND dtype (bf16 shadows for QMOE_BF16, the fp32 masters

@@ -299,11 +299,11 @@ extern "C" int qmoe_gemm_wgrad_split(uint64_t a, uint64_t b, uint64_t c, uint64_
     return 0;
 }
 
-// Inside the layer the pad rows of few-row experts hold zeros only up to a multiple of 16 rows, which is as far as any of the
-// layer's products reaches (the weight gradients; everything else works row by row): at 64 tokens over 64 experts the
-// other pad rows of x, G, U, H and y are 135 MB of zeros beside 1.1 GB of weights.
+// Where the caller allows it, the pad rows of few-row experts hold zeros only up to a multiple of 16 rows, which is as far as
+// any of the layer's products reaches (the weight gradients; everything else works row by row): at 64 tokens over 64 experts
+// the other pad rows of x, G, U, H and y are 135 MB of zeros beside 1.1 GB of weights (247 us with them, 229 without).
 static int layer_pad(const qmoe_route_t* r, const qmoe_experts_t* ex, int engine) {
-    return engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex->experts) ? kStreamPad : kRowPad;
+    return ex->reserved == QMOE_EXPERTS_SHORT_PADS && engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex->experts) ? kStreamPad : kRowPad;
 }
 
 extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
@@ -323,8 +323,10 @@ extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
     }
     if (int rc = qmoe_router_forward(L->x, ex->dtype, L->w_router, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
-    if (int rc = launch_permute(r, L->x, L->x_dispatched, ex->dtype, d, layer_pad(r, ex, engine), stream)) return rc;
-    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, false, stream)) return rc;
+    const int pad = layer_pad(r, ex, engine);
+    if (int rc = launch_permute(r, L->x, L->x_dispatched, ex->dtype, d, pad, stream)) return rc;
+    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, stream))
+        return rc;
     return qmoe_combine(r, L->y_dispatched, L->out, ex->dtype, d, stream);
 }
 
@@ -385,8 +387,10 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
         if (int rc = qmoe_scale_f32(L->scores, L->scores, B->inverse, 0, r->tokens, E, stream)) return rc;
     }
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
-    if (int rc = launch_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, layer_pad(r, ex, engine), stream)) return rc;
-    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, false, stream)) return rc;
+    const int pad = layer_pad(r, ex, engine);
+    if (int rc = launch_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, pad, stream)) return rc;
+    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, stream))
+        return rc;
     return qmoe_combine_residual(r, L->y_dispatched, L->x, L->out, ex->dtype, d, stream);
 }
 

@@ -230,6 +230,7 @@ class SparseMoE:
             setattr(route, name, buf[name].ptr)
         ex = layer.experts
         ex.experts, ex.dtype, ex.engine, ex.width, ex.hidden = E, lib.DTYPE_CODES[dtype], self.engine, d, h
+        ex.reserved = lib.EXPERTS_SHORT_PADS      # the dispatched buffers are this workspace's own
         if dtype == "bfloat16":
             ex.w_gate, ex.w_up, ex.w_down = buf["w_gate"].ptr, buf["w_up"].ptr, buf["w_down"].ptr
             layer.master_gate, layer.master_up, layer.master_down = self._gate.ptr, self._up.ptr, self._down.ptr

@@ -101,3 +101,39 @@ def test_a_layer_of_few_rows_reads_no_pad_row_it_did_not_write():
     for name in ("d_gate", "d_up", "d_down"):
         for a, b in zip(first[name], again[name]):
             assert (a is None and b is None) or np.array_equal(a, b), name
+
+
+@pytest.mark.parametrize("with_norm", [False, True])
+def test_layer_calls_fill_every_pad_row_unless_asked_not_to(with_norm):
+    """The dispatched buffers of a whole-layer (whole-block) call, full of NaN beforehand: every pad row is zero afterwards, as the
+    layout promises, for a caller that has not set ``EXPERTS_SHORT_PADS``; one that has gets the same output."""
+    import ctypes
+
+    from gpu_util import make_layer, to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.layers import MoEFeedForward, RMSNorm, Tensor
+
+    T, d, E, k, h = 70, 136, 6, 2, 264
+    rng = np.random.default_rng(6)
+    x = Tensor(to_device(rng.standard_normal((T, d)), "bfloat16"), (T, d))
+    router = rng.standard_normal((E, d)).astype(np.float32) * 0.05
+    gate, up = (rng.standard_normal((E, h, d)).astype(np.float32) / np.sqrt(d) for _ in range(2))
+    down = rng.standard_normal((E, d, h)).astype(np.float32) / np.sqrt(h)
+    layer = make_layer((T, d), router, gate, up, down, k, engine="tcgen05")
+    call = MoEFeedForward(RMSNorm(d, 1e-6), layer) if with_norm else layer
+    out, _ = call.forward(x)
+    work = layer._saved[0]
+    buf, struct = work["buf"], call._blocks[id(work)]["struct"] if with_norm else work["layer"]
+    experts = struct.layer.experts if with_norm else struct.experts
+    assert experts.reserved == lib.EXPERTS_SHORT_PADS
+    first, experts.reserved = out.storage.tobytes(), 0
+    names = ("x_dispatched", "g", "u", "h", "y_dispatched")
+    for name in names:
+        lib.call("qmoe_memset", buf[name].ptr, 0xFF, buf[name].nbytes, 0)
+    lib.call("qmoe_block_forward" if with_norm else "qmoe_layer_forward", ctypes.byref(struct), 0)
+    assert out.storage.tobytes() == first and lib.device_status() == 0
+    used = int(to_host(buf["offsets"])[E])
+    pads = to_host(buf["row_source"])[:used] < 0
+    for name in names:
+        rows = to_host(buf[name], (work["rows_bound"], -1))[:used]
+        assert np.all(np.isfinite(rows)) and not np.any(rows[pads]), name
