@@ -86,13 +86,13 @@ template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, const float* __restrict__ weight,
                     T* __restrict__ out, const int* __restrict__ dest_row, const int* __restrict__ offsets,
-                    const int* __restrict__ counts, int experts, int pad, long long tokens, int k, long long width, int parts) {
+                    const int* __restrict__ counts, int experts, int pad_bits, long long tokens, int k, long long width, int part_bits) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long i = warp; i < tokens * parts; i += nwarps) {
-        const long long t = i / parts;
-        const int mine = lane + 32 * (int)(i - t * parts), step = 32 * parts;     // this warp's pieces of the row: mine, mine + step, ...
+    for (long long i = warp; i < tokens << part_bits; i += nwarps) {
+        const long long t = i >> part_bits;
+        const int step = 32 << part_bits, mine = lane + (int)(32 * i & (step - 1));     // this warp's pieces of the row: mine, mine + step, ...
         long long rows[KMAX];
 #pragma unroll
         for (int s = 0; s < KMAX; ++s) rows[s] = s < k ? dest_row[t * k + s] : 0;
@@ -119,20 +119,20 @@ permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, 
             }
         }
     }
-    zero_pad_rows<T, VEC>(out, offsets, counts, experts, pad, width, warp, nwarps);
+    zero_pad_rows<T, VEC>(out, offsets, counts, experts, pad_bits, width, (int)warp, (int)nwarps);
 }
 
 // out[t] = round(residual[t] + sum_s w[t, s] * y[dest_row[t, s]]): fp32 sum, one rounding
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 combine_residual_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const int* __restrict__ dest_row,
-                        const T* __restrict__ residual, T* __restrict__ out, long long tokens, int k, long long width, int parts) {
+                        const T* __restrict__ residual, T* __restrict__ out, long long tokens, int k, long long width, int part_bits) {
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long i = warp; i < tokens * parts; i += nwarps) {
-        const long long t = i / parts;
-        const int mine = lane + 32 * (int)(i - t * parts), step = 32 * parts;     // this warp's pieces of the row: mine, mine + step, ...
+    for (long long i = warp; i < tokens << part_bits; i += nwarps) {
+        const long long t = i >> part_bits;
+        const int step = 32 << part_bits, mine = lane + (int)(32 * i & (step - 1));     // this warp's pieces of the row: mine, mine + step, ...
         int rows[KMAX];
         float w[KMAX];
 #pragma unroll
@@ -398,11 +398,12 @@ int qmoe::launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t invers
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_PERMUTE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {x, out, norm_weight}) : can_vec<float>(width, {x, out, norm_weight});
-    const int parts = parts_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
-    const long long warps = r->tokens * parts;
+    const int part_bits = part_bits_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
+    const long long warps = r->tokens << part_bits;
+    const int pad_bits = pad == kRowPad ? 7 : 4;
     const int grid = grid_for_rows(warps > (long long)r->experts * pad / 2 ? warps : (long long)r->experts * pad / 2, 8);
 #define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (const float*)inverse, (const float*)norm_weight, (T*)out,       \
-        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad, (long long)r->tokens, r->top_k, (long long)width, parts)
+        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits)
     if (dtype == QMOE_BF16) { if (vec) BY_K(permute_norm_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(permute_norm_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(permute_norm_kernel, float, true, ARGS(float)); else BY_K(permute_norm_kernel, float, false, ARGS(float)); }
 #undef ARGS
@@ -418,10 +419,10 @@ extern "C" int qmoe_combine_residual(const qmoe_route_t* r, uint64_t y, uint64_t
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_COMBINE, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {y, residual, out}) : can_vec<float>(width, {y, residual, out});
-    const int parts = parts_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
-    const int grid = grid_for_rows(r->tokens * parts, 8);
+    const int part_bits = part_bits_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
+    const int grid = grid_for_rows(r->tokens << part_bits, 8);
 #define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row,           \
-        (const T*)residual, (T*)out, (long long)r->tokens, r->top_k, (long long)width, parts)
+        (const T*)residual, (T*)out, (long long)r->tokens, r->top_k, (long long)width, part_bits)
     if (dtype == QMOE_BF16) { if (vec) BY_K(combine_residual_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(combine_residual_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(combine_residual_kernel, float, true, ARGS(float)); else BY_K(combine_residual_kernel, float, false, ARGS(float)); }
 #undef ARGS
