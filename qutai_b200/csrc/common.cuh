@@ -173,7 +173,7 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
 int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream);
 int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t weight, uint64_t out, int32_t dtype, int64_t width, int pad,
                         uint64_t stream);
-bool router_norm_ok(int64_t tokens, int32_t experts, int64_t width);
+bool router_norm_ok(int64_t tokens, int32_t experts, int64_t width, int32_t x_dtype, uint64_t x, uint64_t scratch);
 int router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
                         int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
 int router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,

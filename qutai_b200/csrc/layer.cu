@@ -377,7 +377,7 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
         if (int rc = qmoe_cast_bf16(L->master_down, ex->w_down, E * hd * d, stream)) return rc;
     }
     // scores = rms_norm(x) . W_r^T = inverse[t] * (x . (W_r * w)^T): the product reads the raw activations
-    if (router_norm_ok(r->tokens, r->experts, d)) {
+    if (router_norm_ok(r->tokens, r->experts, d, ex->dtype, L->x, L->router_partials)) {
         if (int rc = router_forward_norm(L->x, ex->dtype, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, r->tokens, d, r->experts, stream))
             return rc;
     } else {

@@ -124,11 +124,21 @@ router_reduce_dw_kernel(const float* __restrict__ partial, const float* __restri
 // Few tokens (decode): one block per token, a warp per expert in turn, fp32 dot products with the lanes
 // striding over the width and a fixed shuffle tree, so the logits are run-to-run identical.  A tile kernel
 // would put the whole product on one or two SMs and walk the width serially.
-// The warps of a token read every weight row again, from L2: up to 512 tokens that is the shorter way whatever the sizes, and
-// beyond them while it is at most 64 MB (602 tokens, 8 experts, d 512, with the norm: 4 us in one launch, 15 in five).
+// The warps of a token read every weight row again, from L2: up to 512 tokens that is the shorter way whatever the sizes (602
+// tokens, 8 experts, d 512, with the norm: 4 us in one launch, 15 in five).  Beyond them by an estimate of both ways, in us beyond
+// what a launch takes, fitted to 600 .. 65536 tokens, 1 .. 128 experts, widths 64 .. 4096 with L2 flushed: this kernel takes a
+// block's issue per 8 logits (16384 x 16 x 64: 46 us) or the weight reads (32768 x 16 x 2048: 293); three times that when the
+// width is no multiple of 4, half as much again with the norm; the tile kernel a chain of `width` products per tile until its
+// tiles fill the machine (16 and 212); the tensor cores two launches and little else (bf16, 16384 x 16 x 64: 13, against 50 here).
 constexpr long long kSmallRouterTokens = 512, kSmallRouterProducts = 1ll << 24;
-bool small_router(long long tokens, int experts, long long width) {
-    return tokens <= kSmallRouterTokens || tokens * experts * width <= kSmallRouterProducts;
+bool small_router(long long tokens, int experts, long long width, int x_dtype, bool tensor_cores, bool norm) {
+    if (tokens <= kSmallRouterTokens) return true;
+    if (tokens * experts * width > kSmallRouterProducts && !(x_dtype == QMOE_F32 && experts <= 16)) return false;
+    const double T = (double)tokens, d = (double)width;
+    const double blocks = T * (4.5e-4 * ((experts + 7) / 8) + 1e-4 * experts), reads = T * experts * (3e-5 + 2.7e-7 * d);
+    const double here = (blocks > reads ? blocks : reads) * (width % 4 ? 3 : 1) * (norm ? 1.5 : 1);
+    const double there = tensor_cores ? 6 + 5.6e-3 * d + 6e-7 * T * d : 7.5e-2 * d * (T > 30000 ? T / 30000 : 1);
+    return here <= there + (norm ? 9 : 0);     // with the norm: three launches more
 }
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
@@ -220,8 +230,8 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
     if (tokens <= 0 || width <= 0 || experts <= 0) return fail_arg("router_forward: sizes must be positive");
     if (x_dtype != QMOE_F32 && x_dtype != QMOE_BF16) return fail_arg("router_forward: bad dtype %d", x_dtype);
     cudaStream_t stream = (cudaStream_t)stream_;
-    // fp32 rows over up to 16 experts: the tile kernel's 128 x 16 tiles take 31 us for 2048 tokens of width 512 over 8, this 5
-    if (small_router(tokens, experts, width) || (x_dtype == QMOE_F32 && experts <= 16)) {
+    const bool tensor_cores = tc_router_ok(x_dtype, experts, width, x, scratch);
+    if (small_router(tokens, experts, width, x_dtype, tensor_cores, false)) {
         TimedScope timed(KC_ROUTER_GEMM, stream);
         const dim3 grid((unsigned)tokens, (unsigned)((experts + 7) / 8));
         if (x_dtype == QMOE_BF16)
@@ -233,7 +243,7 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
         QMOE_LAUNCH_CHECK("router_small_kernel");
         return 0;
     }
-    if (!tc_router_ok(x_dtype, experts, width, x, scratch))
+    if (!tensor_cores)
         return simt_router_logits(x, x_dtype, w_router, scores, tokens, width, experts, stream);
     TimedScope timed(KC_ROUTER_GEMM, stream);
     const RouterScratch r = plan_scratch(tokens, experts, width);
@@ -243,7 +253,9 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
     return tc_router_forward(x, scratch + r.w3, scores, tokens, width, experts, r.S, stream);
 }
 
-bool qmoe::router_norm_ok(int64_t tokens, int32_t experts, int64_t width) { return small_router(tokens, experts, width); }
+bool qmoe::router_norm_ok(int64_t tokens, int32_t experts, int64_t width, int32_t x_dtype, uint64_t x, uint64_t scratch) {
+    return small_router(tokens, experts, width, x_dtype, tc_router_ok(x_dtype, experts, width, x, scratch), true);
+}
 
 // inverse[t] and the logits of the normalised rows in one launch (tokens within router_norm_ok)
 int qmoe::router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,

@@ -438,6 +438,24 @@ def test_router_forward_backward_fp32_semantics(T, d, E, dtype):
     assert lib.device_status() == 0
 
 
+@pytest.mark.parametrize("T,d,E,tensor_cores", [(512, 64, 64, 0), (513, 512, 8, 0), (2048, 64, 64, 1), (16384, 64, 16, 1), (4096, 256, 8, 0)])
+def test_router_logits_of_many_tokens_leave_the_kernel_for_few(T, d, E, tensor_cores):
+    """bf16 logits beyond 512 tokens take the kernel with a warp per logit only where that is the shorter way; both sides of the
+    line are exact to fp32 sums."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(T + E)
+    x, w = oracle.round_bf16(rng.standard_normal((T, d))), (rng.standard_normal((E, d)) * 0.05).astype(np.float32)
+    xd, wd, scores = to_device(x, "bfloat16"), to_device(w, "float32"), DeviceStorage(T * E, "float32")
+    scratch = DeviceStorage(int(lib.load().qmoe_router_scratch_bytes(T, E, d)) // 4 + 64, "float32")
+    before = lib.load().qmoe_tensor_core_launch_count()
+    lib.call("qmoe_router_forward", xd.ptr, lib.QMOE_BF16, wd.ptr, scores.ptr, scratch.ptr, T, d, E, 0)
+    assert lib.load().qmoe_tensor_core_launch_count() - before == tensor_cores
+    assert rel(to_host(scores, (T, E)), x @ w.astype(np.float64).T) <= 1e-5
+
+
 def test_launch_variants_of_the_weight_gradients_agree_bit_for_bit(kernel_variant):
     """One launch for the three weight gradients (default) against one launch each (the comparison form of
     ``qmoe_test_select_variant``): the same tiles in a different order give the same bits."""
