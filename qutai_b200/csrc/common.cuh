@@ -196,7 +196,7 @@ int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
 // the same two forward products for few rows per expert (gemm_stream.cu)
 // pad_rows: every pad row holds zeros afterwards; else (QMOE_EXPERTS_SHORT_PADS) only those up to a multiple of kStreamPad rows of each expert
 constexpr int kStreamPad = 16;
-bool stream_shape_ok(const qmoe_route_t* r, int experts);
+bool stream_shape_ok(const qmoe_route_t* r, const qmoe_experts_t* ex);
 int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows,
                           cudaStream_t stream);
 int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows,

@@ -4,8 +4,8 @@
 //
 // The kernel for many rows (gemm_tcgen05.cu) gives every expert tiles of 256 rows: an expert with six rows still costs
 // the tensor time of 256 and stages 128 rows of activations beside every 128 rows of weights.  Here both follow the
-// expert's own row count, and what bounds a product is HBM: 128 KiB of weight tiles in flight per SM.  64 rows over 64 experts,
-// top 6, 2048 x 1408: SwiGLU 144 -> 113 us (738 MB: 6.5 TB/s), down product 72 -> 60.
+// expert's own row count, and what bounds a product is HBM: 96 KiB of weight tiles in flight per SM (STREAM_NT), 128 KiB in
+// the other two.  64 rows over 64 experts, top 6, 2048 x 1408: SwiGLU 144 -> 113 us (738 MB: 6.5 TB/s), down product 72 -> 60.
 //
 // One persistent CTA per SM, 6 warps: warp 0 asks TMA for the tiles, warp 1 issues the MMAs, warps 2-5 convert the
 // accumulators (lane = output column, TMEM column = row of the expert) and store them; two accumulator sets, so a
@@ -251,10 +251,20 @@ int stream_launch(const StreamParams& p, cudaStream_t stream) {
 
 // Few rows per expert, on average.  SwiGLU and down product together, here against the kernel for many rows (us, L2 flushed):
 // 32 experts, 2048 x 1408: 136 / 146 at 16 rows, 143 / 145 at 96, 159 / 150 at 128; 16 experts, 1024 x 2048: 68 / 78, 71 / 78,
-// 82 / 80; 8 experts, 1024 x 2816: 60 / 68, 66 / 69, 66 / 70.
-constexpr long long kStreamRowsPerExpert = 96;
-bool stream_shape_ok(const qmoe_route_t* r, int experts) {
-    return r->tokens * r->top_k <= kStreamRowsPerExpert * experts && !kernel_variant(QMOE_VARIANT_NO_STREAM_GEMM);
+// 82 / 80; 8 experts, 1024 x 2816: 60 / 68, 66 / 69, 66 / 70.  30 shapes of 4 .. 64 experts at 24 .. 96 rows: 0.65 .. 1.00 of the
+// other's time under uniform load, and 0.70 .. 1.05 with lognormal load (sigma 1).  Two things lose:
+//   * a few tiles with a long contraction each, whose time is what one SM can fetch: the other kernel splits a tile over two (8
+//     experts, 2048 x 264, 24 tiles of gate and up: 39 / 41 at 24 rows, 41 / 39 at 96, with lognormal load 43 / 39; 960 x 320
+//     35 / 37 at every count).  They change over at 24 rows.
+//   * a load that has collapsed onto a few experts, which this side of the launch cannot see: all 6016 rows on one of 64
+//     experts 125 / 98.
+// The mean is of the whole route.  An expert-parallel view counts the tokens of all ranks over its own experts and so
+// changes over earlier than it need, by the number of ranks.
+constexpr long long kStreamRowsPerExpert = 96, kStreamRowsOfFewTiles = 24;
+bool stream_shape_ok(const qmoe_route_t* r, const qmoe_experts_t* ex) {
+    const long long tiles = (long long)ex->experts * ceil_div(ex->hidden, SM_ROWS);
+    const long long rows = tiles * 4 <= sm_count() && ex->width > 1536 ? kStreamRowsOfFewTiles : kStreamRowsPerExpert;
+    return r->tokens * r->top_k <= rows * ex->experts && !kernel_variant(QMOE_VARIANT_NO_STREAM_GEMM);
 }
 
 int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows,

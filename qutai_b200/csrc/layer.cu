@@ -70,7 +70,7 @@ static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
         return fail_arg("expert_forward: null buffer address");
     cudaStream_t stream = (cudaStream_t)stream_;
     const long long d = ex->width, hd = ex->hidden;
-    const bool tc = engine == QMOE_ENGINE_TCGEN05, few_rows = tc && stream_shape_ok(r, ex->experts);
+    const bool tc = engine == QMOE_ENGINE_TCGEN05, few_rows = tc && stream_shape_ok(r, ex);
     if (parts & QMOE_FWD_UP) {
         if (few_rows) {
             TimedScope timed(KC_EXPERT_GEMM, stream);
@@ -303,7 +303,7 @@ extern "C" int qmoe_gemm_wgrad_split(uint64_t a, uint64_t b, uint64_t c, uint64_
 // any of the layer's products reaches (the weight gradients; everything else works row by row): at 64 tokens over 64 experts
 // the other pad rows of x, G, U, H and y are 135 MB of zeros beside 1.1 GB of weights (247 us with them, 229 without).
 static int layer_pad(const qmoe_route_t* r, const qmoe_experts_t* ex, int engine) {
-    return ex->reserved == QMOE_EXPERTS_SHORT_PADS && engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex->experts) ? kStreamPad : kRowPad;
+    return ex->reserved == QMOE_EXPERTS_SHORT_PADS && engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex) ? kStreamPad : kRowPad;
 }
 
 extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
