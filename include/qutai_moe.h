@@ -292,9 +292,10 @@ int qmoe_expert_backward_parts(const qmoe_route_t* route, const qmoe_experts_t* 
  * the arguments (src/qutai/backends/cuda.py:305-362): A is [M, K] ([K, M] when transpose_a),
  * B is [K, N] ([N, K] when transpose_b); dtypes per operand; accumulate adds into C.  Like upstream's
  * dispatcher (:346-355) it picks a kernel by shape and dtype: bf16 x bf16 without accumulate runs on the
- * tcgen05 kernels when the sizes are multiples of 8 and the addresses of 16 bytes — A . B^T and A . B with a
- * bf16 result and M a multiple of 128, A^T . B with an fp32 result (a weight gradient); everything else on
- * the CUDA cores. */
+ * tcgen05 kernels when the addresses and the row pitches are multiples of 16 bytes — A . B^T and A . B with a
+ * bf16 result, N and K multiples of 8, and M a multiple of 128 or (with K >= 64) any number above it; A^T . B with
+ * an fp32 result (a weight gradient), M and N multiples of 8, and K a multiple of 8 or any number from 128 on (then
+ * in pieces that are added in fp32); everything else on the CUDA cores. */
 int qmoe_gemm(uint64_t a, int32_t a_dtype, uint64_t b, int32_t b_dtype, uint64_t c, int32_t c_dtype,
               int64_t m, int64_t k, int64_t n, int32_t transpose_a, int32_t transpose_b,
               int32_t accumulate, uint64_t stream);

@@ -181,6 +181,9 @@ qmoe_route_t one_group_route(long long rows) {
 // one long product grows with k, that of an FMA chain with its root (2-norm, from the exact product: 602 rows 5.7e-7 in one
 // product, 1.8e-7 in a chain; 8191 rows 9.1e-6 and 9.6e-7); an eighth of k, between 64 and 512 rows, keeps the sum below the chain's.
 constexpr long long kRaggedContraction = 128;
+// Ragged rows with an inner size of less than one k-block are the CUDA cores' too: a tensor-core launch takes 9 .. 11 us
+// (L2 flushed) before there is work, 4503 x 32 x 64 9 us there and 11 here, 60001 x 16 x 16 11 and 19; at 64 they are even (4503 x 64 x 64 11 and 11).
+constexpr long long kRaggedInner = 64;
 int ragged_sum_rows(long long k) {
     const long long rows = (k / 8 + 63) / 64 * 64;
     return (int)(rows < 64 ? 64 : rows > 512 ? 512 : rows);
@@ -190,10 +193,10 @@ int ragged_sum_rows(long long k) {
 
 // Plain product.  bf16 x bf16 in the three forms a linear layer needs goes to the tcgen05 kernels (A [M, K] . B[N, K]^T and
 // A [M, K] . B [K, N] with bf16 results; A [K, M]^T . B [K, N] with fp32 results: a weight gradient); everything else, and
-// every accumulating call, to the CUDA-core kernel.  The rows of the batch (M >= 128, one tile, of the first two; K of the
-// third, from kRaggedContraction on) need be no multiple of anything: TMA fills the last tile with zeros and its rows past the
-// end are not stored.
-// What must be a multiple of 8 is what a row pitch is made of (16 bytes): K and N of the first two, M and N of the third.
+// every accumulating call, to the CUDA-core kernel.  The rows of the batch (M, beyond one tile and from K =
+// kRaggedInner on, of the first two; K, from kRaggedContraction on, of the third) need be no multiple of anything: TMA fills the
+// last tile with zeros and its rows past the end are not stored.  What must be a multiple of 8 is what a row pitch is made of (16 bytes): K and N of the
+// first two, M and N of the third.
 // 602 rows, 512 x 512: 40 us on the CUDA cores (74 for the weight gradient), 10 .. 14 here (21).
 extern "C" int qmoe_gemm(uint64_t a, int32_t a_dtype, uint64_t b, int32_t b_dtype, uint64_t c, int32_t c_dtype, int64_t m,
                          int64_t k, int64_t n, int32_t transpose_a, int32_t transpose_b, int32_t accumulate, uint64_t stream_) {
@@ -205,7 +208,7 @@ extern "C" int qmoe_gemm(uint64_t a, int32_t a_dtype, uint64_t b, int32_t b_dtyp
     cudaStream_t stream = (cudaStream_t)stream_;
     const bool aligned = !((a | b | c) & 15u) && n % 8 == 0 && (transpose_a ? m : k) % 8 == 0 && m < (1ll << 30) && k < (1ll << 30) && n < (1ll << 30);
     if (a_dtype == QMOE_BF16 && b_dtype == QMOE_BF16 && aligned && !accumulate && !kernel_variant(QMOE_VARIANT_PLAIN_GEMM_ON_CUDA_CORES)) {
-        if (!transpose_a && c_dtype == QMOE_BF16 && m >= kRowPad) {
+        if (!transpose_a && c_dtype == QMOE_BF16 && (m % kRowPad == 0 || (m > kRowPad && k >= kRaggedInner))) {
             TimedScope timed(KC_EXPERT_GEMM, stream);
             const qmoe_route_t r = one_group_route(m);
             return transpose_b ? tc_rows_nt(&r, 1, a, b, c, k, n, stream, nullptr, m) : tc_rows_nn(&r, 1, a, b, 0, 0, c, k, n, stream, nullptr, m);

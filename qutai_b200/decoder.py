@@ -57,7 +57,7 @@ def _accumulate(parameter, storage, stream):
 class Linear:
     """``y = x W^T`` without bias (upstream ``Projection`` + ``linear``, src/qutai/lm/layers.py:35-74, :260-272):
     ``weight`` [out, in] float32, bf16 operand copy, bf16 activations; the three products go through ``qmoe_gemm``
-    (tensor cores when the row count is a multiple of 128)."""
+    (tensor cores from 128 rows on, whatever their number)."""
 
     def __init__(self, width_in, width_out, *, std, seed, stream=0):
         storage = DeviceStorage(width_out * width_in, "float32")

@@ -333,3 +333,20 @@ def test_short_ragged_weight_gradients_stay_on_the_cuda_cores(rows):
     assert lib.load().qmoe_tensor_core_launch_count() == before
     g64, x64 = g.astype(np.float64), x.astype(np.float64)
     assert np.all(np.abs(to_host(out, (64, 72)) - g64.T @ x64) <= rows * 2.0 ** -24 * (np.abs(g64).T @ np.abs(x64)) * 1.01)
+
+
+@pytest.mark.parametrize("rows,inner,tensor_cores", [(129, 32, 0), (4503, 56, 0), (129, 64, 1), (256, 8, 1), (128, 32, 1), (127, 64, 0)])
+def test_thin_ragged_products_stay_on_the_cuda_cores(rows, inner, tensor_cores):
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(rows + inner)
+    x, w = (oracle.round_bf16(rng.standard_normal((n, inner))) for n in (rows, 72))
+    xs, ws, out = to_device(x, "bfloat16"), to_device(w, "bfloat16"), DeviceStorage(rows * 72, "bfloat16")
+    before = lib.load().qmoe_tensor_core_launch_count()
+    lib.call("qmoe_gemm", xs.ptr, lib.QMOE_BF16, ws.ptr, lib.QMOE_BF16, out.ptr, lib.QMOE_BF16, rows, inner, 72, 0, 1, 0, 0)
+    assert lib.load().qmoe_tensor_core_launch_count() - before == tensor_cores
+    exact = x.astype(np.float64) @ w.astype(np.float64).T
+    # one rounding to bf16 of an fp32 sum
+    assert np.all(np.abs(to_host(out, exact.shape) - exact) <= 2.0 ** -8 * np.abs(exact) + inner * 2.0 ** -23 * (np.abs(x) @ np.abs(w).T))
