@@ -173,6 +173,10 @@ head_loss_gradient_kernel(T* __restrict__ logits, const long long* __restrict__ 
 // row's maximum, and the second pass writes (8188 rows x 32000: 305 -> 202 us = 5.2 TB/s).  What bounds it is HBM (one read, one write) with the exponential units
 // (two per element, 16 a clock and SM) just below; the kernel above spends 25 instructions per element, a 64-bit column
 // compare among them, and was bound by their issue.
+// Short rows stay with the kernel above: one piece per thread leaves nothing to overlap, and merging the threads' maxima costs
+// more than the second pass (whole forward, 32752 rows of 64 columns: 504 classes 198 us there, 214 here; 2000 265 and 273; 2504
+// 323 and 308; 4000 355 and 327).
+constexpr long long kTwoPassVocab = 2048;
 constexpr float kLog2e = 1.4426950408889634f;
 __device__ __forceinline__ float exp2_approx(float x) {
     float y;
@@ -322,7 +326,7 @@ int launch_loss_pass(T* logits, const long long* labels, const float* factor, fl
     if (bytes <= kMaxCachedRowBytes) {
         auto kernel = head_loss_gradient_kernel<T, true>;
         if constexpr (sizeof(T) == 2)
-            if (vocab % 8 == 0 && ((uintptr_t)logits & 15u) == 0) kernel = head_loss_gradient_bf16_kernel;
+            if (vocab >= kTwoPassVocab && vocab % 8 == 0 && ((uintptr_t)logits & 15u) == 0) kernel = head_loss_gradient_bf16_kernel;
         const int smem = (int)((bytes + 15) / 16 * 16);
         QMOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxCachedRowBytes));
         kernel<<<(unsigned)rows, kThreads, smem, stream>>>(logits, labels, factor, row_loss, rows, vocab, time, write_gradient);

@@ -176,3 +176,51 @@ def test_projection_loss_keeps_the_upstream_signature_and_record_shape():
     assert oracle.elementwise_err(to_host(d_hidden, g["hidden"].shape), g["d_hidden"]) <= FP32_ELEMENT_TOL
     again = projection_loss(hidden, weight, None, 7, prepared_labels=prepare_labels(labels))
     assert to_host(again.storage)[0] == to_host(loss.storage)[0]
+
+
+@pytest.mark.parametrize("vocab", [40, 2040, 2048, 2056, 8200, 32000])
+def test_loss_pass_over_infinities_and_extreme_logits(vocab):
+    """The bf16 loss pass on rows that hold what its running maximum has to get past: -inf in single places, in whole pieces and
+    in all places but one, the type's largest and lowest values, +inf, NaN, and a row that is not counted.  Both kernels (the
+    one for long rows begins at 2048 classes), and vocabularies shorter than a block."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(vocab)
+    largest = (2.0 - 2.0 ** -7) * 2.0 ** 127
+    z = oracle.round_bf16(rng.standard_normal((12, vocab)) * 3).astype(np.float64)
+    labels = rng.integers(1, vocab, size=12)
+    z[1, ::3] = -np.inf
+    z[2, : vocab // 2] = -np.inf
+    z[3], z[3, vocab // 2] = -np.inf, 1.5
+    z[4, labels[4]] = -np.inf
+    z[5, 0] = largest
+    z[6, 1:] = -largest
+    z[7], z[7, vocab - 1] = -largest, largest
+    z[8, 3] = np.inf
+    z[9, 5] = np.nan
+    z[10] = -np.inf
+    z[11, 7], labels[11] = np.nan, -100
+    with np.errstate(invalid="ignore", divide="ignore", over="ignore"):
+        peak = z.max(axis=1, keepdims=True)
+        weights = np.exp(z - peak)
+        p = weights / weights.sum(axis=1, keepdims=True)
+        loss = (np.log(weights.sum(axis=1)) - (z[np.arange(12), np.maximum(labels, 0)] - peak[:, 0]))
+    p[np.arange(11), labels[:11]] -= 1.0
+    p[11], loss[11] = 0.0, 0.0
+    logits, ids = to_device(z, "bfloat16"), to_device(labels, "int64")
+    row_loss, total, factor, one = DeviceStorage(12, "float32"), DeviceStorage(1, "float32"), DeviceStorage(1, "float32"), to_device(np.ones(1), "float32")
+    lib.call("qmoe_head_loss", logits.ptr, lib.QMOE_BF16, ids.ptr, row_loss.ptr, total.ptr, 12, vocab, 0, 0)
+    got = to_host(row_loss)
+    assert np.array_equal(np.isnan(got), np.isnan(loss)) and np.array_equal(np.isinf(got), np.abs(loss) > 3.4e38)
+    finite = np.isfinite(loss) & (np.abs(loss) < 3.4e38)
+    assert np.all(np.abs(got[finite] - loss[finite]) <= 1e-5 * np.maximum(1.0, np.abs(loss[finite])))
+    lib.call("qmoe_head_gradient", logits.ptr, lib.QMOE_BF16, ids.ptr, one.ptr, factor.ptr, 1, 12, vocab, 0, 0)
+    gradient = to_host(logits, (12, vocab))
+    for row in range(12):
+        if np.isnan(p[row]).any():
+            assert np.isnan(gradient[row]).all(), row
+        else:       # bf16 results: half a step of the value, and the fp32 error of p beside its 1
+            assert np.all(np.abs(gradient[row] - p[row]) <= 2.0 ** -8 * np.abs(p[row]) + 1e-6), row
+    assert lib.device_status() == 0
