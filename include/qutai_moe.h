@@ -119,7 +119,8 @@ enum {
     QMOE_VARIANT_NARROW_SCATTER = 2,    /* 64-byte instead of 256-byte row pieces in the peer-memory scatter epilogues */
     QMOE_VARIANT_PLAIN_GEMM_ON_CUDA_CORES = 3, /* qmoe_gemm never takes the tensor-core kernels */
     QMOE_VARIANT_NO_STREAM_GEMM = 4,    /* expert products of few rows on the kernel for many rows */
-    QMOE_VARIANT_COUNT = 5
+    QMOE_VARIANT_NO_FLOAT32_TILES = 5,  /* float32 products on the general CUDA-core kernel, never on 128 x 128 tiles */
+    QMOE_VARIANT_COUNT = 6
 };
 int qmoe_test_select_variant(int32_t which, int32_t value);
 

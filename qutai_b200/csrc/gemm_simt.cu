@@ -252,6 +252,7 @@ simt_tile_kernel(SimtGemmArgs g) {
 // kernel spread better: 48 tiles with K = 512 take 66 us there and 66 .. 70 here, 64 tiles 66 and 59 .. 72, 128 tiles 113 and
 // 61 .. 72).
 bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
+    if (kernel_variant(QMOE_VARIANT_NO_FLOAT32_TILES)) return false;
     if (g.accumulate || (g.mode != SG_PLAIN && g.mode != SG_ROWS && g.mode != SG_K)) return false;
     const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
     if ((!a_kfast && g.a_rs != 1) || (!b_kfast && g.b_cs != 1)) return false;

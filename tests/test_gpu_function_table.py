@@ -1,6 +1,7 @@
 """The per-op backend function table (``qutai_b200.cuda_lm``) against the oracle, written after the
 upstream GPU tests of the same functions (tests/test_lm_moe.py:140-162,
 tests/test_lm_bfloat16.py:129-167, tests/test_gemm_precision.py)."""
+import ctypes
 import os
 
 import numpy as np
@@ -273,20 +274,40 @@ def test_gemm_takes_ragged_row_counts_to_the_tensor_cores(rows, inner, cols, ker
     assert lib.device_status() == 0
 
 
-@pytest.mark.parametrize("m,k,n", [(128, 16, 128), (1000, 37, 900), (4097, 100, 132), (700, 260, 1028)])
-@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
-def test_float32_gemm_in_every_orientation(m, k, n, ta, tb):
-    """float32 products on the 128 x 128 tiles (and, for pitches that are no whole 16 bytes, on the general kernel): one
-    fp32 FMA chain per output, so the error is at most k roundings of sums of |a||b|."""
+# Whether a float32 product runs on the 128 x 128 tiles: the last column.  Ragged edges, an inner size that is no multiple of the
+# 16-deep slice (100, 20, 36) or, where no pitch is made of it, of a 16-byte piece (37), narrow and few tiles.
+@pytest.mark.parametrize("m,k,n,ta,tb,tiles", [
+    *((m, k, n, ta, tb, True) for m, k, n in ((1028, 100, 1156), (1284, 20, 1284), (9476, 4, 132), (1160, 520, 1032)) for ta in (0, 1) for tb in (0, 1)),
+    (1284, 37, 1156, 1, 0, True), (1284, 3, 1156, 1, 0, True), (1281, 36, 1155, 0, 1, True),
+    (1284, 37, 1156, 0, 1, False), (1284, 37, 1156, 1, 1, False), (1282, 36, 1156, 1, 0, False),
+    *((m, k, n, ta, tb, False) for m, k, n in ((128, 16, 128), (1000, 37, 900), (4097, 100, 132), (700, 260, 1028)) for ta in (0, 1) for tb in (0, 1)),
+    (9600, 36, 64, 0, 1, False), (64, 36, 9600, 0, 1, False)])
+def test_float32_gemm_in_every_orientation(m, k, n, ta, tb, tiles, kernel_variant):
+    """float32 products on the 128 x 128 tiles and on the general kernel: one fp32 FMA chain per output in the same order, so the
+    same bits, and an error of at most k roundings of sums of |a||b|.  The
+    dispatch rule is restated here, so that no case misses the kernel it is for."""
     from gpu_util import to_device, to_host
     from qutai_b200 import lib
     from qutai_b200.storage import DeviceStorage
 
+    sms = ctypes.c_int()
+    lib.call("qmoe_device_info", ctypes.byref(sms), ctypes.byref(ctypes.c_int()), ctypes.byref(ctypes.c_int()), ctypes.byref(ctypes.c_uint64()))
+    pitches = (m if ta else k, k if tb else n)
+    assert tiles == (min(m, n) > 64 and all(pitch % 4 == 0 for pitch in pitches) and -(-m // 128) * -(-n // 128) * 2 >= sms.value)
     rng = np.random.default_rng(m + k + n)
     a, b = (rng.standard_normal(shape).astype(np.float32) for shape in ((k, m) if ta else (m, k), (n, k) if tb else (k, n)))
-    out, sa, sb = DeviceStorage(m * n, "float32"), to_device(a, "float32"), to_device(b, "float32")
-    lib.call("qmoe_gemm", sa.ptr, lib.QMOE_F32, sb.ptr, lib.QMOE_F32, out.ptr, lib.QMOE_F32, m, k, n, ta, tb, 0, 0)
-    got = to_host(out, (m, n))
+    sa, sb = to_device(a, "float32"), to_device(b, "float32")
+
+    def product():
+        out = DeviceStorage((m + 1) * n, "float32")
+        lib.call("qmoe_memset", out.ptr, 0x3C, out.nbytes, 0)
+        lib.call("qmoe_gemm", sa.ptr, lib.QMOE_F32, sb.ptr, lib.QMOE_F32, out.ptr, lib.QMOE_F32, m, k, n, ta, tb, 0, 0)
+        return out
+
+    first = product()
+    kernel_variant(lib.VARIANT_NO_FLOAT32_TILES)
+    assert first.tobytes() == product().tobytes()                     # the row behind the result included
+    got = to_host(first, (m + 1, n))[:m]
     a64, b64 = (a.T if ta else a).astype(np.float64), (b.T if tb else b).astype(np.float64)
     bound = k * 2.0 ** -24 * (np.abs(a64) @ np.abs(b64)) * 1.01
     assert np.all(np.abs(got - a64 @ b64) <= bound)

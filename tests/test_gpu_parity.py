@@ -438,6 +438,35 @@ def test_router_forward_backward_fp32_semantics(T, d, E, dtype):
     assert lib.device_status() == 0
 
 
+@pytest.mark.parametrize("T,d,E,k,h", [(2048, 512, 8, 2, 1024), (700, 264, 5, 3, 520)])
+def test_float32_layer_on_tiles_gives_the_bits_of_the_general_kernel(T, d, E, k, h, kernel_variant):
+    """A float32 layer with uneven counts (one expert liked by most tokens, one by none), forward and backward: the products per
+    128-row tile, the two-segment input gradient and the weight gradients of a row range per expert, on 128 x 128 tiles and on
+    the general kernel, in sizes that fill the tiles and in ragged ones."""
+    from gpu_util import make_layer, run_layer
+    from qutai_b200 import lib
+
+    rng = np.random.default_rng(T)
+    x, grad_y = (rng.standard_normal((T, d)).astype(np.float32) for _ in range(2))
+    x[:, 0] = 1.0
+    router = rng.standard_normal((E, d)).astype(np.float32) * 0.05
+    router[0, 0], router[1, 0] = 3.0, -100.0
+    gate, up = (rng.standard_normal((E, h, d)).astype(np.float32) / np.sqrt(d) for _ in range(2))
+    down = rng.standard_normal((E, d, h)).astype(np.float32) / np.sqrt(h)
+    results = []
+    for general in (False, True):
+        if general:
+            kernel_variant(lib.VARIANT_NO_FLOAT32_TILES)
+        results.append(run_layer(make_layer(x.shape, router, gate, up, down, k), x, grad_y, 0.1, "float32"))
+    tiles, general = results
+    assert tiles["counts"] == general["counts"] and tiles["counts"][0] > T * k // E and tiles["counts"][1] == 0
+    for name in ("y", "dx", "d_router"):
+        assert np.array_equal(tiles[name], general[name]), name
+    for name in ("d_gate", "d_up", "d_down"):
+        for got, want in zip(tiles[name], general[name]):
+            assert (got is None and want is None) or np.array_equal(got, want), name
+
+
 @pytest.mark.parametrize("T,d,E,tensor_cores", [(512, 64, 64, 0), (513, 512, 8, 0), (2048, 64, 64, 1), (16384, 64, 16, 1), (4096, 256, 8, 0)])
 def test_router_logits_of_many_tokens_leave_the_kernel_for_few(T, d, E, tensor_cores):
     """bf16 logits beyond 512 tokens take the kernel with a warp per logit only where that is the shorter way; both sides of the
