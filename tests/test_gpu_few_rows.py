@@ -8,11 +8,18 @@ from oracle import moe_oracle as oracle
 pytestmark = pytest.mark.gpu
 
 
+# 64 experts, 50 rows on average: enough tiles of 256 columns for the down product that holds two weight tiles per stage
+MANY = (0, 127, 128, 129, 300, 1, 15, 17) + (33, 0, 64, 31, 49, 96, 2, 48) * 7
+
+
 @pytest.mark.parametrize("counts,width,hidden", [
     ((0, 1, 15, 16, 17), 64, 128),           # around one 16-row step, an expert without rows
     ((127, 128, 129, 0, 3), 72, 136),        # around one 128-row chunk, widths that fill no tile
     ((300, 2, 0, 40, 33), 264, 1032),        # an expert with three chunks, several k blocks and tiles
     ((1,), 2048, 8),                         # one row, the narrowest hidden width
+    (MANY, 648, 136),                        # the last 256-column tile of the down product holds 136, one full weight tile and 8 columns
+    (MANY, 584, 136),                        # it holds 72: the second weight tile lies outside, at the last expert behind the last weight
+    (MANY, 768, 200),                        # whole tiles
 ])
 def test_streamed_products_match_the_kernel_for_many_rows(counts, width, hidden, kernel_variant):
     import ctypes
@@ -22,6 +29,8 @@ def test_streamed_products_match_the_kernel_for_many_rows(counts, width, hidden,
     from qutai_b200.storage import DeviceStorage
 
     experts, tokens = len(counts), sum(counts)
+    if counts is MANY:      # the rule for two weight tiles per stage
+        assert 32 * experts < tokens <= 96 * experts and -(-width // 256) * experts >= lib.device_info()["sm_count"]
     rng = np.random.default_rng(tokens + width)
     choice = np.repeat(np.arange(experts), counts)
     scores = np.zeros((tokens, experts), dtype=np.float32)

@@ -1,7 +1,6 @@
 """The per-op backend function table (``qutai_b200.cuda_lm``) against the oracle, written after the
 upstream GPU tests of the same functions (tests/test_lm_moe.py:140-162,
 tests/test_lm_bfloat16.py:129-167, tests/test_gemm_precision.py)."""
-import ctypes
 import os
 
 import numpy as np
@@ -290,10 +289,8 @@ def test_float32_gemm_in_every_orientation(m, k, n, ta, tb, tiles, kernel_varian
     from qutai_b200 import lib
     from qutai_b200.storage import DeviceStorage
 
-    sms = ctypes.c_int()
-    lib.call("qmoe_device_info", ctypes.byref(sms), ctypes.byref(ctypes.c_int()), ctypes.byref(ctypes.c_int()), ctypes.byref(ctypes.c_uint64()))
     pitches = (m if ta else k, k if tb else n)
-    assert tiles == (min(m, n) > 64 and all(pitch % 4 == 0 for pitch in pitches) and -(-m // 128) * -(-n // 128) * 2 >= sms.value)
+    assert tiles == (min(m, n) > 64 and all(pitch % 4 == 0 for pitch in pitches) and -(-m // 128) * -(-n // 128) * 2 >= lib.device_info()["sm_count"])
     rng = np.random.default_rng(m + k + n)
     a, b = (rng.standard_normal(shape).astype(np.float32) for shape in ((k, m) if ta else (m, k), (n, k) if tb else (k, n)))
     sa, sb = to_device(a, "float32"), to_device(b, "float32")
