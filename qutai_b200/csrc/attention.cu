@@ -30,10 +30,9 @@ namespace {
 constexpr int D = 64;                 // head width
 constexpr int BLOCK = 128;            // query rows of a CTA = key positions of a block
 constexpr int TILE_BYTES = BLOCK * D * 2;          // 16 KiB: 128 rows x 128 bytes
-constexpr int THREADS = 192;              // forward: TMA warp, MMA warp, four row warps
-// Row warps per 32 rows of the backward kernels, which share the columns of a block between them
-constexpr int DQ_PARTS = 1, DKV_PARTS = 2;
-constexpr int DQ_THREADS = 64 + 128 * DQ_PARTS, DKV_THREADS = 64 + 128 * DKV_PARTS;
+constexpr int THREADS = 192;              // forward, dq: TMA warp, MMA warp, four row warps
+// Row warps per 32 rows of the dk, dv kernel, which share the columns of a block between them
+constexpr int DKV_PARTS = 2, DKV_THREADS = 64 + 128 * DKV_PARTS;
 constexpr float LOG2E = 1.4426950408889634f;
 enum { STATUS_ATTENTION_WAIT = 301 };
 
@@ -318,7 +317,7 @@ constexpr int DQ_KV = 64, DQ_TILE = DQ_KV * 128, DQ_STAGES = 3;
 constexpr int DQ_TILES = 2 * TILE_BYTES + 2 * DQ_STAGES * DQ_TILE;
 constexpr int DQ_SMEM = DQ_TILES + 128;
 
-__global__ void __launch_bounds__(DQ_THREADS, 2)
+__global__ void __launch_bounds__(THREADS, 2)
 attention_dq_kernel(const __grid_constant__ AttentionParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -341,7 +340,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
     }
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int w = 0; w < BARS; ++w) mbar_init(bar(w), w == DS_FULL ? 4 * DQ_PARTS : 1);
+        for (int w = 0; w < BARS; ++w) mbar_init(bar(w), w == DS_FULL ? 4 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         prefetch_map(&p.map_q); prefetch_map(&p.map_k2); prefetch_map(&p.map_v2); prefetch_map(&p.map_do);
     }
@@ -414,7 +413,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < DQ_KV / 16; ++kk)
-                    umma_bf16_ts(tmem_dq, tmem + (uint32_t)(j & 1) * DQ_KV + p_column<DQ_KV / DQ_PARTS>(kk),
+                    umma_bf16_ts(tmem_dq, tmem + (uint32_t)(j & 1) * DQ_KV + p_column<DQ_KV>(kk),
                                  make_desc(k_tile + st * DQ_TILE + kk * 2048, 8192, 1024), idesc_dq, (j | kk) ? 1u : 0u);
                 umma_commit(bar(KV_EMPTY + st));
                 if (j == n - 1) umma_commit(bar(DQ_DONE));
@@ -423,8 +422,8 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
         }
         if (ok) wait.all(bar(DQ_DONE), 0);         // the last commit has arrived
     } else {
-        constexpr int COLS = DQ_KV / DQ_PARTS;     // columns of a block per thread
-        const int quad = warp & 3, row = quad * 32 + lane, part = (warp - 2) >> 2;
+        constexpr int COLS = DQ_KV;                // columns of a block per thread
+        const int quad = warp & 3, row = quad * 32 + lane;
         const int tq = i * BLOCK + row;
         const bool live = tq < p.time;
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
@@ -443,15 +442,15 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
                     delta += __uint_as_float(aw[e] << 16) * __uint_as_float(ow[e] << 16) +
                              __uint_as_float(aw[e] & 0xffff0000u) * __uint_as_float(ow[e] & 0xffff0000u);
             }
-            if (part == 0) p.delta[at] = delta;
+            p.delta[at] = delta;
             lse2 = p.lse[at] * LOG2E;
         }
         const float scale2 = 0.125f * LOG2E;
         const uint64_t scale_pair = pair2(scale2, scale2), lse_pair = pair2(-lse2, -lse2), delta_pair = pair2(-delta, -delta);
         bool ok = true;
         for (int j = 0; ok && j < n; ++j) {
-            const uint32_t tmem_s = tmem + (uint32_t)(j & 1) * DQ_KV + lane_base + part * COLS;
-            const int first = j * DQ_KV + part * COLS - i * BLOCK;       // first key position of this thread, from the CTA's first query
+            const uint32_t tmem_s = tmem + (uint32_t)(j & 1) * DQ_KV + lane_base;
+            const int first = j * DQ_KV - i * BLOCK;                     // first key position of the block, from the CTA's first query
             const bool masked = first + COLS - 1 > quad * 32;            // some row of this warp may not see some of these columns
             uint32_t s[COLS], dp[COLS], packed[COLS / 2];
             ok = wait.all(bar(S_FULL + (j & 1)), (uint32_t)(j >> 1) & 1u);
@@ -471,7 +470,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
-            for (int c = 0; c < COLS; c += 32) tmem_ld32(tmem_dp + lane_base + part * COLS + c, dp + c);
+            for (int c = 0; c < COLS; c += 32) tmem_ld32(tmem_dp + lane_base + c, dp + c);
             tmem_ld_wait();
             // dS without the 1/8 of the scores, which the last step applies to dQ (a power of two: the same bits)
 #pragma unroll
@@ -489,8 +488,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
             }
 #pragma unroll
             for (int c = 0; c < COLS; c += 2) packed[c >> 1] = pack2(__uint_as_float(s[c]), __uint_as_float(s[c + 1]));
-            if (COLS == 64) tmem_st32(tmem_s, packed);
-            else tmem_st16(tmem_s, packed);
+            tmem_st32(tmem_s, packed);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -501,7 +499,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
             tc_fence_after();
             uint4* dst = reinterpret_cast<uint4*>(p.out + at * D);
 #pragma unroll
-            for (int c = part; c < 2; c += DQ_PARTS) {
+            for (int c = 0; c < 2; ++c) {
                 uint32_t r[32];
                 tmem_ld32(tmem_dq + lane_base + c * 32, r);
                 tmem_ld_wait();
@@ -896,7 +894,7 @@ extern "C" int qmoe_attention_backward(const qmoe_attention_t* a, uint64_t strea
     QMOE_CUDA(cudaFuncSetAttribute(attention_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
     QMOE_CUDA(cudaFuncSetAttribute(attention_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DKV_SMEM));
     p.out = (__nv_bfloat16*)a->dq; p.out2 = nullptr;
-    attention_dq_kernel<<<(unsigned)(blocks * a->heads * a->batch), DQ_THREADS, DQ_SMEM, stream>>>(p);
+    attention_dq_kernel<<<(unsigned)(blocks * a->heads * a->batch), THREADS, DQ_SMEM, stream>>>(p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("attention_dq_kernel");
     p.out = (__nv_bfloat16*)a->dk; p.out2 = (__nv_bfloat16*)a->dv;
