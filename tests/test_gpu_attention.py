@@ -172,3 +172,31 @@ def test_attention_gradients_of_a_key_that_no_query_sees(time):
     for name in ("dk", "dv"):
         assert np.all(np.isfinite(got[name])) and not np.any(got[name][0, hidden]), name
     check(dict(got, dq=dq), dict(out=out, dq=dq, dk=dk, dv=dv))       # dq holds 0 * inf, as a product with that key does
+
+
+@pytest.mark.parametrize("time", [130, 300])
+def test_attention_rows_with_infinities_and_nan_stay_by_themselves(time):
+    """Query rows that hold NaN and infinities give NaN rows; every other row of the output keeps its bits, in the same block and in
+    others."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.attention import attention_forward
+    from qutai_b200.layers import Tensor
+
+    heads, kv_heads = 2, 1
+    q, k, v, _ = attention_inputs(1, time, heads, kv_heads, seed=time, scale=1.0)
+
+    def rows(values):
+        tensors = [Tensor(to_device(a, "bfloat16"), a.shape) for a in (values, k, v)]
+        out, lse = attention_forward(*tensors, heads, kv_heads)
+        assert lib.device_status() == 0
+        return to_host(out, q.shape)[0], to_host(lse, (time, heads))
+
+    wild = q.copy()
+    wild[0, 5, 3], wild[0, 64, 64:], wild[0, 127, 7], wild[0, time - 1, 0] = np.nan, np.inf, -np.inf, np.nan
+    (plain, plain_lse), (got, got_lse) = rows(q), rows(wild)
+    bad = np.zeros((time, heads), dtype=bool)
+    bad[5, 0] = bad[64, 1] = bad[127, 0] = bad[time - 1, 0] = True
+    wide = np.repeat(bad, 64, axis=1)
+    assert np.isnan(got[wide]).all() and np.isnan(got_lse[bad]).all()
+    assert np.array_equal(got[~wide], plain[~wide]) and np.array_equal(got_lse[~bad], plain_lse[~bad])
