@@ -433,8 +433,9 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     // An epilogue warp hands its accumulator back as soon as its last read of it has arrived in registers, before the stores
     // of what it read, and without release semantics across the pair: a release at cluster scope waits until every global
     // store of the thread has been acknowledged (weight gradients over 375 rows per expert, 16 x 3 x 1024 x 2048: 145 us with
-    // both, 130 without).  Nothing but tensor memory is handed over, and the reads
-    // of it are complete.
+    // both, 130 without).  Nothing but tensor memory is handed over, and for that PTX asks for no release: the reads are complete
+    // (tcgen05.wait::ld by every lane), tcgen05.fence::before_thread_sync orders them before the arrival, and the issuer's
+    // tcgen05.fence::after_thread_sync, once it has seen the phase end, orders its next product after it.
     auto release_accumulator = [&](int acc) {
         tc_fence_before();
         __syncwarp();
@@ -549,21 +550,32 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     int next_stage = stage + 1;
                     uint32_t next_phase = phase;
                     if (next_stage == STAGES) { next_stage = 0; next_phase ^= 1u; }
-#pragma unroll
-                    for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                    auto product = [&](int kk) {
                         // K-major: 128-byte rows, 8-row groups 1024 B apart, +32 B per 16 k.
                         // MN-major: 64-wide chunks 8 KiB apart (LBO), 8-k groups 1024 B apart, +2 KiB per 16 k.
                         const uint64_t adesc = A_MN ? make_desc(sa + kk * 2048, CHUNK_BYTES, 1024)
                                                     : make_desc(sa + kk * 32, 16, 1024);
                         const uint64_t bdesc = B_MN ? make_desc(sb + kk * 2048, CHUNK_BYTES, 1024)
                                                     : make_desc(sb + kk * 32, 16, 1024);
-                        // the look at the next stage's barrier goes between the MMAs, where the tensor pipe has work queued,
-                        // rather than after the last one, where its latency would leave the pipe idle
-                        if (kk == BK / UMMA_K - 1) ready = kb + 1 < tile.kblocks && mbar_try(full_bar(next_stage), next_phase);
-                        // WGRAD: rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten)
-                        if (MODE == MODE_WGRAD && kb * BK + kk * UMMA_K >= tile.depth) continue;
                         if (CTAS == 2) umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
                         else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
+                    };
+                    // the look at the next stage's barrier goes between the MMAs, where the tensor pipe has work queued,
+                    // rather than after the last one, where its latency would leave the pipe idle
+                    auto look_ahead = [&] { ready = kb + 1 < tile.kblocks && mbar_try(full_bar(next_stage), next_phase); };
+                    if (MODE == MODE_WGRAD && (kb + 1) * BK > tile.depth) {
+                        // rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten); in a
+                        // branch of its own, since a test per product held up the issue (4096 rows per expert: 421 -> 430 us)
+                        look_ahead();
+#pragma unroll
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            if (kb * BK + kk * UMMA_K < tile.depth) product(kk);
+                    } else {
+#pragma unroll
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                            if (kk == BK / UMMA_K - 1) look_ahead();
+                            product(kk);
+                        }
                     }
                     commit(empty_bar(stage));  // the stage is free once these MMAs have read it
                     stage = next_stage; phase = next_phase;
@@ -861,7 +873,8 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     float* to = C + (long long)(c * 32) * ldc;
                     // The common case without a test per store and with one running address: over a short contraction a tile waits
                     // for the instructions of these warps (375 rows per expert, 16 x 3 x 1024 x 2048: 130 -> 95 us, where the bytes
-                    // take 62; 32768 rows over 64 experts, 2048 x 1408: 3.31 -> 3.10 ms).
+                    // take 62; both changes to the epilogue, L2 flushed: 148 -> 101).  Over a long one it makes no difference: 32768
+                    // rows over 64 experts, 2048 x 1408, 2.75 ms before and after.
                     if (row_ok && valid >= 32) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i, to += ldc) *to = __uint_as_float(r[i]);

@@ -28,7 +28,8 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
 // ---- permute: dispatched[dest_row[t, s]] = x[t] for every slot, pads zero ------------------------
 // Organised by TOKEN: a warp reads one token row once and writes its k copies, so the source is
 // read T*d instead of A*d times (the k copies of a token lie far apart in the dispatched layout and
-// would miss L2).  Pad rows are zeroed afterwards by the warps that find row_source[r] < 0.
+// would miss L2).  Pad rows are zeroed afterwards, a warp per row, from the experts' offsets and counts: up to the next multiple
+// of 2^pad_bits rows.
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restrict__ dest_row,
