@@ -54,6 +54,42 @@ def test_router_scratch_never_shrinks_with_more_tokens(library_path, experts, wi
     assert size(0, experts, width) == size(-1, experts, width) == size(1, 0, width) == 0
 
 
+@pytest.mark.parametrize("ids", [[0], [5, 5, 5], [3, 1, 3, 0, 9, 1, 3], [7, 6, 5, 4, 3, 2, 1, 0]])
+def test_token_tables_list_every_token_with_its_positions(library_path, ids):
+    from array import array
+
+    values, distinct, starts, positions = (array("q", data) for data in (ids, [-1] * 10, [-1] * 11, [-1] * len(ids)))
+    segments = ctypes.c_int64()
+    addresses = [a.buffer_info()[0] for a in (values, distinct, starts, positions)]
+    lib.call("qmoe_token_tables", addresses[0], len(ids), 10, *addresses[1:], ctypes.byref(segments))
+    found = segments.value
+    assert list(distinct[:found]) == sorted(set(ids))
+    for i, token in enumerate(distinct[:found]):
+        assert list(positions[starts[i]:starts[i + 1]]) == [p for p, t in enumerate(ids) if t == token]
+    for bad in (10, -1):
+        values[0] = bad
+        with pytest.raises(ValueError, match="vocabulary"):
+            lib.call("qmoe_token_tables", addresses[0], len(ids), 10, *addresses[1:], ctypes.byref(segments))
+    with pytest.raises(ValueError):
+        lib.call("qmoe_token_tables", addresses[0], 0, 10, *addresses[1:], ctypes.byref(segments))
+
+
+def test_token_ids_of_every_kind_become_64_bit_integers():
+    """What ``int()`` turns into an integer is a token id; one beyond 64 bits is outside every vocabulary."""
+    from array import array
+
+    import numpy as np
+
+    from qutai_b200.decoder import _integers
+
+    for rows in ([[1, 2], [3, 4]], [(1, 2), (3, 4)], np.array([[1, 2], [3, 4]], dtype=np.int32), [array("i", [1, 2]), array("q", [3, 4])],
+                 [[1.0, 2.9], ["3", 4]], [[True, 2], [np.int8(3), np.float32(4.5)]], [range(1, 3), b"\x03\x04"]):
+        assert list(_integers(rows, 3)) == [1, 2, 3, 4, 0, 0, 0]
+    assert list(_integers([[2 ** 63, -2 ** 70, 5]], 0)) == [-1, -1, 5]
+    with pytest.raises(ValueError):
+        _integers([[float("nan")]], 0)
+
+
 def test_ctypes_structures_match_the_c_layout(tmp_path):
     source = tmp_path / "layout.c"
     fields = {"qmoe_route_t": [f[0] for f in lib.Route._fields_],
