@@ -248,7 +248,7 @@ simt_tile_kernel(SimtGemmArgs g) {
 // What the 128 x 128 kernel takes: fp32 operands and results, each operand contiguous along one of its axes with whole
 // 16-byte pieces, no accumulation, more than 64 rows and columns (fewer are one tile of the general kernel, and half of the work
 // here is on what does not exist: 40000 x 1024 x 16 columns 140 us there and 280 here, 32 columns 271 and 282, 64 columns 281
-// and 281 .. 300), and a tile for every second SM (with fewer, the four times smaller tiles of the general
+// and 281 .. 300), an inner size of at least one slice (9472 x 4 x 128: 8 us there, 10 here), and a tile for every second SM (with fewer, the four times smaller tiles of the general
 // kernel spread better: 48 tiles with K = 512 take 66 us there and 66 .. 70 here, 64 tiles 66 and 59 .. 72, 128 tiles 113 and
 // 61 .. 72).
 bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
@@ -259,7 +259,7 @@ bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
     const long long a_pitch = a_kfast ? g.a_rs : g.a_cs, b_pitch = b_kfast ? g.b_cs : g.b_rs;
     if (a_pitch % 4 || b_pitch % 4 || g.b_slab % 4) return false;
     if (((uintptr_t)g.A | (uintptr_t)g.B | (uintptr_t)g.A2 | (uintptr_t)g.B2) & 15u) return false;
-    if (g.N <= 64 || m_extent <= 64) return false;
+    if (g.N <= 64 || m_extent <= 64 || (g.mode != SG_K && g.K < TILE_K)) return false;
     return (long long)ceil_div(g.N, TILE) * ceil_div(m_extent, TILE) * groups * 2 >= sm_count();
 }
 

@@ -276,9 +276,9 @@ def test_gemm_takes_ragged_row_counts_to_the_tensor_cores(rows, inner, cols, ker
 # Whether a float32 product runs on the 128 x 128 tiles: the last column.  Ragged edges, an inner size that is no multiple of the
 # 16-deep slice (100, 20, 36) or, where no pitch is made of it, of a 16-byte piece (37), narrow and few tiles.
 @pytest.mark.parametrize("m,k,n,ta,tb,tiles", [
-    *((m, k, n, ta, tb, True) for m, k, n in ((1028, 100, 1156), (1284, 20, 1284), (9476, 4, 132), (1160, 520, 1032)) for ta in (0, 1) for tb in (0, 1)),
-    (1284, 37, 1156, 1, 0, True), (1284, 3, 1156, 1, 0, True), (1281, 36, 1155, 0, 1, True),
-    (1284, 37, 1156, 0, 1, False), (1284, 37, 1156, 1, 1, False), (1282, 36, 1156, 1, 0, False),
+    *((m, k, n, ta, tb, True) for m, k, n in ((1028, 100, 1156), (1284, 20, 1284), (9476, 16, 132), (1160, 520, 1032)) for ta in (0, 1) for tb in (0, 1)),
+    (1284, 37, 1156, 1, 0, True), (1284, 17, 1156, 1, 0, True), (1281, 36, 1155, 0, 1, True),
+    (9476, 4, 132, 0, 1, False), (1284, 15, 1156, 1, 0, False), (1284, 37, 1156, 0, 1, False), (1284, 37, 1156, 1, 1, False), (1282, 36, 1156, 1, 0, False),
     *((m, k, n, ta, tb, False) for m, k, n in ((128, 16, 128), (1000, 37, 900), (4097, 100, 132), (700, 260, 1028)) for ta in (0, 1) for tb in (0, 1)),
     (9600, 36, 64, 0, 1, False), (64, 36, 9600, 0, 1, False)])
 def test_float32_gemm_in_every_orientation(m, k, n, ta, tb, tiles, kernel_variant):
@@ -290,7 +290,7 @@ def test_float32_gemm_in_every_orientation(m, k, n, ta, tb, tiles, kernel_varian
     from qutai_b200.storage import DeviceStorage
 
     pitches = (m if ta else k, k if tb else n)
-    assert tiles == (min(m, n) > 64 and all(pitch % 4 == 0 for pitch in pitches) and -(-m // 128) * -(-n // 128) * 2 >= lib.device_info()["sm_count"])
+    assert tiles == (min(m, n) > 64 and k >= 16 and all(pitch % 4 == 0 for pitch in pitches) and -(-m // 128) * -(-n // 128) * 2 >= lib.device_info()["sm_count"])
     rng = np.random.default_rng(m + k + n)
     a, b = (rng.standard_normal(shape).astype(np.float32) for shape in ((k, m) if ta else (m, k), (n, k) if tb else (k, n)))
     sa, sb = to_device(a, "float32"), to_device(b, "float32")
