@@ -139,6 +139,8 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_wait();
+    chain_next();      // the tensor memory is this block's
     const uint32_t tmem = s_tmem_base;
     const uint32_t tmem_s = tmem, tmem_o = tmem + 128, tmem_p = tmem + 192;    // 128 + 64 + 64 (bf16 pairs) columns
     const Wait wait{&s_abort, p.status};
@@ -351,6 +353,8 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_wait();
+    chain_next();      // the tensor memory is this block's
     const uint32_t tmem = s_tmem_base;
     // S of block j in columns 64 (j & 1) ..; the rows put dS (bf16 pairs) back over the columns they read
     const uint32_t tmem_dp = tmem + 2 * DQ_KV, tmem_dq = tmem + 3 * DQ_KV;
@@ -572,6 +576,8 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_wait();
+    chain_next();      // the tensor memory is this block's
     const uint32_t tmem = s_tmem_base;
     // everything with key positions as rows (lanes) and query positions as columns: S^T of iteration it in columns
     // 128 (it & 1) .., over which the rows put back P^T and dS^T (bf16 pairs); one dP^T
@@ -869,7 +875,7 @@ extern "C" int qmoe_attention_forward(const qmoe_attention_t* a, uint64_t stream
     p.batch = a->batch; p.time = a->time; p.heads = a->heads; p.kv_heads = a->kv_heads;
     QMOE_CUDA(cudaFuncSetAttribute(attention_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FORWARD_SMEM));
     const int blocks = (a->time + BLOCK - 1) / BLOCK;
-    attention_forward_kernel<<<(unsigned)(blocks * a->heads * a->batch), THREADS, FORWARD_SMEM, stream>>>(p);
+    chained(attention_forward_kernel, (unsigned)(blocks * a->heads * a->batch), THREADS, FORWARD_SMEM, stream, p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("attention_forward_kernel");
     return 0;
@@ -894,24 +900,22 @@ extern "C" int qmoe_attention_backward(const qmoe_attention_t* a, uint64_t strea
     QMOE_CUDA(cudaFuncSetAttribute(attention_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
     QMOE_CUDA(cudaFuncSetAttribute(attention_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DKV_SMEM));
     p.out = (__nv_bfloat16*)a->dq; p.out2 = nullptr;
-    attention_dq_kernel<<<(unsigned)(blocks * a->heads * a->batch), THREADS, DQ_SMEM, stream>>>(p);
+    chained(attention_dq_kernel, (unsigned)(blocks * a->heads * a->batch), THREADS, DQ_SMEM, stream, p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("attention_dq_kernel");
     p.out = (__nv_bfloat16*)a->dk; p.out2 = (__nv_bfloat16*)a->dv;
     p.split = dkv_split(a, blocks);
     cudaLaunchConfig_t config = {};
-    cudaLaunchAttribute cluster[1];
+    cudaLaunchAttribute attributes[2] = {chain_attribute()};
     config.gridDim = dim3((unsigned)(blocks * a->kv_heads * a->batch * p.split));
     config.blockDim = dim3(DKV_THREADS);
     config.dynamicSmemBytes = DKV_SMEM;
     config.stream = stream;
-    if (p.split > 1) {
-        cluster[0].id = cudaLaunchAttributeClusterDimension;
-        cluster[0].val.clusterDim.x = (unsigned)p.split;
-        cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
-        config.attrs = cluster;
-        config.numAttrs = 1;
-    }
+    config.attrs = attributes;
+    config.numAttrs = p.split > 1 ? 2 : 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = (unsigned)p.split;
+    attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
     QMOE_CUDA(cudaLaunchKernelEx(&config, attention_dkv_kernel, p));
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("attention_dkv_kernel");

@@ -18,6 +18,7 @@ template <typename T> __device__ __forceinline__ float ldf(const T* p, long long
 template <typename TA, typename TB, typename TC, int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__(256)
 simt_gemm_kernel(SimtGemmArgs g) {
+    chain_wait();      // no chain_next: see chained
     constexpr int BK = 16;
     static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
     __shared__ float As[BK][BM + 4];
@@ -161,6 +162,7 @@ struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice 
 template <bool A_KFAST, bool B_KFAST>
 __global__ void __launch_bounds__(256, 2)
 simt_tile_kernel(SimtGemmArgs g) {
+    chain_wait();      // no chain_next: see chained
     __shared__ __align__(16) float As[2][TILE_K][TILE_PITCH];
     __shared__ __align__(16) float Bs[2][TILE_K][TILE_PITCH];
     const long long m0 = (long long)blockIdx.y * TILE, n0 = (long long)blockIdx.x * TILE;
@@ -266,10 +268,10 @@ bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
 int launch_tiles(const SimtGemmArgs& g, long long m_extent, int groups, cudaStream_t stream) {
     const dim3 grid(ceil_div(g.N, TILE), ceil_div(m_extent, TILE), groups);
     const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
-    if (a_kfast && b_kfast) simt_tile_kernel<true, true><<<grid, 256, 0, stream>>>(g);
-    else if (a_kfast) simt_tile_kernel<true, false><<<grid, 256, 0, stream>>>(g);
-    else if (b_kfast) simt_tile_kernel<false, true><<<grid, 256, 0, stream>>>(g);
-    else simt_tile_kernel<false, false><<<grid, 256, 0, stream>>>(g);
+    if (a_kfast && b_kfast) chained(simt_tile_kernel<true, true>, grid, 256, 0, stream, g);
+    else if (a_kfast) chained(simt_tile_kernel<true, false>, grid, 256, 0, stream, g);
+    else if (b_kfast) chained(simt_tile_kernel<false, true>, grid, 256, 0, stream, g);
+    else chained(simt_tile_kernel<false, false>, grid, 256, 0, stream, g);
     QMOE_LAUNCH_CHECK("simt_tile_kernel");
     return 0;
 }
@@ -277,6 +279,7 @@ int launch_tiles(const SimtGemmArgs& g, long long m_extent, int groups, cudaStre
 // sum S partial [S][n] slabs in a fixed order
 __global__ void __launch_bounds__(256)
 reduce_partials_kernel(const float* __restrict__ partials, float* __restrict__ out, long long n, int splits) {
+    chain_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.f;
@@ -288,10 +291,10 @@ template <typename TA, typename TB, typename TC>
 int launch_typed(const SimtGemmArgs& g, long long m_extent, int groups, cudaStream_t stream) {
     if (g.N <= 16) {
         dim3 grid(ceil_div(g.N, 16), ceil_div(m_extent, 128), groups);
-        simt_gemm_kernel<TA, TB, TC, 128, 16, 2, 4><<<grid, 256, 0, stream>>>(g);
+        chained(simt_gemm_kernel<TA, TB, TC, 128, 16, 2, 4>, grid, 256, 0, stream, g);
     } else {
         dim3 grid(ceil_div(g.N, 64), ceil_div(m_extent, 64), groups);
-        simt_gemm_kernel<TA, TB, TC, 64, 64, 4, 4><<<grid, 256, 0, stream>>>(g);
+        chained(simt_gemm_kernel<TA, TB, TC, 64, 64, 4, 4>, grid, 256, 0, stream, g);
     }
     QMOE_LAUNCH_CHECK("simt_gemm_kernel");
     return 0;
@@ -320,7 +323,7 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
 }
 
 int launch_reduce_partials(const float* partials, float* out, long long n, int splits, cudaStream_t stream) {
-    reduce_partials_kernel<<<ceil_div(n, 256), 256, 0, stream>>>(partials, out, n, splits);
+    chained(reduce_partials_kernel, ceil_div(n, 256), 256, 0, stream, partials, out, n, splits);
     QMOE_LAUNCH_CHECK("reduce_partials_kernel");
     return 0;
 }

@@ -95,11 +95,6 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
     auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
 
-    for (int e = threadIdx.x; e <= p.experts; e += STREAM_THREADS) {
-        int tiles = 0;
-        for (int j = 0; j < e; ++j) tiles += (p.counts[j] + kRowPad - 1) / kRowPad;
-        s_first[e] = tiles * p.m_tiles;
-    }
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
@@ -110,6 +105,12 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(STREAM_TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    chain_wait();      // what follows reads global memory; no chain_next: see chained
+    for (int e = threadIdx.x; e <= p.experts; e += STREAM_THREADS) {
+        int tiles = 0;
+        for (int j = 0; j < e; ++j) tiles += (p.counts[j] + kRowPad - 1) / kRowPad;
+        s_first[e] = tiles * p.m_tiles;
     }
     tc_fence_before();
     __syncthreads();
@@ -241,7 +242,7 @@ int stream_launch(const StreamParams& p, cudaStream_t stream) {
         QMOE_CUDA(cudaFuncSetAttribute(stream_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamCfg<MODE>::SMEM_BYTES));
         configured[dev] = true;
     }
-    stream_gemm_kernel<MODE><<<sm_count(), STREAM_THREADS, StreamCfg<MODE>::SMEM_BYTES, stream>>>(p);
+    chained(stream_gemm_kernel<MODE>, sm_count(), STREAM_THREADS, StreamCfg<MODE>::SMEM_BYTES, stream, p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("stream_gemm_kernel");
     return 0;

@@ -351,29 +351,6 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
     auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
 
-    if (!STARTS_IN_SHARED) {
-        // nothing to fill: the table reads the offsets
-    } else if (p.plain_rows > 0) {
-        if (threadIdx.x == 0) { s_start_table[0] = 0; s_start_table[1] = (p.plain_rows + kRowPad - 1) / kRowPad; }
-    } else {
-        for (int i = threadIdx.x; i <= p.experts; i += NUM_THREADS) s_start_table[i] = p.offsets[i] / kRowPad;
-    }
-    if (MODE == MODE_WGRAD) {
-        // Tiles of large experts cost more (longer contraction).  Walking the experts from large to
-        // small and dealing tiles round-robin gives every CTA the same mix of long and short tiles.
-        if (p.plain_rows > 0) {
-            if (threadIdx.x == 0) { s_order[0] = 0; s_pair[0] = p.plain_rows; }
-        } else for (int i = threadIdx.x; i < p.experts; i += NUM_THREADS) {
-            const int mine = p.counts[i];
-            s_pair[i] = mine;
-            int rank = 0;
-            for (int j = 0; j < p.experts; ++j) {
-                const int other = p.counts[j];
-                rank += (other > mine || (other == mine && j < i)) ? 1 : 0;
-            }
-            s_order[rank] = i;
-        }
-    }
     if (threadIdx.x == 0) {
         s_abort = 0;
         // CTAS == 2: the copies of both CTAs count on the first CTA's full barrier; the MMA issuer (first
@@ -400,8 +377,33 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
     }
+    chain_wait();      // what follows reads global memory
+    if (!STARTS_IN_SHARED) {
+        // nothing to fill: the table reads the offsets
+    } else if (p.plain_rows > 0) {
+        if (threadIdx.x == 0) { s_start_table[0] = 0; s_start_table[1] = (p.plain_rows + kRowPad - 1) / kRowPad; }
+    } else {
+        for (int i = threadIdx.x; i <= p.experts; i += NUM_THREADS) s_start_table[i] = p.offsets[i] / kRowPad;
+    }
+    if (MODE == MODE_WGRAD) {
+        // Tiles of large experts cost more (longer contraction).  Walking the experts from large to
+        // small and dealing tiles round-robin gives every CTA the same mix of long and short tiles.
+        if (p.plain_rows > 0) {
+            if (threadIdx.x == 0) { s_order[0] = 0; s_pair[0] = p.plain_rows; }
+        } else for (int i = threadIdx.x; i < p.experts; i += NUM_THREADS) {
+            const int mine = p.counts[i];
+            s_pair[i] = mine;
+            int rank = 0;
+            for (int j = 0; j < p.experts; ++j) {
+                const int other = p.counts[j];
+                rank += (other > mine || (other == mine && j < i)) ? 1 : 0;
+            }
+            s_order[rank] = i;
+        }
+    }
     tc_fence_before();
     __syncthreads();
+    chain_next();      // the tensor memory is this block's
     if (CTAS == 2) {
         // pair-tiles of the experts before e; an odd last 128-row tile takes a pair-tile of its own
         if (MODE != MODE_WGRAD) for (int i = threadIdx.x; i <= p.experts; i += NUM_THREADS) {
@@ -1040,7 +1042,7 @@ int launch(const GemmParams& p, cudaStream_t stream) {
     if (dev >= 64) return fail_arg("device ordinal beyond 63");
     auto kernel = grouped_gemm_kernel<MODE, A_MN, B_MN, CTAS>;
     cudaLaunchConfig_t config = {};
-    cudaLaunchAttribute attribute[1];
+    cudaLaunchAttribute attribute[2];
     config.blockDim = dim3(NUM_THREADS);
     config.dynamicSmemBytes = SMEM_BYTES;
     config.stream = stream;
@@ -1049,9 +1051,10 @@ int launch(const GemmParams& p, cudaStream_t stream) {
         attribute[0].val.clusterDim.x = 2;
         attribute[0].val.clusterDim.y = 1;
         attribute[0].val.clusterDim.z = 1;
-        config.attrs = attribute;
-        config.numAttrs = 1;
     }
+    config.attrs = attribute;
+    config.numAttrs = CTAS == 2 ? 1 : 0;      // the occupancy question is about the cluster alone
+    attribute[config.numAttrs] = chain_attribute();
     if (!grid_of[dev]) {
         QMOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         int grid = sm_count();
@@ -1067,6 +1070,7 @@ int launch(const GemmParams& p, cudaStream_t stream) {
         grid_of[dev] = grid;
     }
     config.gridDim = dim3((unsigned)grid_of[dev]);
+    ++config.numAttrs;
     QMOE_CUDA(cudaLaunchKernelEx(&config, kernel, p));
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("grouped_gemm_kernel");

@@ -60,6 +60,7 @@ __device__ __forceinline__ long long label_of(const long long* labels, long long
 __global__ void __launch_bounds__(1024) head_count_kernel(const long long* __restrict__ labels, long long rows, int time,
                                                           long long vocab, float* __restrict__ factor, int* __restrict__ group,
                                                           int rows_bound) {
+    chain_begin();
     __shared__ int tmp[32];
     int mine = 0;
     for (long long r = threadIdx.x; r < rows; r += blockDim.x) mine += label_of(labels, r, time, vocab) != -100;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(1024) head_count_kernel(const long long* __res
 // (backward != 0).  16-byte pieces.
 __global__ void __launch_bounds__(256) head_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, long long dst_rows,
                                                         long long rows, int time, long long pieces, int backward) {
+    chain_begin();
     const long long total = dst_rows * pieces;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long row = i / pieces, piece = i - row * pieces;
@@ -101,6 +103,7 @@ template <typename T, bool CACHED>
 __global__ void __launch_bounds__(kThreads)
 head_loss_gradient_kernel(T* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ factor,
                           float* __restrict__ row_loss, long long rows, long long vocab, int time, int write_gradient) {
+    chain_begin();
     extern __shared__ __align__(16) uint8_t cache_raw[];
     __shared__ float tmp[kWarps];
     T* cache = reinterpret_cast<T*>(cache_raw);
@@ -191,6 +194,7 @@ __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
 __global__ void __launch_bounds__(kThreads, 3)
 head_loss_gradient_bf16_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ factor,
                                float* __restrict__ row_loss, long long rows, long long vocab, int time, int write_gradient) {
+    chain_begin();
     extern __shared__ __align__(16) uint8_t cache_raw[];
     __shared__ float tmp[kWarps];
     uint4* cache = reinterpret_cast<uint4*>(cache_raw);
@@ -273,6 +277,7 @@ head_loss_gradient_bf16_kernel(__nv_bfloat16* __restrict__ logits, const long lo
 // loss[0] = factor * sum_r row_loss[r], one block, fixed order
 __global__ void __launch_bounds__(1024) head_mean_kernel(const float* __restrict__ row_loss, const float* __restrict__ factor,
                                                          float* __restrict__ loss, long long rows) {
+    chain_begin();
     __shared__ float tmp[32];
     float mine = 0.f;
     for (long long r = threadIdx.x; r < rows; r += blockDim.x) mine += row_loss[r];
@@ -289,6 +294,7 @@ __global__ void __launch_bounds__(1024) head_mean_kernel(const float* __restrict
 // values[i] *= scalar[0]
 template <typename T>
 __global__ void __launch_bounds__(256) head_scale_kernel(T* __restrict__ values, const float* __restrict__ scalar, long long n) {
+    chain_begin();
     const float s = scalar[0];
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         Act<T>::store(values + i, Act<T>::load(values + i) * s);
@@ -329,9 +335,9 @@ int launch_loss_pass(T* logits, const long long* labels, const float* factor, fl
             if (vocab >= kTwoPassVocab && vocab % 8 == 0 && ((uintptr_t)logits & 15u) == 0) kernel = head_loss_gradient_bf16_kernel;
         const int smem = (int)((bytes + 15) / 16 * 16);
         QMOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxCachedRowBytes));
-        kernel<<<(unsigned)rows, kThreads, smem, stream>>>(logits, labels, factor, row_loss, rows, vocab, time, write_gradient);
+        chained(kernel, (unsigned)rows, kThreads, smem, stream, logits, labels, factor, row_loss, rows, vocab, time, write_gradient);
     } else {
-        head_loss_gradient_kernel<T, false><<<(unsigned)rows, kThreads, 0, stream>>>(logits, labels, factor, row_loss, rows, vocab, time,
+        chained(head_loss_gradient_kernel<T, false>, (unsigned)rows, kThreads, 0, stream, logits, labels, factor, row_loss, rows, vocab, time,
                                                                                       write_gradient);
     }
     QMOE_LAUNCH_CHECK("head_loss_gradient_kernel");
@@ -348,6 +354,7 @@ int launch_loss_gradient(const qmoe_head_t* h, long long rows, cudaStream_t stre
 template <typename T>
 __global__ void __launch_bounds__(256) head_rows_range_kernel(const T* __restrict__ src, T* __restrict__ dst, long long start,
                                                               long long count, long long width, int time, int backward) {
+    chain_begin();
     const long long total = count * width;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long row = start + i / width, at = ((row / (time - 1)) * time + row % (time - 1)) * width + i % width;
@@ -357,6 +364,7 @@ __global__ void __launch_bounds__(256) head_rows_range_kernel(const T* __restric
 }
 // out[0] = scale * sum of values (fixed order); scale = numerator[0] / denominator when numerator is given
 __global__ void __launch_bounds__(1024) head_sum_kernel(const float* __restrict__ values, float* __restrict__ out, long long n) {
+    chain_begin();
     __shared__ float tmp[32];
     float mine = 0.f;
     for (long long r = threadIdx.x; r < n; r += blockDim.x) mine += values[r];
@@ -370,6 +378,7 @@ __global__ void __launch_bounds__(1024) head_sum_kernel(const float* __restrict_
     }
 }
 __global__ void head_factor_kernel(const float* __restrict__ gradient, float count, float* __restrict__ factor) {
+    chain_begin();
     factor[0] = gradient[0] / count;
 }
 
@@ -384,11 +393,11 @@ extern "C" int qmoe_head_forward(const qmoe_head_t* h, uint64_t stream_) {
     const long long rows = (long long)h->batch * (h->time - 1), element = h->dtype == QMOE_BF16 ? 2 : 4;
     {
         TimedScope timed(KC_OTHER, stream);
-        head_count_kernel<<<1, 1024, 0, stream>>>((const long long*)h->labels, rows, h->time, h->vocab, (float*)h->meta, (int*)(h->meta + 16),
+        chained(head_count_kernel, 1, 1024, 0, stream, (const long long*)h->labels, rows, h->time, h->vocab, (float*)h->meta, (int*)(h->meta + 16),
                                                   (int)h->rows_bound);
         QMOE_LAUNCH_CHECK("head_count_kernel");
         const long long pieces = h->width * element / 16;
-        head_rows_kernel<<<grid_for(h->rows_bound * pieces), 256, 0, stream>>>((const uint4*)h->hidden, (uint4*)h->inputs, h->rows_bound, rows,
+        chained(head_rows_kernel, grid_for(h->rows_bound * pieces), 256, 0, stream, (const uint4*)h->hidden, (uint4*)h->inputs, h->rows_bound, rows,
                                                                                h->time, pieces, 0);
         QMOE_LAUNCH_CHECK("head_rows_kernel");
     }
@@ -408,7 +417,7 @@ extern "C" int qmoe_head_forward(const qmoe_head_t* h, uint64_t stream_) {
     }
     TimedScope timed(KC_HEAD_LOSS, stream);
     if (int rc = h->dtype == QMOE_BF16 ? launch_loss_gradient<__nv_bfloat16>(h, rows, stream) : launch_loss_gradient<float>(h, rows, stream)) return rc;
-    head_mean_kernel<<<1, 1024, 0, stream>>>((const float*)h->row_loss, (const float*)h->meta, (float*)h->loss, rows);
+    chained(head_mean_kernel, 1, 1024, 0, stream, (const float*)h->row_loss, (const float*)h->meta, (float*)h->loss, rows);
     QMOE_LAUNCH_CHECK("head_mean_kernel");
     return 0;
 }
@@ -437,12 +446,12 @@ extern "C" int qmoe_head_backward(const qmoe_head_t* h, uint64_t gradient, uint6
         }
         TimedScope timed(KC_OTHER, stream);
         const long long pieces = h->width * element / 16, hidden_rows = (long long)h->batch * h->time;
-        head_rows_kernel<<<grid_for(hidden_rows * pieces), 256, 0, stream>>>((const uint4*)h->d_inputs, (uint4*)h->d_hidden, hidden_rows, rows,
+        chained(head_rows_kernel, grid_for(hidden_rows * pieces), 256, 0, stream, (const uint4*)h->d_inputs, (uint4*)h->d_hidden, hidden_rows, rows,
                                                                              h->time, pieces, 1);
         QMOE_LAUNCH_CHECK("head_rows_kernel");
         if (gradient) {
-            if (h->dtype == QMOE_BF16) head_scale_kernel<<<grid_for(hidden_rows * h->width), 256, 0, stream>>>((__nv_bfloat16*)h->d_hidden, (const float*)gradient, hidden_rows * h->width);
-            else head_scale_kernel<<<grid_for(hidden_rows * h->width), 256, 0, stream>>>((float*)h->d_hidden, (const float*)gradient, hidden_rows * h->width);
+            if (h->dtype == QMOE_BF16) chained(head_scale_kernel<__nv_bfloat16>, grid_for(hidden_rows * h->width), 256, 0, stream, (__nv_bfloat16*)h->d_hidden, (const float*)gradient, hidden_rows * h->width);
+            else chained(head_scale_kernel<float>, grid_for(hidden_rows * h->width), 256, 0, stream, (float*)h->d_hidden, (const float*)gradient, hidden_rows * h->width);
             QMOE_LAUNCH_CHECK("head_scale_kernel");
         }
     }
@@ -462,7 +471,7 @@ extern "C" int qmoe_head_backward(const qmoe_head_t* h, uint64_t gradient, uint6
         }
         if (gradient) {
             TimedScope timed(KC_OTHER, stream);
-            head_scale_kernel<<<grid_for(h->vocab * h->width), 256, 0, stream>>>((float*)h->d_weight, (const float*)gradient, h->vocab * h->width);
+            chained(head_scale_kernel<float>, grid_for(h->vocab * h->width), 256, 0, stream, (float*)h->d_weight, (const float*)gradient, h->vocab * h->width);
             QMOE_LAUNCH_CHECK("head_scale_kernel");
         }
     }
@@ -479,10 +488,10 @@ extern "C" int qmoe_head_rows(uint64_t values, uint64_t out, int32_t dtype, int6
     TimedScope timed(KC_OTHER, stream);
     // forward: values = hidden, out = the rows; backward: values = the rows' gradient, out = the hidden gradient added to
     if (dtype == QMOE_BF16)
-        head_rows_range_kernel<<<grid_for(count * width), 256, 0, stream>>>((const __nv_bfloat16*)values, (__nv_bfloat16*)out, start, count, width,
+        chained(head_rows_range_kernel<__nv_bfloat16>, grid_for(count * width), 256, 0, stream, (const __nv_bfloat16*)values, (__nv_bfloat16*)out, start, count, width,
                                                                             (int)time, backward);
     else
-        head_rows_range_kernel<<<grid_for(count * width), 256, 0, stream>>>((const float*)values, (float*)out, start, count, width, (int)time,
+        chained(head_rows_range_kernel<float>, grid_for(count * width), 256, 0, stream, (const float*)values, (float*)out, start, count, width, (int)time,
                                                                             backward);
     QMOE_LAUNCH_CHECK("head_rows_range_kernel");
     return 0;
@@ -499,7 +508,7 @@ extern "C" int qmoe_head_loss(uint64_t logits, int32_t dtype, uint64_t labels, u
     if (int rc = dtype == QMOE_BF16 ? launch_loss_pass<__nv_bfloat16>((__nv_bfloat16*)logits, targets, nullptr, (float*)row_loss, rows, vocab, 0, 0, stream)
                                     : launch_loss_pass<float>((float*)logits, targets, nullptr, (float*)row_loss, rows, vocab, 0, 0, stream))
         return rc;
-    head_sum_kernel<<<1, 1024, 0, stream>>>((const float*)row_loss, (float*)out, rows);
+    chained(head_sum_kernel, 1, 1024, 0, stream, (const float*)row_loss, (float*)out, rows);
     QMOE_LAUNCH_CHECK("head_sum_kernel");
     return 0;
 }
@@ -511,7 +520,7 @@ extern "C" int qmoe_head_gradient(uint64_t logits, int32_t dtype, uint64_t label
     if (dtype != QMOE_BF16 && dtype != QMOE_F32) return fail_arg("head_gradient: dtype must be QMOE_F32 or QMOE_BF16");
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_OTHER, stream);
-    head_factor_kernel<<<1, 1, 0, stream>>>((const float*)gradient, (float)count, (float*)factor);
+    chained(head_factor_kernel, 1, 1, 0, stream, (const float*)gradient, (float)count, (float*)factor);
     QMOE_LAUNCH_CHECK("head_factor_kernel");
     const long long* targets = (const long long*)labels + start;
     return dtype == QMOE_BF16 ? launch_loss_pass<__nv_bfloat16>((__nv_bfloat16*)logits, targets, (const float*)factor, nullptr, rows, vocab, 0, 1, stream)

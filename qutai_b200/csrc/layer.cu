@@ -248,6 +248,7 @@ int wgrad_splits(long long m, long long k, long long n) {
 }
 
 __global__ void fill_split_table_kernel(int* table, int splits, int rows_per_split, int rows) {
+    chain_begin();
     const int i = threadIdx.x;
     if (i <= splits) table[i] = i * rows_per_split;
     if (i < splits) {
@@ -257,6 +258,7 @@ __global__ void fill_split_table_kernel(int* table, int splits, int rows_per_spl
 }
 // out = slab 0 + slab 1 + ... in that order, four values per thread
 __global__ void __launch_bounds__(256) sum_slabs_kernel(const float4* __restrict__ slabs, float4* __restrict__ out, int count, long long quads) {
+    chain_begin();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (long long)gridDim.x * blockDim.x) {
         float4 total = slabs[i];
         for (int s = 1; s < count; ++s) {
@@ -287,7 +289,7 @@ extern "C" int qmoe_gemm_wgrad_split(uint64_t a, uint64_t b, uint64_t c, uint64_
     TimedScope timed(KC_WGRAD_GEMM, stream);
     int* table = (int*)partials;
     float* slabs = (float*)partials + kSplitTableInts;
-    fill_split_table_kernel<<<1, 32, 0, stream>>>(table, splits, (int)split_rows(k, splits), (int)k);
+    chained(fill_split_table_kernel, 1, 32, 0, stream, table, splits, (int)split_rows(k, splits), (int)k);
     QMOE_LAUNCH_CHECK("fill_split_table_kernel");
     qmoe_route_t r = {};
     r.rows_bound = k;
@@ -297,7 +299,7 @@ extern "C" int qmoe_gemm_wgrad_split(uint64_t a, uint64_t b, uint64_t c, uint64_
     const long long quads = m * n / 4;
     long long blocks = (quads + 255) / 256;
     if (blocks > 8ll * sm_count()) blocks = 8ll * sm_count();
-    sum_slabs_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const float4*)slabs, (float4*)c, splits, quads);
+    chained(sum_slabs_kernel, (unsigned)blocks, 256, 0, stream, (const float4*)slabs, (float4*)c, splits, quads);
     QMOE_LAUNCH_CHECK("sum_slabs_kernel");
     return 0;
 }

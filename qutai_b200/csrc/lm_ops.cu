@@ -56,6 +56,7 @@ template <typename TX, typename TO, bool VEC>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_kernel(const TX* __restrict__ x, const float* __restrict__ weight, TO* __restrict__ out, float* __restrict__ inverse,
                 long long rows, long long width, float eps) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5), nwarps = (long long)gridDim.x * kWarpsPerBlock;
     for (long long r = warp; r < rows; r += nwarps) {
@@ -98,6 +99,7 @@ template <typename TG, typename TX, bool VEC>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_dx_kernel(const TG* __restrict__ gradient, const TX* __restrict__ x, const float* __restrict__ weight,
                    const float* __restrict__ inverse, TX* __restrict__ dx, long long rows, long long width) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5), nwarps = (long long)gridDim.x * kWarpsPerBlock;
     for (long long r = warp; r < rows; r += nwarps) {
@@ -137,6 +139,7 @@ template <typename TG, typename TX, bool VEC>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_dw_partial_kernel(const TG* __restrict__ gradient, const TX* __restrict__ x, const float* __restrict__ inverse,
                            float* __restrict__ partial, long long rows, long long width) {
+    chain_begin();
     const long long first = (long long)blockIdx.x * kSlabRows;
     const long long last = first + kSlabRows < rows ? first + kSlabRows : rows;
     if (VEC) {   // a thread owns eight neighbouring columns; the rows are added in order, four of them in flight
@@ -171,6 +174,7 @@ rms_norm_dw_partial_kernel(const TG* __restrict__ gradient, const TX* __restrict
 // their sums are added in the order of w: the same tree on every run.
 __global__ void __launch_bounds__(kThreads)
 sum_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, long long slabs, long long width) {
+    chain_begin();
     __shared__ float part[kWarpsPerBlock][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (long long c0 = (long long)blockIdx.x * 32; c0 < width; c0 += (long long)gridDim.x * 32) {
@@ -195,6 +199,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 rope_kernel(const T* __restrict__ values, T* __restrict__ out, long long pairs, int time, int heads, int dim, float theta,
             int offset, int inverse) {
+    chain_begin();
     const int half = dim / 2;
     const float step = -2.f * log2f(theta) / (float)dim;
     for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < pairs; i += (long long)gridDim.x * kThreads) {
@@ -215,6 +220,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 rope_heads_kernel(const T* __restrict__ values, T* __restrict__ out, long long positions, int time, int heads, int dim, float theta,
                   int offset, int inverse) {
+    chain_begin();
     const int groups = dim / 8;
     const float step = -2.f * log2f(theta) / (float)dim;
     for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < positions * groups; i += (long long)gridDim.x * kThreads) {
@@ -246,6 +252,7 @@ template <typename TO>
 __global__ void __launch_bounds__(kThreads)
 embedding_kernel(const float* __restrict__ weight, const long long* __restrict__ ids, TO* __restrict__ out, long long count,
                  long long width, long long vocab) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5), nwarps = (long long)gridDim.x * kWarpsPerBlock;
     for (long long i = warp; i < count; i += nwarps) {
@@ -262,6 +269,7 @@ __global__ void __launch_bounds__(kThreads)
 embedding_backward_kernel(const TG* __restrict__ gradient, const long long* __restrict__ tokens, const long long* __restrict__ starts,
                           const long long* __restrict__ positions, float* __restrict__ d_weight, long long segments, long long width,
                           long long vocab, long long count, int parts) {
+    chain_begin();
     // A warp owns (segment, part): columns [part * span, (part + 1) * span) of the token's row.
     // A frequent token has thousands of positions (Zipf-distributed ids put a third of a batch on one token); its
     // row is walked by `parts` warps side by side, each adding the positions in the order given, four rows in flight.
@@ -342,8 +350,8 @@ extern "C" int qmoe_rms_norm(uint64_t x, int32_t x_dtype, uint64_t weight, uint6
     const bool vec = width % 8 == 0 && !((x | out | weight) & 31u);
 #define QMOE_RMS_FORWARD(TX, TO)                                                                                               \
     do {                                                                                                                       \
-        if (vec) rms_norm_kernel<TX, TO, true><<<grid, kThreads, 0, stream>>>((const TX*)x, w, (TO*)out, inv, rows, width, (float)eps);  \
-        else rms_norm_kernel<TX, TO, false><<<grid, kThreads, 0, stream>>>((const TX*)x, w, (TO*)out, inv, rows, width, (float)eps);     \
+        if (vec) chained(rms_norm_kernel<TX, TO, true>, grid, kThreads, 0, stream, (const TX*)x, w, (TO*)out, inv, rows, width, (float)eps);  \
+        else chained(rms_norm_kernel<TX, TO, false>, grid, kThreads, 0, stream, (const TX*)x, w, (TO*)out, inv, rows, width, (float)eps);     \
     } while (0)
     if (x_dtype == QMOE_BF16 && out_dtype == QMOE_F32) QMOE_RMS_FORWARD(__nv_bfloat16, float);
     else if (x_dtype == QMOE_BF16) QMOE_RMS_FORWARD(__nv_bfloat16, __nv_bfloat16);
@@ -374,10 +382,10 @@ extern "C" int qmoe_rms_norm_backward(uint64_t gradient, int32_t g_dtype, uint64
     const bool vec = width % 8 == 0 && !((gradient | x | dx | weight | partials) & 31u);
 #define QMOE_RMS_BACKWARD(TG, TX)                                                                                              \
     do {                                                                                                                       \
-        if (vec) rms_norm_dx_kernel<TG, TX, true><<<grid, kThreads, 0, stream>>>((const TG*)gradient, (const TX*)x, w, inv, (TX*)dx, rows, width);   \
-        else rms_norm_dx_kernel<TG, TX, false><<<grid, kThreads, 0, stream>>>((const TG*)gradient, (const TX*)x, w, inv, (TX*)dx, rows, width);      \
-        if (vec) rms_norm_dw_partial_kernel<TG, TX, true><<<(unsigned)slabs, kThreads, 0, stream>>>((const TG*)gradient, (const TX*)x, inv, part, rows, width); \
-        else rms_norm_dw_partial_kernel<TG, TX, false><<<(unsigned)slabs, kThreads, 0, stream>>>((const TG*)gradient, (const TX*)x, inv, part, rows, width); \
+        if (vec) chained(rms_norm_dx_kernel<TG, TX, true>, grid, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, w, inv, (TX*)dx, rows, width);   \
+        else chained(rms_norm_dx_kernel<TG, TX, false>, grid, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, w, inv, (TX*)dx, rows, width);      \
+        if (vec) chained(rms_norm_dw_partial_kernel<TG, TX, true>, (unsigned)slabs, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, inv, part, rows, width); \
+        else chained(rms_norm_dw_partial_kernel<TG, TX, false>, (unsigned)slabs, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, inv, part, rows, width); \
     } while (0)
     if (g_dtype == QMOE_BF16 && x_dtype == QMOE_BF16) QMOE_RMS_BACKWARD(__nv_bfloat16, __nv_bfloat16);
     else if (g_dtype == QMOE_BF16) QMOE_RMS_BACKWARD(__nv_bfloat16, float);
@@ -385,7 +393,7 @@ extern "C" int qmoe_rms_norm_backward(uint64_t gradient, int32_t g_dtype, uint64
     else QMOE_RMS_BACKWARD(float, float);
 #undef QMOE_RMS_BACKWARD
     QMOE_LAUNCH_CHECK("rms_norm_dx_kernel");
-    sum_partials_kernel<<<(unsigned)((width + 31) / 32), kThreads, 0, stream>>>(part, (float*)d_weight, slabs, width);
+    chained(sum_partials_kernel, (unsigned)((width + 31) / 32), kThreads, 0, stream, part, (float*)d_weight, slabs, width);
     QMOE_LAUNCH_CHECK("sum_partials_kernel");
     return 0;
 }
@@ -400,16 +408,16 @@ extern "C" int qmoe_rope(uint64_t values, uint64_t out, int32_t dtype, int64_t b
     const long long pairs = batch * time * heads * (dim / 2), positions = batch * time;
     const bool by_position = dim % 8 == 0 && !((values | out) & 31u);
     if (by_position && dtype == QMOE_BF16)
-        rope_heads_kernel<<<flat_grid(positions * (dim / 8)), kThreads, 0, stream>>>((const __nv_bfloat16*)values, (__nv_bfloat16*)out, positions,
+        chained(rope_heads_kernel<__nv_bfloat16>, flat_grid(positions * (dim / 8)), kThreads, 0, stream, (const __nv_bfloat16*)values, (__nv_bfloat16*)out, positions,
                                                                                      (int)time, heads, dim, (float)theta, offset, inverse);
     else if (by_position)
-        rope_heads_kernel<<<flat_grid(positions * (dim / 8)), kThreads, 0, stream>>>((const float*)values, (float*)out, positions, (int)time,
+        chained(rope_heads_kernel<float>, flat_grid(positions * (dim / 8)), kThreads, 0, stream, (const float*)values, (float*)out, positions, (int)time,
                                                                                      heads, dim, (float)theta, offset, inverse);
     else if (dtype == QMOE_BF16)
-        rope_kernel<<<flat_grid(pairs), kThreads, 0, stream>>>((const __nv_bfloat16*)values, (__nv_bfloat16*)out, pairs, (int)time, heads, dim,
+        chained(rope_kernel<__nv_bfloat16>, flat_grid(pairs), kThreads, 0, stream, (const __nv_bfloat16*)values, (__nv_bfloat16*)out, pairs, (int)time, heads, dim,
                                                                (float)theta, offset, inverse);
     else
-        rope_kernel<<<flat_grid(pairs), kThreads, 0, stream>>>((const float*)values, (float*)out, pairs, (int)time, heads, dim, (float)theta,
+        chained(rope_kernel<float>, flat_grid(pairs), kThreads, 0, stream, (const float*)values, (float*)out, pairs, (int)time, heads, dim, (float)theta,
                                                                offset, inverse);
     QMOE_LAUNCH_CHECK("rope_kernel");
     return 0;
@@ -423,9 +431,9 @@ extern "C" int qmoe_embedding(uint64_t weight, uint64_t ids, uint64_t out, int32
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_ELEMENTWISE, stream);
     if (out_dtype == QMOE_BF16)
-        embedding_kernel<<<row_grid(count), kThreads, 0, stream>>>((const float*)weight, (const long long*)ids, (__nv_bfloat16*)out, count, width, vocab);
+        chained(embedding_kernel<__nv_bfloat16>, row_grid(count), kThreads, 0, stream, (const float*)weight, (const long long*)ids, (__nv_bfloat16*)out, count, width, vocab);
     else
-        embedding_kernel<<<row_grid(count), kThreads, 0, stream>>>((const float*)weight, (const long long*)ids, (float*)out, count, width, vocab);
+        chained(embedding_kernel<float>, row_grid(count), kThreads, 0, stream, (const float*)weight, (const long long*)ids, (float*)out, count, width, vocab);
     QMOE_LAUNCH_CHECK("embedding_kernel");
     return 0;
 }
@@ -471,7 +479,7 @@ extern "C" int qmoe_embedding_backward(uint64_t gradient, int32_t g_dtype, uint6
     const int parts = vec ? (int)((width + 255) / 256) : 1;
     const int grid = row_grid(segments * parts);
 #define QMOE_EMBEDDING_BACKWARD(TG, VEC)                                                                                              \
-    embedding_backward_kernel<TG, VEC><<<grid, kThreads, 0, stream>>>((const TG*)gradient, (const long long*)tokens, (const long long*)starts, \
+    chained(embedding_backward_kernel<TG, VEC>, grid, kThreads, 0, stream, (const TG*)gradient, (const long long*)tokens, (const long long*)starts, \
                                                                       (const long long*)positions, (float*)d_weight, segments, width, vocab, \
                                                                       count, parts)
     if (g_dtype == QMOE_BF16) {

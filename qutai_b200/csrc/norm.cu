@@ -42,6 +42,7 @@ template <int N> __device__ __forceinline__ void load_f32(const float* p, float*
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kThreads)
 rms_inverse_kernel(const T* __restrict__ x, float* __restrict__ inverse, long long tokens, long long width, float eps) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -71,6 +72,7 @@ rms_inverse_kernel(const T* __restrict__ x, float* __restrict__ inverse, long lo
 __global__ void __launch_bounds__(kThreads)
 scale_kernel(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ row_scale,
              const float* __restrict__ col_scale, long long rows, long long cols) {
+    chain_begin();
     const long long n = rows * cols;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / cols;
@@ -87,6 +89,7 @@ __global__ void __launch_bounds__(kThreads)
 permute_norm_kernel(const T* __restrict__ x, const float* __restrict__ inverse, const float* __restrict__ weight,
                     T* __restrict__ out, const int* __restrict__ dest_row, const int* __restrict__ offsets,
                     const int* __restrict__ counts, int experts, int pad_bits, long long tokens, int k, long long width, int part_bits) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -127,6 +130,7 @@ template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 combine_residual_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const int* __restrict__ dest_row,
                         const T* __restrict__ residual, T* __restrict__ out, long long tokens, int k, long long width, int part_bits) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -189,6 +193,7 @@ unpermute_norm_backward_kernel(const T* __restrict__ dxd, const float* __restric
                                const int* __restrict__ dest_row, const T* __restrict__ x, const float* __restrict__ inverse,
                                const float* __restrict__ weight, const T* __restrict__ grad_out, T* __restrict__ dx,
                                float* __restrict__ partials, long long tokens, int k, long long width) {
+    chain_begin();
     extern __shared__ float s_dw[];  // [warps][width]
     const int lane = threadIdx.x & 31, warp_in_block = threadIdx.x >> 5;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + warp_in_block;
@@ -314,6 +319,7 @@ int backward_grid(long long tokens, long long width) {
 // out[c] = sum over rows of partials[row, c] in a fixed order: 32 strided partial sums per column, then those 32 in order
 __global__ void __launch_bounds__(1024)
 reduce_rows_kernel(const float* __restrict__ partials, float* __restrict__ out, int rows, long long width) {
+    chain_begin();
     __shared__ float s_part[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const long long c = (long long)blockIdx.x * 32 + tx;
@@ -337,11 +343,11 @@ using namespace qmoe;
 
 #define BY_K(KERNEL, T, V, ...)                                                   \
     do {                                                                          \
-        if (r->top_k <= 1) KERNEL<T, V, 1> __VA_ARGS__;                            \
-        else if (r->top_k <= 2) KERNEL<T, V, 2> __VA_ARGS__;                       \
-        else if (r->top_k <= 4) KERNEL<T, V, 4> __VA_ARGS__;                       \
-        else if (r->top_k <= 6) KERNEL<T, V, 6> __VA_ARGS__;                       \
-        else KERNEL<T, V, 8> __VA_ARGS__;                                          \
+        if (r->top_k <= 1) chained(KERNEL<T, V, 1>, __VA_ARGS__);                            \
+        else if (r->top_k <= 2) chained(KERNEL<T, V, 2>, __VA_ARGS__);                       \
+        else if (r->top_k <= 4) chained(KERNEL<T, V, 4>, __VA_ARGS__);                       \
+        else if (r->top_k <= 6) chained(KERNEL<T, V, 6>, __VA_ARGS__);                       \
+        else chained(KERNEL<T, V, 8>, __VA_ARGS__);                                          \
     } while (0)
 #define BY_TYPE(KERNEL, ...)                                                       \
     do {                                                                          \
@@ -359,14 +365,14 @@ extern "C" int qmoe_rms_inverse(uint64_t x, int32_t dtype, uint64_t inverse, int
     const int grid = grid_for_rows(tokens, 8);
     if (dtype == QMOE_BF16) {
         if (can_vec<__nv_bfloat16>(width, {x}))
-            rms_inverse_kernel<__nv_bfloat16, true><<<grid, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (float*)inverse, tokens, width, (float)eps);
+            chained(rms_inverse_kernel<__nv_bfloat16, true>, grid, kThreads, 0, stream, (const __nv_bfloat16*)x, (float*)inverse, tokens, width, (float)eps);
         else
-            rms_inverse_kernel<__nv_bfloat16, false><<<grid, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (float*)inverse, tokens, width, (float)eps);
+            chained(rms_inverse_kernel<__nv_bfloat16, false>, grid, kThreads, 0, stream, (const __nv_bfloat16*)x, (float*)inverse, tokens, width, (float)eps);
     } else {
         if (can_vec<float>(width, {x}))
-            rms_inverse_kernel<float, true><<<grid, kThreads, 0, stream>>>((const float*)x, (float*)inverse, tokens, width, (float)eps);
+            chained(rms_inverse_kernel<float, true>, grid, kThreads, 0, stream, (const float*)x, (float*)inverse, tokens, width, (float)eps);
         else
-            rms_inverse_kernel<float, false><<<grid, kThreads, 0, stream>>>((const float*)x, (float*)inverse, tokens, width, (float)eps);
+            chained(rms_inverse_kernel<float, false>, grid, kThreads, 0, stream, (const float*)x, (float*)inverse, tokens, width, (float)eps);
     }
     QMOE_LAUNCH_CHECK("rms_inverse_kernel");
     return 0;
@@ -379,7 +385,7 @@ extern "C" int qmoe_scale_f32(uint64_t in, uint64_t out, uint64_t row_scale, uin
     TimedScope timed(KC_NORM, stream);
     const long long n = rows * cols;
     const long long blocks = (n + kThreads - 1) / kThreads, cap = (long long)sm_count() * 8;
-    scale_kernel<<<(int)(blocks < cap ? blocks : cap), kThreads, 0, stream>>>((const float*)in, (float*)out, (const float*)row_scale,
+    chained(scale_kernel, (int)(blocks < cap ? blocks : cap), kThreads, 0, stream, (const float*)in, (float*)out, (const float*)row_scale,
                                                                              (const float*)col_scale, rows, cols);
     QMOE_LAUNCH_CHECK("scale_kernel");
     return 0;
@@ -402,8 +408,8 @@ int qmoe::launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t invers
     const long long warps = r->tokens << part_bits;
     const int pad_bits = pad == kRowPad ? 7 : 4;
     const int grid = grid_for_rows(warps > (long long)r->experts * pad / 2 ? warps : (long long)r->experts * pad / 2, 8);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (const float*)inverse, (const float*)norm_weight, (T*)out,       \
-        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits)
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)x, (const float*)inverse, (const float*)norm_weight, (T*)out,       \
+        (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits
     if (dtype == QMOE_BF16) { if (vec) BY_K(permute_norm_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(permute_norm_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(permute_norm_kernel, float, true, ARGS(float)); else BY_K(permute_norm_kernel, float, false, ARGS(float)); }
 #undef ARGS
@@ -421,8 +427,8 @@ extern "C" int qmoe_combine_residual(const qmoe_route_t* r, uint64_t y, uint64_t
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {y, residual, out}) : can_vec<float>(width, {y, residual, out});
     const int part_bits = part_bits_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
     const int grid = grid_for_rows(r->tokens << part_bits, 8);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row,           \
-        (const T*)residual, (T*)out, (long long)r->tokens, r->top_k, (long long)width, part_bits)
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row,           \
+        (const T*)residual, (T*)out, (long long)r->tokens, r->top_k, (long long)width, part_bits
     if (dtype == QMOE_BF16) { if (vec) BY_K(combine_residual_kernel, __nv_bfloat16, true, ARGS(__nv_bfloat16)); else BY_K(combine_residual_kernel, __nv_bfloat16, false, ARGS(__nv_bfloat16)); }
     else { if (vec) BY_K(combine_residual_kernel, float, true, ARGS(float)); else BY_K(combine_residual_kernel, float, false, ARGS(float)); }
 #undef ARGS
@@ -457,7 +463,7 @@ extern "C" int qmoe_unpermute_norm_backward(const qmoe_route_t* r, uint64_t d_di
     do {                                                                                                                       \
         auto kernel = unpermute_norm_backward_kernel<T, V, K>;                                                                 \
         if (smem > 48 * 1024) QMOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        kernel<<<grid, kThreads, smem, stream>>>((const T*)d_dispatched, (const float*)extra_f32, extra_row_scaled,            \
+        chained(kernel, grid, kThreads, smem, stream, (const T*)d_dispatched, (const float*)extra_f32, extra_row_scaled,            \
             (const int*)r->dest_row,                                                                                           \
             (const T*)x, (const float*)inverse, (const float*)norm_weight, (const T*)grad_out, (T*)dx, (float*)partials,      \
             (long long)r->tokens, r->top_k, (long long)width);                                                                 \
@@ -472,7 +478,7 @@ extern "C" int qmoe_unpermute_norm_backward(const qmoe_route_t* r, uint64_t d_di
 #undef LAUNCH_K
 #undef LAUNCH
     QMOE_LAUNCH_CHECK("unpermute_norm_backward_kernel");
-    reduce_rows_kernel<<<(int)((width + 31) / 32), 1024, 0, stream>>>((const float*)partials, (float*)d_norm_weight, grid, width);
+    chained(reduce_rows_kernel, (int)((width + 31) / 32), 1024, 0, stream, (const float*)partials, (float*)d_norm_weight, grid, width);
     QMOE_LAUNCH_CHECK("reduce_rows_kernel");
     return 0;
 }

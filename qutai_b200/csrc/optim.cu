@@ -49,6 +49,7 @@ __device__ __forceinline__ void adamw_element(float& p, float g, float& m, float
 __global__ void __launch_bounds__(kOptimThreads)
 adamw_multi_kernel(const Item* __restrict__ items, int count, long long total_chunks, float lr, float b1, float b2,
                    float eps, float decay) {
+    chain_begin();
     for (long long chunk = blockIdx.x; chunk < total_chunks; chunk += gridDim.x) {
         const Item it = items[find_item(items, count, chunk)];
         const long long base = (chunk - it.first_chunk) * kChunk;
@@ -94,6 +95,7 @@ adamw_multi_kernel(const Item* __restrict__ items, int count, long long total_ch
 constexpr int kNormBlocks = 1024;
 __global__ void __launch_bounds__(kOptimThreads)
 grad_square_sum_kernel(const Item* __restrict__ items, int count, long long total_chunks, double* __restrict__ partial) {
+    chain_begin();
     __shared__ double s_sum[kOptimThreads];
     double sum = 0.0;
     for (long long chunk = blockIdx.x; chunk < total_chunks; chunk += gridDim.x) {
@@ -125,6 +127,7 @@ grad_square_sum_kernel(const Item* __restrict__ items, int count, long long tota
 // upstream: `if norm > max_norm: scale = max_norm / norm`, src/qutai/nn/optimizers.py:27-30)
 __global__ void __launch_bounds__(kNormBlocks)
 grad_norm_finish_kernel(const double* __restrict__ partial, int blocks, double max_norm, double* __restrict__ result) {
+    chain_begin();
     __shared__ double s_sum[kNormBlocks];
     s_sum[threadIdx.x] = (int)threadIdx.x < blocks ? partial[threadIdx.x] : 0.0;
     __syncthreads();
@@ -141,6 +144,7 @@ grad_norm_finish_kernel(const double* __restrict__ partial, int blocks, double m
 
 __global__ void __launch_bounds__(kOptimThreads)
 grad_scale_kernel(const Item* __restrict__ items, int count, long long total_chunks, const double* __restrict__ result) {
+    chain_begin();
     const double factor = result[1];
     if (factor == 1.0) return;
     const float f = (float)factor;
@@ -207,7 +211,7 @@ extern "C" int qmoe_adamw_multi(qmoe_optim_item_t* items, int32_t count, uint64_
     long long chunks = 0;
     if (int rc = stage_table(items, count, table, true, &chunks, stream)) return rc;
     TimedScope timed(KC_OPTIMIZER, stream);
-    adamw_multi_kernel<<<stream_grid(chunks), kOptimThreads, 0, stream>>>((const Item*)table, count, chunks, learning_rate,
+    chained(adamw_multi_kernel, stream_grid(chunks), kOptimThreads, 0, stream, (const Item*)table, count, chunks, learning_rate,
                                                                          beta1, beta2, eps, weight_decay);
     QMOE_LAUNCH_CHECK("adamw_multi_kernel");
     return 0;
@@ -224,11 +228,11 @@ extern "C" int qmoe_clip_grad_norm(qmoe_optim_item_t* items, int32_t count, uint
     double* result = (double*)scratch;       // [0] norm, [1] factor
     double* partial = result + 2;            // [kNormBlocks]
     const int blocks = (int)(chunks < kNormBlocks ? chunks : kNormBlocks);
-    grad_square_sum_kernel<<<blocks, kOptimThreads, 0, stream>>>((const Item*)table, count, chunks, partial);
+    chained(grad_square_sum_kernel, blocks, kOptimThreads, 0, stream, (const Item*)table, count, chunks, partial);
     QMOE_LAUNCH_CHECK("grad_square_sum_kernel");
-    grad_norm_finish_kernel<<<1, kNormBlocks, 0, stream>>>(partial, blocks, max_norm, result);
+    chained(grad_norm_finish_kernel, 1, kNormBlocks, 0, stream, partial, blocks, max_norm, result);
     QMOE_LAUNCH_CHECK("grad_norm_finish_kernel");
-    grad_scale_kernel<<<stream_grid(chunks), kOptimThreads, 0, stream>>>((const Item*)table, count, chunks, result);
+    chained(grad_scale_kernel, stream_grid(chunks), kOptimThreads, 0, stream, (const Item*)table, count, chunks, result);
     QMOE_LAUNCH_CHECK("grad_scale_kernel");
     return 0;
 }

@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(kThreads)
 permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restrict__ dest_row,
                const int* __restrict__ offsets, const int* __restrict__ counts, int experts, int pad_bits, long long tokens, int k,
                long long width, int part_bits) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -85,6 +86,7 @@ template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 combine_kernel(const T* __restrict__ y, const float* __restrict__ gate_w, const int* __restrict__ dest_row,
                T* __restrict__ out, long long tokens, int k, long long width, int part_bits) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -138,6 +140,7 @@ combine_backward_kernel(const T* __restrict__ g, const T* __restrict__ y, const 
                         const int* __restrict__ dest_row, const int* __restrict__ row_source,
                         const int* __restrict__ meta, T* __restrict__ dy, float* __restrict__ dw, long long tokens,
                         int k, long long width) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -205,6 +208,7 @@ template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 unpermute_kernel(const T* __restrict__ dxd, const float* __restrict__ extra, const int* __restrict__ dest_row,
                  T* __restrict__ dx, long long tokens, int k, long long width) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -278,6 +282,7 @@ template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kThreads)
 swiglu_kernel(const T* __restrict__ G, const T* __restrict__ U, T* __restrict__ H,
               const int* __restrict__ meta, long long hidden) {
+    chain_begin();
     using P = Piece<T, WIDE>;
     const long long n = (long long)meta[0] * hidden / P::N;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -294,6 +299,7 @@ template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kThreads)
 swiglu_backward_kernel(const T* __restrict__ dH, const T* __restrict__ G, const T* __restrict__ U,
                        T* __restrict__ dG, T* __restrict__ dU, const int* __restrict__ meta, long long hidden) {
+    chain_begin();
     using P = Piece<T, WIDE>;
     const long long n = (long long)meta[0] * hidden / P::N;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -315,6 +321,7 @@ swiglu_backward_kernel(const T* __restrict__ dH, const T* __restrict__ G, const 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 silu_kernel(const T* __restrict__ v, const T* __restrict__ g, T* __restrict__ out, long long n, int backward) {
+    chain_begin();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float x = Act<T>::load(v + i);
         const float s = sigmoid_stable(x);
@@ -324,6 +331,7 @@ silu_kernel(const T* __restrict__ v, const T* __restrict__ g, T* __restrict__ ou
 
 __global__ void __launch_bounds__(kThreads)
 cast_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
+    chain_begin();
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long n8 = n / 8;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride) {
@@ -342,6 +350,7 @@ cast_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst,
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 add_kernel(const T* a, const T* b, T* out, long long n, long long pieces) {
+    chain_begin();
     constexpr int N = Vec16<T>::N;
     const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
     for (long long i = first; i < pieces; i += stride) {
@@ -366,6 +375,7 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 normal_fill_kernel(T* __restrict__ out, long long n, float mean, float std, unsigned long long seed) {
+    chain_begin();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long h = mix64(mix64(seed) ^ (unsigned long long)i);
         const float u1 = ((float)(h >> 40) + 1.0f) * (1.0f / 16777216.0f);       // (0, 1]
@@ -412,7 +422,7 @@ int launch_swiglu(const qmoe_route_t* r, uint64_t g, uint64_t u, uint64_t h, int
     TimedScope timed(KC_SWIGLU, stream);
     const bool wide = !((g | u | h) & 15u);
     const int grid = grid_for_elems(r->rows_bound * hidden / (wide ? (dtype == QMOE_BF16 ? 8 : 4) : 1));
-#define SWIGLU(T, W) swiglu_kernel<T, W><<<grid, kThreads, 0, stream>>>((const T*)g, (const T*)u, (T*)h, (const int*)r->meta, hidden)
+#define SWIGLU(T, W) chained(swiglu_kernel<T, W>, grid, kThreads, 0, stream, (const T*)g, (const T*)u, (T*)h, (const int*)r->meta, hidden)
     if (dtype == QMOE_BF16) { if (wide) SWIGLU(__nv_bfloat16, true); else SWIGLU(__nv_bfloat16, false); }
     else { if (wide) SWIGLU(float, true); else SWIGLU(float, false); }
 #undef SWIGLU
@@ -426,7 +436,7 @@ int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint6
     const bool wide = !((dh | g | u | dg | du) & 15u);
     const int grid = grid_for_elems(r->rows_bound * hidden / (wide ? (dtype == QMOE_BF16 ? 8 : 4) : 1));
 #define SWIGLU(T, W) \
-    swiglu_backward_kernel<T, W><<<grid, kThreads, 0, stream>>>((const T*)dh, (const T*)g, (const T*)u, (T*)dg, (T*)du, (const int*)r->meta, hidden)
+    chained(swiglu_backward_kernel<T, W>, grid, kThreads, 0, stream, (const T*)dh, (const T*)g, (const T*)u, (T*)dg, (T*)du, (const int*)r->meta, hidden)
     if (dtype == QMOE_BF16) { if (wide) SWIGLU(__nv_bfloat16, true); else SWIGLU(__nv_bfloat16, false); }
     else { if (wide) SWIGLU(float, true); else SWIGLU(float, false); }
 #undef SWIGLU
@@ -454,14 +464,14 @@ int qmoe::launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_
     const long long warps = r->tokens << part_bits;
     const int pad_bits = pad == kRowPad ? 7 : 4;
     const int grid = grid_for_rows(warps > (long long)r->experts * pad / 2 ? warps : (long long)r->experts * pad / 2);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits)
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits
 #define BY_K(T, V)                                                  \
     do {                                                            \
-        if (r->top_k <= 1) permute_kernel<T, V, 1> ARGS(T);         \
-        else if (r->top_k <= 2) permute_kernel<T, V, 2> ARGS(T);    \
-        else if (r->top_k <= 4) permute_kernel<T, V, 4> ARGS(T);    \
-        else if (r->top_k <= 6) permute_kernel<T, V, 6> ARGS(T);    \
-        else permute_kernel<T, V, 8> ARGS(T);                       \
+        if (r->top_k <= 1) chained(permute_kernel<T, V, 1>, ARGS(T));         \
+        else if (r->top_k <= 2) chained(permute_kernel<T, V, 2>, ARGS(T));    \
+        else if (r->top_k <= 4) chained(permute_kernel<T, V, 4>, ARGS(T));    \
+        else if (r->top_k <= 6) chained(permute_kernel<T, V, 6>, ARGS(T));    \
+        else chained(permute_kernel<T, V, 8>, ARGS(T));                       \
     } while (0)
     if (dtype == QMOE_BF16) { if (vec) BY_K(__nv_bfloat16, true); else BY_K(__nv_bfloat16, false); }
     else { if (vec) BY_K(float, true); else BY_K(float, false); }
@@ -481,14 +491,14 @@ extern "C" int qmoe_combine(const qmoe_route_t* r, uint64_t y, uint64_t out, int
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {y, out}) : can_vec<float>(width, {y, out});
     const int part_bits = part_bits_per_row(r->tokens, vec ? width * (dtype == QMOE_BF16 ? 2 : 4) / 16 : width);
     const int grid = grid_for_rows(r->tokens << part_bits);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row, (T*)out, (long long)r->tokens, r->top_k, (long long)width, part_bits)
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row, (T*)out, (long long)r->tokens, r->top_k, (long long)width, part_bits
 #define BY_K(T, V)                                                  \
     do {                                                            \
-        if (r->top_k <= 1) combine_kernel<T, V, 1> ARGS(T);         \
-        else if (r->top_k <= 2) combine_kernel<T, V, 2> ARGS(T);    \
-        else if (r->top_k <= 4) combine_kernel<T, V, 4> ARGS(T);    \
-        else if (r->top_k <= 6) combine_kernel<T, V, 6> ARGS(T);    \
-        else combine_kernel<T, V, 8> ARGS(T);                       \
+        if (r->top_k <= 1) chained(combine_kernel<T, V, 1>, ARGS(T));         \
+        else if (r->top_k <= 2) chained(combine_kernel<T, V, 2>, ARGS(T));    \
+        else if (r->top_k <= 4) chained(combine_kernel<T, V, 4>, ARGS(T));    \
+        else if (r->top_k <= 6) chained(combine_kernel<T, V, 6>, ARGS(T));    \
+        else chained(combine_kernel<T, V, 8>, ARGS(T));                       \
     } while (0)
     if (dtype == QMOE_BF16) { if (vec) BY_K(__nv_bfloat16, true); else BY_K(__nv_bfloat16, false); }
     else { if (vec) BY_K(float, true); else BY_K(float, false); }
@@ -507,14 +517,14 @@ extern "C" int qmoe_combine_backward(const qmoe_route_t* r, uint64_t g, uint64_t
     TimedScope timed(KC_COMBINE_BWD, stream);
     const bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {g, y, dy}) : can_vec<float>(width, {g, y, dy});
     const int grid = grid_for_rows(r->tokens > (long long)r->experts * 64 ? r->tokens : (long long)r->experts * 64);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)g, (const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row, (const int*)r->row_source, (const int*)r->meta, (T*)dy, (float*)dw, (long long)r->tokens, r->top_k, (long long)width)
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)g, (const T*)y, (const float*)r->gate_weights, (const int*)r->dest_row, (const int*)r->row_source, (const int*)r->meta, (T*)dy, (float*)dw, (long long)r->tokens, r->top_k, (long long)width
 #define BY_K(T, V)                                                           \
     do {                                                                     \
-        if (r->top_k <= 1) combine_backward_kernel<T, V, 1> ARGS(T);         \
-        else if (r->top_k <= 2) combine_backward_kernel<T, V, 2> ARGS(T);    \
-        else if (r->top_k <= 4) combine_backward_kernel<T, V, 4> ARGS(T);    \
-        else if (r->top_k <= 6) combine_backward_kernel<T, V, 6> ARGS(T);    \
-        else combine_backward_kernel<T, V, 8> ARGS(T);                       \
+        if (r->top_k <= 1) chained(combine_backward_kernel<T, V, 1>, ARGS(T));         \
+        else if (r->top_k <= 2) chained(combine_backward_kernel<T, V, 2>, ARGS(T));    \
+        else if (r->top_k <= 4) chained(combine_backward_kernel<T, V, 4>, ARGS(T));    \
+        else if (r->top_k <= 6) chained(combine_backward_kernel<T, V, 6>, ARGS(T));    \
+        else chained(combine_backward_kernel<T, V, 8>, ARGS(T));                       \
     } while (0)
     if (dtype == QMOE_BF16) { if (vec) BY_K(__nv_bfloat16, true); else BY_K(__nv_bfloat16, false); }
     else { if (vec) BY_K(float, true); else BY_K(float, false); }
@@ -534,14 +544,14 @@ extern "C" int qmoe_unpermute_reduce(const qmoe_route_t* r, uint64_t dxd, uint64
     bool vec = dtype == QMOE_BF16 ? can_vec<__nv_bfloat16>(width, {dxd, dx}) : can_vec<float>(width, {dxd, dx});
     if (extra && (!aligned16(extra) || (width * 4) % 16)) vec = false;
     const int grid = grid_for_rows(r->tokens);
-#define ARGS(T) <<<grid, kThreads, 0, stream>>>((const T*)dxd, (const float*)extra, (const int*)r->dest_row, (T*)dx, (long long)r->tokens, r->top_k, (long long)width)
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)dxd, (const float*)extra, (const int*)r->dest_row, (T*)dx, (long long)r->tokens, r->top_k, (long long)width
 #define BY_K(T, V)                                                    \
     do {                                                              \
-        if (r->top_k <= 1) unpermute_kernel<T, V, 1> ARGS(T);         \
-        else if (r->top_k <= 2) unpermute_kernel<T, V, 2> ARGS(T);    \
-        else if (r->top_k <= 4) unpermute_kernel<T, V, 4> ARGS(T);    \
-        else if (r->top_k <= 6) unpermute_kernel<T, V, 6> ARGS(T);    \
-        else unpermute_kernel<T, V, 8> ARGS(T);                       \
+        if (r->top_k <= 1) chained(unpermute_kernel<T, V, 1>, ARGS(T));         \
+        else if (r->top_k <= 2) chained(unpermute_kernel<T, V, 2>, ARGS(T));    \
+        else if (r->top_k <= 4) chained(unpermute_kernel<T, V, 4>, ARGS(T));    \
+        else if (r->top_k <= 6) chained(unpermute_kernel<T, V, 6>, ARGS(T));    \
+        else chained(unpermute_kernel<T, V, 8>, ARGS(T));                       \
     } while (0)
     if (dtype == QMOE_BF16) { if (vec) BY_K(__nv_bfloat16, true); else BY_K(__nv_bfloat16, false); }
     else { if (vec) BY_K(float, true); else BY_K(float, false); }
@@ -557,7 +567,7 @@ extern "C" int qmoe_cast_bf16(uint64_t src, uint64_t dst, int64_t n, uint64_t st
     if (n == 0) return 0;
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_CAST, stream);
-    cast_bf16_kernel<<<grid_for_elems(n / 8 + 1), kThreads, 0, stream>>>((const float*)src, (__nv_bfloat16*)dst, n);
+    chained(cast_bf16_kernel, grid_for_elems(n / 8 + 1), kThreads, 0, stream, (const float*)src, (__nv_bfloat16*)dst, n);
     QMOE_LAUNCH_CHECK("cast_bf16_kernel");
     return 0;
 }
@@ -570,10 +580,10 @@ extern "C" int qmoe_silu(uint64_t values, uint64_t gradient, uint64_t out, int32
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_SWIGLU, stream);
     if (dtype == QMOE_BF16)
-        silu_kernel<__nv_bfloat16><<<grid_for_elems(n), kThreads, 0, stream>>>(
+        chained(silu_kernel<__nv_bfloat16>, grid_for_elems(n), kThreads, 0, stream, 
             (const __nv_bfloat16*)values, (const __nv_bfloat16*)gradient, (__nv_bfloat16*)out, n, backward);
     else
-        silu_kernel<float><<<grid_for_elems(n), kThreads, 0, stream>>>((const float*)values, (const float*)gradient,
+        chained(silu_kernel<float>, grid_for_elems(n), kThreads, 0, stream, (const float*)values, (const float*)gradient,
                                                                         (float*)out, n, backward);
     QMOE_LAUNCH_CHECK("silu_kernel");
     return 0;
@@ -589,9 +599,9 @@ extern "C" int qmoe_add(uint64_t a, uint64_t b, uint64_t out, int32_t dtype, int
     const long long pieces = aligned ? n / (dtype == QMOE_BF16 ? 8 : 4) : 0;
     const int grid = grid_for_elems(aligned ? pieces + 8 : n);
     if (dtype == QMOE_BF16)
-        add_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n, pieces);
+        chained(add_kernel<__nv_bfloat16>, grid, kThreads, 0, stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n, pieces);
     else
-        add_kernel<float><<<grid, kThreads, 0, stream>>>((const float*)a, (const float*)b, (float*)out, n, pieces);
+        chained(add_kernel<float>, grid, kThreads, 0, stream, (const float*)a, (const float*)b, (float*)out, n, pieces);
     QMOE_LAUNCH_CHECK("add_kernel");
     return 0;
 }
@@ -604,10 +614,10 @@ extern "C" int qmoe_normal_fill(uint64_t out, int32_t dtype, int64_t n, double m
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_OTHER, stream);
     if (dtype == QMOE_BF16)
-        normal_fill_kernel<__nv_bfloat16><<<grid_for_elems(n), kThreads, 0, stream>>>((__nv_bfloat16*)out, n, (float)mean,
+        chained(normal_fill_kernel<__nv_bfloat16>, grid_for_elems(n), kThreads, 0, stream, (__nv_bfloat16*)out, n, (float)mean,
                                                                                        (float)std, seed);
     else
-        normal_fill_kernel<float><<<grid_for_elems(n), kThreads, 0, stream>>>((float*)out, n, (float)mean, (float)std, seed);
+        chained(normal_fill_kernel<float>, grid_for_elems(n), kThreads, 0, stream, (float*)out, n, (float)mean, (float)std, seed);
     QMOE_LAUNCH_CHECK("normal_fill_kernel");
     return 0;
 }
@@ -618,6 +628,7 @@ namespace {
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, const int* __restrict__ index, int rows,
                    long long row_vecs, int src_rows) {
+    chain_begin();
     const long long total = (long long)rows * row_vecs;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int row = (int)(i / row_vecs);
@@ -629,6 +640,7 @@ gather_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, const
 __global__ void __launch_bounds__(256)
 gather_words_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, const int* __restrict__ index, int rows,
                     long long row_words, int src_rows) {
+    chain_begin();
     const long long total = (long long)rows * row_words;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int row = (int)(i / row_words);
@@ -649,11 +661,11 @@ extern "C" int qmoe_gather_rows(uint64_t src, uint64_t dst, uint64_t index, int3
     TimedScope timed(KC_OTHER, stream);
     if (row_bytes % 16 == 0 && !((src | dst) & 15u)) {
         const long long total = (long long)rows * (row_bytes / 16);
-        gather_rows_kernel<<<(int)((total + 255) / 256 > 1184 ? 1184 : (total + 255) / 256), 256, 0, stream>>>(
+        chained(gather_rows_kernel, (int)((total + 255) / 256 > 1184 ? 1184 : (total + 255) / 256), 256, 0, stream, 
             (const uint4*)src, (uint4*)dst, (const int*)index, rows, row_bytes / 16, src_rows);
     } else {
         const long long total = (long long)rows * (row_bytes / 4);
-        gather_words_kernel<<<(int)((total + 255) / 256 > 1184 ? 1184 : (total + 255) / 256), 256, 0, stream>>>(
+        chained(gather_words_kernel, (int)((total + 255) / 256 > 1184 ? 1184 : (total + 255) / 256), 256, 0, stream, 
             (const uint32_t*)src, (uint32_t*)dst, (const int*)index, rows, row_bytes / 4, src_rows);
     }
     QMOE_LAUNCH_CHECK("gather_rows_kernel");

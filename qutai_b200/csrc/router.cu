@@ -64,6 +64,7 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& hi, __nv_bfloat16
 __global__ void __launch_bounds__(256)
 router_split_w_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ w3, __nv_bfloat16* __restrict__ wbwd, int E, int S,
                       long long d) {
+    chain_begin();
     const long long n = (long long)S * d;
     const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -80,6 +81,7 @@ router_split_w_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ w
 __global__ void __launch_bounds__(256)
 router_split_ds_kernel(float* __restrict__ ds, const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S,
                        int* __restrict__ tables, int splits, long long rows_per_split) {
+    chain_begin();
     if (blockIdx.x == 0 && threadIdx.x <= splits) {
         const int i = threadIdx.x;
         tables[i] = (int)(i * rows_per_split);  // offsets[splits + 1]
@@ -109,6 +111,7 @@ router_split_ds_kernel(float* __restrict__ ds, const float* __restrict__ row_sca
 __global__ void __launch_bounds__(256)
 router_reduce_dw_kernel(const float* __restrict__ partial, const float* __restrict__ col_scale, float* __restrict__ dw, int E, int S, long long d,
                         int splits) {
+    chain_begin();
     const long long n = (long long)E * d;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long e = i / d, j = i - e * d;
@@ -154,6 +157,7 @@ template <typename T, bool NORM>
 __global__ void __launch_bounds__(256)
 router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float* __restrict__ scores, int E, long long d,
                     const float* __restrict__ norm_weight, float eps, float* __restrict__ inverse) {
+    chain_begin();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.y * 8 + warp;
     if (e >= E) return;
@@ -235,10 +239,10 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
         TimedScope timed(KC_ROUTER_GEMM, stream);
         const dim3 grid((unsigned)tokens, (unsigned)((experts + 7) / 8));
         if (x_dtype == QMOE_BF16)
-            router_small_kernel<__nv_bfloat16, false><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (const float*)w_router, (float*)scores,
+            chained(router_small_kernel<__nv_bfloat16, false>, grid, 256, 0, stream, (const __nv_bfloat16*)x, (const float*)w_router, (float*)scores,
                                                                                 experts, width, nullptr, 0.f, nullptr);
         else
-            router_small_kernel<float, false><<<grid, 256, 0, stream>>>((const float*)x, (const float*)w_router, (float*)scores, experts, width,
+            chained(router_small_kernel<float, false>, grid, 256, 0, stream, (const float*)x, (const float*)w_router, (float*)scores, experts, width,
                                                                         nullptr, 0.f, nullptr);
         QMOE_LAUNCH_CHECK("router_small_kernel");
         return 0;
@@ -247,7 +251,7 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
         return simt_router_logits(x, x_dtype, w_router, scores, tokens, width, experts, stream);
     TimedScope timed(KC_ROUTER_GEMM, stream);
     const RouterScratch r = plan_scratch(tokens, experts, width);
-    router_split_w_kernel<<<elem_grid((long long)r.S * width), 256, 0, stream>>>(
+    chained(router_split_w_kernel, elem_grid((long long)r.S * width), 256, 0, stream, 
         (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, r.S, width);
     QMOE_LAUNCH_CHECK("router_split_w_kernel");
     return tc_router_forward(x, scratch + r.w3, scores, tokens, width, experts, r.S, stream);
@@ -264,10 +268,10 @@ int qmoe::router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, ui
     TimedScope timed(KC_ROUTER_GEMM, stream);
     const dim3 grid((unsigned)tokens, (unsigned)((experts + 7) / 8));
     if (x_dtype == QMOE_BF16)
-        router_small_kernel<__nv_bfloat16, true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (const float*)w_router, (float*)scores, experts, width,
+        chained(router_small_kernel<__nv_bfloat16, true>, grid, 256, 0, stream, (const __nv_bfloat16*)x, (const float*)w_router, (float*)scores, experts, width,
                                                                            (const float*)norm_weight, (float)eps, (float*)inverse);
     else
-        router_small_kernel<float, true><<<grid, 256, 0, stream>>>((const float*)x, (const float*)w_router, (float*)scores, experts, width,
+        chained(router_small_kernel<float, true>, grid, 256, 0, stream, (const float*)x, (const float*)w_router, (float*)scores, experts, width,
                                                                    (const float*)norm_weight, (float)eps, (float*)inverse);
     QMOE_LAUNCH_CHECK("router_small_kernel");
     return 0;
@@ -304,10 +308,10 @@ int qmoe::router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t
     const int S = r.S;
     int* tables = (int*)(scratch + r.tables);
     // the weight terms are rebuilt here as well: the scratch may have been used by another layer since the forward
-    router_split_w_kernel<<<elem_grid((long long)S * width), 256, 0, stream>>>(
+    chained(router_split_w_kernel, elem_grid((long long)S * width), 256, 0, stream, 
         (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, S, width);
     QMOE_LAUNCH_CHECK("router_split_w_kernel");
-    router_split_ds_kernel<<<elem_grid(tokens * S), 256, 0, stream>>>((float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6),
+    chained(router_split_ds_kernel, elem_grid(tokens * S), 256, 0, stream, (float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6),
                                                                       tokens, experts, S, tables, r.splits, r.rows_per_split);
     QMOE_LAUNCH_CHECK("router_split_ds_kernel");
     if (dx_router)
@@ -315,7 +319,7 @@ int qmoe::router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t
     if (d_w_router) {
         if (int rc = tc_split_wgrad(scratch + r.ds6, 6ll * S, x, scratch + r.partial, tables, tables + r.splits + 1, r.splits,
                                     tokens, 3ll * S, width, stream)) return rc;
-        router_reduce_dw_kernel<<<elem_grid((long long)experts * width), 256, 0, stream>>>(
+        chained(router_reduce_dw_kernel, elem_grid((long long)experts * width), 256, 0, stream, 
             (const float*)(scratch + r.partial), (const float*)col_scale, (float*)d_w_router, experts, S, width, r.splits);
         QMOE_LAUNCH_CHECK("router_reduce_dw_kernel");
     }

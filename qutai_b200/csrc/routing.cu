@@ -86,6 +86,7 @@ route_topk_kernel(const float* __restrict__ scores, float* __restrict__ probs,
                   float* __restrict__ gate_w, int* __restrict__ expert_idx,
                   int* __restrict__ block_counts, float* __restrict__ block_colsum,
                   long long T, int E, int k) {
+    chain_begin();
     __shared__ int s_cnt[kMaxExperts];
     __shared__ float s_col[kWarps][32 * EPL];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -170,6 +171,7 @@ route_scan_kernel(const int* __restrict__ block_counts, const float* __restrict_
                   int* __restrict__ block_base, int* __restrict__ counts, int* __restrict__ offsets,
                   int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util,
                   float* __restrict__ aux, int nblk, long long T, int E, int k) {
+    chain_begin();
     __shared__ int s_seg[kScanThreads];
     __shared__ double s_segcs[kScanThreads];
     __shared__ int s_cnt[kMaxExperts];
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(kPackWarps * 32)
 route_pack_kernel(const int* __restrict__ expert_idx, const int* __restrict__ block_base,
                   const int* __restrict__ offsets, int* __restrict__ dest_row,
                   int* __restrict__ row_source, long long T, int E, int k) {
+    chain_begin();
     __shared__ int s_hist[kPackWarps][kMaxExperts];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < kPackWarps * kMaxExperts; i += blockDim.x) (&s_hist[0][0])[i] = 0;
@@ -281,6 +284,7 @@ route_small_kernel(const float* __restrict__ scores, float* __restrict__ probs, 
                    int* __restrict__ dest_row, int* row_source, int* __restrict__ counts, int* __restrict__ offsets,
                    int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util, float* __restrict__ aux,
                    float* __restrict__ block_colsum, int T, int E, int k, long long rows_bound) {
+    chain_begin();
     // [warp][expert]: probability sums, then assignments; one more column, so that a warp reading one expert's 32 entries
     // meets 32 banks
     __shared__ union { float col[kWarps][32 * EPL + 1]; int hist[kWarps][32 * EPL + 1]; } s;
@@ -359,6 +363,7 @@ __global__ void route_export_kernel(const int* __restrict__ expert_idx, const in
                                     long long* indices, long long* ids, long long* slots,
                                     long long* locations, long long* counts64, long long A, int E,
                                     int k, long long capacity) {
+    chain_begin();
     const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (a < E && counts64) counts64[a] = counts[a];
     if (a >= A) return;
@@ -376,6 +381,7 @@ route_backward_kernel(const float* __restrict__ probs, const float* __restrict__
                       const int* __restrict__ expert_idx, const float* __restrict__ util,
                       const float* __restrict__ grad_w, const float* __restrict__ grad_aux,
                       float* __restrict__ d_scores, long long T, int E, int k) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= T) return;
@@ -454,28 +460,28 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
     float* bs = (float*)r->block_colsum;
     const int epl = (E + 31) / 32;
     if (T <= kSmallRouteTokens) {
-#define ARGS <<<1, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, (int*)r->dest_row, (int*)r->row_source, (int*)r->counts, (int*)r->offsets, \
-        (int*)r->tile_expert, (int*)r->meta, (float*)r->utilization, (float*)r->aux, bs, (int)T, E, k, (long long)r->rows_bound)
-        if (epl <= 1) route_small_kernel<1> ARGS;
-        else if (epl <= 2) route_small_kernel<2> ARGS;
-        else if (epl <= 4) route_small_kernel<4> ARGS;
-        else route_small_kernel<8> ARGS;
+#define ARGS 1, kWarps * 32, 0, stream, sc, probs, gw, eidx, (int*)r->dest_row, (int*)r->row_source, (int*)r->counts, (int*)r->offsets, \
+        (int*)r->tile_expert, (int*)r->meta, (float*)r->utilization, (float*)r->aux, bs, (int)T, E, k, (long long)r->rows_bound
+        if (epl <= 1) chained(route_small_kernel<1>, ARGS);
+        else if (epl <= 2) chained(route_small_kernel<2>, ARGS);
+        else if (epl <= 4) chained(route_small_kernel<4>, ARGS);
+        else chained(route_small_kernel<8>, ARGS);
 #undef ARGS
         QMOE_LAUNCH_CHECK("route_small_kernel");
         return 0;
     }
     QMOE_CUDA(cudaMemsetAsync((void*)r->row_source, 0xff, (size_t)r->rows_bound * sizeof(int), stream));
-    if (epl <= 1) route_topk_kernel<1><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
-    else if (epl <= 2) route_topk_kernel<2><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
-    else if (epl <= 4) route_topk_kernel<4><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
-    else route_topk_kernel<8><<<nblk, kWarps * 32, 0, stream>>>(sc, probs, gw, eidx, bc, bs, T, E, k);
+    if (epl <= 1) chained(route_topk_kernel<1>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
+    else if (epl <= 2) chained(route_topk_kernel<2>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
+    else if (epl <= 4) chained(route_topk_kernel<4>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
+    else chained(route_topk_kernel<8>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
     QMOE_LAUNCH_CHECK("route_topk_kernel");
-    route_scan_kernel<<<1, kScanThreads, 0, stream>>>(bc, bs, (int*)r->block_base, (int*)r->counts,
+    chained(route_scan_kernel, 1, kScanThreads, 0, stream, bc, bs, (int*)r->block_base, (int*)r->counts,
                                                       (int*)r->offsets, (int*)r->tile_expert,
                                                       (int*)r->meta, (float*)r->utilization,
                                                       (float*)r->aux, nblk, T, E, k);
     QMOE_LAUNCH_CHECK("route_scan_kernel");
-    route_pack_kernel<<<nblk, kPackWarps * 32, 0, stream>>>(eidx, (const int*)r->block_base,
+    chained(route_pack_kernel, nblk, kPackWarps * 32, 0, stream, eidx, (const int*)r->block_base,
                                                         (const int*)r->offsets, (int*)r->dest_row,
                                                         (int*)r->row_source, T, E, k);
     QMOE_LAUNCH_CHECK("route_pack_kernel");
@@ -491,7 +497,7 @@ extern "C" int qmoe_route_export_i64(const qmoe_route_t* r, uint64_t indices, ui
     cudaStream_t stream = (cudaStream_t)stream_;
     TimedScope timed(KC_OTHER, stream);
     const long long n = A > r->experts ? A : r->experts;
-    route_export_kernel<<<ceil_div(n, 256), 256, 0, stream>>>(
+    chained(route_export_kernel, ceil_div(n, 256), 256, 0, stream, 
         (const int*)r->expert_index, (const int*)r->dest_row, (const int*)r->offsets,
         (const int*)r->counts, (long long*)indices, (long long*)ids, (long long*)slots,
         (long long*)locations, (long long*)counts, A, r->experts, r->top_k, capacity);
@@ -509,7 +515,7 @@ extern "C" int qmoe_route_backward(const qmoe_route_t* r, uint64_t grad_weights,
         QMOE_CUDA(cudaMemsetAsync((void*)d_scores, 0, (size_t)r->tokens * r->experts * sizeof(float), stream));
         return 0;
     }
-    route_backward_kernel<<<ceil_div(r->tokens, 8), 256, 0, stream>>>(
+    chained(route_backward_kernel, ceil_div(r->tokens, 8), 256, 0, stream, 
         (const float*)r->probs, (const float*)r->gate_weights, (const int*)r->expert_index,
         (const float*)r->utilization, (const float*)grad_weights, (const float*)grad_aux,
         (float*)d_scores, r->tokens, r->experts, r->top_k);
