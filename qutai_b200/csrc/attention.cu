@@ -18,8 +18,9 @@
 // The products of the next block are issued before the rows have finished with this one (S has a second buffer in the
 // backward and is taken into registers at once in the forward), so the row warps rarely wait for the tensor cores; what
 // bounds them is the exponential unit, 1024 cycles per 128 x 128 block and SM, and the latency of their own chain beside it.
-// 4 sequences x 2048 positions, 16 heads in 4 groups (L2 flushed): forward 142 -> 79 us, backward 470 -> 181 against the form
-// with P and dS in shared memory and one block in flight.
+// 4 sequences x 2048 positions, 16 heads in 4 groups: forward and backward 606 -> 250 us against the form with P and dS in shared memory and
+// one block in flight, 241 with O rescaled behind the exponentials and delta from coalesced loads; 3 x 1501 positions,
+// forward: 72, 37 and 32.
 // Every wait is bounded; on expiry the CTA records a code in the library's status word and leaves.
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -62,6 +63,11 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 __device__ __forceinline__ float exp2_fast(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {      // like fmaxf: a number rather than a NaN
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
     return y;
 }
 // 32 accumulator columns of one row, scaled, as 64 bytes of bf16
@@ -225,36 +231,23 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
             }
             float peak4[4] = {__uint_as_float(s[0]), __uint_as_float(s[1]), __uint_as_float(s[2]), __uint_as_float(s[3])};
 #pragma unroll
-            for (int c = 4; c < BLOCK; ++c) peak4[c & 3] = fmaxf(peak4[c & 3], __uint_as_float(s[c]));
-            const float peak = fmaxf(fmaxf(peak4[0], peak4[1]), fmaxf(peak4[2], peak4[3]));
+            for (int c = 4; c < BLOCK; c += 2) peak4[(c >> 1) & 3] = max3(peak4[(c >> 1) & 3], __uint_as_float(s[c]), __uint_as_float(s[c + 1]));
+            const float peak = fmaxf(max3(peak4[0], peak4[1], peak4[2]), peak4[3]);
             // The base of the exponentials is the maximum so far.  (Letting it lag behind by up to 2^8 would leave O alone in
             // most blocks, but then the largest probability of a row is no longer an exact 1 in bf16: 2.05e-3 instead of
             // 1.74e-3 from the exact result for scores of standard deviation 4.)
+            float alpha = 1.f;
             if (j == 0) {
                 m = peak;
             } else {
-                if (__any_sync(0xffffffffu, peak > m)) {
-                    const float m_new = fmaxf(m, peak), alpha = exp2_fast((m - m_new) * scale2);
-                    m = m_new;
-                    l *= alpha;
-                    ok = wait.all(bar(O_DONE), (uint32_t)(j - 1) & 1u);
-                    if (!ok) break;
-                    tc_fence_after();
-#pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t o[16];
-                        tmem_ld16(tmem_o + lane_base + c * 16, o);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-                        tmem_st16(tmem_o + lane_base + c * 16, o);
-                    }
-                }
+                const float m_new = fmaxf(m, peak);
+                alpha = exp2_fast((m - m_new) * scale2);
+                m = m_new;
+                l *= alpha;
             }
             // Subtract, then multiply: a single fma against m * scale2 saves an instruction, but that product is rounded, so the
             // largest probability becomes 2^(up to half an ulp of the base) instead of 1 (scores of 2e5: out 2.2e-3 instead of
-            // 2.9e-5 from the exact result, and dq, whose terms cancel, 0.31 instead of 7e-3; forward at 4 x 2048, 16 heads: 77
-            // us with it, 79 like this).
+            // 2.9e-5 from the exact result, and dq, whose terms cancel, 0.31 instead of 7e-3).
             const uint64_t minus_m = pair2(-m, -m);
             uint64_t total2[2] = {0, 0};
             uint32_t packed[BLOCK / 2];
@@ -266,10 +259,29 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
                 total2[(c >> 1) & 1] = add2(total2[(c >> 1) & 1], pair2(p0, p1));
                 packed[c >> 1] = pack2(p0, p1);
             }
-            if (j > 0) {   // the product that reads the P of the block before is done
+            if (j > 0) {
+                // the product that reads the P of the block before is done: O is whole, and the place of P free.  Only here, behind
+                // the exponentials: their registers are free for O by now, and the wait is over before it begins (before them, with
+                // 16 columns at a time, wait and rescaling took 900 of a block's 3400 cycles)
                 ok = wait.all(bar(O_DONE), (uint32_t)(j - 1) & 1u);
                 if (!ok) break;
                 tc_fence_after();
+                if (__any_sync(0xffffffffu, alpha != 1.f)) {
+                    uint32_t o[D];
+                    tmem_ld32(tmem_o + lane_base, o);
+                    tmem_ld32(tmem_o + lane_base + 32, o + 32);
+                    tmem_ld_wait();
+                    const uint64_t alpha_pair = pair2(alpha, alpha);
+#pragma unroll
+                    for (int e = 0; e < D; e += 2) {
+                        float o0, o1;
+                        unpair2(mul2(pair2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), alpha_pair), o0, o1);
+                        o[e] = __float_as_uint(o0);
+                        o[e + 1] = __float_as_uint(o1);
+                    }
+                    tmem_st32(tmem_o + lane_base, o);
+                    tmem_st32(tmem_o + lane_base + 32, o + 32);
+                }
             }
             tmem_st32(tmem_p + lane_base, packed);
             tmem_st32(tmem_p + lane_base + 32, packed + 32);
@@ -432,22 +444,35 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
         const bool live = tq < p.time;
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         const long long at = ((long long)b * p.time + (live ? tq : 0)) * p.heads + h;
-        // delta = sum_j grad_out * out of this row (kept for the dk, dv kernel), lse of this row
+        // delta = sum_j grad_out * out of this row (kept for the dk, dv kernel), lse of this row.  Eight lanes read a row, four rows
+        // per access, and all accesses are on their way before the first sum (a row per lane, 16 bytes at a time: 3 us of
+        // the 10 .. 30 of a CTA before its first block).
         float delta = 0.f, lse2 = 0.f;
-        if (live) {
-            const uint4* go = reinterpret_cast<const uint4*>(p.grad_out + at * D);
-            const uint4* oo = reinterpret_cast<const uint4*>(p.out_in + at * D);
+        {
+            uint4 a[8], o[8];
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c) {
-                const uint4 a = go[c], o = oo[c];
-                const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, ow[4] = {o.x, o.y, o.z, o.w};
+            for (int r = 0; r < 8; ++r) {
+                const int t = i * BLOCK + quad * 32 + r * 4 + (lane >> 3);
+                const long long from = (((long long)b * p.time + (t < p.time ? t : 0)) * p.heads + h) * (D / 8) + (lane & 7);
+                a[r] = reinterpret_cast<const uint4*>(p.grad_out)[from];
+                o[r] = reinterpret_cast<const uint4*>(p.out_in)[from];
+            }
+            if (live) lse2 = p.lse[at] * LOG2E;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const uint32_t aw[4] = {a[r].x, a[r].y, a[r].z, a[r].w}, ow[4] = {o[r].x, o[r].y, o[r].z, o[r].w};
+                float sum = 0.f;
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    delta += __uint_as_float(aw[e] << 16) * __uint_as_float(ow[e] << 16) +
-                             __uint_as_float(aw[e] & 0xffff0000u) * __uint_as_float(ow[e] & 0xffff0000u);
+                    sum += __uint_as_float(aw[e] << 16) * __uint_as_float(ow[e] << 16) +
+                           __uint_as_float(aw[e] & 0xffff0000u) * __uint_as_float(ow[e] & 0xffff0000u);
+#pragma unroll
+                for (int off = 1; off < 8; off *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+                const float mine = __shfl_sync(0xffffffffu, sum, (lane & 3) * 8);      // of row 4 r + (lane & 3)
+                if ((lane >> 2) == r) delta = mine;
             }
-            p.delta[at] = delta;
-            lse2 = p.lse[at] * LOG2E;
+            if (live) p.delta[at] = delta;
+            else delta = 0.f;
         }
         const float scale2 = 0.125f * LOG2E;
         const uint64_t scale_pair = pair2(scale2, scale2), lse_pair = pair2(-lse2, -lse2), delta_pair = pair2(-delta, -delta);
