@@ -55,9 +55,8 @@ struct TimedScope {  // records a pair of events around the launches made while 
 // start.  It stands behind chain_wait, so at most two kernels are there at a time and whatever lies two launches back is
 // complete, and, in a kernel that allocates tensor memory, behind the allocation: the next kernel, if it allocates too, would
 // else be able to take the columns first and wait, holding them, for this one.  Without chain_next a kernel lets the next one
-// start as its CTAs leave; so do the CUDA-core products (with it the CTAs of the next one fill whatever places come free first,
-// two on some SMs and none on others: a float32 layer of 2048 rows 1122 us before, 1308 with it), and the products for few
-// rows (64 rows over 64 experts, replayed: 162 us before, 167 with it).
+// start as its CTAs leave: so do the products for few rows (64 rows over 64 experts, replayed: 162 us before, 167 with it) and the
+// general CUDA-core products; the 128 x 128 tiles are launched in the ordinary way (see there).
 // 3001 rows, 16 experts, forward and backward (27 launches): 461 us in ordinary launches, 432 like this.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -202,6 +201,9 @@ struct SimtGemmArgs {
 // dtype codes QMOE_F32 / QMOE_BF16 for A, B, C; m_extent = rows the grid must cover
 int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtype, long long m_extent, int groups,
                      cudaStream_t stream);
+// up to kSimtProducts products of one mode, one set of groups and the same operand types (m_extent: g.M), in one launch where they take the tiles
+constexpr int kSimtProducts = 3;
+int launch_simt_gemms(const SimtGemmArgs* g, int count, int a_dtype, int b_dtype, int c_dtype, int groups, cudaStream_t stream);
 
 // ---- cross-file entry points -----------------------------------------------------------------
 // qmoe_permute / qmoe_permute_norm with the pad rows zeroed only up to a multiple of `pad` rows per expert

@@ -159,13 +159,24 @@ struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice 
     }
 };
 
+// Products that share a launch: their tiles follow one another in blockIdx.x.  A product of 256 tiles leaves the last round of the
+// 296 CTAs that are resident (two per SM) part empty; gate and up together, and the three weight gradients, do so once
+// (a layer of 2048 rows, 512 x 1024, 8 experts, forward and backward: 1113 us with a launch each, 1035 like this).
+struct SimtTileArgs {
+    SimtGemmArgs product[kSimtProducts];
+    int end[kSimtProducts];       // tiles of the products up to and including this one
+    int columns[kSimtProducts];   // tiles side by side
+};
+
 template <bool A_KFAST, bool B_KFAST>
 __global__ void __launch_bounds__(256, 2)
-simt_tile_kernel(SimtGemmArgs g) {
-    chain_wait();      // no chain_next: see chained
+simt_tile_kernel(const __grid_constant__ SimtTileArgs args) {
+    const int tile = (int)blockIdx.x, which = tile < args.end[0] ? 0 : tile < args.end[1] ? 1 : 2;
+    const SimtGemmArgs& g = args.product[which];
+    const int local = tile - (which ? args.end[which - 1] : 0);
     __shared__ __align__(16) float As[2][TILE_K][TILE_PITCH];
     __shared__ __align__(16) float Bs[2][TILE_K][TILE_PITCH];
-    const long long m0 = (long long)blockIdx.y * TILE, n0 = (long long)blockIdx.x * TILE;
+    const long long m0 = (long long)(local / args.columns[which]) * TILE, n0 = (long long)(local % args.columns[which]) * TILE;
     long long M = g.M, k_begin = 0, k_end = g.K, b_offset = 0;
     float* C = (float*)g.C;
     if (g.mode == SG_ROWS) {
@@ -265,13 +276,28 @@ bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
     return (long long)ceil_div(g.N, TILE) * ceil_div(m_extent, TILE) * groups * 2 >= sm_count();
 }
 
-int launch_tiles(const SimtGemmArgs& g, long long m_extent, int groups, cudaStream_t stream) {
-    const dim3 grid(ceil_div(g.N, TILE), ceil_div(m_extent, TILE), groups);
+// m_extent 0: every product's own M
+int launch_tiles(const SimtGemmArgs* products, int count, long long m_extent, int groups, cudaStream_t stream) {
+    SimtTileArgs args = {};
+    long long tiles = 0;
+    for (int i = 0; i < kSimtProducts; ++i) {
+        if (i < count) {
+            args.product[i] = products[i];
+            args.columns[i] = ceil_div(products[i].N, TILE);
+            tiles += (long long)args.columns[i] * ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE);
+        }
+        args.end[i] = (int)tiles;
+    }
+    if (tiles >= (1ll << 31)) return fail_arg("gemm: too many tiles");
+    const SimtGemmArgs& g = products[0];
+    const dim3 grid((unsigned)tiles, 1, (unsigned)groups);
+    // ordinary launches: in a chain the CTAs are handed out while those of the kernel before leave, two to some SMs and none to
+    // others, which costs these kernels, as long as their slowest SM, more than the gap (the layer above: 1113 us)
     const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
-    if (a_kfast && b_kfast) chained(simt_tile_kernel<true, true>, grid, 256, 0, stream, g);
-    else if (a_kfast) chained(simt_tile_kernel<true, false>, grid, 256, 0, stream, g);
-    else if (b_kfast) chained(simt_tile_kernel<false, true>, grid, 256, 0, stream, g);
-    else chained(simt_tile_kernel<false, false>, grid, 256, 0, stream, g);
+    if (a_kfast && b_kfast) simt_tile_kernel<true, true><<<grid, 256, 0, stream>>>(args);
+    else if (a_kfast) simt_tile_kernel<true, false><<<grid, 256, 0, stream>>>(args);
+    else if (b_kfast) simt_tile_kernel<false, true><<<grid, 256, 0, stream>>>(args);
+    else simt_tile_kernel<false, false><<<grid, 256, 0, stream>>>(args);
     QMOE_LAUNCH_CHECK("simt_tile_kernel");
     return 0;
 }
@@ -309,7 +335,7 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
     const int key = (a_dtype << 2) | (b_dtype << 1) | c_dtype;
     switch (key) {
         case 0:
-            if (tile_kernel_ok(g, m_extent, groups)) return launch_tiles(g, m_extent, groups, stream);
+            if (tile_kernel_ok(g, m_extent, groups)) return launch_tiles(&g, 1, m_extent, groups, stream);
             return launch_typed<float, float, float>(g, m_extent, groups, stream);
         case 1: return launch_typed<float, float, bf>(g, m_extent, groups, stream);
         case 2: return launch_typed<float, bf, float>(g, m_extent, groups, stream);
@@ -320,6 +346,16 @@ int launch_simt_gemm(const SimtGemmArgs& g, int a_dtype, int b_dtype, int c_dtyp
         case 7: return launch_typed<bf, bf, bf>(g, m_extent, groups, stream);
     }
     return fail_arg("bad dtype combination");
+}
+
+int launch_simt_gemms(const SimtGemmArgs* g, int count, int a_dtype, int b_dtype, int c_dtype, int groups, cudaStream_t stream) {
+    bool together = count <= kSimtProducts && a_dtype == QMOE_F32 && b_dtype == QMOE_F32 && c_dtype == QMOE_F32;
+    for (int i = 0; together && i < count; ++i)
+        together = tile_kernel_ok(g[i], g[i].M, groups) && (g[i].a_cs == 1) == (g[0].a_cs == 1) && (g[i].b_rs == 1) == (g[0].b_rs == 1);
+    if (together) return launch_tiles(g, count, 0, groups, stream);
+    for (int i = 0; i < count; ++i)
+        if (int rc = launch_simt_gemm(g[i], a_dtype, b_dtype, c_dtype, g[i].M, groups, stream)) return rc;
+    return 0;
 }
 
 int launch_reduce_partials(const float* partials, float* out, long long n, int splits, cudaStream_t stream) {

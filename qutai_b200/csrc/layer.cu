@@ -27,8 +27,7 @@ int check_experts(const qmoe_route_t* r, const qmoe_experts_t* ex, int* engine) 
 }
 
 // C[rows, N] = A[rows, K] . op(B_e) on CUDA cores; b_kfast: B_e is [N, K] ("x W^T"), else [K, N]
-int simt_rows(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c,
-              long long K, long long N, bool b_kfast, cudaStream_t stream) {
+SimtGemmArgs simt_rows_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c, long long K, long long N, bool b_kfast) {
     SimtGemmArgs g = {};
     g.A = (const void*)a; g.B = (const void*)b; g.A2 = (const void*)a2; g.B2 = (const void*)b2; g.C = (void*)c;
     g.M = r->rows_bound; g.N = N; g.K = K;
@@ -37,12 +36,15 @@ int simt_rows(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint6
     g.ldc = N; g.mode = SG_ROWS;
     g.tile_expert = (const int*)r->tile_expert; g.meta = (const int*)r->meta;
     g.b_slab = K * N;
-    return launch_simt_gemm(g, ex->dtype, ex->dtype, ex->dtype, r->rows_bound, 1, stream);
+    return g;
+}
+int simt_rows(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c,
+              long long K, long long N, bool b_kfast, cudaStream_t stream) {
+    return launch_simt_gemm(simt_rows_args(r, a, b, a2, b2, c, K, N, b_kfast), ex->dtype, ex->dtype, ex->dtype, r->rows_bound, 1, stream);
 }
 
 // C_e[M, N] (fp32) = A_e^T . B_e, A [rows, M], B [rows, N]
-int simt_wgrad(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint64_t b, uint64_t c, long long M, long long N,
-               cudaStream_t stream) {
+SimtGemmArgs simt_wgrad_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t c, long long M, long long N) {
     SimtGemmArgs g = {};
     g.A = (const void*)a; g.B = (const void*)b; g.C = (void*)c;
     g.M = M; g.N = N; g.K = 0;
@@ -51,7 +53,7 @@ int simt_wgrad(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint
     g.ldc = N; g.mode = SG_K;
     g.offsets = (const int*)r->offsets; g.counts = (const int*)r->counts;
     g.c_slab = M * N;
-    return launch_simt_gemm(g, ex->dtype, ex->dtype, QMOE_F32, M, ex->experts, stream);
+    return g;
 }
 
 }  // namespace
@@ -81,8 +83,8 @@ static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
         } else {
             {
                 TimedScope timed(KC_EXPERT_GEMM, stream);
-                if (int rc = simt_rows(r, ex, x, ex->w_gate, 0, 0, g, d, hd, true, stream)) return rc;
-                if (int rc = simt_rows(r, ex, x, ex->w_up, 0, 0, u, d, hd, true, stream)) return rc;
+                const SimtGemmArgs both[2] = {simt_rows_args(r, x, ex->w_gate, 0, 0, g, d, hd, true), simt_rows_args(r, x, ex->w_up, 0, 0, u, d, hd, true)};
+                if (int rc = launch_simt_gemms(both, 2, ex->dtype, ex->dtype, ex->dtype, 1, stream)) return rc;
             }
             if (int rc = launch_swiglu(r, g, u, h, ex->dtype, hd, stream)) return rc;
         }
@@ -146,9 +148,9 @@ extern "C" int qmoe_expert_backward_parts(const qmoe_route_t* r, const qmoe_expe
         if (tc) {  // all three in one launch
             if (int rc = tc_wgrad3(r, ex->experts, dy, h, x, d_g, d_u, d_w_down, d_w_gate, d_w_up, d, hd, stream)) return rc;
         } else {
-            if (int rc = simt_wgrad(r, ex, dy, h, d_w_down, d, hd, stream)) return rc;
-            if (int rc = simt_wgrad(r, ex, d_g, x, d_w_gate, hd, d, stream)) return rc;
-            if (int rc = simt_wgrad(r, ex, d_u, x, d_w_up, hd, d, stream)) return rc;
+            const SimtGemmArgs three[3] = {simt_wgrad_args(r, dy, h, d_w_down, d, hd), simt_wgrad_args(r, d_g, x, d_w_gate, hd, d),
+                                           simt_wgrad_args(r, d_u, x, d_w_up, hd, d)};
+            if (int rc = launch_simt_gemms(three, 3, ex->dtype, ex->dtype, QMOE_F32, ex->experts, stream)) return rc;
         }
     }
     if ((parts & QMOE_BWD_ACTIVATIONS) && !skip_dx && dx == dy) {  // dX overwrites dY: only after dY's last reader (dWd)
