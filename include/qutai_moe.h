@@ -80,6 +80,9 @@ int qmoe_stream_destroy(uint64_t stream);
 int qmoe_event_create(uint64_t* event);
 int qmoe_event_destroy(uint64_t event);
 int qmoe_event_record(uint64_t event, uint64_t stream);
+/* counts[0 .. experts) to pinned host memory of qmoe_host_alloc, written by a kernel of `stream` (no copy engine, whose queue may
+ * hold the caller's own large copies), and, unless event is 0, that event recorded behind it.  Capturable with event 0. */
+int qmoe_publish_counts(uint64_t counts, void* host, int32_t experts, uint64_t event, uint64_t stream);
 int qmoe_stream_wait_event(uint64_t stream, uint64_t event);
 int qmoe_event_sync(uint64_t event);                       /* host waits for the event only */
 /* CUDA graphs (no upstream counterpart: its runtime launches kernel by kernel,

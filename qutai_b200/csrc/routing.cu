@@ -271,6 +271,12 @@ route_pack_kernel(const int* __restrict__ expert_idx, const int* __restrict__ bl
     }
 }
 
+// counts to pinned host memory
+__global__ void publish_counts_kernel(const int* __restrict__ counts, int* __restrict__ host, int experts) {
+    chain_begin();
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) host[e] = counts[e];
+}
+
 // ---- few tokens (decoding): the whole routing in one block -------------------------------------------
 // At 64 tokens the three kernels above and the fill of row_source are four launches of which none has work for more than
 // one or two SMs; here the same steps meet at block barriers (64 tokens, 64 experts, top 6: 31 us in four launches with one
@@ -485,6 +491,16 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
                                                         (const int*)r->offsets, (int*)r->dest_row,
                                                         (int*)r->row_source, T, E, k);
     QMOE_LAUNCH_CHECK("route_pack_kernel");
+    return 0;
+}
+
+extern "C" int qmoe_publish_counts(uint64_t counts, void* host, int32_t experts, uint64_t event, uint64_t stream_) {
+    if (!counts || !host) return fail_arg("publish_counts: null address");
+    if (experts <= 0) return fail_arg("publish_counts: experts must be positive");
+    cudaStream_t stream = (cudaStream_t)stream_;
+    chained(publish_counts_kernel, 1, experts < 256 ? (experts + 31) / 32 * 32 : 256, 0, stream, (const int*)counts, (int*)host, experts);
+    QMOE_LAUNCH_CHECK("publish_counts_kernel");
+    if (event) QMOE_CUDA(cudaEventRecord((cudaEvent_t)event, stream));
     return 0;
 }
 

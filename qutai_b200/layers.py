@@ -243,13 +243,11 @@ class SparseMoE:
             setattr(layer, name, buf[name].ptr)
         layer.dx_dispatched = buf["dy_dispatched"].ptr  # dX reuses dY's buffer (written after its last reader)
         if self._counts_host is None:
-            host, event, routed, side = ctypes.c_void_p(), ctypes.c_uint64(), ctypes.c_uint64(), ctypes.c_uint64()
+            host, event = ctypes.c_void_p(), ctypes.c_uint64()
             lib.call("qmoe_host_alloc", ctypes.byref(host), 4 * E)
             lib.call("qmoe_event_create", ctypes.byref(event))
-            lib.call("qmoe_event_create", ctypes.byref(routed))
-            lib.call("qmoe_stream_create", ctypes.byref(side))
             self._counts_host = ctypes.cast(host, ctypes.POINTER(ctypes.c_int32))
-            self._counts_event, self._routed_event, self._copy_stream = event.value, routed.value, side.value
+            self._counts_address, self._counts_event = host.value, event.value
         grad_views = [Tensor(buf["d_w_router"], (E, d))]
         for i in range(E):
             grad_views.append((Tensor(buf["d_w_gate"].view(i * h * d, h * d), (h, d)),
@@ -298,8 +296,6 @@ class SparseMoE:
         keep = self._operands_current(work)
         if keep:
             layer.master_gate = layer.master_up = layer.master_down = 0   # keep the bf16 copies of the last forward
-        if self._counts_valid is True:  # the previous forward's counts have left before routing overwrites them
-            lib.call("qmoe_stream_wait_event", self.stream, self._counts_event)
         lib.call("qmoe_layer_forward", ctypes.byref(layer), self.stream)
         layer.master_gate, layer.master_up, layer.master_down = masters
         if not keep:
@@ -310,14 +306,10 @@ class SparseMoE:
         return Tensor(out, shape), Tensor(buf["aux"], ())
 
     def _publish_counts(self, buf):
-        """Start the host's copy of the counts of the forward just enqueued.  It travels on a stream of its own: a
+        """Start the host's copy of the counts of the forward just enqueued.  A kernel writes them to pinned memory: a
         device-to-host copy queued on the caller's stream would wait behind whatever large copy-out the caller
         has in flight on the same copy engine, and every kernel after it would wait too."""
-        lib.call("qmoe_event_record", self._routed_event, self.stream)
-        lib.call("qmoe_stream_wait_event", self._copy_stream, self._routed_event)
-        lib.call("qmoe_memcpy_d2h", ctypes.cast(self._counts_host, ctypes.c_void_p), buf["counts"].ptr,
-                 4 * self.n_experts, self._copy_stream)
-        lib.call("qmoe_event_record", self._counts_event, self._copy_stream)
+        lib.call("qmoe_publish_counts", buf["counts"].ptr, self._counts_address, self.n_experts, self._counts_event, self.stream)
         self._counts_valid = True
 
     def _release_aliased_gradients(self, work):
@@ -351,8 +343,7 @@ class SparseMoE:
         lib.call("qmoe_graph_begin", self.stream)
         try:
             lib.call("qmoe_layer_forward", ctypes.byref(layer), self.stream)
-            lib.call("qmoe_memcpy_d2h", ctypes.cast(self._counts_host, ctypes.c_void_p), buf["counts"].ptr,
-                     4 * self.n_experts, self.stream)
+            lib.call("qmoe_publish_counts", buf["counts"].ptr, self._counts_address, self.n_experts, 0, self.stream)
         except Exception:
             lib.load().qmoe_graph_abandon(self.stream)
             raise
@@ -493,8 +484,6 @@ class MoEFeedForward:
             layer.master_gate = layer.master_up = layer.master_down = 0
         struct.layer = layer
         struct.norm_weight, struct.norm_eps = self.ffn_norm.weight.storage.ptr, self.ffn_norm.eps
-        if moe._counts_valid is True:
-            lib.call("qmoe_stream_wait_event", moe.stream, moe._counts_event)
         lib.call("qmoe_block_forward", ctypes.byref(struct), moe.stream)
         layer.master_gate, layer.master_up, layer.master_down = masters
         if not keep:

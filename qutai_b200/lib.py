@@ -109,6 +109,7 @@ SIGNATURES = {
     "qmoe_event_create": (c_int, [POINTER(c_uint64)]),
     "qmoe_event_destroy": (c_int, [_U]),
     "qmoe_event_record": (c_int, [_U, _U]),
+    "qmoe_publish_counts": (c_int, [_U, c_void_p, c_int32, _U, _U]),
     "qmoe_stream_wait_event": (c_int, [_U, _U]),
     "qmoe_event_sync": (c_int, [_U]),
     "qmoe_launch_count": (c_int64, []),
@@ -226,6 +227,8 @@ def library_path():
 def load(path=None):
     """Load the shared library (once) and attach the signatures."""
     global _library
+    if path is None and _library is not None:
+        return _library
     with _lock:
         if _library is not None and path is None:
             return _library
@@ -255,8 +258,16 @@ def check(code):
     raise RuntimeError(f"{message} [code {code}]")
 
 
+_functions = {}     # the library's functions by name, as `call` first met them
+
+
 def call(name, *args):
-    check(getattr(load(), name)(*args))
+    function = _functions.get(name)
+    if function is None:
+        function = _functions[name] = getattr(load(), name)
+    code = function(*args)
+    if code:
+        check(code)
 
 
 def rows_bound(tokens, experts, top_k):

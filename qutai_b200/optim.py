@@ -10,6 +10,8 @@ are those storages need not convert its weights again (``SparseMoE.operand_shado
 from __future__ import annotations
 
 import ctypes
+import struct
+from itertools import chain
 from math import isfinite
 
 from . import lib
@@ -23,6 +25,9 @@ def _parameters(source):
     return tuple(dict.fromkeys(source))
 
 
+_ITEM = "5Q2q2f"       # lib.OptimItem: values, grad, exp_avg, exp_avg_sq, shadow, size, first_chunk, c1, c2
+
+
 class _Table:
     """Host item array plus the device buffer it is copied into, grown on demand."""
 
@@ -34,9 +39,7 @@ class _Table:
             self.capacity = max(64, 2 * len(rows))
             self.items = (lib.OptimItem * self.capacity)()
             self.device = DeviceStorage(int(lib.load().qmoe_optim_table_bytes(self.capacity)) // 4, "int32")
-        for item, (values, grad, average, square, shadow, size, c1, c2) in zip(self.items, rows):
-            item.values, item.grad, item.exp_avg, item.exp_avg_sq, item.shadow = values, grad, average, square, shadow
-            item.size, item.first_chunk, item.c1, item.c2 = size, 0, c1, c2
+        struct.pack_into(_ITEM * len(rows), self.items, 0, *chain.from_iterable(rows))
         return self.items, len(rows), self.device.ptr
 
 
@@ -51,7 +54,7 @@ def clip_grad_norm(parameters, max_norm=1.0, *, stream=0, scratch=None):
     if any(g.dtype != "float32" for g in gradients):
         raise ValueError("gradients must be float32")
     table = _Table()
-    items, count, device = table.fill([(0, g.storage.ptr, 0, 0, 0, g.storage.size, 1.0, 1.0) for g in gradients])
+    items, count, device = table.fill([(0, g.storage.ptr, 0, 0, 0, g.storage.size, 0, 1.0, 1.0) for g in gradients])
     scratch = scratch or DeviceStorage(int(lib.load().qmoe_clip_scratch_bytes()) // 4, "int32")
     lib.call("qmoe_clip_grad_norm", items, count, device, float(max_norm), scratch.ptr, stream)
     host = (ctypes.c_double * 2)()
@@ -130,7 +133,7 @@ class AdamW:
                 raise ValueError("a shadow must be a bfloat16 storage of its parameter's size")
             rows.append((parameter.storage.ptr, gradient.storage.ptr, self.averages[parameter].ptr,
                          self.square_averages[parameter].ptr, shadow.ptr if shadow is not None else 0,
-                         parameter.storage.size, 1 - beta1 ** step, 1 - beta2 ** step))
+                         parameter.storage.size, 0, 1 - beta1 ** step, 1 - beta2 ** step))
             self.steps[parameter] = step
             updated.append((parameter.storage, shadow))
         if not rows:

@@ -32,14 +32,10 @@ _cached_bytes = 0
 CACHE_LIMIT_BYTES = int(os.environ.get("QUTAI_MOE_CACHE_BYTES", 64 << 30))
 
 
-def _bucket(nbytes):
-    step = 512 if nbytes < (1 << 16) else 1 << 16
-    return max(step, (nbytes + step - 1) // step * step)
-
-
 def _allocate(nbytes):
     global _cached_bytes
-    size = _bucket(nbytes)
+    step = 512 if nbytes < (1 << 16) else 1 << 16
+    size = (nbytes + step - 1) // step * step or step
     free = _cache.get(size)
     if free:
         _cached_bytes -= size
@@ -70,7 +66,11 @@ def _release(address, size):
         _cached_bytes -= oldest
         if not blocks:
             del _cache[oldest]
-    _cache.setdefault(size, []).append(address)
+    free = _cache.get(size)
+    if free is None:
+        _cache[size] = [address]
+    else:
+        free.append(address)
     _cached_bytes += size
 
 
@@ -96,12 +96,13 @@ class DeviceStorage:
     device = "cuda"
 
     def __init__(self, size, dtype="float32", *, ptr=None, owner=None):
-        if dtype not in lib.ITEM_BYTES:
+        item = lib.ITEM_BYTES.get(dtype)
+        if item is None:
             raise ValueError(f"unsupported dtype {dtype!r}")
         if size < 0:
             raise ValueError("size must not be negative")
         self.size, self.dtype = int(size), dtype
-        self.nbytes = self.size * lib.ITEM_BYTES[dtype]
+        self.nbytes = self.size * item
         self._owner = owner
         self._block = None
         self._parent = None        # a view shares the generation counter of the storage it was cut from; an owning
@@ -110,7 +111,7 @@ class DeviceStorage:
         self._generation = 0
         self._synced = {}          # id(source root) -> generation of the source this storage was last derived from
         if ptr is None:
-            self.ptr, self._block = _allocate(max(self.nbytes, 1))
+            self.ptr, self._block = _allocate(self.nbytes)
         else:
             self.ptr = int(ptr)
 
