@@ -56,7 +56,8 @@ struct StreamTile { int expert, n0, row0, columns; };   // `columns`: rows of th
 
 // tiles of expert e: m_tiles weight tiles x its 128-row chunks, the chunks of one weight tile side by side (the second
 // finds the weights in L2)
-__device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const int* first, int t, int columns) {
+// (first, row0, rows: each expert's first tile, first dispatched row and rows, in shared memory)
+__device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const int* first, const int* row0, const int* rows, int t, int columns) {
     int lo = 0, hi = p.experts;        // largest e with first[e] <= t
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -66,8 +67,8 @@ __device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const i
     StreamTile tile;
     tile.expert = lo;
     tile.n0 = local / chunks * columns;
-    tile.row0 = p.offsets[lo] + chunk * kRowPad;
-    const int left = p.counts[lo] - chunk * kRowPad;
+    tile.row0 = row0[lo] + chunk * kRowPad;
+    const int left = rows[lo] - chunk * kRowPad;
     tile.columns = left >= kRowPad ? kRowPad : (left + kStreamPad - 1) / kStreamPad * kStreamPad;
     return tile;
 }
@@ -85,7 +86,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     using Config = StreamCfg<MODE>;
     constexpr int STAGES = Config::STAGES, STAGE_BYTES = Config::STAGE_BYTES, W_TILES = Config::W_TILES;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ int s_first[kMaxExperts + 1];     // first tile of each expert
+    __shared__ int s_first[kMaxExperts + 1], s_row0[kMaxExperts], s_rows[kMaxExperts];     // see stream_tile
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,10 +108,28 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     chain_wait();      // what follows reads global memory; no chain_next: see chained
-    for (int e = threadIdx.x; e <= p.experts; e += STREAM_THREADS) {
-        int tiles = 0;
-        for (int j = 0; j < e; ++j) tiles += (p.counts[j] + kRowPad - 1) / kRowPad;
-        s_first[e] = tiles * p.m_tiles;
+    // The tables in one round trip to L2: a thread per expert loads, a warp sums up (every thread adding up the counts before its
+    // expert, a chain of L2 latencies, took two microseconds of the two launches of 64 rows over 64 experts, 201 us).
+    for (int e = threadIdx.x; e < p.experts; e += STREAM_THREADS) {
+        const int count = p.counts[e];
+        s_rows[e] = count;
+        s_row0[e] = p.offsets[e];
+        s_first[e + 1] = (count + kRowPad - 1) / kRowPad * p.m_tiles;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int before = 0;
+        for (int e0 = 0; e0 < p.experts; e0 += 32) {
+            int sum = e0 + lane < p.experts ? s_first[e0 + lane + 1] : 0;
+#pragma unroll
+            for (int step = 1; step < 32; step *= 2) {
+                const int other = __shfl_up_sync(0xffffffffu, sum, step);
+                if (lane >= step) sum += other;
+            }
+            if (e0 + lane < p.experts) s_first[e0 + lane + 1] = before + sum;
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) s_first[0] = 0;
     }
     tc_fence_before();
     __syncthreads();
@@ -125,7 +144,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
             int stage = 0;
             uint32_t phase = 0;
             for (int t = blockIdx.x; t < total && !*abort_flag; t += gridDim.x) {
-                const StreamTile tile = stream_tile(p, s_first, t, Config::COLUMNS);
+                const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS);
                 const int boxes = (tile.columns + X_BOX - 1) / X_BOX, w_row = tile.expert * p.N + tile.n0;
                 for (int kb = 0; kb < kblocks; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { gave_up(STATUS_STREAM_PRODUCER); break; }
@@ -144,7 +163,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
         uint32_t phase = 0;
         bool ok = true;
         for (int t = blockIdx.x; ok && t < total; t += gridDim.x, ++iter) {
-            const StreamTile tile = stream_tile(p, s_first, t, Config::COLUMNS);
+            const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS);
             const uint32_t idesc = make_idesc<false, false, SM_ROWS>(tile.columns), acc = tmem + (uint32_t)(iter & 1) * 256;
             ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(iter & 1), ((uint32_t)(iter >> 1) & 1u) ^ 1u, abort_flag));
             tc_fence_after();
@@ -172,7 +191,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
         const int quad = warp & 3;
         int iter = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++iter) {
-            const StreamTile tile = stream_tile(p, s_first, t, Config::COLUMNS);
+            const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS);
             const int a = iter & 1, n = tile.n0 + quad * 32 + lane;
             if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(a), (uint32_t)(iter >> 1) & 1u, abort_flag))) {
                 if (lane == 0) gave_up(STATUS_STREAM_EPILOGUE);
