@@ -158,27 +158,27 @@ struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice 
     }
 };
 
-// Products that share a launch (SEVERAL): their tiles follow one another in blockIdx.x.  A product of 256 tiles leaves the last
-// round of the 296 CTAs that are resident (two per SM) part empty; gate and up together, and the three weight gradients, do so
-// once (a layer of 2048 rows, 512 x 1024, 8 experts, forward and backward: 1109 us with a launch each, 1083 like this; 512 rows,
-// 1024 x 800, 16 experts 1445 and 1333).  One product alone is addressed without the index: through it the strides take
-// registers, and the spills cost 2 % of 2048 rows, 1024 x 2048.
+// Products that share a launch: their tiles follow one another in blockIdx.x.  A product of 256 tiles leaves the last round of the
+// 296 CTAs that are resident (two per SM) part empty; gate and up together, and the three weight gradients, do so once.  A
+// product alone takes the same way: with its strides in registers, as the index leaves them, the kernel is faster than with them
+// in the constant bank.  Forward and backward, us at the start, with the products together but single ones addressed without the
+// index, and like this: 2048 rows, 512 x 1024, 8 experts 1112, 1068, 1038; 512 rows, 1024 x 800, 16 experts 1456, 1336, 1314;
+// 2048 rows, 1024 x 2048, 8 experts 3462, 3488, 3486.
 struct SimtTileArgs {
     SimtGemmArgs product[kSimtProducts];
     int end[kSimtProducts];       // tiles of the products up to and including this one
     int columns[kSimtProducts];   // tiles side by side
 };
 
-template <bool A_KFAST, bool B_KFAST, bool SEVERAL>
+template <bool A_KFAST, bool B_KFAST>
 __global__ void __launch_bounds__(256, 2)
 simt_tile_kernel(const __grid_constant__ SimtTileArgs args) {
-    const int tile = (int)blockIdx.x, which = !SEVERAL || tile < args.end[0] ? 0 : tile < args.end[1] ? 1 : 2;
+    const int tile = (int)blockIdx.x, which = tile < args.end[0] ? 0 : tile < args.end[1] ? 1 : 2;
     const SimtGemmArgs& g = args.product[which];
-    const int local = tile - (which ? args.end[which - 1] : 0);      // one product: its tiles are the grid
+    const int local = tile - (which ? args.end[which - 1] : 0);
     __shared__ __align__(16) float As[2][TILE_K][TILE_PITCH];
     __shared__ __align__(16) float Bs[2][TILE_K][TILE_PITCH];
-    const long long m0 = (long long)(SEVERAL ? local / args.columns[which] : (int)blockIdx.y) * TILE;
-    const long long n0 = (long long)(SEVERAL ? local % args.columns[which] : (int)blockIdx.x) * TILE;
+    const long long m0 = (long long)(local / args.columns[which]) * TILE, n0 = (long long)(local % args.columns[which]) * TILE;
     long long M = g.M, k_begin = 0, k_end = g.K, b_offset = 0;
     float* C = (float*)g.C;
     if (g.mode == SG_ROWS) {
@@ -292,18 +292,15 @@ int launch_tiles(const SimtGemmArgs* products, int count, long long m_extent, in
     }
     if (tiles >= (1ll << 31)) return fail_arg("gemm: too many tiles");
     const SimtGemmArgs& g = products[0];
-    const dim3 grid = count > 1 ? dim3((unsigned)tiles, 1, (unsigned)groups)
-                                : dim3((unsigned)args.columns[0], (unsigned)(tiles / args.columns[0]), (unsigned)groups);
+    const dim3 grid((unsigned)tiles, 1, (unsigned)groups);
     // Ordinary launches, as for the general kernel: in a chain the CTAs are handed out while those of the kernel before leave, two
     // to some SMs and none to others, which costs kernels that are as long as their slowest SM more than the gap (the layer above: 1113
     // us; 700 rows, 320 x 300, 4 experts, on the general kernel: 346 us, in a chain 445).
     const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
-    if (a_kfast && b_kfast && count > 1) simt_tile_kernel<true, true, true><<<grid, 256, 0, stream>>>(args);
-    else if (a_kfast && b_kfast) simt_tile_kernel<true, true, false><<<grid, 256, 0, stream>>>(args);
-    else if (a_kfast) simt_tile_kernel<true, false, false><<<grid, 256, 0, stream>>>(args);
-    else if (b_kfast) simt_tile_kernel<false, true, false><<<grid, 256, 0, stream>>>(args);
-    else if (count > 1) simt_tile_kernel<false, false, true><<<grid, 256, 0, stream>>>(args);
-    else simt_tile_kernel<false, false, false><<<grid, 256, 0, stream>>>(args);
+    if (a_kfast && b_kfast) simt_tile_kernel<true, true><<<grid, 256, 0, stream>>>(args);
+    else if (a_kfast) simt_tile_kernel<true, false><<<grid, 256, 0, stream>>>(args);
+    else if (b_kfast) simt_tile_kernel<false, true><<<grid, 256, 0, stream>>>(args);
+    else simt_tile_kernel<false, false><<<grid, 256, 0, stream>>>(args);
     QMOE_LAUNCH_CHECK("simt_tile_kernel");
     return 0;
 }
