@@ -483,10 +483,6 @@ int qmoe_rms_norm_backward(uint64_t gradient, int32_t g_dtype, uint64_t x, int32
  * the other way round with inverse != 0 (its own backward).  Replaces `rope` (lm_rope). */
 int qmoe_rope(uint64_t values, uint64_t out, int32_t dtype, int64_t batch, int64_t time, int32_t heads, int32_t dim,
               double theta, int32_t offset, int32_t inverse, uint64_t stream);
-/* bf16.  inverse 0: packed [batch][time][heads + 2 kv_heads][dim] (queries, keys and values side by side) -> q, k (both rotated) and v as
- * dense tensors; inverse 1: q, k (rotated back) and v -> packed.  The rotation of qmoe_rope; dim a multiple of 8, addresses of 16. */
-int qmoe_rope_qkv(uint64_t packed, uint64_t q, uint64_t k, uint64_t v, int64_t batch, int64_t time, int32_t heads, int32_t kv_heads, int32_t dim,
-                  double theta, int32_t offset, int32_t inverse, uint64_t stream);
 /* out[i, :] = weight[ids[i], :] (ids i64; an id outside [0, vocab) gives a zero row).  Replaces `embedding` (lm_embedding). */
 int qmoe_embedding(uint64_t weight, uint64_t ids, uint64_t out, int32_t out_dtype, int64_t count, int64_t width,
                    int64_t vocab, uint64_t stream);

@@ -247,62 +247,6 @@ rope_heads_kernel(const T* __restrict__ values, T* __restrict__ out, long long p
     }
 }
 
-// Rows of queries, keys and values side by side [position][heads + 2 kv_heads][dim], as one product with the three stacked
-// weights makes them, into the tensors that attention reads, queries and keys rotated on the way (SPLIT); or the other way
-// round, the rotations taken back: the gradients of the three side by side, as the stacked products of the backward read them.
-// The same rotation as above, to the bit.  HBM-bound, every value read and written once: a thread owns eight elements of a position in
-// QKV_HEADS heads, whose loads are all on their way before the first store.  With it a block has one projection instead of three and
-// two rotations forward, and backward one input gradient and one weight gradient instead of three each and two
-// additions (a decoder step of 2 x 301 positions, two blocks of width 512: 1178 -> 1037 us).
-constexpr int QKV_HEADS = 8;
-template <bool SPLIT>
-__global__ void __launch_bounds__(kThreads)
-rope_qkv_kernel(__nv_bfloat16* packed, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* v, long long positions, int time, int heads, int kv_heads,
-                int dim, float theta, int offset) {
-    chain_begin();
-    const int groups = dim / 8, all = heads + 2 * kv_heads;
-    const float step = -2.f * log2f(theta) / (float)dim;
-    for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < positions * groups; i += (long long)gridDim.x * kThreads) {
-        const int group = (int)(i % groups);
-        const long long position = i / groups, t = position % time;
-        const int first = (int)blockIdx.y * QKV_HEADS, end = min(first + QKV_HEADS, all);
-        float s[4], c[4];
-        if (first < heads + kv_heads) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float angle = (float)(offset + t) * exp2f(step * (float)(4 * group + e));
-                if (!SPLIT) angle = -angle;
-                sincosf(angle, &s[e], &c[e]);
-            }
-        }
-        float f[QKV_HEADS][8];
-        auto side = [&](int h) { return packed + (position * all + h) * dim + 8 * group; };
-        auto alone = [&](int h) {
-            if (h < heads) return q + (position * heads + h) * dim + 8 * group;
-            if (h < heads + kv_heads) return k + (position * kv_heads + h - heads) * dim + 8 * group;
-            return v + (position * kv_heads + h - heads - kv_heads) * dim + 8 * group;
-        };
-#pragma unroll
-        for (int n = 0; n < QKV_HEADS; ++n)
-            if (first + n < end) load8((const __nv_bfloat16*)(SPLIT ? side(first + n) : alone(first + n)), f[n]);
-#pragma unroll
-        for (int n = 0; n < QKV_HEADS; ++n) {
-            if (first + n >= end) break;
-            if (first + n < heads + kv_heads) {
-                float r[8];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    r[2 * e] = f[n][2 * e] * c[e] - f[n][2 * e + 1] * s[e];
-                    r[2 * e + 1] = f[n][2 * e] * s[e] + f[n][2 * e + 1] * c[e];
-                }
-                store8(SPLIT ? alone(first + n) : side(first + n), r);
-            } else {
-                store8(SPLIT ? alone(first + n) : side(first + n), f[n]);
-            }
-        }
-    }
-}
-
 // out[i, :] = weight[ids[i], :]   (lm_embedding)
 template <typename TO>
 __global__ void __launch_bounds__(kThreads)
@@ -476,24 +420,6 @@ extern "C" int qmoe_rope(uint64_t values, uint64_t out, int32_t dtype, int64_t b
         chained(rope_kernel<float>, flat_grid(pairs), kThreads, 0, stream, (const float*)values, (float*)out, pairs, (int)time, heads, dim, (float)theta,
                                                                offset, inverse);
     QMOE_LAUNCH_CHECK("rope_kernel");
-    return 0;
-}
-
-extern "C" int qmoe_rope_qkv(uint64_t packed, uint64_t q, uint64_t k, uint64_t v, int64_t batch, int64_t time, int32_t heads, int32_t kv_heads,
-                             int32_t dim, double theta, int32_t offset, int32_t inverse, uint64_t stream_) {
-    if (!packed || !q || !k || !v) return fail_arg("rope_qkv: null address");
-    if ((packed | q | k | v) & 15u) return fail_arg("rope_qkv: addresses must be multiples of 16 bytes");
-    if (batch <= 0 || time <= 0 || heads <= 0 || kv_heads <= 0 || dim <= 0 || dim % 8 || theta <= 0)
-        return fail_arg("rope_qkv: sizes must be positive, dim a multiple of 8, theta positive");
-    if ((long long)heads + 2ll * kv_heads > 65535ll * QKV_HEADS) return fail_arg("rope_qkv: too many heads");
-    cudaStream_t stream = (cudaStream_t)stream_;
-    TimedScope timed(KC_ELEMENTWISE, stream);
-    const long long positions = batch * time;
-    const dim3 grid((unsigned)flat_grid(positions * (dim / 8)), (unsigned)((heads + 2 * kv_heads + QKV_HEADS - 1) / QKV_HEADS));
-    auto at = [](uint64_t address) { return (__nv_bfloat16*)address; };
-    if (inverse) chained(rope_qkv_kernel<false>, grid, kThreads, 0, stream, at(packed), at(q), at(k), at(v), positions, (int)time, heads, kv_heads, dim, (float)theta, offset);
-    else chained(rope_qkv_kernel<true>, grid, kThreads, 0, stream, at(packed), at(q), at(k), at(v), positions, (int)time, heads, kv_heads, dim, (float)theta, offset);
-    QMOE_LAUNCH_CHECK("rope_qkv_kernel");
     return 0;
 }
 

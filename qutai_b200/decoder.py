@@ -59,13 +59,12 @@ class Linear:
     ``weight`` [out, in] float32, bf16 operand copy, bf16 activations; the three products go through ``qmoe_gemm``
     (tensor cores from 128 rows on, whatever their number)."""
 
-    def __init__(self, width_in, width_out, *, std, seed, stream=0, operand=None):
-        """``operand``: where the bf16 copy of the weight lies, if not in a buffer of its own."""
+    def __init__(self, width_in, width_out, *, std, seed, stream=0):
         storage = DeviceStorage(width_out * width_in, "float32")
         storage.fill_normal(0.0, std, 0x5EED if seed is None else seed, stream)
         self.weight = Tensor(storage, (width_out, width_in), requires_grad=True)
         self.width_in, self.width_out, self.stream = width_in, width_out, stream
-        self._operand = DeviceStorage(storage.size, "bfloat16") if operand is None else operand
+        self._operand = DeviceStorage(storage.size, "bfloat16")
 
     def parameters(self):
         return (self.weight,)
@@ -76,34 +75,27 @@ class Linear:
             self._operand.mark_derived_from(self.weight.storage)
         return self._operand
 
+    def _gemm(self, a, b, c, m, k, n, ta, tb, c_dtype):
+        lib.call("qmoe_gemm", a.ptr, lib.QMOE_BF16, b.ptr, lib.QMOE_BF16, c.ptr, c_dtype, m, k, n, ta, tb, 0, self.stream)
+
     def forward(self, x, rows):
         y = DeviceStorage(rows * self.width_out, "bfloat16")
-        _product(x, self.operand(), y, rows, self.width_in, self.width_out, 0, 1, lib.QMOE_BF16, self.stream)
+        self._gemm(x, self.operand(), y, rows, self.width_in, self.width_out, 0, 1, lib.QMOE_BF16)
         return y
 
     def backward(self, dy, x, rows):
         """Input gradient [rows, in] (bf16); the weight gradient [out, in] (float32) is accumulated into ``weight.grad``."""
-        dx, dw = _linear_backward(dy, x, self.operand(), rows, self.width_in, self.width_out, self.stream)
+        dx = DeviceStorage(rows * self.width_in, "bfloat16")
+        self._gemm(dy, self.operand(), dx, rows, self.width_out, self.width_in, 0, 0, lib.QMOE_BF16)
+        dw = DeviceStorage(self.weight.storage.size, "float32")
+        partials = lib.load().qmoe_gemm_wgrad_partials(self.width_out, rows, self.width_in)
+        if partials:    # few output tiles, many rows: the rows are cut into ranges that run side by side
+            scratch = DeviceStorage(partials, "float32")
+            lib.call("qmoe_gemm_wgrad_split", dy.ptr, x.ptr, dw.ptr, scratch.ptr, self.width_out, rows, self.width_in, self.stream)
+        else:
+            self._gemm(dy, x, dw, self.width_out, rows, self.width_in, 1, 0, lib.QMOE_F32)
         _accumulate(self.weight, dw, self.stream)
         return dx
-
-
-def _product(a, b, c, m, k, n, ta, tb, c_dtype, stream):
-    lib.call("qmoe_gemm", a.ptr, lib.QMOE_BF16, b.ptr, lib.QMOE_BF16, c.ptr, c_dtype, m, k, n, ta, tb, 0, stream)
-
-
-def _linear_backward(dy, x, operand, rows, width_in, width_out, stream):
-    """Input gradient [rows, in] (bf16) and weight gradient [out, in] (float32) of ``y = x W^T``."""
-    dx = DeviceStorage(rows * width_in, "bfloat16")
-    _product(dy, operand, dx, rows, width_out, width_in, 0, 0, lib.QMOE_BF16, stream)
-    dw = DeviceStorage(width_out * width_in, "float32")
-    partials = lib.load().qmoe_gemm_wgrad_partials(width_out, rows, width_in)
-    if partials:    # few output tiles, many rows: the rows are cut into ranges that run side by side
-        scratch = DeviceStorage(partials, "float32")
-        lib.call("qmoe_gemm_wgrad_split", dy.ptr, x.ptr, dw.ptr, scratch.ptr, width_out, rows, width_in, stream)
-    else:
-        _product(dy, x, dw, width_out, rows, width_in, 1, 0, lib.QMOE_F32, stream)
-    return dx, dw
 
 
 def _integers(rows, room):
@@ -142,10 +134,7 @@ def _add(a, b, stream):
 
 
 class GQA:
-    """Grouped-query attention with rotary embedding (src/qutai/lm/layers.py:316-349).  The bf16 copies of the query, key and
-    value weights lie one behind the other, so the three projections are one product, and so are their input gradients
-    (whose sum it forms in fp32) and their weight gradients; ``qmoe_rope_qkv`` goes between the rows side by side and the
-    tensors that attention reads."""
+    """Grouped-query attention with rotary embedding (src/qutai/lm/layers.py:316-349)."""
 
     def __init__(self, config, *, seed, stream=0):
         width = config.d_model
@@ -153,33 +142,27 @@ class GQA:
         self.dim = width // config.n_heads
         kv_width = config.n_kv_heads * self.dim
         s = (lambda k: None if seed is None else seed + k)
-        self._stacked = DeviceStorage((width + 2 * kv_width) * width, "bfloat16")
-        part = lambda row, rows: self._stacked.view(row * width, rows * width)
-        self.q = Linear(width, width, std=0.02, seed=s(0), stream=stream, operand=part(0, width))
-        self.k = Linear(width, kv_width, std=0.02, seed=s(1), stream=stream, operand=part(width, kv_width))
-        self.v = Linear(width, kv_width, std=0.02, seed=s(2), stream=stream, operand=part(width + kv_width, kv_width))
+        self.q = Linear(width, width, std=0.02, seed=s(0), stream=stream)
+        self.k = Linear(width, kv_width, std=0.02, seed=s(1), stream=stream)
+        self.v = Linear(width, kv_width, std=0.02, seed=s(2), stream=stream)
         self.out = Linear(width, width, std=0.02 / sqrt(2 * config.n_layers), seed=s(3), stream=stream)
         self.width, self.kv_width, self.stream = width, kv_width, stream
 
     def parameters(self):
         return tuple(p for layer in (self.q, self.k, self.v, self.out) for p in layer.parameters())
 
-    def _operand(self):
-        for layer in (self.q, self.k, self.v):
-            layer.operand()
-        return self._stacked
-
-    def _rope(self, packed, q, k, v, batch, time, inverse):
-        lib.call("qmoe_rope_qkv", packed.ptr, q.ptr, k.ptr, v.ptr, batch, time, self.heads, self.kv_heads, self.dim, float(self.theta), 0,
-                 inverse, self.stream)
+    def _rope(self, values, batch, time, heads, inverse):
+        out = DeviceStorage(values.size, "bfloat16")
+        lib.call("qmoe_rope", values.ptr, out.ptr, lib.QMOE_BF16, batch, time, heads, self.dim, float(self.theta), 0, 1 if inverse else 0,
+                 self.stream)
+        return out
 
     def forward(self, x, batch, time):
         rows = batch * time
         view = lambda storage, width: Tensor(storage, (batch, time, width))
-        packed = DeviceStorage(rows * (self.width + 2 * self.kv_width), "bfloat16")
-        _product(x, self._operand(), packed, rows, self.width, self.width + 2 * self.kv_width, 0, 1, lib.QMOE_BF16, self.stream)
-        q, k, v = (DeviceStorage(rows * width, "bfloat16") for width in (self.width, self.kv_width, self.kv_width))
-        self._rope(packed, q, k, v, batch, time, 0)
+        q = self._rope(self.q.forward(x, rows), batch, time, self.heads, False)
+        k = self._rope(self.k.forward(x, rows), batch, time, self.kv_heads, False)
+        v = self.v.forward(x, rows)
         qt, kt, vt = view(q, self.width), view(k, self.kv_width), view(v, self.kv_width)
         attended, lse = attention_forward(qt, kt, vt, self.heads, self.kv_heads, self.stream)
         saved = (x, qt, kt, vt, attended, lse)
@@ -190,15 +173,11 @@ class GQA:
         x, qt, kt, vt, attended, lse = saved
         d_attended = self.out.backward(dy, attended, rows)
         dq, dk, dv = attention_backward(d_attended, qt, kt, vt, attended, lse, self.heads, self.kv_heads, self.stream)
-        width, out = self.width, self.width + 2 * self.kv_width
-        packed = DeviceStorage(rows * out, "bfloat16")
-        self._rope(packed, dq, dk, dv, batch, time, 1)
-        dx, dw = _linear_backward(packed, x, self._operand(), rows, width, out, self.stream)
-        row = 0
-        for layer in (self.q, self.k, self.v):
-            _accumulate(layer.weight, dw.view(row * width, layer.width_out * width), self.stream)
-            row += layer.width_out
-        return dx
+        dq = self._rope(dq, batch, time, self.heads, True)
+        dk = self._rope(dk, batch, time, self.kv_heads, True)
+        dx = self.q.backward(dq, x, rows)
+        dx = _add(dx, self.k.backward(dk, x, rows), self.stream)
+        return _add(dx, self.v.backward(dv, x, rows), self.stream)
 
 
 class Block:

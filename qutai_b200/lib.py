@@ -166,7 +166,6 @@ SIGNATURES = {
     "qmoe_rms_norm": (c_int, [_U, _I32, _U, _U, _I32, _U, _I64, _I64, c_double, _U]),
     "qmoe_rms_norm_partials": (c_int64, [_I64, _I64]),
     "qmoe_rms_norm_backward": (c_int, [_U, _I32, _U, _I32, _U, _U, _U, _U, _U, _I64, _I64, _U]),
-    "qmoe_rope_qkv": (c_int, [_U, _U, _U, _U, _I64, _I64, _I32, _I32, _I32, c_double, _I32, _I32, _U]),
     "qmoe_rope": (c_int, [_U, _U, _I32, _I64, _I64, _I32, _I32, c_double, _I32, _I32, _U]),
     "qmoe_embedding": (c_int, [_U, _U, _U, _I32, _I64, _I64, _I64, _U]),
     "qmoe_token_tables": (c_int, [c_void_p, _I64, _I64, c_void_p, c_void_p, c_void_p, POINTER(c_int64)]),
