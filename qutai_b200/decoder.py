@@ -290,19 +290,7 @@ class Decoder:
         return tuple(p for p in self.parameters() if id(p) not in skip)
 
     def parameters(self):
-        """The tensors of ``named_parameters``, in its order."""
-        result = [self.embedding.weight]
-        for block in self.blocks:
-            attn, ffn = block.attn, block.ffn
-            result += (block.attn_norm.weight, block.ffn_norm.weight, attn.q.weight, attn.k.weight, attn.v.weight, attn.out.weight,
-                       ffn.router.weight)
-            if self.world > 1:
-                result += [parameter for _, parameter in ffn.named_expert_parameters()]
-                continue
-            for expert in ffn.experts:
-                result += (expert.gate.weight, expert.up.weight, expert.down.weight)
-        result.append(self.norm.weight)
-        return tuple(result)
+        return tuple(parameter for _, parameter in self.named_parameters())
 
     def zero_grad(self):
         for parameter in self.parameters():
