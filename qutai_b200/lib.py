@@ -226,8 +226,9 @@ def library_path():
 def load(path=None):
     """Load the shared library (once) and attach the signatures."""
     global _library
-    if path is None and _library is not None:
-        return _library
+    loaded = _library
+    if path is None and loaded is not None:
+        return loaded
     with _lock:
         if _library is not None and path is None:
             return _library
@@ -257,16 +258,8 @@ def check(code):
     raise RuntimeError(f"{message} [code {code}]")
 
 
-_functions = {}     # the library's functions by name, as `call` first met them
-
-
 def call(name, *args):
-    function = _functions.get(name)
-    if function is None:
-        function = _functions[name] = getattr(load(), name)
-    code = function(*args)
-    if code:
-        check(code)
+    check(getattr(load(), name)(*args))
 
 
 def rows_bound(tokens, experts, top_k):
