@@ -67,8 +67,12 @@ inline cudaLaunchAttribute chain_attribute() {
     attribute.val.programmaticStreamSerializationAllowed = 1;
     return attribute;
 }
-template <typename... Parameters, typename... Arguments>
-inline cudaError_t chained(void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Arguments... arguments) {
+// The arguments convert to the kernel's parameters as in an ordinary launch: a pointer of another type does not.  A launch that
+// fails is found by the QMOE_LAUNCH_CHECK behind it.
+template <typename T> struct AsGiven { using type = T; };
+template <typename... Parameters>
+inline void chained(void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
+                    typename AsGiven<Parameters>::type... arguments) {
     cudaLaunchAttribute attribute = chain_attribute();
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
@@ -77,7 +81,7 @@ inline cudaError_t chained(void (*kernel)(Parameters...), dim3 grid, dim3 block,
     config.stream = stream;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, Parameters(arguments)...);
+    (void)cudaLaunchKernelEx(&config, kernel, arguments...);
 }
 
 // ---- small device helpers -------------------------------------------------------------------

@@ -1,0 +1,39 @@
+"""Kernels launched in a chain (``chained`` in csrc/common.cuh): what the launch accepts, and the rule that every such kernel waits
+for the one before it.  No GPU: the first compiles, the second reads the sources."""
+import subprocess
+
+import pytest
+
+from qutai_b200 import build
+
+LAUNCHES = """
+#include <type_traits>
+#include "common.cuh"
+using namespace qmoe;
+__global__ void kernel(const float* in, __nv_bfloat16* out, long long n, int m) {}
+template <typename... A, typename = decltype(chained(kernel, 1, 32, 0, nullptr, std::declval<A>()...))>
+std::true_type accepted(int);
+template <typename... A>
+std::false_type accepted(...);
+template <typename... A>
+constexpr bool takes = decltype(accepted<A...>(0))::value;
+static_assert(takes<const float*, __nv_bfloat16*, long long, int>, "the kernel's own types");
+static_assert(takes<float*, __nv_bfloat16*, int, long long>, "conversions that any call makes");
+static_assert(!takes<__nv_bfloat16*, float*, long long, int>, "two pointers swapped");
+static_assert(!takes<const int*, __nv_bfloat16*, long long, int>, "a pointer of another type");
+static_assert(!takes<const float*, const __nv_bfloat16*, long long, int>, "const dropped");
+static_assert(!takes<const float*, __nv_bfloat16*, float*, int>, "a pointer for a size");
+static_assert(!takes<unsigned long, __nv_bfloat16*, long long, int>, "a number for a pointer");
+"""
+
+
+def test_a_chained_launch_checks_the_types_of_its_arguments(tmp_path):
+    try:
+        nvcc = build.nvcc_path()
+    except RuntimeError:
+        pytest.skip("no nvcc on this machine")
+    source = tmp_path / "launches.cu"
+    source.write_text(LAUNCHES)
+    done = subprocess.run([nvcc, *build.ARCH_FLAGS, "-std=c++17", "--expt-relaxed-constexpr", "-I", build.INCLUDE, "-I", build.CSRC, "-c",
+                           str(source), "-o", str(tmp_path / "launches.o")], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    assert done.returncode == 0, done.stdout
