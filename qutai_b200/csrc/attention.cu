@@ -129,6 +129,7 @@ attention_forward_kernel(const __grid_constant__ AttentionParams p) {
     uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + 5 * TILE_BYTES + 8 * BARS);
     volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + 5 * TILE_BYTES + 8 * BARS + 4);
     if (base & 1023u) {   // the operand tiles need the alignment the declaration asks for
+        chain_wait();
         if (threadIdx.x == 0) atomicExch(p.status, STATUS_ATTENTION_WAIT + 1);
         return;
     }
@@ -349,6 +350,7 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
     uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + DQ_TILES + 8 * BARS);
     volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + DQ_TILES + 8 * BARS + 4);
     if (base & 1023u) {
+        chain_wait();
         if (threadIdx.x == 0) atomicExch(p.status, STATUS_ATTENTION_WAIT + 1);
         return;
     }
@@ -581,6 +583,7 @@ attention_dkv_kernel(const __grid_constant__ AttentionParams p) {
     uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 8 * BARS);
     volatile int& s_abort = *reinterpret_cast<volatile int*>(smem_raw + DKV_TILES + DKV_STAGES * DKV_ROW_BYTES + 8 * BARS + 4);
     if (base & 1023u) {
+        chain_wait();
         if (threadIdx.x == 0) atomicExch(p.status, STATUS_ATTENTION_WAIT + 1);
         return;
     }

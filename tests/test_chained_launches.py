@@ -1,5 +1,7 @@
 """Kernels launched in a chain (``chained`` in csrc/common.cuh): what the launch accepts, and the rule that every such kernel waits
 for the one before it.  No GPU: the first compiles, the second reads the sources."""
+import os
+import re
 import subprocess
 
 import pytest
@@ -37,3 +39,40 @@ def test_a_chained_launch_checks_the_types_of_its_arguments(tmp_path):
     done = subprocess.run([nvcc, *build.ARCH_FLAGS, "-std=c++17", "--expt-relaxed-constexpr", "-I", build.INCLUDE, "-I", build.CSRC, "-c",
                            str(source), "-o", str(tmp_path / "launches.o")], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     assert done.returncode == 0, done.stdout
+
+
+def kernels():
+    """``(name, body)`` of every kernel in the sources, and the names of those that are launched with <<<>>>."""
+    found, ordinary = [], set()
+    for name in build.SOURCES:
+        with open(os.path.join(build.CSRC, name)) as file:
+            text = re.sub(r"//[^\n]*", "", file.read())
+        ordinary |= set(re.findall(r"(\w+)\s*(?:<[^;{}<>]*>)?\s*<<<", text))
+        for match in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*\)\s*)?(\w+)\s*\(", text):
+            start = position = text.index("{", match.end())
+            depth = 0
+            while True:
+                depth += {"{": 1, "}": -1}.get(text[position], 0)
+                position += 1
+                if depth == 0:
+                    break
+            found.append((match.group(1), text[start + 1:position - 1]))
+        assert len(re.findall(r"__global__", text)) == len(re.findall(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*\)\s*)?\w+\s*\(", text)), name
+    return found, ordinary
+
+
+def test_every_kernel_of_the_chain_waits_before_it_works_or_leaves():
+    found, ordinary = kernels()
+    chained = [(name, body) for name, body in found if name not in ordinary]
+    assert len(chained) > 40 and ordinary
+    late = []
+    for name, body in chained:
+        body = re.sub(r"\[&\]\([^)]*\)\s*\{[^{}]*\}", "", body)           # what a lambda returns leaves no kernel
+        if "chain_begin();" in body:
+            good = body.lstrip().startswith("chain_begin();")
+        else:   # set up first: no way out and no status word written before the wait, and the next one let go only behind it
+            wait = body.find("chain_wait();")
+            good = wait >= 0 and not re.search(r"\breturn\b|atomicExch|__ldg|chain_next", body[:wait])
+        if not good:
+            late.append(name)
+    assert not late
