@@ -200,3 +200,34 @@ def test_attention_rows_with_infinities_and_nan_stay_by_themselves(time):
     wide = np.repeat(bad, 64, axis=1)
     assert np.isnan(got[wide]).all() and np.isnan(got_lse[bad]).all()
     assert np.array_equal(got[~wide], plain[~wide]) and np.array_equal(got_lse[~bad], plain_lse[~bad])
+
+
+@pytest.mark.parametrize("batch,time,heads,kv_heads", [(1, 1, 1, 1), (2, 129, 4, 2), (1, 300, 2, 1)])
+def test_attention_delta_is_summed_in_the_order_of_the_row(batch, time, heads, kv_heads):
+    """delta = sum of grad_out * out: products of two bf16 numbers are exact in fp32, the pairs of a row are rounded once and
+    added from the first to the last, so numpy gives the same bits."""
+    import ctypes
+
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.attention import attention_forward
+    from qutai_b200.layers import Tensor
+    from qutai_b200.storage import DeviceStorage
+
+    rng = np.random.default_rng(time)
+    q, k, v, grad = (oracle.round_bf16(rng.standard_normal((batch, time, 64 * h))).astype(np.float32) for h in (heads, kv_heads, kv_heads, heads))
+    tensors = [Tensor(to_device(x, "bfloat16"), x.shape) for x in (q, k, v)]
+    out, lse = attention_forward(*tensors, heads, kv_heads)
+    a = lib.Attention()
+    a.batch, a.time, a.heads, a.kv_heads, a.dim, a.dtype = batch, time, heads, kv_heads, 64, lib.QMOE_BF16
+    gradients = [DeviceStorage(x.size, "bfloat16") for x in (q, k, v)]
+    delta, gradient = DeviceStorage(lse.size, "float32"), to_device(grad, "bfloat16")
+    a.q, a.k, a.v = (tensor.storage.ptr for tensor in tensors)
+    a.dq, a.dk, a.dv = (storage.ptr for storage in gradients)
+    a.out, a.lse, a.grad_out, a.delta = out.ptr, lse.ptr, gradient.ptr, delta.ptr
+    lib.call("qmoe_attention_backward", ctypes.byref(a), 0)
+    products = to_host(out, (-1, 64)).astype(np.float32) * grad.reshape(-1, 64)
+    want = np.zeros(len(products), dtype=np.float32)
+    for column in range(0, 64, 2):
+        want += products[:, column] + products[:, column + 1]
+    assert np.array_equal(to_host(delta, (-1,)).astype(np.float32), want)
