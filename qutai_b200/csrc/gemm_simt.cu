@@ -6,6 +6,8 @@
 //    kernel does not take.
 // One generic kernel: arbitrary element strides for both operands, optional second (A2, B2) segment
 // accumulated into the same tile, and three ways of grouping by expert.
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -159,26 +161,39 @@ struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice 
 };
 
 // Products that share a launch: their tiles follow one another in blockIdx.x.  A product of 256 tiles leaves the last round of the
-// 296 CTAs that are resident (two per SM) part empty; gate and up together, and the three weight gradients, do so once.  A
-// product alone takes the same way: with its strides in registers, as the index leaves them, the kernel is faster than with them
-// in the constant bank.  Forward and backward, us at the start, with the products together but single ones addressed without the
-// index, and like this: 2048 rows, 512 x 1024, 8 experts 1112, 1068, 1038; 512 rows, 1024 x 800, 16 experts 1456, 1336, 1314;
-// 2048 rows, 1024 x 2048, 8 experts 3462, 3488, 3486.
+// 296 CTAs that are resident (two per SM) part empty; the three weight gradients together do so once.
 struct SimtTileArgs {
     SimtGemmArgs product[kSimtProducts];
     int end[kSimtProducts];       // tiles of the products up to and including this one
     int columns[kSimtProducts];   // tiles side by side
 };
+template <bool ALONE> using TileArgs = std::conditional_t<ALONE, SimtGemmArgs, SimtTileArgs>;
+__device__ __forceinline__ int product_index(const SimtGemmArgs&) { return 0; }
+__device__ __forceinline__ int product_index(const SimtTileArgs& args) {
+    const int tile = (int)blockIdx.x;
+    return tile < args.end[0] ? 0 : tile < args.end[1] ? 1 : 2;
+}
+__device__ __forceinline__ const SimtGemmArgs& product_at(const SimtGemmArgs& args, int) { return args; }
+__device__ __forceinline__ const SimtGemmArgs& product_at(const SimtTileArgs& args, int which) { return args.product[which]; }
+__device__ __forceinline__ void tile_at(const SimtGemmArgs&, int, long long& m0, long long& n0) {
+    m0 = (long long)blockIdx.y * TILE;
+    n0 = (long long)blockIdx.x * TILE;
+}
+__device__ __forceinline__ void tile_at(const SimtTileArgs& args, int which, long long& m0, long long& n0) {
+    const int local = (int)blockIdx.x - (which ? args.end[which - 1] : 0);
+    m0 = (long long)(local / args.columns[which]) * TILE;
+    n0 = (long long)(local % args.columns[which]) * TILE;
+}
 
-template <bool A_KFAST, bool B_KFAST>
+template <bool A_KFAST, bool B_KFAST, bool ALONE>
 __global__ void __launch_bounds__(256, 2)
-simt_tile_kernel(const __grid_constant__ SimtTileArgs args) {
-    const int tile = (int)blockIdx.x, which = tile < args.end[0] ? 0 : tile < args.end[1] ? 1 : 2;
-    const SimtGemmArgs& g = args.product[which];
-    const int local = tile - (which ? args.end[which - 1] : 0);
+simt_tile_kernel(const __grid_constant__ TileArgs<ALONE> args) {
+    const int which = product_index(args);
+    const SimtGemmArgs& g = product_at(args, which);
     __shared__ __align__(16) float As[2][TILE_K][TILE_PITCH];
     __shared__ __align__(16) float Bs[2][TILE_K][TILE_PITCH];
-    const long long m0 = (long long)(local / args.columns[which]) * TILE, n0 = (long long)(local % args.columns[which]) * TILE;
+    long long m0, n0;
+    tile_at(args, which, m0, n0);
     long long M = g.M, k_begin = 0, k_end = g.K, b_offset = 0;
     float* C = (float*)g.C;
     if (g.mode == SG_ROWS) {
@@ -278,8 +293,7 @@ bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
     return (long long)ceil_div(g.N, TILE) * ceil_div(m_extent, TILE) * groups * 2 >= sm_count();
 }
 
-// m_extent 0: every product's own M
-int launch_tiles(const SimtGemmArgs* products, int count, long long m_extent, int groups, cudaStream_t stream) {
+int launch_tiles_together(const SimtGemmArgs* products, int count, long long m_extent, int groups, cudaStream_t stream) {
     SimtTileArgs args = {};
     long long tiles = 0;
     for (int i = 0; i < kSimtProducts; ++i) {
@@ -294,14 +308,39 @@ int launch_tiles(const SimtGemmArgs* products, int count, long long m_extent, in
     const SimtGemmArgs& g = products[0];
     const dim3 grid((unsigned)tiles, 1, (unsigned)groups);
     // Ordinary launches, as for the general kernel: in a chain the CTAs are handed out while those of the kernel before leave, two
-    // to some SMs and none to others, which costs kernels that are as long as their slowest SM more than the gap (the layer above: 1113
-    // us; 700 rows, 320 x 300, 4 experts, on the general kernel: 346 us, in a chain 445).
+    // to some SMs and none to others, which costs kernels that are as long as their slowest SM more than the gap (2048
+    // rows, 512 x 1024, 8 experts, forward and backward: 1038 us, in a chain 1113; 700 rows, 320 x 300, 4 experts, on the general kernel: 346 and 445).
     const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
-    if (a_kfast && b_kfast) simt_tile_kernel<true, true><<<grid, 256, 0, stream>>>(args);
-    else if (a_kfast) simt_tile_kernel<true, false><<<grid, 256, 0, stream>>>(args);
-    else if (b_kfast) simt_tile_kernel<false, true><<<grid, 256, 0, stream>>>(args);
-    else simt_tile_kernel<false, false><<<grid, 256, 0, stream>>>(args);
+    if (a_kfast && b_kfast) simt_tile_kernel<true, true, false><<<grid, 256, 0, stream>>>(args);
+    else if (a_kfast) simt_tile_kernel<true, false, false><<<grid, 256, 0, stream>>>(args);
+    else if (b_kfast) simt_tile_kernel<false, true, false><<<grid, 256, 0, stream>>>(args);
+    else simt_tile_kernel<false, false, false><<<grid, 256, 0, stream>>>(args);
     QMOE_LAUNCH_CHECK("simt_tile_kernel");
+    return 0;
+}
+
+constexpr int kMaxGridY = 65535;      // of a launch
+
+// m_extent 0: every product's own M.  Which products share a launch, or take that form of the kernel by themselves, was measured
+// (medians of 15, all forms in one job): the index that finds a tile's product costs registers, and at 128 of them spills.  x W^T spills
+// nothing without it, and two such products one after the other are faster than together (gate, up and down of 2048 rows, 1024 x 2048, 8
+// experts, top 2: 1172 us, with the index 1262; a single 4096 x 1024 x 1024: 192 and 210).  So are single products with A transposed
+// (2048 x 776 x 1500, B as it is 153 and 162, transposed 153 and 156).  Single products of plain A and B are not (dX and d_h; 2049 x 776 x
+// 1500: 164 and 159), nor are the three weight gradients of a call (512 x 1024: 330 us one after the other, 299 together).  Forward and
+// backward, 2048 rows, 8 experts, every product alone, every product with the index, and like this: 512 x 1024 1122, 1047 and 1026 us;
+// 1024 x 2048 3474, 3498 and 3409; 512 rows, 1024 x 800, 16 experts 908, 824 and 822.
+int launch_tiles(const SimtGemmArgs* products, int count, long long m_extent, int groups, cudaStream_t stream) {
+    const bool a_kfast = products[0].a_cs == 1, b_kfast = products[0].b_rs == 1;
+    bool alone = a_kfast ? b_kfast : count == 1;
+    for (int i = 0; i < count; ++i) alone = alone && ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE) <= kMaxGridY;
+    if (!alone) return launch_tiles_together(products, count, m_extent, groups, stream);
+    for (int i = 0; i < count; ++i) {
+        const dim3 grid(ceil_div(products[i].N, TILE), ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE), groups);
+        if (a_kfast) simt_tile_kernel<true, true, true><<<grid, 256, 0, stream>>>(products[i]);
+        else if (b_kfast) simt_tile_kernel<false, true, true><<<grid, 256, 0, stream>>>(products[i]);
+        else simt_tile_kernel<false, false, true><<<grid, 256, 0, stream>>>(products[i]);
+        QMOE_LAUNCH_CHECK("simt_tile_kernel");
+    }
     return 0;
 }
 

@@ -310,6 +310,25 @@ def test_float32_gemm_in_every_orientation(m, k, n, ta, tb, tiles, kernel_varian
     assert np.all(np.abs(got - a64 @ b64) <= bound)
 
 
+def test_float32_gemm_with_more_row_tiles_than_a_grid_axis():
+    """x W^T goes one product per launch with a row of tiles per step of the grid's y axis, which ends at 65535; beyond, the tiles
+    follow one another in x.  The rows around that line and the last ones, to k roundings of sums of |a||b|."""
+    from gpu_util import to_device, to_host
+    from qutai_b200 import lib
+    from qutai_b200.storage import DeviceStorage
+
+    m, k, n = 65535 * 128 + 5, 16, 68
+    a, out = DeviceStorage(m * k, "float32"), DeviceStorage(m * n, "float32")
+    a.fill_normal(0.0, 1.0, 7)
+    b = np.random.default_rng(7).standard_normal((n, k)).astype(np.float32)
+    sb = to_device(b, "float32")
+    lib.call("qmoe_gemm", a.ptr, lib.QMOE_F32, sb.ptr, lib.QMOE_F32, out.ptr, lib.QMOE_F32, m, k, n, 0, 1, 0, 0)
+    for first, rows in ((0, 130), (m - 140, 140)):
+        x = to_host(a.view(first * k, rows * k), (rows, k)).astype(np.float64)
+        got = to_host(out.view(first * n, rows * n), (rows, n))
+        assert np.all(np.abs(got - x @ b.T.astype(np.float64)) <= k * 2.0 ** -24 * (np.abs(x) @ np.abs(b.T.astype(np.float64))) * 1.01)
+
+
 @pytest.mark.parametrize("rows,cols_out,cols_in", [(129, 64, 72), (301, 264, 512), (602, 512, 136), (1001, 1024, 264), (4503, 128, 256)])
 def test_ragged_weight_gradients_are_as_exact_as_an_fma_chain(rows, cols_out, cols_in, kernel_variant):
     """bf16 operands, fp32 result, a row count that is no multiple of 8: the tensor cores take the rows in pieces that are added
