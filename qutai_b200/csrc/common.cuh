@@ -55,7 +55,8 @@ struct TimedScope {  // records a pair of events around the launches made while 
 // start.  It stands behind chain_wait, so at most two kernels are there at a time and whatever lies two launches back is
 // complete, and, in a kernel that allocates tensor memory, behind the allocation: the next kernel, if it allocates too, would
 // else be able to take the columns first and wait, holding them, for this one.  Without chain_next a kernel lets the next one
-// start as its CTAs leave: so do the products for few rows (64 rows over 64 experts, replayed: 162 us before, 167 with it).  The
+// start as its CTAs leave: so do the permutation, the backward of the combine (both in permute.cu) and the products for few rows (64 rows over 64
+// experts, replayed: 162 us before, 167 with it).  The
 // CUDA-core products are launched in the ordinary way (see there).
 // 3001 rows, 16 experts, forward and backward (27 launches): 461 us in ordinary launches, 432 like this.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

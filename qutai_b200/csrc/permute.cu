@@ -30,12 +30,15 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
 // read T*d instead of A*d times (the k copies of a token lie far apart in the dispatched layout and
 // would miss L2).  Pad rows are zeroed afterwards, a warp per row, from the experts' offsets and counts: up to the next multiple
 // of 2^pad_bits rows.
+// The next kernel does not start early: these CTAs hold unequal numbers of pad rows and finish unevenly, and where they do first the
+// next kernel's CTAs would crowd (1003 rows of 2048 floats, 64 experts, top 6, us in ordinary launches, with chain_next and without: permute after
+// permute 16.7, 20.0 and 14.3; combine, its backward and the gather of the input gradient 52.8, 57.4 and 48.3).
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restrict__ dest_row,
                const int* __restrict__ offsets, const int* __restrict__ counts, int experts, int pad_bits, long long tokens, int k,
                long long width, int part_bits) {
-    chain_begin();
+    chain_wait();      // no chain_next, see above
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -140,7 +143,7 @@ combine_backward_kernel(const T* __restrict__ g, const T* __restrict__ y, const 
                         const int* __restrict__ dest_row, const int* __restrict__ row_source,
                         const int* __restrict__ meta, T* __restrict__ dy, float* __restrict__ dw, long long tokens,
                         int k, long long width) {
-    chain_begin();
+    chain_wait();      // no chain_next: as in the permutation
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
