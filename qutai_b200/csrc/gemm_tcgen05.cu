@@ -120,7 +120,7 @@ struct Tile {
 template <bool IN_SHARED> struct StartTable {
     const int* shared;
     const int* offsets;
-    __device__ __forceinline__ int operator[](int e) const { return IN_SHARED ? shared[e] : __ldg(offsets + e) / kRowPad; }
+    __device__ __forceinline__ int operator[](int e) const { return IN_SHARED ? shared[e] : offsets[e] / kRowPad; }
 };
 template <int MODE, int CTAS> constexpr bool starts_in_shared() { return !(MODE == MODE_DSWIGLU && CTAS == 2); }
 
