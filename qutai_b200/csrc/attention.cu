@@ -16,10 +16,12 @@
 //   at or after it, everything transposed (lanes = key positions):  S^T = K Q^T, dP^T = V dO^T -> rows: P^T, dS^T ->
 //   dV += P^T dO, dK += dS^T Q.
 // The products of the next block are issued before the rows have finished with this one (S has a second buffer in the
-// backward and is taken into registers at once in the forward), so the row warps rarely wait for the tensor cores; what
-// bounds them is the exponential unit, 1024 cycles per 128 x 128 block and SM, and the latency of their own chain beside it.
+// backward and is taken into registers at once in the forward).  What bounds them: the forward and dq the chain of a row warp (load, maximum,
+// exponentials, store, barrier) beside the exponential unit, which alone is 1024 cycles per 128 x 128 block and SM; dk, dv the handshakes
+// of an iteration between row warps, MMA warp and TMA (500 of 2650 cycles per block in waits; without exponentials, row
+// values and the dV and dK products it still took 72 of its 97 us).
 // 4 sequences x 2048 positions, 16 heads in 4 groups: forward and backward 606 -> 250 us against the form with P and dS in shared memory and
-// one block in flight, 241 with O rescaled behind the exponentials and delta from coalesced loads; 3 x 1501 positions,
+// one block in flight, 242 with O rescaled behind the exponentials and delta from coalesced loads; 3 x 1501 positions,
 // forward: 72, 37 and 32.
 // Every wait is bounded; on expiry the CTA records a code in the library's status word and leaves.
 #include "common.cuh"
@@ -449,8 +451,8 @@ attention_dq_kernel(const __grid_constant__ AttentionParams p) {
         // delta = sum_j grad_out * out of this row (kept for the dk, dv kernel), lse of this row.  Eight lanes read a row, four rows
         // per access, and all accesses are on their way before the first sum (a row per lane, 16 bytes at a time: 3 us of
         // the 10 .. 30 of a CTA before its first block).  The pairs of a row are added in their order, from lane to lane, as one thread
-        // per row would add them: the order is part of the result (4 sequences x 2048 positions, forward and backward: 247 us with a
-        // row per thread, 235 like this, 239 with each lane's eight products summed first).
+        // per row would add them: the order is part of the result (4 sequences x 2048 positions, 16 heads, this
+        // kernel alone: 78 us with a row per thread, 75 like this; each lane's eight products summed first would save another 1 us).
         float delta = 0.f, lse2 = 0.f;
         {
             uint4 a[8], o[8];

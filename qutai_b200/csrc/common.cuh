@@ -55,10 +55,14 @@ struct TimedScope {  // records a pair of events around the launches made while 
 // start.  It stands behind chain_wait, so at most two kernels are there at a time and whatever lies two launches back is
 // complete, and, in a kernel that allocates tensor memory, behind the allocation: the next kernel, if it allocates too, would
 // else be able to take the columns first and wait, holding them, for this one.  Without chain_next a kernel lets the next one
-// start as its CTAs leave: so do the permutation, the backward of the combine (both in permute.cu) and the products for few rows (64 rows over 64
-// experts, replayed: 162 us before, 167 with it).  The
-// CUDA-core products are launched in the ordinary way (see there).
-// 3001 rows, 16 experts, forward and backward (27 launches): 461 us in ordinary launches, 432 like this.
+// start as its CTAs leave: so do the permutation, the backward of the combine (both in permute.cu) and the products for few rows (L2 flushed before
+// every call, without it and with it: 64 rows over 64 experts, replayed, 215 us both; one row 63.5 and 61.5; a prefill of 1003 rows 283 and
+// 284).  The CUDA-core products are launched in the ordinary way (see there).
+// 3001 rows, 16 experts, forward and backward (27 launches): 472 us in ordinary launches, 440 like this; 64 rows over 64 experts, replayed, L2
+// flushed: 220 and 215.
+// The wait is a volatile statement that clobbers memory, and griddepcontrol.wait is what orders the kernel's loads behind the writes of the
+// one before; no load is declared free of order (no __ldg, loads in inline PTX are volatile), and parameters that are const __restrict__ are read
+// behind it in program order.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() { chain_wait(); chain_next(); }

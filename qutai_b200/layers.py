@@ -191,7 +191,7 @@ class SparseMoE:
         if self._counts_valid == "stream":  # the last forward was a graph replay: its copy is a node of the graph
             lib.call("qmoe_stream_sync", self.stream)
         else:
-            lib.call("qmoe_event_sync", self._counts_event)  # waits for the forward's routing only, not for later work
+            lib.call("qmoe_event_sync", self._counts_event)  # recorded behind the whole forward; later work is not waited for
         return tuple(self._counts_host[i] for i in range(self.n_experts))
 
     # ------------------------------------------------------------------------------------------
