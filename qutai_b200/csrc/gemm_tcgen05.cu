@@ -450,10 +450,9 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
     if (warp == 0 || warp == B_PRODUCER_WARP) {
         // ------------------------------ TMA producers -----------------------------
         // Two threads: one asks for the A boxes of every stage (and announces the stage's bytes), the other for the B
-        // boxes.  Issuing a TMA instruction costs its thread of the order of a hundred cycles whatever the box holds;
-        // with announce + A + B in one thread a k-block took that thread longer than its 512 cycles of tensor work.
+        // boxes: with announce + A + B in one thread a k-block took that thread longer than its 512 cycles of tensor work.
         const bool does_a = warp == 0;
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
@@ -523,72 +522,64 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        if (lane == 0 && cta_rank == 0) {
+        // The warp stays together and one elected lane issues.  Inside a test of the lane number every tcgen05 and TMA instruction
+        // took its thread of the order of a hundred cycles (operands moved to uniform registers lane by lane), and 578 .. 606
+        // cycles passed per k-block, whose tensor work is 512; like this 520 .. 530 where DRAM keeps up (8188 x 32000 x 1024).
+        // Where the power limit sets the clock it is worth less: 16384 rows, 8 experts, 1024 x 2816, forward and backward 1827 ->
+        // 1791 us; 3001 rows, 16 experts, 1024 x 2048, 440 -> 434 (three weight gradients 97.6 -> 94.4, dX 60.8 -> 58.7).
+        if (cta_rank == 0) {
             int stage = 0;
             uint32_t phase = 0;
             int iter = 0;
+            bool ok = true;
             // a pair's commit reaches the barrier of both CTAs
             auto commit = [&](uint32_t bar) {
                 if (CTAS == 2) umma_commit_both(bar);
                 else umma_commit(bar);
             };
-            for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
+            for (int t = first_tile, piece = 0; ok && t < total_tiles; next_tile(t, piece)) {
                 const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
                 if (!tile.valid) continue;
                 const int acc = accumulator(iter);
                 const uint32_t acc_phase = accumulator_phase(iter);
-                bool ok = mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag);
+                ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag));
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)acc * BN;
                 const uint32_t idesc = make_idesc<A_MN, B_MN, BM * CTAS>(tile.bn);
-                bool ready = false;   // the stage of this k-block was seen full while the k-block before it was issued
                 for (int kb = 0; ok && kb < tile.kblocks; ++kb) {
-                    if (!ready) {
-                        ok = mbar_wait(full_bar(stage), phase, abort_flag);
-                        if (!ok) break;
-                    }
+                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag));
+                    if (!ok) break;
                     tc_fence_after();
                     const uint32_t sa = base + stage * STAGE_BYTES, sb = sa + A_STAGE_BYTES;
-                    int next_stage = stage + 1;
-                    uint32_t next_phase = phase;
-                    if (next_stage == STAGES) { next_stage = 0; next_phase ^= 1u; }
-                    auto product = [&](int kk) {
-                        // K-major: 128-byte rows, 8-row groups 1024 B apart, +32 B per 16 k.
-                        // MN-major: 64-wide chunks 8 KiB apart (LBO), 8-k groups 1024 B apart, +2 KiB per 16 k.
-                        const uint64_t adesc = A_MN ? make_desc(sa + kk * 2048, CHUNK_BYTES, 1024)
-                                                    : make_desc(sa + kk * 32, 16, 1024);
-                        const uint64_t bdesc = B_MN ? make_desc(sb + kk * 2048, CHUNK_BYTES, 1024)
-                                                    : make_desc(sb + kk * 32, 16, 1024);
-                        if (CTAS == 2) umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
-                        else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
-                    };
-                    // the look at the next stage's barrier goes between the MMAs, where the tensor pipe has work queued,
-                    // rather than after the last one, where its latency would leave the pipe idle
-                    auto look_ahead = [&] { ready = kb + 1 < tile.kblocks && mbar_try(full_bar(next_stage), next_phase); };
-                    if (MODE == MODE_WGRAD && (kb + 1) * BK > tile.depth) {
-                        // rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten); in a
-                        // branch of its own, since a test per product held up the issue (4096 rows per expert: 421 -> 430 us)
-                        look_ahead();
+                    if (elect_one()) {
+                        auto product = [&](int kk) {
+                            // K-major: 128-byte rows, 8-row groups 1024 B apart, +32 B per 16 k.
+                            // MN-major: 64-wide chunks 8 KiB apart (LBO), 8-k groups 1024 B apart, +2 KiB per 16 k.
+                            const uint64_t adesc = A_MN ? make_desc(sa + kk * 2048, CHUNK_BYTES, 1024)
+                                                        : make_desc(sa + kk * 32, 16, 1024);
+                            const uint64_t bdesc = B_MN ? make_desc(sb + kk * 2048, CHUNK_BYTES, 1024)
+                                                        : make_desc(sb + kk * 32, 16, 1024);
+                            if (CTAS == 2) umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
+                            else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
+                        };
+                        if (MODE == MODE_WGRAD && (kb + 1) * BK > tile.depth) {
+                            // rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten)
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                            if (kb * BK + kk * UMMA_K < tile.depth) product(kk);
-                    } else {
+                            for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                                if (kb * BK + kk * UMMA_K < tile.depth) product(kk);
+                        } else {
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-                            if (kk == BK / UMMA_K - 1) look_ahead();
-                            product(kk);
+                            for (int kk = 0; kk < BK / UMMA_K; ++kk) product(kk);
                         }
+                        commit(empty_bar(stage));  // the stage is free once these MMAs have read it
+                        if (kb + 1 == tile.kblocks) commit(tfull_bar(acc));
                     }
-                    commit(empty_bar(stage));  // the stage is free once these MMAs have read it
-                    stage = next_stage; phase = next_phase;
+                    __syncwarp();
+                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
-                if (!ok) {
-                    if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, STATUS_WAIT_MMA); }
-                    break;
-                }
-                commit(tfull_bar(acc));
                 ++iter;
             }
+            if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, STATUS_WAIT_MMA); }
         }
     } else if (MODE == MODE_DSWIGLU) {
         // ------------------------------ epilogue of dSwiGLU -------------------------

@@ -96,9 +96,7 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, 
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// One commit that arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair.  The issuing thread
-// pays about ninety cycles for every tcgen05 instruction whatever its size, and a k-block of four MMAs has 512 cycles
-// of tensor work: a second commit per k-block made the issuer, not the tensor pipe, the limit.
+// One commit that arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair.
 __device__ __forceinline__ void umma_commit_both(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(bar), "h"((uint16_t)3) : "memory");
