@@ -102,6 +102,7 @@ struct alignas(64) GemmParams {
     int plain_rows;       // > 0: one group of this many rows (any number) instead of the expert groups of `offsets` and `counts`
     int transpose_out;    // WGRAD: bit i set = problem i stores the [M, N] product of each expert as [N, M]
     int problems;         // WGRAD: 1, or 3 products of the same shape (outputs out0, out1, out2) sharing the tile queue
+    int columns_first;    // one group: tiles that follow one another share their rows (else their columns)
     int sum_rows;         // WGRAD: > 0 (a multiple of 64): the contraction in pieces of this many rows, their products added in fp32
     int group_stride;     // ROUTER: accumulator columns [0,S), [S,2S), [2S,3S) hold the three bf16 terms of the weights
 };
@@ -147,8 +148,8 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         rem -= turn * per_product;
         const int e = s_order[slot];
         tile.expert = e;
-        tile.row0 = (rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
-        tile.n0 = (rem / p.m_tiles) * BN;
+        tile.row0 = (p.columns_first ? rem / p.n_tiles : rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
+        tile.n0 = (p.columns_first ? rem % p.n_tiles : rem / p.m_tiles) * BN;
         int count = s_pair[e];            // WGRAD keeps the row counts in this table
         tile.krow0 = s_start[e] * kRowPad;
         if (p.sum_rows > 0) {
@@ -171,12 +172,12 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         const int e = lo;
         const int groups = first_of(e + 1) - first_of(e);
         const int local = t - (first_of(e) - first) * p.n_tiles;
-        const int m_tile = (local % groups) * CTAS + cta_rank;  // 128-row tile inside the expert
+        const int m_tile = (p.columns_first ? local / p.n_tiles : local % groups) * CTAS + cta_rank;  // 128-row tile inside the expert
         const int start = s_start[e];
         tile.expert = e;
         tile.row0 = (start + m_tile) * BM;
         tile.rows_valid = m_tile < s_start[e + 1] - start;
-        tile.n0 = (local / groups) * (MODE == MODE_SWIGLU ? 128 : BN);
+        tile.n0 = (p.columns_first ? local % p.n_tiles : local / groups) * (MODE == MODE_SWIGLU ? 128 : BN);
         tile.kblocks = ((p.K + BK - 1) / BK) * p.segments;
         tile.krow0 = 0;
     }
@@ -1093,7 +1094,6 @@ int tc_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t 
     return launch<MODE_SWIGLU, false, false>(p, stream);
 }
 
-// C [rows, N] = A [rows, K] . B_e^T with B stacked [E*N, K]; `rows` > 0: one group whose last tile may be ragged
 void set_scatter(GemmParams& p, const TcScatter* scatter) {
     if (!scatter) return;
     p.scatter_ret = scatter->ret;
@@ -1101,11 +1101,20 @@ void set_scatter(GemmParams& p, const TcScatter* scatter) {
     for (int i = 0; i < 16; ++i) p.scatter_base[i] = scatter->base[i];
 }
 
+// Which operand's panels the tiles of one group that run side by side share.  Down a column of tiles every tile has rows of A of its
+// own: all of A then passes through each round of the grid, which is once too often for every round but one when A does not stay in
+// the L2 (126 MB; half of it, since results pass through as well).  Along a row of tiles the same happens to B, so the larger
+// operand goes through once.  The head over 32000 classes, 8188 rows of 1024, whose logit gradients are 524 MB: its weight gradient
+// (500 tiles) 430 -> 390 us, the gradient of its input (128 tiles) even.
+bool columns_first(long long a_elements, long long b_elements) { return a_elements > b_elements && a_elements * 2 > (64ll << 20); }
+
+// C [rows, N] = A [rows, K] . B_e^T with B stacked [E*N, K]; `rows` > 0: one group whose last tile may be ragged
 int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N,
                cudaStream_t stream, const TcScatter* scatter, long long rows) {
     GemmParams p = {};
     set_scatter(p, scatter);
     p.plain_rows = (int)rows;
+    p.columns_first = rows > 0 && columns_first(rows * K, N * K);
     if (int rc = make_map(&p.map_a, a, (uint64_t)K, (uint64_t)r->rows_bound, BM)) return rc;
     const int ctas = gemm_ctas();
     if (int rc = make_map(&p.map_b, b, (uint64_t)K, (uint64_t)experts * N, BN / ctas)) return rc;
@@ -1123,6 +1132,7 @@ int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
     GemmParams p = {};
     set_scatter(p, scatter);
     p.plain_rows = (int)rows;
+    p.columns_first = rows > 0 && columns_first(rows * K, N * K);
     if (int rc = make_map(&p.map_a, a, (uint64_t)K, (uint64_t)r->rows_bound, BM)) return rc;
     if (int rc = make_map(&p.map_b, b, (uint64_t)N, (uint64_t)experts * K, 64)) return rc;
     p.map_a2 = p.map_a; p.map_b2 = p.map_b;
@@ -1254,7 +1264,11 @@ int tc_wgrad3(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t h_act, u
 int tc_wgrad1(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t out, long long M, long long N, cudaStream_t stream,
               int groups, long long slab, int sum_rows) {
     GemmParams p = {};
-    if (!r->offsets) { p.plain_rows = (int)r->rows_bound; p.sum_rows = sum_rows; }
+    if (!r->offsets) {
+        p.plain_rows = (int)r->rows_bound;
+        p.sum_rows = sum_rows;
+        p.columns_first = columns_first(r->rows_bound * M, r->rows_bound * N);
+    }
     if (out & 15u || (N * 4) % 16) return fail_arg("weight-gradient output must be 16-byte aligned with a 16-byte row pitch");
     const int ctas = gemm_ctas();
     const uint64_t rows = (uint64_t)r->rows_bound;
