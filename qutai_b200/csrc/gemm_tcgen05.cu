@@ -2,9 +2,9 @@
 // operands staged in shared memory by TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast),
 // fp32 accumulators in tensor memory (TMEM), read back with tcgen05.ld for the epilogue.
 //
-// One persistent kernel, one CTA per SM, 10 warps; the expert products run as CTA PAIRS (CTAS = 2: the two
+// One persistent kernel, one CTA per SM, 11 warps; the expert products run as CTA PAIRS (CTAS = 2: the two
 // CTAs of a cluster share one 256 x 256 tile, tcgen05.mma.cta_group::2), the small router products with one
-// CTA per 128 x 256 tile:
+// CTA per 128 x 256 tile, products of a few tiles with one CTA per 128 x 64 tile:
 //   warp 0      TMA producer (one lane): fills a ring of {A 128x64, B 256x64 or this CTA's 128x64 half} bf16
 //               tiles (4 stages of 48 KiB, or 6 stages of 32 KiB per CTA of a pair; two fewer in dSwiGLU, whose
 //               epilogue stages its own operands in shared memory)
@@ -60,17 +60,19 @@ constexpr int B_PRODUCER_WARP = 2 + EPILOGUE_WARPS;
 constexpr int MODE_DSWIGLU_ID = 3;
 constexpr int BOX_BYTES = 32 * 64 * 2;            // one 32 x 64 bf16 box of the dSwiGLU epilogue (4 KiB, 128-byte rows)
 constexpr int BARRIER_BYTES = 512;
-template <int CTAS, int MODE> struct Cfg {
+// TN = 64:  one CTA owns a 128 x 64 tile (16 + 8 KiB per stage, 8 stages): products that are a few tiles of the other sizes.
+template <int CTAS, int MODE, int TN> struct Cfg {
     static constexpr bool STAGED = MODE == MODE_DSWIGLU_ID;
-    static constexpr int STAGES = CTAS == 2 ? (STAGED ? 5 : 6) : (STAGED ? 3 : 4);
-    static constexpr int B_STAGE_BYTES = (CTAS == 2 ? BN / 2 : BN) * BK * 2;
+    static constexpr int STAGES = TN < BN ? 8 : CTAS == 2 ? (STAGED ? 5 : 6) : (STAGED ? 3 : 4);
+    static constexpr int B_STAGE_BYTES = TN / CTAS * BK * 2;
+    static constexpr uint32_t TMEM_COLS = 2 * TN;             // two accumulators
     static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
     static constexpr int EPI_WARP_BYTES = 32 * 80;            // transpose buffer of one epilogue warp (not dSwiGLU)
     static constexpr int EPI_SLICE_BYTES = 4 * BOX_BYTES;     // dSwiGLU: two {G, U} buffers for each two warps on the same rows
     static constexpr int EPI_BYTES = STAGED ? (EPILOGUE_WARPS / 2) * EPI_SLICE_BYTES : EPILOGUE_WARPS * EPI_WARP_BYTES;  // a multiple of 1 KiB either way
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + EPI_BYTES + BARRIER_BYTES;
 };
-constexpr uint32_t TMEM_COLS = 512;
+constexpr int NARROW_TN = 64;
 
 enum { MODE_PLAIN = 0, MODE_SWIGLU = 1, MODE_WGRAD = 2, MODE_DSWIGLU = MODE_DSWIGLU_ID, MODE_ROUTER = 4, MODE_PLAIN_F32 = 5 };
 enum { STATUS_WAIT_PRODUCER = 101, STATUS_WAIT_MMA = 102, STATUS_WAIT_EPILOGUE = 103 };
@@ -127,7 +129,7 @@ template <int MODE, int CTAS> constexpr bool starts_in_shared() { return !(MODE 
 
 // s_start[e]: first 128-row tile of expert e.  s_pair[e] (CTAS == 2): first 256-row pair-tile of expert e, an
 // expert with an odd number of 128-row tiles gets a last pair-tile whose second half is not stored.
-template <int MODE, bool B_MN, int CTAS>
+template <int MODE, bool B_MN, int CTAS, int TN>
 __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTable<starts_in_shared<MODE, CTAS>()>& s_start,
                                             const int* s_pair, const int* s_order, int t, int cta_rank, int piece = 0) {
     Tile tile;
@@ -149,7 +151,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         const int e = s_order[slot];
         tile.expert = e;
         tile.row0 = (p.columns_first ? rem / p.n_tiles : rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
-        tile.n0 = (p.columns_first ? rem % p.n_tiles : rem / p.m_tiles) * BN;
+        tile.n0 = (p.columns_first ? rem % p.n_tiles : rem / p.m_tiles) * TN;
         int count = s_pair[e];            // WGRAD keeps the row counts in this table
         tile.krow0 = s_start[e] * kRowPad;
         if (p.sum_rows > 0) {
@@ -177,12 +179,12 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         tile.expert = e;
         tile.row0 = (start + m_tile) * BM;
         tile.rows_valid = m_tile < s_start[e + 1] - start;
-        tile.n0 = (p.columns_first ? local % p.n_tiles : local / groups) * (MODE == MODE_SWIGLU ? 128 : BN);
+        tile.n0 = (p.columns_first ? local % p.n_tiles : local / groups) * (MODE == MODE_SWIGLU ? 128 : TN);
         tile.kblocks = ((p.K + BK - 1) / BK) * p.segments;
         tile.krow0 = 0;
     }
     // MN-major B arrives in 64-column boxes, so a narrow last tile simply loads and multiplies half of them
-    tile.bn = (B_MN && MODE != MODE_SWIGLU && p.N - tile.n0 <= BN / 2) ? BN / 2 : BN;
+    tile.bn = (TN == BN && B_MN && MODE != MODE_SWIGLU && p.N - tile.n0 <= BN / 2) ? BN / 2 : TN;
     return tile;
 }
 
@@ -326,10 +328,11 @@ __device__ __forceinline__ void scatter_rows256(uint32_t stage, int lane, const 
 // Each stages its own 128 rows of A and half of the B tile, the pair's first CTA issues one
 // cta_group::2 MMA per k-step that reads both halves, and each CTA converts the 128 x 256 accumulator
 // that lands in its own tensor memory.  Per SM and k-step that is 32 KiB of operands instead of 48 KiB.
-template <int MODE, bool A_MN, bool B_MN, int CTAS>
+template <int MODE, bool A_MN, bool B_MN, int CTAS, int TN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
-    using Config = Cfg<CTAS, MODE>;
+    using Config = Cfg<CTAS, MODE, TN>;
+    constexpr uint32_t TMEM_COLS = Config::TMEM_COLS;
     constexpr int STAGES = Config::STAGES, B_STAGE_BYTES = Config::B_STAGE_BYTES, STAGE_BYTES = Config::STAGE_BYTES;
     extern __shared__ uint8_t smem_raw[];
     constexpr bool STARTS_IN_SHARED = starts_in_shared<MODE, CTAS>();
@@ -457,7 +460,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
             int stage = 0;
             uint32_t phase = 0;
             for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
-                const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
+                const Tile tile = decode_tile<MODE, B_MN, CTAS, TN>(p, s_start, s_pair, s_order, t, cta_rank, piece);
                 if (!tile.valid) continue;
                 const int kb_per_seg = tile.kblocks / (MODE == MODE_WGRAD ? 1 : p.segments);
                 for (int kb = 0; kb < tile.kblocks; ++kb) {
@@ -488,7 +491,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                             for (int j = 0; j < BM / 64; ++j) load(ma, sa + j * CHUNK_BYTES, tile.row0 + 64 * j, krow);
                         } else {
 #pragma unroll
-                            for (int j = 0; j < BN / CTAS / 64; ++j)
+                            for (int j = 0; j < TN / CTAS / 64; ++j)
                                 if (64 * j < bn_mine) load(mb, sb + j * CHUNK_BYTES, n_mine + 64 * j, krow);
                         }
                     } else {
@@ -511,7 +514,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                             }
                         } else if (B_MN) {
 #pragma unroll
-                            for (int j = 0; j < BN / CTAS / 64; ++j)
+                            for (int j = 0; j < TN / CTAS / 64; ++j)
                                 if (64 * j < bn_mine) load(mb, sb + j * CHUNK_BYTES, n_mine + 64 * j, tile.expert * p.b_rows + k0);
                         } else {
                             load(mb, sb, k0, tile.expert * p.b_rows + n_mine);
@@ -539,13 +542,13 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 else umma_commit(bar);
             };
             for (int t = first_tile, piece = 0; ok && t < total_tiles; next_tile(t, piece)) {
-                const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
+                const Tile tile = decode_tile<MODE, B_MN, CTAS, TN>(p, s_start, s_pair, s_order, t, cta_rank, piece);
                 if (!tile.valid) continue;
                 const int acc = accumulator(iter);
                 const uint32_t acc_phase = accumulator_phase(iter);
                 ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag));
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)acc * BN;
+                const uint32_t tmem_d = tmem_base + (uint32_t)acc * TN;
                 const uint32_t idesc = make_idesc<A_MN, B_MN, BM * CTAS>(tile.bn);
                 for (int kb = 0; ok && kb < tile.kblocks; ++kb) {
                     ok = __all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag));
@@ -618,7 +621,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         int iter = 0;
         bool gave_up = false;
         for (int t = first_tile; t < total_tiles && !*abort_flag && !gave_up; t += tile_stride) {
-            const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank);
+            const Tile tile = decode_tile<MODE, B_MN, CTAS, TN>(p, s_start, s_pair, s_order, t, cta_rank);
             if (!tile.valid) continue;
             const int c_end = chunks_of(tile);
             if (leader && c_end > 0 && !on_its_way) {  // only the first chunk of the kernel is not prefetched
@@ -632,7 +635,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 break;
             }
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN + (uint32_t)side * 32u;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * TN + (uint32_t)side * 32u;
             bool released = false;
 #pragma unroll 1
             for (int c = 0; c < c_end; ++c) {
@@ -645,7 +648,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     if (next_c >= c_end) {
                         next_c = next_last = 0;
                         for (int u = t + tile_stride; u < total_tiles; u += tile_stride) {
-                            next_tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, u, cta_rank);
+                            next_tile = decode_tile<MODE, B_MN, CTAS, TN>(p, s_start, s_pair, s_order, u, cta_rank);
                             next_last = chunks_of(next_tile);
                             if (next_last > 0) break;
                         }
@@ -717,7 +720,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         const int half = (warp - 2) >> 2;  // which half of the tile's columns this warp converts
         int iter = 0;
         for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
-            const Tile tile = decode_tile<MODE, B_MN, CTAS>(p, s_start, s_pair, s_order, t, cta_rank, piece);
+            const Tile tile = decode_tile<MODE, B_MN, CTAS, TN>(p, s_start, s_pair, s_order, t, cta_rank, piece);
             if (!tile.valid) continue;
             const int acc = accumulator(iter);
             const uint32_t acc_phase = accumulator_phase(iter);
@@ -726,7 +729,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 break;
             }
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * TN;
             const long long row = (long long)tile.row0 + quad * 32 + lane;
             // Row-major pointers of this warp's 32 rows (row0w) for the coalesced paths: a warp moves a
             // 32-row x 32-column bf16 block as 8 rows x 64 contiguous bytes per instruction, transposing
@@ -889,7 +892,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     tmem_ld32(taddr + c * 32, r);
                     if (MODE == MODE_WGRAD && piece > 0) {
                         uint32_t sum[32];
-                        tmem_ld32(taddr + BN + c * 32, sum);
+                        tmem_ld32(taddr + TN + c * 32, sum);
                         tmem_ld_wait();
 #pragma unroll
                         for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(sum[i]) + __uint_as_float(r[i]));
@@ -898,7 +901,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     }
                     last_read(c + 1 == c_end);
                     if (MODE == MODE_WGRAD && piece + 1 < pieces) {
-                        tmem_st32(taddr + BN + c * 32, r);
+                        tmem_st32(taddr + TN + c * 32, r);
                         tmem_st_wait();
                         continue;
                     }
@@ -1022,17 +1025,17 @@ int make_map_3d(CUtensorMap* out, uint64_t ptr, uint64_t inner, uint64_t mid, ui
 
 namespace {
 
-template <int MODE, bool A_MN, bool B_MN, int CTAS = 1>
-int launch(const GemmParams& p, cudaStream_t stream) {
+template <int MODE, bool A_MN, bool B_MN, int CTAS = 1, int TN = BN>
+int launch(const GemmParams& p, cudaStream_t stream, long long tiles = 0) {     // tiles: how many there are, where the host knows
     static int grid_of[64] = {0};  // per device: blocks to launch (0: not configured yet)
-    constexpr int SMEM_BYTES = Cfg<CTAS, MODE>::SMEM_BYTES;
+    constexpr int SMEM_BYTES = Cfg<CTAS, MODE, TN>::SMEM_BYTES;
     // a block has 227 KiB, its static tables included: two or three of (kMaxExperts + 1) ints plus two words
     static_assert(SMEM_BYTES + (starts_in_shared<MODE, CTAS>() ? 3 : 1) * 4 * (kMaxExperts + 1) + 16 <= 227 * 1024,
                   "operand ring + epilogue staging + tables exceed the shared memory of a block");
     int dev = 0;
     QMOE_CUDA(cudaGetDevice(&dev));
     if (dev >= 64) return fail_arg("device ordinal beyond 63");
-    auto kernel = grouped_gemm_kernel<MODE, A_MN, B_MN, CTAS>;
+    auto kernel = grouped_gemm_kernel<MODE, A_MN, B_MN, CTAS, TN>;
     cudaLaunchConfig_t config = {};
     cudaLaunchAttribute attribute[2];
     config.blockDim = dim3(NUM_THREADS);
@@ -1061,7 +1064,7 @@ int launch(const GemmParams& p, cudaStream_t stream) {
         }
         grid_of[dev] = grid;
     }
-    config.gridDim = dim3((unsigned)grid_of[dev]);
+    config.gridDim = dim3((unsigned)(tiles > 0 && tiles * CTAS < grid_of[dev] ? tiles * CTAS : grid_of[dev]));
     ++config.numAttrs;
     QMOE_CUDA(cudaLaunchKernelEx(&config, kernel, p));
     count_tensor_core_launch();
@@ -1108,6 +1111,17 @@ void set_scatter(GemmParams& p, const TcScatter* scatter) {
 // (500 tiles) 430 -> 390 us, the gradient of its input (128 tiles) even.
 bool columns_first(long long a_elements, long long b_elements) { return a_elements > b_elements && a_elements * 2 > (64ll << 20); }
 
+// Products that leave most of the chip idle in tiles of 256 x 256: in tiles of 128 x 64 as long as each has an SM of its own.  What bounds them
+// is the latency of one tile (set-up, first loads, its k-blocks, its epilogue), and a tile of an eighth of the size has a quarter of the epilogue and
+// no partner to wait for; the sums are the same bits.  us, launches back to back, 256 x 256 and 128 x 64: 602 x 512 x 512 (x W^T) 8.8 and 5.5,
+// 1024 x 1024 x 1024 11.5 and 7.8, 2048 x 2048 x 256 15.8 and 11.3, 128 x 4096 x 1024 24.3 and 18.0, 8192 x 1024 x 64 10.3 and 7.5, 602 x 8000 x 512
+// 41.5 and 32.2, 130 x 64 x 64 5.2 and 3.6; g W the same; weight gradients of 602 rows, 512 x 512, 15.2 and 8.7, of 8192 rows, 512 x 256, 43.5 and 36.7.
+// A k-block brings 24 KiB for a quarter of the products, 384 cycles at the 64 bytes a cycle that an SM gets from the L2 against
+// 512: a second round of tiles would cost more than a tile of 256 x 256.
+bool narrow_tiles(long long rows, long long columns) {
+    return !kernel_variant(QMOE_VARIANT_SINGLE_CTA_GEMM) && (long long)ceil_div(rows, BM) * ceil_div(columns, NARROW_TN) <= sm_count();
+}
+
 // C [rows, N] = A [rows, K] . B_e^T with B stacked [E*N, K]; `rows` > 0: one group whose last tile may be ragged
 int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N,
                cudaStream_t stream, const TcScatter* scatter, long long rows) {
@@ -1117,11 +1131,13 @@ int tc_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
     p.columns_first = rows > 0 && columns_first(rows * K, N * K);
     if (int rc = make_map(&p.map_a, a, (uint64_t)K, (uint64_t)r->rows_bound, BM)) return rc;
     const int ctas = gemm_ctas();
-    if (int rc = make_map(&p.map_b, b, (uint64_t)K, (uint64_t)experts * N, BN / ctas)) return rc;
+    const bool narrow = !scatter && narrow_tiles(r->rows_bound, N);
+    if (int rc = make_map(&p.map_b, b, (uint64_t)K, (uint64_t)experts * N, narrow ? NARROW_TN : BN / ctas)) return rc;
     p.map_a2 = p.map_a; p.map_b2 = p.map_b;
     p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
-    p.out0 = (void*)c; p.ldc = N; p.experts = experts; p.n_tiles = ceil_div(N, BN);
+    p.out0 = (void*)c; p.ldc = N; p.experts = experts; p.n_tiles = ceil_div(N, narrow ? NARROW_TN : BN);
     p.N = (int)N; p.K = (int)K; p.b_rows = (int)N; p.segments = 1;
+    if (narrow) return launch<MODE_PLAIN, false, false, 1, NARROW_TN>(p, stream, (long long)ceil_div(r->rows_bound, BM) * p.n_tiles);
     if (ctas == 2) return launch<MODE_PLAIN, false, false, 2>(p, stream);
     return launch<MODE_PLAIN, false, false>(p, stream);
 }
@@ -1143,8 +1159,10 @@ int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
         p.segments = 2;
     }
     p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
-    p.out0 = (void*)c; p.ldc = N; p.experts = experts; p.n_tiles = ceil_div(N, BN);
+    const bool narrow = !scatter && narrow_tiles(r->rows_bound, N);
+    p.out0 = (void*)c; p.ldc = N; p.experts = experts; p.n_tiles = ceil_div(N, narrow ? NARROW_TN : BN);
     p.N = (int)N; p.K = (int)K; p.b_rows = (int)K;
+    if (narrow) return launch<MODE_PLAIN, false, true, 1, NARROW_TN>(p, stream, (long long)ceil_div(r->rows_bound, BM) * p.n_tiles);
     if (gemm_ctas() == 2) return launch<MODE_PLAIN, false, true, 2>(p, stream);
     return launch<MODE_PLAIN, false, true>(p, stream);
 }
@@ -1277,8 +1295,10 @@ int tc_wgrad1(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t out, long 
     p.map_a2 = p.map_a; p.map_b2 = p.map_b; p.map_a3 = p.map_a; p.map_b3 = p.map_b;
     p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
     p.out0 = (void*)out; p.ldc = N; p.c_slab = slab; p.experts = groups; p.problems = 1;
-    p.m_tiles = ceil_div(M, BM * ctas); p.n_tiles = ceil_div(N, BN);
+    const bool narrow = groups == 1 && narrow_tiles(M, N);
+    p.m_tiles = ceil_div(M, narrow ? BM : BM * ctas); p.n_tiles = ceil_div(N, narrow ? NARROW_TN : BN);
     p.M = (int)M; p.N = (int)N; p.K = 0; p.segments = 1;
+    if (narrow) return launch<MODE_WGRAD, true, true, 1, NARROW_TN>(p, stream, (long long)p.m_tiles * p.n_tiles);
     if (ctas == 2) return launch<MODE_WGRAD, true, true, 2>(p, stream);
     return launch<MODE_WGRAD, true, true>(p, stream);
 }
