@@ -50,6 +50,22 @@ template <> struct Raw8<__nv_bfloat16> {
     __device__ __forceinline__ void unpack(float* f) const { Vec16<__nv_bfloat16>::unpack(v, f); }
 };
 
+// the same for four
+template <typename T> struct Raw4;
+template <> struct Raw4<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void unpack(float* f) const { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
+};
+template <> struct Raw4<__nv_bfloat16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void unpack(float* f) const {
+        f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+        f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+    }
+};
+
 // out[r, :] = x[r, :] * inverse[r] * weight, inverse[r] = 1 / sqrt(mean(x[r, :]^2) + eps).  VEC: width a multiple of 8 and
 // 32-byte aligned rows.
 template <typename TX, typename TO, bool VEC>
@@ -142,24 +158,34 @@ rms_norm_dw_partial_kernel(const TG* __restrict__ gradient, const TX* __restrict
     chain_begin();
     const long long first = (long long)blockIdx.x * kSlabRows;
     const long long last = first + kSlabRows < rows ? first + kSlabRows : rows;
-    if (VEC) {   // a thread owns eight neighbouring columns; the rows are added in order, four of them in flight
-        for (long long c = (long long)threadIdx.x * 8; c < width; c += 8ll * kThreads) {
-            float total[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (long long r0 = first; r0 < last; r0 += 4) {
-                float g[4][8], v[4][8], inv[4];
+    // A thread owns four neighbouring columns; the rows are added in order, sixteen (8 of fp32) of them in flight.  A slab is a chain of round
+    // trips to memory: with four rows in flight and eight columns per thread, 602 x 512 13.4 us and 8192 x 1024 19, like this 4.5 and 12.9.
+    if (VEC) {
+        constexpr int kFlight = sizeof(TG) + sizeof(TX) == 4 ? 16 : 8;
+        for (long long c = (long long)threadIdx.x * 4; c < width; c += 4ll * kThreads) {
+            float total[4] = {0.f, 0.f, 0.f, 0.f};
+            for (long long r0 = first; r0 < last; r0 += kFlight) {
+                Raw4<TG> g[kFlight];
+                Raw4<TX> v[kFlight];
+                float inv[kFlight];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const long long r = r0 + u < last ? r0 + u : last - 1;
-                    load8(gradient + r * width + c, g[u]);
-                    load8(x + r * width + c, v[u]);
-                    inv[u] = r0 + u < last ? inverse[r] : 0.f;
-                }
+                for (int u = 0; u < kFlight; ++u)
+                    if (r0 + u < last) {
+                        g[u].load(gradient + (r0 + u) * width + c);
+                        v[u].load(x + (r0 + u) * width + c);
+                        inv[u] = inverse[r0 + u];
+                    }
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < kFlight; ++u)
+                    if (r0 + u < last) {
+                        float a[4], b[4];
+                        g[u].unpack(a);
+                        v[u].unpack(b);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) total[j] = fmaf(g[u][j] * v[u][j], inv[u], total[j]);
+                        for (int j = 0; j < 4; ++j) total[j] = fmaf(a[j] * b[j], inv[u], total[j]);
+                    }
             }
-            store8(partial + (long long)blockIdx.x * width + c, total);
+            *reinterpret_cast<float4*>(partial + (long long)blockIdx.x * width + c) = make_float4(total[0], total[1], total[2], total[3]);
         }
         return;
     }
