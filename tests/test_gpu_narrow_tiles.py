@@ -39,12 +39,7 @@ def test_narrow_tiles_give_the_bits_of_wide_tiles(form, rows, inner, columns, ke
     assert narrow.tobytes() == product().tobytes()
     x, y = (to_host(value, like.shape) for value, like in zip((a, b), _operands(form, rows, inner, columns)))
     exact = {"nt": lambda: x @ y.T, "nn": lambda: x @ y, "tn": lambda: x.T @ y}[form]()
-<<<<<<< Updated upstream
     # bfloat16 has 8 significant bits: rounding moves a value by up to 2^-8 of itself (half of the last place, 2^-9, just below a power of
     # two); what is added in tensor memory loses its low bits, 2^-22 of the running sum per 16 products
     bound = (2.0 ** -8 if kind == "bfloat16" else 0.0) * np.abs(exact) + 2.0 ** -22 * (k / 16 + 4) * (np.abs(x).max() * np.abs(y).max() * np.sqrt(k) * 4)
-=======
-    # bfloat16 rounds by 2^-9; what is added in tensor memory loses its low bits, 2^-22 of the running sum per 16 products
-    bound = (2.0 ** -9 if kind == "bfloat16" else 0.0) * np.abs(exact) + 2.0 ** -22 * (k / 16 + 4) * (np.abs(x).max() * np.abs(y).max() * np.sqrt(k) * 4)
->>>>>>> Stashed changes
     assert (np.abs(to_host(narrow, (m, n)) - exact) <= bound).all()
