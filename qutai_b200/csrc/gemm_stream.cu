@@ -31,10 +31,12 @@ constexpr uint32_t STREAM_TMEM = 512;                  // two sets of two 128-co
 enum { STREAM_SWIGLU = 0, STREAM_NT = 1, STREAM_NT2 = 2 };
 enum { STATUS_STREAM_PRODUCER = 111, STATUS_STREAM_MMA = 112, STATUS_STREAM_EPILOGUE = 113 };
 
-template <int MODE> struct StreamCfg {
+// FEW: at most X_BOX rows per expert, one box of activations per stage, and the room for more stages
+template <int MODE, bool FEW> struct StreamCfg {
     static constexpr int W_TILES = MODE == STREAM_NT ? 1 : 2;
-    static constexpr int STAGE_BYTES = W_TILES * W_BYTES + X_BYTES;
-    static constexpr int STAGES = MODE == STREAM_NT ? 6 : 4;
+    static constexpr int MOST_ROWS = FEW ? X_BOX : kRowPad;                       // of an expert in a tile
+    static constexpr int STAGE_BYTES = W_TILES * W_BYTES + (FEW ? X_BOX_BYTES : X_BYTES);
+    static constexpr int STAGES = MODE == STREAM_NT ? (FEW ? 11 : 6) : FEW ? 6 : 4;
     static constexpr int COLUMNS = MODE == STREAM_NT2 ? 2 * SM_ROWS : SM_ROWS;    // output columns of a tile
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 };
@@ -56,8 +58,8 @@ struct StreamTile { int expert, n0, row0, columns; };   // `columns`: rows of th
 
 // tiles of expert e: m_tiles weight tiles x its 128-row chunks, the chunks of one weight tile side by side (the second
 // finds the weights in L2)
-// (first, row0, rows: each expert's first tile, first dispatched row and rows, in shared memory)
-__device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const int* first, const int* row0, const int* rows, int t, int columns) {
+// (first, row0, rows: each expert's first tile, first dispatched row and rows, in shared memory; most_rows: what a stage has room for)
+__device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const int* first, const int* row0, const int* rows, int t, int columns, int most_rows) {
     int lo = 0, hi = p.experts;        // largest e with first[e] <= t
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -69,7 +71,7 @@ __device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const i
     tile.n0 = local / chunks * columns;
     tile.row0 = row0[lo] + chunk * kRowPad;
     const int left = rows[lo] - chunk * kRowPad;
-    tile.columns = left >= kRowPad ? kRowPad : (left + kStreamPad - 1) / kStreamPad * kStreamPad;
+    tile.columns = left >= most_rows ? most_rows : (left + kStreamPad - 1) / kStreamPad * kStreamPad;
     return tile;
 }
 
@@ -80,10 +82,10 @@ __device__ __forceinline__ float logistic(float v) {   // 1 / (1 + 2^(-v log2 e)
     return r;
 }
 
-template <int MODE>
+template <int MODE, bool FEW>
 __global__ void __launch_bounds__(STREAM_THREADS, 1)
 stream_gemm_kernel(const __grid_constant__ StreamParams p) {
-    using Config = StreamCfg<MODE>;
+    using Config = StreamCfg<MODE, FEW>;
     constexpr int STAGES = Config::STAGES, STAGE_BYTES = Config::STAGE_BYTES, W_TILES = Config::W_TILES;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_first[kMaxExperts + 1], s_row0[kMaxExperts], s_rows[kMaxExperts];     // see stream_tile
@@ -144,7 +146,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
             int stage = 0;
             uint32_t phase = 0;
             for (int t = blockIdx.x; t < total && !*abort_flag; t += gridDim.x) {
-                const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS);
+                const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS, Config::MOST_ROWS);
                 const int boxes = (tile.columns + X_BOX - 1) / X_BOX, w_row = tile.expert * p.N + tile.n0;
                 for (int kb = 0; kb < kblocks; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { gave_up(STATUS_STREAM_PRODUCER); break; }
@@ -159,39 +161,47 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
             }
         }
     } else if (warp == 1) {
-        int stage = 0, iter = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; ok && t < total; t += gridDim.x, ++iter) {
-            const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS);
-            const uint32_t idesc = make_idesc<false, false, SM_ROWS>(tile.columns), acc = tmem + (uint32_t)(iter & 1) * 256;
-            ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(iter & 1), ((uint32_t)(iter >> 1) & 1u) ^ 1u, abort_flag));
-            tc_fence_after();
-            for (int kb = 0; ok && kb < kblocks; ++kb) {
-                ok = __all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag));
-                if (!ok) break;
+        // One elected lane walks the blocks and looks at the next stage's barrier before the last MMA of this one, while the tensor pipe has work
+        // queued: an MMA of 128 weight rows takes 66 cycles for up to 32 columns and 81 for 128, eight of them 530 .. 650 per k-block, and the
+        // waits, votes and elections of a whole warp came on top (4 rows, 8 experts, 1024 x 2816: 42.9 us a call, like this 40.6).
+        if (elect_one()) {
+            int stage = 0, iter = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; ok && t < total; t += gridDim.x, ++iter) {
+                const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS, Config::MOST_ROWS);
+                const uint32_t idesc = make_idesc<false, false, SM_ROWS>(tile.columns), acc = tmem + (uint32_t)(iter & 1) * 256;
+                ok = mbar_wait(tempty_bar(iter & 1), ((uint32_t)(iter >> 1) & 1u) ^ 1u, abort_flag);
                 tc_fence_after();
-                const uint32_t w = base + stage * STAGE_BYTES, x = w + W_TILES * W_BYTES;
-                if (elect_one()) {
+                bool ready = false;      // the stage of this k-block was seen full while the one before it was issued
+                for (int kb = 0; ok && kb < kblocks; ++kb) {
+                    if (!ready) ok = mbar_wait(full_bar(stage), phase, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t w = base + stage * STAGE_BYTES, x = w + W_TILES * W_BYTES;
+                    int next_stage = stage + 1;
+                    uint32_t next_phase = phase;
+                    if (next_stage == STAGES) { next_stage = 0; next_phase ^= 1u; }
 #pragma unroll
                     for (int which = 0; which < W_TILES; ++which)
 #pragma unroll
-                        for (int kk = 0; kk < SK / 16; ++kk)
+                        for (int kk = 0; kk < SK / 16; ++kk) {
+                            if (which == W_TILES - 1 && kk == SK / 16 - 1) ready = kb + 1 < kblocks && mbar_try(full_bar(next_stage), next_phase);
                             umma_bf16(acc + which * 128, make_desc(w + which * W_BYTES + kk * 32, 16, 1024), make_desc(x + kk * 32, 16, 1024), idesc,
                                       (kb | kk) ? 1u : 0u);
+                        }
                     umma_commit(empty_bar(stage));
                     if (kb == kblocks - 1) umma_commit(tfull_bar(iter & 1));
+                    stage = next_stage; phase = next_phase;
                 }
-                __syncwarp();
-                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             }
+            if (!ok) gave_up(STATUS_STREAM_MMA);
         }
-        if (!ok && lane == 0) gave_up(STATUS_STREAM_MMA);
     } else {
         const int quad = warp & 3;
         int iter = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++iter) {
-            const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS);
+            const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS, Config::MOST_ROWS);
             const int a = iter & 1, n = tile.n0 + quad * 32 + lane;
             if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(a), (uint32_t)(iter >> 1) & 1u, abort_flag))) {
                 if (lane == 0) gave_up(STATUS_STREAM_EPILOGUE);
@@ -251,20 +261,35 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     }
 }
 
-template <int MODE>
+template <int MODE, bool FEW = false>
 int stream_launch(const StreamParams& p, cudaStream_t stream) {
     static bool configured[64] = {};      // per device, like the kernels of gemm_tcgen05.cu
+    constexpr int SMEM_BYTES = StreamCfg<MODE, FEW>::SMEM_BYTES;
+    static_assert(SMEM_BYTES + 3 * 4 * (kMaxExperts + 1) + 16 <= 227 * 1024, "the stages and the tables exceed the shared memory of a block");
     int dev = 0;
     QMOE_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return fail_arg("device ordinal beyond 63");
     if (!configured[dev]) {
-        QMOE_CUDA(cudaFuncSetAttribute(stream_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamCfg<MODE>::SMEM_BYTES));
+        QMOE_CUDA(cudaFuncSetAttribute(stream_gemm_kernel<MODE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         configured[dev] = true;
     }
-    chained(stream_gemm_kernel<MODE>, sm_count(), STREAM_THREADS, StreamCfg<MODE>::SMEM_BYTES, stream, p);
+    chained(stream_gemm_kernel<MODE, FEW>, sm_count(), STREAM_THREADS, SMEM_BYTES, stream, p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("stream_gemm_kernel");
     return 0;
+}
+
+// The form with more stages: up to X_BOX tokens (a token goes to an expert once, so no expert has more rows than there are tokens), and with the
+// experts that uniform load reaches on average at most two tiles per SM.  There a tile's time is what one SM has on its way; with more tiles
+// HBM is the limit, and the more is asked for at once the less it gives.  us a call, 128 KiB of weights in flight per SM and 192: 8 experts,
+// 1024 x 2816, 4 rows 40.9 and 40.6, 32 rows 52.2 and 51.4, 1 row of 4096 x 2816 67.9 and 62.8, 64 experts, 2048 x 1408, 1 row 46.9 and 45.1, but
+// 16 rows 169.9 and 172.8, 32 rows 196.6 and 203.2.
+bool few_tokens(const qmoe_route_t* r, int experts, long long tiles_per_expert) {
+    if (r->tokens > X_BOX) return false;
+    const double hit = r->top_k < experts ? (double)r->top_k / experts : 1.0;
+    double missed = 1.0;
+    for (long long t = 0; t < r->tokens; ++t) missed *= 1.0 - hit;
+    return (1.0 - missed) * experts * (double)tiles_per_expert <= 2.0 * sm_count();
 }
 
 }  // namespace
@@ -298,7 +323,7 @@ int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
     p.out0 = (__nv_bfloat16*)g; p.out1 = (__nv_bfloat16*)u; p.out2 = (__nv_bfloat16*)h;
     p.experts = ex->experts; p.m_tiles = ceil_div((long long)hd, SM_ROWS); p.N = (int)hd; p.K = (int)d;
     p.pad_rows = pad_rows;
-    return stream_launch<STREAM_SWIGLU>(p, stream);
+    return few_tokens(r, ex->experts, p.m_tiles) ? stream_launch<STREAM_SWIGLU, true>(p, stream) : stream_launch<STREAM_SWIGLU>(p, stream);
 }
 
 int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows,
@@ -318,7 +343,7 @@ int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, u
         return stream_launch<STREAM_NT2>(p, stream);
     }
     p.m_tiles = ceil_div(N, SM_ROWS);
-    return stream_launch<STREAM_NT>(p, stream);
+    return few_tokens(r, experts, p.m_tiles) ? stream_launch<STREAM_NT, true>(p, stream) : stream_launch<STREAM_NT>(p, stream);
 }
 
 }  // namespace qmoe
