@@ -526,64 +526,77 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        // The warp stays together and one elected lane issues.  Inside a test of the lane number every tcgen05 and TMA instruction
-        // took its thread of the order of a hundred cycles (operands moved to uniform registers lane by lane), and 578 .. 606
-        // cycles passed per k-block, whose tensor work is 512; like this 520 .. 530 where DRAM keeps up (8188 x 32000 x 1024).
-        // Where the power limit sets the clock it is worth less: 16384 rows, 8 experts, 1024 x 2816, forward and backward 1827 ->
-        // 1791 us; 3001 rows, 16 experts, 1024 x 2048, 440 -> 434 (three weight gradients 97.6 -> 94.4, dX 60.8 -> 58.7).
-        if (cta_rank == 0) {
+        // One elected lane.  Inside a test of the lane number every tcgen05 and TMA instruction took its thread of the order of a
+        // hundred cycles (operands moved to uniform registers lane by lane), and 578 .. 606 cycles passed per k-block, whose tensor work is 512;
+        // like this 520 .. 530 where DRAM keeps up (8188 x 32000 x 1024).  Where the power limit sets the clock it is worth less: 16384 rows,
+        // 8 experts, 1024 x 2816, forward and backward 1827 -> 1791 us; 3001 rows, 16 experts, 1024 x 2048, 440 -> 434 (three weight gradients
+        // 97.6 -> 94.4, dX 60.8 -> 58.7).  The lane walks the k-blocks by itself: a warp that waits, votes and elects per k-block is as
+        // fast on 256 columns, but not on 128 x 64 tiles (weight gradient of 4096 rows, 1024 x 512, 21.5 us, like this 15.7).
+        if (cta_rank == 0 && elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             int iter = 0;
-            bool ok = true;
             // a pair's commit reaches the barrier of both CTAs
             auto commit = [&](uint32_t bar) {
                 if (CTAS == 2) umma_commit_both(bar);
                 else umma_commit(bar);
             };
-            for (int t = first_tile, piece = 0; ok && t < total_tiles; next_tile(t, piece)) {
+            for (int t = first_tile, piece = 0; t < total_tiles && !*abort_flag; next_tile(t, piece)) {
                 const Tile tile = decode_tile<MODE, B_MN, CTAS, TN>(p, s_start, s_pair, s_order, t, cta_rank, piece);
                 if (!tile.valid) continue;
                 const int acc = accumulator(iter);
                 const uint32_t acc_phase = accumulator_phase(iter);
-                ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag));
+                bool ok = mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag);
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)acc * TN;
                 const uint32_t idesc = make_idesc<A_MN, B_MN, BM * CTAS>(tile.bn);
+                bool ready = false;   // the stage of this k-block was seen full while the k-block before it was issued
                 for (int kb = 0; ok && kb < tile.kblocks; ++kb) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag));
-                    if (!ok) break;
+                    if (!ready) {
+                        ok = mbar_wait(full_bar(stage), phase, abort_flag);
+                        if (!ok) break;
+                    }
                     tc_fence_after();
                     const uint32_t sa = base + stage * STAGE_BYTES, sb = sa + A_STAGE_BYTES;
-                    if (elect_one()) {
-                        auto product = [&](int kk) {
-                            // K-major: 128-byte rows, 8-row groups 1024 B apart, +32 B per 16 k.
-                            // MN-major: 64-wide chunks 8 KiB apart (LBO), 8-k groups 1024 B apart, +2 KiB per 16 k.
-                            const uint64_t adesc = A_MN ? make_desc(sa + kk * 2048, CHUNK_BYTES, 1024)
-                                                        : make_desc(sa + kk * 32, 16, 1024);
-                            const uint64_t bdesc = B_MN ? make_desc(sb + kk * 2048, CHUNK_BYTES, 1024)
-                                                        : make_desc(sb + kk * 32, 16, 1024);
-                            if (CTAS == 2) umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
-                            else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
-                        };
-                        if (MODE == MODE_WGRAD && (kb + 1) * BK > tile.depth) {
-                            // rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten)
+                    int next_stage = stage + 1;
+                    uint32_t next_phase = phase;
+                    if (next_stage == STAGES) { next_stage = 0; next_phase ^= 1u; }
+                    auto product = [&](int kk) {
+                        // K-major: 128-byte rows, 8-row groups 1024 B apart, +32 B per 16 k.
+                        // MN-major: 64-wide chunks 8 KiB apart (LBO), 8-k groups 1024 B apart, +2 KiB per 16 k.
+                        const uint64_t adesc = A_MN ? make_desc(sa + kk * 2048, CHUNK_BYTES, 1024)
+                                                    : make_desc(sa + kk * 32, 16, 1024);
+                        const uint64_t bdesc = B_MN ? make_desc(sb + kk * 2048, CHUNK_BYTES, 1024)
+                                                    : make_desc(sb + kk * 32, 16, 1024);
+                        if (CTAS == 2) umma_bf16_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
+                        else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb | kk) ? 1u : 0u);
+                    };
+                    // the look at the next stage's barrier goes between the MMAs, where the tensor pipe has work queued,
+                    // rather than after the last one, where its latency would leave the pipe idle
+                    auto look_ahead = [&] { ready = kb + 1 < tile.kblocks && mbar_try(full_bar(next_stage), next_phase); };
+                    if (MODE == MODE_WGRAD && (kb + 1) * BK > tile.depth) {
+                        // rows past the next multiple of 16 need not be there (the forward for few rows leaves them unwritten)
+                        look_ahead();
 #pragma unroll
-                            for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                                if (kb * BK + kk * UMMA_K < tile.depth) product(kk);
-                        } else {
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                            if (kb * BK + kk * UMMA_K < tile.depth) product(kk);
+                    } else {
 #pragma unroll
-                            for (int kk = 0; kk < BK / UMMA_K; ++kk) product(kk);
+                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                            if (kk == BK / UMMA_K - 1) look_ahead();
+                            product(kk);
                         }
-                        commit(empty_bar(stage));  // the stage is free once these MMAs have read it
-                        if (kb + 1 == tile.kblocks) commit(tfull_bar(acc));
                     }
-                    __syncwarp();
-                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                    commit(empty_bar(stage));  // the stage is free once these MMAs have read it
+                    stage = next_stage; phase = next_phase;
                 }
+                if (!ok) {
+                    if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, STATUS_WAIT_MMA); }
+                    break;
+                }
+                commit(tfull_bar(acc));
                 ++iter;
             }
-            if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, STATUS_WAIT_MMA); }
         }
     } else if (MODE == MODE_DSWIGLU) {
         // ------------------------------ epilogue of dSwiGLU -------------------------
@@ -1115,7 +1128,7 @@ bool columns_first(long long a_elements, long long b_elements) { return a_elemen
 // is the latency of one tile (set-up, first loads, its k-blocks, its epilogue), and a tile of an eighth of the size has a quarter of the epilogue and
 // no partner to wait for; the sums are the same bits.  us, launches back to back, 256 x 256 and 128 x 64: 602 x 512 x 512 (x W^T) 8.8 and 5.5,
 // 1024 x 1024 x 1024 11.5 and 7.8, 2048 x 2048 x 256 15.8 and 11.3, 128 x 4096 x 1024 24.3 and 18.0, 8192 x 1024 x 64 10.3 and 7.5, 602 x 8000 x 512
-// 41.5 and 32.2, 130 x 64 x 64 5.2 and 3.6; g W the same; weight gradients of 602 rows, 512 x 512, 15.2 and 8.7, of 8192 rows, 512 x 256, 43.5 and 36.7.
+// 41.5 and 32.2, 130 x 64 x 64 5.2 and 3.6; g W the same; weight gradients of 602 rows, 512 x 512, 15.2 and 8.7, of 8192 rows, 512 x 256, 43.5 and 25.9.
 // A k-block brings 24 KiB for a quarter of the products, 384 cycles at the 64 bytes a cycle that an SM gets from the L2 against
 // 512: a second round of tiles would cost more than a tile of 256 x 256.
 bool narrow_tiles(long long rows, long long columns) {
