@@ -51,13 +51,13 @@ struct TimedScope {  // records a pair of events around the launches made while 
 // for about two microseconds: the first drains, its writes are flushed, the second is fetched, its CTAs start and set themselves
 // up.  With programmatic dependent launch the second is set up meanwhile and only waits, at chain_wait, until the first has
 // completed and its writes are visible.  Every thread of a kernel that is launched through `chained` calls chain_wait before its
-// first access to global memory; only its own parameters may be read earlier.  chain_next lets the next kernel of the stream
+// first access to global memory, with one exception below; only its own parameters may be read earlier.  chain_next lets the next kernel of the stream
 // start.  It stands behind chain_wait, so at most two kernels are there at a time and whatever lies two launches back is
 // complete, and, in a kernel that allocates tensor memory, behind the allocation: the next kernel, if it allocates too, would
 // else be able to take the columns first and wait, holding them, for this one.  Without chain_next a kernel lets the next one
-// start as its CTAs leave: so do the permutation, the backward of the combine (both in permute.cu) and the products for few rows (L2 flushed before
-// every call, without it and with it: 64 rows over 64 experts, replayed, 215 us both; one row 63.5 and 61.5; a prefill of 1003 rows 283 and
-// 284).  The CUDA-core products are launched in the ordinary way (see there).
+// start as its CTAs leave: so do the backward of the combine, the permutation unless a product for few rows follows (permute.cu), and those products unless
+// the down product follows for few tokens (gemm_stream.cu).  The CUDA-core products are launched in the ordinary way (see there).
+// One kernel reads before its wait: a product for few rows fetches tables and weights that nothing within the last launch wrote (gemm_stream.cu).
 // 3001 rows, 16 experts, forward and backward (27 launches): 472 us in ordinary launches, 440 like this; 64 rows over 64 experts, replayed, L2
 // flushed: 220 and 215.
 // The wait is a volatile statement that clobbers memory, and griddepcontrol.wait is what orders the kernel's loads behind the writes of the
@@ -215,8 +215,8 @@ constexpr int kSimtProducts = 3;
 int launch_simt_gemms(const SimtGemmArgs* g, int count, int a_dtype, int b_dtype, int c_dtype, int groups, cudaStream_t stream);
 
 // ---- cross-file entry points -----------------------------------------------------------------
-// qmoe_permute / qmoe_permute_norm with the pad rows zeroed only up to a multiple of `pad` rows per expert
-int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream);
+// qmoe_permute / qmoe_permute_norm with the pad rows zeroed only up to a multiple of `pad` rows per expert; let_next: the next kernel may start early
+int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, bool let_next, uint64_t stream);
 int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t weight, uint64_t out, int32_t dtype, int64_t width, int pad,
                         uint64_t stream);
 bool router_norm_ok(int64_t tokens, int32_t experts, int64_t width, int32_t x_dtype, uint64_t x, uint64_t scratch);
@@ -241,11 +241,13 @@ int tc_rows_nn(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint6
                long long N, cudaStream_t stream, const TcScatter* scatter = nullptr, long long rows = 0);
 // the same two forward products for few rows per expert (gemm_stream.cu)
 // pad_rows: every pad row holds zeros afterwards; else (QMOE_EXPERTS_SHORT_PADS) only those up to a multiple of kStreamPad rows of each expert
+// early: the kernel before on the stream is this call's own and wrote neither the tables nor the weights (see the kernel)
 constexpr int kStreamPad = 16;
 bool stream_shape_ok(const qmoe_route_t* r, const qmoe_experts_t* ex);
-int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows,
+bool stream_down_early(const qmoe_route_t* r, const qmoe_experts_t* ex);     // the down product starts beside the up product's tail
+int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows, bool early, bool let_next,
                           cudaStream_t stream);
-int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows,
+int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows, bool early,
                    cudaStream_t stream);
 int tc_dswiglu(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t w_down, uint64_t g, uint64_t u, uint64_t dg,
                uint64_t du, long long d, long long h, cudaStream_t stream);

@@ -51,6 +51,8 @@ struct alignas(64) StreamParams {
     __nv_bfloat16* out1;           // SWIGLU: U
     __nv_bfloat16* out2;           // SWIGLU: H
     int experts, m_tiles, N, K;
+    int early;                     // what lies two launches back wrote the tables and the weights: see the wait
+    int let_next;                  // the next kernel is the down product of the same call: it may start early
     int pad_rows;                  // zero every pad row; else those from `columns` on are left as they are
 };
 
@@ -109,7 +111,13 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(STREAM_TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    chain_wait();      // what follows reads global memory; no chain_next: see chained
+    // `early`: the kernel before is this call's own (the permutation, or the product that forms H), writes neither tables nor weights and lets
+    // this one start behind its own wait, so whatever wrote those lies at least two launches back and is complete.  The tables and the first
+    // stages' weights are then fetched beside the kernel before; what that one writes (the activations), and whatever this one writes, waits.
+    // us a call without it and with it: 4 rows, 8 experts, 1024 x 2816, 45.9 and 43.4 (46.0 of 47.2 with the up product alone), 16 rows, 4 experts,
+    // 512 x 264, 24.1 and 21.2.  64 rows over 64 experts, replayed on one stream 200 and 195, but on several at a time 158.6 and 160.6: CTAs that
+    // wait for the tail of the up product keep other streams' kernels from those SMs.  So the down product starts early for few tokens alone.
+    if (!p.early) chain_wait();
     // The tables in one round trip to L2: a thread per expert loads, a warp sums up (every thread adding up the counts before its
     // expert is a chain of L2 latencies: 64 rows over 64 experts, replayed, L2 flushed before every call, 217 us and 215 like this).
     for (int e = threadIdx.x; e < p.experts; e += STREAM_THREADS) {
@@ -142,25 +150,51 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     auto gave_up = [&](int code) { if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, code); } };
 
     if (warp == 0) {
+        auto ask_weights = [&](int stage, int kb, int w_row) {
+            const uint32_t w = base + stage * STAGE_BYTES, bar = full_bar(stage);
+            tma_load_2d(&p.map_w, w, bar, kb * SK, w_row);
+            if (MODE == STREAM_SWIGLU) tma_load_2d(&p.map_w2, w + W_BYTES, bar, kb * SK, w_row);
+            if (MODE == STREAM_NT2) tma_load_2d(&p.map_w, w + W_BYTES, bar, kb * SK, w_row + SM_ROWS);
+        };
+        auto ask_rows = [&](int stage, int kb, int row0, int boxes) {
+            const uint32_t x = base + stage * STAGE_BYTES + W_TILES * W_BYTES, bar = full_bar(stage);
+            for (int j = 0; j < boxes; ++j) tma_load_2d(&p.map_x, x + j * X_BOX_BYTES, bar, kb * SK, row0 + j * X_BOX);
+        };
+        int ahead = 0;       // k-blocks of the first tile whose weights were asked for before the wait
+        StreamTile first_tile = {};
+        if (p.early) {
+            if ((int)blockIdx.x < total) {
+                first_tile = stream_tile(p, s_first, s_row0, s_rows, (int)blockIdx.x, Config::COLUMNS, Config::MOST_ROWS);
+                ahead = kblocks < STAGES ? kblocks : STAGES;
+            }
+            const int boxes = (first_tile.columns + X_BOX - 1) / X_BOX;
+            if (lane == 0)
+                for (int kb = 0; kb < ahead; ++kb) {      // the stages are empty
+                    mbar_expect_tx(full_bar(kb), W_TILES * W_BYTES + boxes * X_BOX_BYTES);
+                    ask_weights(kb, kb, first_tile.expert * p.N + first_tile.n0);
+                }
+            chain_wait();
+            if (lane == 0)
+                for (int kb = 0; kb < ahead; ++kb) ask_rows(kb, kb, first_tile.row0, boxes);
+        }
         if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            for (int t = blockIdx.x; t < total && !*abort_flag; t += gridDim.x) {
+            int stage = ahead == STAGES ? 0 : ahead;
+            uint32_t phase = ahead == STAGES ? 1 : 0;
+            for (int t = blockIdx.x; t < total && !*abort_flag; t += gridDim.x, ahead = 0) {
                 const StreamTile tile = stream_tile(p, s_first, s_row0, s_rows, t, Config::COLUMNS, Config::MOST_ROWS);
-                const int boxes = (tile.columns + X_BOX - 1) / X_BOX, w_row = tile.expert * p.N + tile.n0;
-                for (int kb = 0; kb < kblocks; ++kb) {
+                const int boxes = (tile.columns + X_BOX - 1) / X_BOX;
+                for (int kb = ahead; kb < kblocks; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { gave_up(STATUS_STREAM_PRODUCER); break; }
-                    const uint32_t w = base + stage * STAGE_BYTES, x = w + W_TILES * W_BYTES, bar = full_bar(stage);
-                    mbar_expect_tx(bar, W_TILES * W_BYTES + boxes * X_BOX_BYTES);
-                    tma_load_2d(&p.map_w, w, bar, kb * SK, w_row);
-                    if (MODE == STREAM_SWIGLU) tma_load_2d(&p.map_w2, w + W_BYTES, bar, kb * SK, w_row);
-                    if (MODE == STREAM_NT2) tma_load_2d(&p.map_w, w + W_BYTES, bar, kb * SK, w_row + SM_ROWS);
-                    for (int j = 0; j < boxes; ++j) tma_load_2d(&p.map_x, x + j * X_BOX_BYTES, bar, kb * SK, tile.row0 + j * X_BOX);
+                    mbar_expect_tx(full_bar(stage), W_TILES * W_BYTES + boxes * X_BOX_BYTES);
+                    ask_weights(stage, kb, tile.expert * p.N + tile.n0);
+                    ask_rows(stage, kb, tile.row0, boxes);
                     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
+        if (p.early) chain_wait();
+        if (p.let_next) chain_next();      // the tensor memory is this block's
         // One elected lane walks the blocks and looks at the next stage's barrier before the last MMA of this one, while the tensor pipe has work
         // queued: an MMA of 128 weight rows takes 66 cycles for up to 32 columns and 81 for 128, eight of them 530 .. 650 per k-block, and the
         // waits, votes and elections of a whole warp came on top (4 rows, 8 experts, 1024 x 2816: 42.9 us a call, like this 40.6).
@@ -198,6 +232,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
             if (!ok) gave_up(STATUS_STREAM_MMA);
         }
     } else {
+        if (p.early) chain_wait();
         const int quad = warp & 3;
         int iter = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++iter) {
@@ -306,13 +341,14 @@ bool few_tokens(const qmoe_route_t* r, int experts, long long tiles_per_expert) 
 // The mean is of the whole route.  An expert-parallel view counts the tokens of all ranks over its own experts and so
 // changes over earlier than it need, by the number of ranks.
 constexpr long long kStreamRowsPerExpert = 96, kStreamRowsOfFewTiles = 24;
+bool stream_down_early(const qmoe_route_t* r, const qmoe_experts_t* ex) { return few_tokens(r, ex->experts, ceil_div(ex->hidden, SM_ROWS)); }
 bool stream_shape_ok(const qmoe_route_t* r, const qmoe_experts_t* ex) {
     const long long tiles = (long long)ex->experts * ceil_div(ex->hidden, SM_ROWS);
     const long long rows = tiles * 4 <= sm_count() && ex->width > 1536 ? kStreamRowsOfFewTiles : kStreamRowsPerExpert;
     return r->tokens * r->top_k <= rows * ex->experts && !kernel_variant(QMOE_VARIANT_NO_STREAM_GEMM);
 }
 
-int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows,
+int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, bool pad_rows, bool early, bool let_next,
                           cudaStream_t stream) {
     StreamParams p = {};
     const uint64_t d = (uint64_t)ex->width, hd = (uint64_t)ex->hidden, E = (uint64_t)ex->experts;
@@ -322,11 +358,11 @@ int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
     p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
     p.out0 = (__nv_bfloat16*)g; p.out1 = (__nv_bfloat16*)u; p.out2 = (__nv_bfloat16*)h;
     p.experts = ex->experts; p.m_tiles = ceil_div((long long)hd, SM_ROWS); p.N = (int)hd; p.K = (int)d;
-    p.pad_rows = pad_rows;
+    p.pad_rows = pad_rows; p.early = early; p.let_next = let_next;
     return few_tokens(r, ex->experts, p.m_tiles) ? stream_launch<STREAM_SWIGLU, true>(p, stream) : stream_launch<STREAM_SWIGLU>(p, stream);
 }
 
-int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows,
+int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows, bool early,
                    cudaStream_t stream) {
     StreamParams p = {};
     if (int rc = make_map_2d(&p.map_w, b, (uint64_t)K, (uint64_t)experts * N, SM_ROWS)) return rc;
@@ -334,7 +370,7 @@ int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, u
     if (int rc = make_map_2d(&p.map_x, a, (uint64_t)K, (uint64_t)r->rows_bound, X_BOX)) return rc;
     p.offsets = (const int*)r->offsets; p.counts = (const int*)r->counts; p.status = device_status_address();
     p.out0 = (__nv_bfloat16*)c;
-    p.experts = experts; p.N = (int)N; p.K = (int)K; p.pad_rows = pad_rows;
+    p.experts = experts; p.N = (int)N; p.K = (int)K; p.pad_rows = pad_rows; p.early = early;
     // Two weight tiles per stage where that leaves a tile for every SM and an expert's rows take more than one box of
     // activations: 64 experts, 94 rows on average, 1408 -> 2048 columns: 81 us with one, 74 with two; but 16 experts, 96 rows,
     // 2048 -> 1024 columns (64 tiles of 256): 27 with one, 32 with two.

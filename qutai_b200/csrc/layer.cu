@@ -61,9 +61,10 @@ SimtGemmArgs simt_wgrad_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint
 
 using namespace qmoe;
 
-// pad_rows: see stream_swiglu_forward (the kernels for many rows always write whole 128-row tiles)
+// pad_rows: see stream_swiglu_forward (the kernels for many rows always write whole 128-row tiles); behind_permute: the launch before this
+// call was the caller's permutation of the same route
 static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u, uint64_t h, uint64_t y,
-                          int32_t parts, bool pad_rows, uint64_t stream_) {
+                          int32_t parts, bool pad_rows, bool behind_permute, uint64_t stream_) {
     int engine = 0;
     if (int rc = check_experts(r, ex, &engine)) return rc;
     if (!(parts & (QMOE_FWD_UP | QMOE_FWD_DOWN)) || (parts & ~(QMOE_FWD_UP | QMOE_FWD_DOWN)))
@@ -73,10 +74,11 @@ static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
     cudaStream_t stream = (cudaStream_t)stream_;
     const long long d = ex->width, hd = ex->hidden;
     const bool tc = engine == QMOE_ENGINE_TCGEN05, few_rows = tc && stream_shape_ok(r, ex);
+    const bool down_early = few_rows && parts == (QMOE_FWD_UP | QMOE_FWD_DOWN) && stream_down_early(r, ex);
     if (parts & QMOE_FWD_UP) {
         if (few_rows) {
             TimedScope timed(KC_EXPERT_GEMM, stream);
-            if (int rc = stream_swiglu_forward(r, ex, x, g, u, h, pad_rows, stream)) return rc;
+            if (int rc = stream_swiglu_forward(r, ex, x, g, u, h, pad_rows, behind_permute, down_early, stream)) return rc;
         } else if (tc) {
             TimedScope timed(KC_EXPERT_GEMM, stream);
             if (int rc = tc_swiglu_forward(r, ex, x, g, u, h, stream)) return rc;
@@ -91,7 +93,7 @@ static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
     }
     if (parts & QMOE_FWD_DOWN) {
         TimedScope timed(KC_EXPERT_GEMM, stream);
-        if (few_rows) return stream_rows_nt(r, ex->experts, h, ex->w_down, y, hd, d, pad_rows, stream);
+        if (few_rows) return stream_rows_nt(r, ex->experts, h, ex->w_down, y, hd, d, pad_rows, down_early, stream);
         return tc ? tc_rows_nt(r, ex->experts, h, ex->w_down, y, hd, d, stream)
                   : simt_rows(r, ex, h, ex->w_down, 0, 0, y, hd, d, true, stream);
     }
@@ -100,7 +102,7 @@ static int expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
 
 extern "C" int qmoe_expert_forward_parts(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u,
                                          uint64_t h, uint64_t y, int32_t parts, uint64_t stream) {
-    return expert_forward(r, ex, x, g, u, h, y, parts, true, stream);
+    return expert_forward(r, ex, x, g, u, h, y, parts, true, false, stream);
 }
 
 extern "C" int qmoe_expert_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t x, uint64_t g, uint64_t u,
@@ -331,8 +333,8 @@ extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
     if (int rc = qmoe_router_forward(L->x, ex->dtype, L->w_router, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
     const int pad = layer_pad(r, ex, engine);
-    if (int rc = launch_permute(r, L->x, L->x_dispatched, ex->dtype, d, pad, stream)) return rc;
-    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, stream))
+    if (int rc = launch_permute(r, L->x, L->x_dispatched, ex->dtype, d, pad, engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex), stream)) return rc;
+    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, true, stream))
         return rc;
     return qmoe_combine(r, L->y_dispatched, L->out, ex->dtype, d, stream);
 }
@@ -396,7 +398,7 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
     if (int rc = qmoe_route(r, L->scores, stream)) return rc;
     const int pad = layer_pad(r, ex, engine);
     if (int rc = launch_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, pad, stream)) return rc;
-    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, stream))
+    if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, true, stream))
         return rc;
     return qmoe_combine_residual(r, L->y_dispatched, L->x, L->out, ex->dtype, d, stream);
 }

@@ -30,15 +30,16 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
 // read T*d instead of A*d times (the k copies of a token lie far apart in the dispatched layout and
 // would miss L2).  Pad rows are zeroed afterwards, a warp per row, from the experts' offsets and counts: up to the next multiple
 // of 2^pad_bits rows.
-// The next kernel does not start early: these CTAs hold unequal numbers of pad rows and finish unevenly, and where they do first the
+// The next kernel does not start early, unless it is a product for few rows, which has one small CTA per SM and weights to fetch meanwhile: these CTAs hold unequal numbers of pad rows and finish unevenly, and where they do first the
 // next kernel's CTAs would crowd (1003 rows of 2048 floats, 64 experts, top 6, us in ordinary launches, with chain_next and without: permute after
 // permute 16.7, 20.0 and 14.3; combine, its backward and the gather of the input gradient 52.8, 57.4 and 48.3).
 template <typename T, bool VEC, int KMAX>
 __global__ void __launch_bounds__(kThreads)
 permute_kernel(const T* __restrict__ x, T* __restrict__ out, const int* __restrict__ dest_row,
                const int* __restrict__ offsets, const int* __restrict__ counts, int experts, int pad_bits, long long tokens, int k,
-               long long width, int part_bits) {
-    chain_wait();      // no chain_next, see above
+               long long width, int part_bits, int let_next) {
+    chain_wait();
+    if (let_next) chain_next();      // see above
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
@@ -454,10 +455,10 @@ int launch_swiglu_backward(const qmoe_route_t* r, uint64_t dh, uint64_t g, uint6
 using namespace qmoe;
 
 extern "C" int qmoe_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, uint64_t stream) {
-    return launch_permute(r, x, out, dtype, width, kRowPad, stream);
+    return launch_permute(r, x, out, dtype, width, kRowPad, false, stream);
 }
 
-int qmoe::launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, uint64_t stream_) {
+int qmoe::launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, bool let_next, uint64_t stream_) {
     if (int rc = route_check(r)) return rc;
     if (int rc = check_dtype(dtype)) return rc;
     if (!x || !out || width <= 0) return fail_arg("permute: null address or non-positive width");
@@ -469,7 +470,7 @@ int qmoe::launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_
     const long long warps = r->tokens << part_bits;
     const int pad_bits = pad == kRowPad ? 7 : 4;
     const int grid = grid_for_rows(warps > (long long)r->experts * pad / 2 ? warps : (long long)r->experts * pad / 2);
-#define ARGS(T) grid, kThreads, 0, stream, (const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits
+#define ARGS(T) grid, kThreads, 0, stream, (const T*)x, (T*)out, (const int*)r->dest_row, (const int*)r->offsets, (const int*)r->counts, r->experts, pad_bits, (long long)r->tokens, r->top_k, (long long)width, part_bits, let_next ? 1 : 0
 #define BY_K(T, V)                                                  \
     do {                                                            \
         if (r->top_k <= 1) chained(permute_kernel<T, V, 1>, ARGS(T));         \
