@@ -85,8 +85,11 @@ __global__ void __launch_bounds__(kWarps * 32)
 route_topk_kernel(const float* __restrict__ scores, float* __restrict__ probs,
                   float* __restrict__ gate_w, int* __restrict__ expert_idx,
                   int* __restrict__ block_counts, float* __restrict__ block_colsum,
-                  long long T, int E, int k) {
+                  long long T, int E, int k, int* __restrict__ row_source, long long rows_bound) {
     chain_begin();
+    // every dispatched row a pad row until the packing kernel, two launches on, says otherwise; a memset between two kernels is a gap of 2 us on
+    // both sides of its own 1.4
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rows_bound; i += (long long)gridDim.x * blockDim.x) row_source[i] = -1;
     __shared__ int s_cnt[kMaxExperts];
     __shared__ float s_col[kWarps][32 * EPL];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -476,11 +479,10 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
         QMOE_LAUNCH_CHECK("route_small_kernel");
         return 0;
     }
-    QMOE_CUDA(cudaMemsetAsync((void*)r->row_source, 0xff, (size_t)r->rows_bound * sizeof(int), stream));
-    if (epl <= 1) chained(route_topk_kernel<1>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
-    else if (epl <= 2) chained(route_topk_kernel<2>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
-    else if (epl <= 4) chained(route_topk_kernel<4>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
-    else chained(route_topk_kernel<8>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k);
+    if (epl <= 1) chained(route_topk_kernel<1>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k, (int*)r->row_source, (long long)r->rows_bound);
+    else if (epl <= 2) chained(route_topk_kernel<2>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k, (int*)r->row_source, (long long)r->rows_bound);
+    else if (epl <= 4) chained(route_topk_kernel<4>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k, (int*)r->row_source, (long long)r->rows_bound);
+    else chained(route_topk_kernel<8>, nblk, kWarps * 32, 0, stream, sc, probs, gw, eidx, bc, bs, T, E, k, (int*)r->row_source, (long long)r->rows_bound);
     QMOE_LAUNCH_CHECK("route_topk_kernel");
     chained(route_scan_kernel, 1, kScanThreads, 0, stream, bc, bs, (int*)r->block_base, (int*)r->counts,
                                                       (int*)r->offsets, (int*)r->tile_expert,

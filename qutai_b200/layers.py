@@ -454,7 +454,7 @@ class MoEFeedForward:
             moe = self.ffn
             E, d = moe.n_experts, moe.d_model
             S = DeviceStorage
-            extra = dict(inverse=S(tokens, "float32"), w_router_folded=S(E * d, "float32"), d_norm_weight=S(d, "float32"),
+            extra = dict(inverse=S(tokens, "float32"), w_router_folded=S(E * d, "float32"),
                          norm_partials=S(int(lib.load().qmoe_norm_backward_partials(tokens, d)), "float32"))
             block = dict(struct=lib.Block(), extra=extra, work=work)
             for name, storage in extra.items():
@@ -513,11 +513,12 @@ class MoEFeedForward:
         layer.x, layer.grad_out, layer.grad_aux, layer.dx = x_storage.ptr, g.ptr, 0 if ga is None else ga.ptr, dx.ptr
         struct.layer = layer
         struct.norm_weight, struct.norm_eps = self.ffn_norm.weight.storage.ptr, self.ffn_norm.eps
+        d_norm = DeviceStorage(moe.d_model, "float32")     # handed out below: a buffer of the block would have to be copied
+        struct.d_norm_weight = d_norm.ptr
         lib.call("qmoe_block_backward", ctypes.byref(struct), moe.stream)
         views = work["grad_views"]
         counts = moe.last_counts
-        d_norm = Tensor(block["extra"]["d_norm_weight"].copy(moe.stream), (moe.d_model,))   # the buffer is reused by the next backward
-        _accumulate(self.ffn_norm.weight, d_norm, moe.stream)
+        _accumulate(self.ffn_norm.weight, Tensor(d_norm, (moe.d_model,)), moe.stream)
         _accumulate(moe.router.weight, views[0], moe.stream)
         for i, expert in enumerate(moe.experts):
             if not counts[i]:
