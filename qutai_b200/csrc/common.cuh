@@ -182,6 +182,19 @@ __device__ __forceinline__ void zero_pad_rows(T* out, const int* offsets, const 
     }
 }
 
+// this warp's sum of squares of a row of 16-byte pieces, in every lane: the order is part of the norm's result
+template <typename T> __device__ __forceinline__ float row_square_sum(const T* src, long long width) {
+    constexpr int N = Vec16<T>::N;
+    float total = 0.f;
+    for (int c = threadIdx.x & 31; c < (int)(width / N); c += 32) {
+        float f[N];
+        Vec16<T>::unpack(*reinterpret_cast<const uint4*>(src + (long long)c * N), f);
+#pragma unroll
+        for (int i = 0; i < N; ++i) total = fmaf(f[i], f[i], total);
+    }
+    return warp_sum(total);
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 int sm_count();
 
@@ -222,6 +235,10 @@ int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uin
 bool router_norm_ok(int64_t tokens, int32_t experts, int64_t width, int32_t x_dtype, uint64_t x, uint64_t scratch);
 int router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
                         int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
+// the same on the tensor cores, for any number of tokens (router_tensor_cores): the logits of the normalised rows from the raw ones
+bool router_tensor_cores(int32_t x_dtype, int32_t experts, int64_t width, uint64_t x, uint64_t scratch);
+int router_forward_scaled(uint64_t x, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores, uint64_t scratch,
+                          int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
 int router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t dx_router,
                            uint64_t d_w_router, uint64_t col_scale, uint64_t scratch, int64_t tokens, int64_t width, int32_t experts, uint64_t stream);
 int route_check(const qmoe_route_t* r);
@@ -255,7 +272,7 @@ int tc_wgrad3(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t h_act, u
               uint64_t d_w_down, uint64_t d_w_gate, uint64_t d_w_up, long long d, long long h, cudaStream_t stream);
 int tc_wgrad1(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t out, long long M, long long N, cudaStream_t stream,
               int groups = 1, long long slab = 0, int sum_rows = 0);
-int tc_router_forward(uint64_t x, uint64_t w3, uint64_t scores, long long T, long long d, int E, int S, cudaStream_t stream);
+int tc_router_forward(uint64_t x, uint64_t w3, uint64_t scores, uint64_t row_scale, long long T, long long d, int E, int S, cudaStream_t stream);
 int tc_plain_f32_nn(uint64_t a, uint64_t b, uint64_t c, long long T, long long K, long long N, cudaStream_t stream);
 int tc_split_wgrad(uint64_t a, long long a_pitch, uint64_t b, uint64_t partial, const int* offsets, const int* counts,
                    int splits, long long T, long long M, long long N, cudaStream_t stream);

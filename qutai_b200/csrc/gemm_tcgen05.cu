@@ -86,7 +86,7 @@ struct alignas(64) GemmParams {
     void* out0;           // PLAIN: C bf16; SWIGLU: G; WGRAD: C fp32 (stacked per expert); DSWIGLU: dG
     void* out1;           // SWIGLU: U; DSWIGLU: dU
     void* out2;           // SWIGLU: H
-    const void* in0;      // DSWIGLU: G (saved by the forward)
+    const void* in0;      // DSWIGLU: G (saved by the forward); ROUTER: a factor for every row, or null
     const void* in1;      // DSWIGLU: U
     long long ldc;        // row pitch of the outputs, in elements
     long long c_slab;     // WGRAD: elements per expert
@@ -851,6 +851,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                 // scores = x . (W_hi + W_mid + W_lo)^T: the three partial products sit S columns apart
                 float* C = (float*)p.out0 + row * p.ldc;
                 const int S = p.group_stride;
+                const float scale = p.in0 && row < p.M ? ((const float*)p.in0)[row] : 1.f;
 #pragma unroll 1
                 for (int c = half; c * 32 < S; c += 2) {
                     uint32_t r0[32], r1[32], r2[32];
@@ -862,8 +863,10 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
                     if (row < p.M) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (i < valid)
-                                C[c * 32 + i] = (__uint_as_float(r2[i]) + __uint_as_float(r1[i])) + __uint_as_float(r0[i]);
+                            if (i < valid) {
+                                const float v = (__uint_as_float(r2[i]) + __uint_as_float(r1[i])) + __uint_as_float(r0[i]);
+                                C[c * 32 + i] = v * scale;      // a factor of 1 changes no bit
+                            }
                     }
                 }
             } else if (MODE == MODE_WGRAD && ((p.transpose_out >> tile.problem) & 1)) {
@@ -1201,14 +1204,14 @@ int tc_dswiglu(const qmoe_route_t* r, int experts, uint64_t dy, uint64_t w_down,
     return launch<MODE_DSWIGLU, false, true>(p, stream);
 }
 
-// scores [T, E] (fp32) = x [T, d] . (W_hi + W_mid + W_lo)^T, w3 = [3S, d] bf16 with the three terms S rows apart
-int tc_router_forward(uint64_t x, uint64_t w3, uint64_t scores, long long T, long long d, int E, int S, cudaStream_t stream) {
+// scores [T, E] (fp32) = x [T, d] . (W_hi + W_mid + W_lo)^T (times row_scale[t], when given), w3 = [3S, d] bf16 with the three terms S rows apart
+int tc_router_forward(uint64_t x, uint64_t w3, uint64_t scores, uint64_t row_scale, long long T, long long d, int E, int S, cudaStream_t stream) {
     GemmParams p = {};
     if (int rc = make_map(&p.map_a, x, (uint64_t)d, (uint64_t)T, BM)) return rc;
     if (int rc = make_map(&p.map_b, w3, (uint64_t)d, (uint64_t)3 * S, BN)) return rc;
     p.map_a2 = p.map_a; p.map_b2 = p.map_b;
     p.status = device_status_address();
-    p.out0 = (void*)scores; p.ldc = E; p.experts = 1; p.n_tiles = 1;
+    p.out0 = (void*)scores; p.in0 = (const void*)row_scale; p.ldc = E; p.experts = 1; p.n_tiles = 1;
     p.M = (int)T; p.N = E; p.K = (int)d; p.b_rows = 0; p.segments = 1; p.plain_rows = (int)T; p.group_stride = S;
     return launch<MODE_ROUTER, false, false>(p, stream);
 }

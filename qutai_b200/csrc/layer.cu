@@ -389,6 +389,10 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
     if (router_norm_ok(r->tokens, r->experts, d, ex->dtype, L->x, L->router_partials)) {
         if (int rc = router_forward_norm(L->x, ex->dtype, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, r->tokens, d, r->experts, stream))
             return rc;
+    } else if (router_tensor_cores(ex->dtype, r->experts, d, L->x, L->router_partials)) {
+        if (int rc = router_forward_scaled(L->x, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, L->router_partials, r->tokens, d, r->experts,
+                                           stream))
+            return rc;
     } else {
         if (int rc = qmoe_rms_inverse(L->x, ex->dtype, B->inverse, r->tokens, d, B->norm_eps, stream)) return rc;
         if (int rc = qmoe_scale_f32(L->w_router, B->w_router_folded, 0, B->norm_weight, E, d, stream)) return rc;

@@ -50,20 +50,14 @@ rms_inverse_kernel(const T* __restrict__ x, float* __restrict__ inverse, long lo
         const T* src = x + t * width;
         float total = 0.f;
         if constexpr (VEC) {
-            constexpr int N = Vec16<T>::N;
-            for (int c = lane; c < (int)(width / N); c += 32) {
-                float f[N];
-                Vec16<T>::unpack(*reinterpret_cast<const uint4*>(src + (long long)c * N), f);
-#pragma unroll
-                for (int i = 0; i < N; ++i) total = fmaf(f[i], f[i], total);
-            }
+            total = row_square_sum(src, width);
         } else {
             for (long long c = lane; c < width; c += 32) {
                 const float v = Act<T>::load(src + c);
                 total = fmaf(v, v, total);
             }
+            total = warp_sum(total);
         }
-        total = warp_sum(total);
         if (lane == 0) inverse[t] = rsqrtf(total / (float)width + eps);
     }
 }

@@ -60,27 +60,47 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& hi, __nv_bfloat16
     lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
 }
 
-// W [E, d] fp32 -> w3 [3S, d] = {hi; mid; lo}, wbwd [6S, d] = {hi; hi; hi; mid; mid; 0}; rows E..S-1 zero
-__global__ void __launch_bounds__(256)
-router_split_w_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ w3, __nv_bfloat16* __restrict__ wbwd, int E, int S,
-                      long long d) {
-    chain_begin();
+// Elements first, first + step, ... of W [E, d] fp32 (times col_scale[j], when given) -> w3 [3S, d] = {hi; mid; lo} (forward), or wbwd [6S, d] = {hi; hi; hi; mid; mid; 0}
+// (backward); rows E..S-1 zero
+__device__ __forceinline__ void split_w(const float* __restrict__ w, const float* __restrict__ col_scale, __nv_bfloat16* __restrict__ w3,
+                                        __nv_bfloat16* __restrict__ wbwd, int E, int S, long long d, long long first, long long step) {
     const long long n = (long long)S * d;
     const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    for (long long i = first; i < n; i += step) {
         const long long r = i / d;
         __nv_bfloat16 hi, mid, lo;
-        split3(r < E ? w[i] : 0.f, hi, mid, lo);
-        w3[i] = hi; w3[n + i] = mid; w3[2 * n + i] = lo;
-        wbwd[i] = hi; wbwd[n + i] = hi; wbwd[2 * n + i] = hi; wbwd[3 * n + i] = mid; wbwd[4 * n + i] = mid; wbwd[5 * n + i] = zero;
+        float v = r < E ? w[i] : 0.f;
+        if (col_scale && r < E) v *= col_scale[i - r * d];
+        split3(v, hi, mid, lo);
+        if (w3) { w3[i] = hi; w3[n + i] = mid; w3[2 * n + i] = lo; }
+        if (wbwd) { wbwd[i] = hi; wbwd[n + i] = hi; wbwd[2 * n + i] = hi; wbwd[3 * n + i] = mid; wbwd[4 * n + i] = mid; wbwd[5 * n + i] = zero; }
     }
 }
 
-// ds [T, E] fp32 (first multiplied by row_scale[t] in place, when given) -> ds6 [T, 6S] = {hi | mid | lo | hi | mid | 0}; also the
-// token-block tables of the split contraction
+// What the forward's product needs: the weight terms, by the first w_blocks blocks, and with x the inverse of every row's norm, by a warp per
+// row of the others.  One launch each and one for the weight times the norm weight were three, and the scaled logits a fourth behind the
+// product: block of 3001 rows, 16 experts, 1024 x 2048, forward and backward 429 -> 427 us, with the backward's two below in one.
 __global__ void __launch_bounds__(256)
-router_split_ds_kernel(float* __restrict__ ds, const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S,
-                       int* __restrict__ tables, int splits, long long rows_per_split) {
+router_prepare_kernel(const float* __restrict__ w, const float* __restrict__ col_scale, __nv_bfloat16* __restrict__ w3, int E, int S, long long d, int w_blocks,
+                      const __nv_bfloat16* __restrict__ x, float* __restrict__ inverse, long long tokens, float eps) {
+    chain_begin();
+    if ((int)blockIdx.x < w_blocks) {
+        split_w(w, col_scale, w3, nullptr, E, S, d, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)w_blocks * blockDim.x);
+        return;
+    }
+    const long long warp = (long long)(blockIdx.x - w_blocks) * 8 + (threadIdx.x >> 5), warps = (long long)(gridDim.x - w_blocks) * 8;
+    for (long long t = warp; t < tokens; t += warps) {
+        const float total = row_square_sum(x + t * d, d);
+        if ((threadIdx.x & 31) == 0) inverse[t] = rsqrtf(total / (float)d + eps);
+    }
+}
+
+// What the backward's products need: the weight terms, by the first w_blocks blocks; by the others ds [T, E] fp32 (first multiplied by
+// row_scale[t] in place, when given) -> ds6 [T, 6S] = {hi | mid | lo | hi | mid | 0}; also the token-block tables of the split contraction
+__global__ void __launch_bounds__(256)
+router_split_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ wbwd, long long d, int w_blocks, float* __restrict__ ds,
+                    const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ ds6, long long T, int E, int S,
+                    int* __restrict__ tables, int splits, long long rows_per_split) {
     chain_begin();
     if (blockIdx.x == 0 && threadIdx.x <= splits) {
         const int i = threadIdx.x;
@@ -90,9 +110,13 @@ router_split_ds_kernel(float* __restrict__ ds, const float* __restrict__ row_sca
             tables[splits + 1 + i] = (int)(c < 0 ? 0 : (c > rows_per_split ? rows_per_split : c));  // counts[splits]
         }
     }
+    if ((int)blockIdx.x < w_blocks) {
+        split_w(w, nullptr, nullptr, wbwd, E, S, d, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)w_blocks * blockDim.x);
+        return;
+    }
     const long long n = T * S;
     const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    for (long long i = (long long)(blockIdx.x - w_blocks) * blockDim.x + threadIdx.x; i < n; i += (long long)(gridDim.x - w_blocks) * blockDim.x) {
         const long long t = i / S;
         const int e = (int)(i - t * S);
         __nv_bfloat16 hi, mid, lo;
@@ -251,10 +275,27 @@ extern "C" int qmoe_router_forward(uint64_t x, int32_t x_dtype, uint64_t w_route
         return simt_router_logits(x, x_dtype, w_router, scores, tokens, width, experts, stream);
     TimedScope timed(KC_ROUTER_GEMM, stream);
     const RouterScratch r = plan_scratch(tokens, experts, width);
-    chained(router_split_w_kernel, elem_grid((long long)r.S * width), 256, 0, stream, 
-        (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, r.S, width);
-    QMOE_LAUNCH_CHECK("router_split_w_kernel");
-    return tc_router_forward(x, scratch + r.w3, scores, tokens, width, experts, r.S, stream);
+    const int w_blocks = elem_grid((long long)r.S * width);
+    chained(router_prepare_kernel, w_blocks, 256, 0, stream, (const float*)w_router, nullptr, (__nv_bfloat16*)(scratch + r.w3), experts, r.S, width, w_blocks,
+            nullptr, nullptr, 0, 0.f);
+    QMOE_LAUNCH_CHECK("router_prepare_kernel");
+    return tc_router_forward(x, scratch + r.w3, scores, 0, tokens, width, experts, r.S, stream);
+}
+
+bool qmoe::router_tensor_cores(int32_t x_dtype, int32_t experts, int64_t width, uint64_t x, uint64_t scratch) {
+    return tc_router_ok(x_dtype, experts, width, x, scratch);
+}
+
+int qmoe::router_forward_scaled(uint64_t x, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores, uint64_t scratch,
+                                int64_t tokens, int64_t width, int32_t experts, uint64_t stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    TimedScope timed(KC_ROUTER_GEMM, stream);
+    const RouterScratch r = plan_scratch(tokens, experts, width);
+    const int w_blocks = elem_grid((long long)r.S * width), row_blocks = elem_grid(tokens * 32);
+    chained(router_prepare_kernel, w_blocks + row_blocks, 256, 0, stream, (const float*)w_router, (const float*)norm_weight, (__nv_bfloat16*)(scratch + r.w3),
+            experts, r.S, width, w_blocks, (const __nv_bfloat16*)x, (float*)inverse, tokens, (float)eps);
+    QMOE_LAUNCH_CHECK("router_prepare_kernel");
+    return tc_router_forward(x, scratch + r.w3, scores, inverse, tokens, width, experts, r.S, stream);
 }
 
 bool qmoe::router_norm_ok(int64_t tokens, int32_t experts, int64_t width, int32_t x_dtype, uint64_t x, uint64_t scratch) {
@@ -307,13 +348,10 @@ int qmoe::router_backward_scaled(uint64_t d_scores, uint64_t row_scale, uint64_t
     const RouterScratch r = plan_scratch(tokens, experts, width);
     const int S = r.S;
     int* tables = (int*)(scratch + r.tables);
-    // the weight terms are rebuilt here as well: the scratch may have been used by another layer since the forward
-    chained(router_split_w_kernel, elem_grid((long long)S * width), 256, 0, stream, 
-        (const float*)w_router, (__nv_bfloat16*)(scratch + r.w3), (__nv_bfloat16*)(scratch + r.wbwd), experts, S, width);
-    QMOE_LAUNCH_CHECK("router_split_w_kernel");
-    chained(router_split_ds_kernel, elem_grid(tokens * S), 256, 0, stream, (float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6),
-                                                                      tokens, experts, S, tables, r.splits, r.rows_per_split);
-    QMOE_LAUNCH_CHECK("router_split_ds_kernel");
+    const int w_blocks = elem_grid((long long)S * width);
+    chained(router_split_kernel, w_blocks + elem_grid(tokens * S), 256, 0, stream, (const float*)w_router, (__nv_bfloat16*)(scratch + r.wbwd), width, w_blocks,
+            (float*)d_scores, (const float*)row_scale, (__nv_bfloat16*)(scratch + r.ds6), tokens, experts, S, tables, r.splits, r.rows_per_split);
+    QMOE_LAUNCH_CHECK("router_split_kernel");
     if (dx_router)
         if (int rc = tc_plain_f32_nn(scratch + r.ds6, scratch + r.wbwd, dx_router, tokens, 6ll * S, width, stream)) return rc;
     if (d_w_router) {
