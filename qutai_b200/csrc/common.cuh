@@ -195,6 +195,60 @@ template <typename T> __device__ __forceinline__ float row_square_sum(const T* s
     return warp_sum(total);
 }
 
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+}
+// One router logit by one warp, in every lane: row . w, with the lanes striding over the width and a fixed shuffle tree.  Four 16-byte loads of
+// the weight row and of the token row are in flight per lane and iteration, so the few round trips to L2 overlap.
+// NORM: the logit of the normalised row, inv * (row . (w * norm weight)), with inv = 1 / rms from the same pass over the row.
+template <typename T, bool NORM>
+__device__ __forceinline__ float small_logit(const T* row, const float* we, long long d, const float* norm_weight, float eps, float& inv) {
+    const int lane = threadIdx.x & 31;
+    const bool vec = (d & 3) == 0 && (((uintptr_t)row | (uintptr_t)we | (NORM ? (uintptr_t)norm_weight : 0)) & 15u) == 0;
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, square = 0.f;
+    if (vec) {
+        for (long long j = (long long)lane * 4; j < d; j += 512) {
+            float4 wv[4], xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const long long at = j + 128 * u;
+                const bool in = at < d;
+                wv[u] = in ? load4(we + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                xv[u] = in ? load4(row + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (NORM && in) {
+                    const float4 nv = load4(norm_weight + at);
+                    wv[u].x *= nv.x; wv[u].y *= nv.y; wv[u].z *= nv.z; wv[u].w *= nv.w;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {   // fixed order: the sums do not depend on timing
+                a0 = fmaf(xv[u].x, wv[u].x, a0);
+                a1 = fmaf(xv[u].y, wv[u].y, a1);
+                a2 = fmaf(xv[u].z, wv[u].z, a2);
+                a3 = fmaf(xv[u].w, wv[u].w, a3);
+                if (NORM) square = fmaf(xv[u].w, xv[u].w, fmaf(xv[u].z, xv[u].z, fmaf(xv[u].y, xv[u].y, fmaf(xv[u].x, xv[u].x, square))));
+            }
+        }
+    } else {
+        for (long long j = lane; j < d; j += 32) {
+            const float v = Act<T>::load(row + j);
+            a0 = fmaf(v, NORM ? we[j] * norm_weight[j] : we[j], a0);
+            if (NORM) square = fmaf(v, v, square);
+        }
+    }
+    float acc = (a0 + a1) + (a2 + a3);
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, step);
+    if (NORM) {
+        inv = rsqrtf(warp_sum(square) / (float)d + eps);
+        acc *= inv;
+    }
+    return acc;
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 int sm_count();
 
@@ -232,6 +286,10 @@ int launch_simt_gemms(const SimtGemmArgs* g, int count, int a_dtype, int b_dtype
 int launch_permute(const qmoe_route_t* r, uint64_t x, uint64_t out, int32_t dtype, int64_t width, int pad, bool let_next, uint64_t stream);
 int launch_permute_norm(const qmoe_route_t* r, uint64_t x, uint64_t inverse, uint64_t weight, uint64_t out, int32_t dtype, int64_t width, int pad,
                         uint64_t stream);
+// router_forward (with norm_weight router_forward_norm) and the routing in one launch, for a handful of logits (router_route_ok)
+bool router_route_ok(const qmoe_route_t* r);
+int router_route_small(const qmoe_route_t* r, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
+                       int64_t width, uint64_t stream);
 bool router_norm_ok(int64_t tokens, int32_t experts, int64_t width, int32_t x_dtype, uint64_t x, uint64_t scratch);
 int router_forward_norm(uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse, uint64_t scores,
                         int64_t tokens, int64_t width, int32_t experts, uint64_t stream);

@@ -330,8 +330,12 @@ extern "C" int qmoe_layer_forward(const qmoe_layer_t* L, uint64_t stream) {
         if (int rc = qmoe_cast_bf16(L->master_up, ex->w_up, E * hd * d, stream)) return rc;
         if (int rc = qmoe_cast_bf16(L->master_down, ex->w_down, E * hd * d, stream)) return rc;
     }
-    if (int rc = qmoe_router_forward(L->x, ex->dtype, L->w_router, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
-    if (int rc = qmoe_route(r, L->scores, stream)) return rc;
+    if (router_route_ok(r)) {
+        if (int rc = router_route_small(r, L->x, ex->dtype, L->w_router, 0, 0.0, 0, L->scores, d, stream)) return rc;
+    } else {
+        if (int rc = qmoe_router_forward(L->x, ex->dtype, L->w_router, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
+        if (int rc = qmoe_route(r, L->scores, stream)) return rc;
+    }
     const int pad = layer_pad(r, ex, engine);
     if (int rc = launch_permute(r, L->x, L->x_dispatched, ex->dtype, d, pad, engine == QMOE_ENGINE_TCGEN05 && stream_shape_ok(r, ex), stream)) return rc;
     if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, true, stream))
@@ -386,7 +390,10 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
         if (int rc = qmoe_cast_bf16(L->master_down, ex->w_down, E * hd * d, stream)) return rc;
     }
     // scores = rms_norm(x) . W_r^T = inverse[t] * (x . (W_r * w)^T): the product reads the raw activations
-    if (router_norm_ok(r->tokens, r->experts, d, ex->dtype, L->x, L->router_partials)) {
+    const bool with_routing = router_route_ok(r);
+    if (with_routing) {
+        if (int rc = router_route_small(r, L->x, ex->dtype, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, d, stream)) return rc;
+    } else if (router_norm_ok(r->tokens, r->experts, d, ex->dtype, L->x, L->router_partials)) {
         if (int rc = router_forward_norm(L->x, ex->dtype, L->w_router, B->norm_weight, B->norm_eps, B->inverse, L->scores, r->tokens, d, r->experts, stream))
             return rc;
     } else if (router_tensor_cores(ex->dtype, r->experts, d, L->x, L->router_partials)) {
@@ -399,7 +406,8 @@ extern "C" int qmoe_block_forward(const qmoe_block_t* B, uint64_t stream) {
         if (int rc = qmoe_router_forward(L->x, ex->dtype, B->w_router_folded, L->scores, L->router_partials, r->tokens, d, r->experts, stream)) return rc;
         if (int rc = qmoe_scale_f32(L->scores, L->scores, B->inverse, 0, r->tokens, E, stream)) return rc;
     }
-    if (int rc = qmoe_route(r, L->scores, stream)) return rc;
+    if (!with_routing)
+        if (int rc = qmoe_route(r, L->scores, stream)) return rc;
     const int pad = layer_pad(r, ex, engine);
     if (int rc = launch_permute_norm(r, L->x, B->inverse, B->norm_weight, L->x_dispatched, ex->dtype, d, pad, stream)) return rc;
     if (int rc = expert_forward(r, ex, L->x_dispatched, L->g, L->u, L->h, L->y_dispatched, QMOE_FWD_UP | QMOE_FWD_DOWN, pad == kRowPad, true, stream))

@@ -167,16 +167,7 @@ bool small_router(long long tokens, int experts, long long width, int x_dtype, b
     const double there = tensor_cores ? 6 + 5.6e-3 * d + 6e-7 * T * d : 7.5e-2 * d * (T > 30000 ? T / 30000 : 1);
     return here <= there + (norm ? 9 : 0);     // with the norm: three launches more
 }
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
-    const uint2 v = *reinterpret_cast<const uint2*>(p);
-    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
-                       __uint_as_float(v.y & 0xffff0000u));
-}
-// grid (tokens, ceil(E / 8)): warp w of block (t, g) computes scores[t, 8 g + w].  Four 16-byte loads of the weight
-// row and of the token row are in flight per lane and iteration, so the few round trips to L2 overlap.
-// NORM: the logits of the normalised row, inverse * (x . (w * norm weight)), with inverse = 1 / rms from the same pass over
-// the row (kept for the later kernels): four launches in one.
+// grid (tokens, ceil(E / 8)): warp w of block (t, g) computes scores[t, 8 g + w]
 template <typename T, bool NORM>
 __global__ void __launch_bounds__(256)
 router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float* __restrict__ scores, int E, long long d,
@@ -185,48 +176,9 @@ router_small_kernel(const T* __restrict__ x, const float* __restrict__ w, float*
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.y * 8 + warp;
     if (e >= E) return;
-    const T* row = x + (long long)blockIdx.x * d;
-    const float* we = w + (long long)e * d;
-    const bool vec = (d & 3) == 0 && (((uintptr_t)row | (uintptr_t)we | (NORM ? (uintptr_t)norm_weight : 0)) & 15u) == 0;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, square = 0.f;
-    if (vec) {
-        for (long long j = (long long)lane * 4; j < d; j += 512) {
-            float4 wv[4], xv[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const long long at = j + 128 * u;
-                const bool in = at < d;
-                wv[u] = in ? load4(we + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-                xv[u] = in ? load4(row + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-                if (NORM && in) {
-                    const float4 nv = load4(norm_weight + at);
-                    wv[u].x *= nv.x; wv[u].y *= nv.y; wv[u].z *= nv.z; wv[u].w *= nv.w;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {   // fixed order: the sums do not depend on timing
-                a0 = fmaf(xv[u].x, wv[u].x, a0);
-                a1 = fmaf(xv[u].y, wv[u].y, a1);
-                a2 = fmaf(xv[u].z, wv[u].z, a2);
-                a3 = fmaf(xv[u].w, wv[u].w, a3);
-                if (NORM) square = fmaf(xv[u].w, xv[u].w, fmaf(xv[u].z, xv[u].z, fmaf(xv[u].y, xv[u].y, fmaf(xv[u].x, xv[u].x, square))));
-            }
-        }
-    } else {
-        for (long long j = lane; j < d; j += 32) {
-            const float v = Act<T>::load(row + j);
-            a0 = fmaf(v, NORM ? we[j] * norm_weight[j] : we[j], a0);
-            if (NORM) square = fmaf(v, v, square);
-        }
-    }
-    float acc = (a0 + a1) + (a2 + a3);
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, step);
-    if (NORM) {
-        const float inv = rsqrtf(warp_sum(square) / (float)d + eps);
-        acc *= inv;
-        if (lane == 0 && e == 0) inverse[blockIdx.x] = inv;
-    }
+    float inv = 0.f;
+    const float acc = small_logit<T, NORM>(x + (long long)blockIdx.x * d, w + (long long)e * d, d, norm_weight, eps, inv);
+    if (NORM && lane == 0 && e == 0) inverse[blockIdx.x] = inv;
     if (lane == 0) scores[(long long)blockIdx.x * E + e] = acc;
 }
 

@@ -288,12 +288,10 @@ __global__ void publish_counts_kernel(const int* __restrict__ counts, int* __res
 constexpr long long kSmallRouteTokens = 128;
 static_assert(kSmallRouteTokens * kMaxTopK <= kWarps * 32, "a slice of assignments is one per lane");
 template <int EPL>
-__global__ void __launch_bounds__(kWarps * 32, 1)
-route_small_kernel(const float* __restrict__ scores, float* __restrict__ probs, float* __restrict__ gate_w, int* __restrict__ expert_idx,
-                   int* __restrict__ dest_row, int* row_source, int* __restrict__ counts, int* __restrict__ offsets,
-                   int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util, float* __restrict__ aux,
-                   float* __restrict__ block_colsum, int T, int E, int k, long long rows_bound) {
-    chain_begin();
+__device__ __forceinline__ void route_small(const float* scores, float* __restrict__ probs, float* __restrict__ gate_w, int* __restrict__ expert_idx,
+                                            int* __restrict__ dest_row, int* row_source, int* __restrict__ counts, int* __restrict__ offsets,
+                                            int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util, float* __restrict__ aux,
+                                            float* __restrict__ block_colsum, int T, int E, int k, long long rows_bound) {
     // [warp][expert]: probability sums, then assignments; one more column, so that a warp reading one expert's 32 entries
     // meets 32 banks
     __shared__ union { float col[kWarps][32 * EPL + 1]; int hist[kWarps][32 * EPL + 1]; } s;
@@ -365,6 +363,42 @@ route_small_kernel(const float* __restrict__ scores, float* __restrict__ probs, 
         dest_row[a] = dest;
         row_source[dest] = a;      // after the fill above: barriers lie between
     }
+}
+
+template <int EPL>
+__global__ void __launch_bounds__(kWarps * 32, 1)
+route_small_kernel(const float* __restrict__ scores, float* __restrict__ probs, float* __restrict__ gate_w, int* __restrict__ expert_idx,
+                   int* __restrict__ dest_row, int* row_source, int* __restrict__ counts, int* __restrict__ offsets,
+                   int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util, float* __restrict__ aux,
+                   float* __restrict__ block_colsum, int T, int E, int k, long long rows_bound) {
+    chain_begin();
+    route_small<EPL>(scores, probs, gate_w, expert_idx, dest_row, row_source, counts, offsets, tile_expert, meta, util, aux, block_colsum, T, E, k, rows_bound);
+}
+
+// The logits of a handful of tokens and their routing in one launch, a warp per logit.  us a call, in two launches and one: 4 rows, 8 experts,
+// 1024 x 2816, norm to residual, called step by step 45.2 and 42.7 (its launches bound the host), the device alone 38.9 and 39.1; 1 row of
+// 2048, 32 experts, 32.7 and 33.1.  A second logit per warp is a second round trip: 8 rows, 8 experts, 39.8 and 41.5, 2 rows, 32 experts, 41.9 and 45.0.
+constexpr int kRouterRouteLogits = kWarps;
+template <typename X, bool NORM>
+__global__ void __launch_bounds__(kWarps * 32, 1)
+router_route_small_kernel(const X* __restrict__ x, const float* __restrict__ w, long long d, const float* __restrict__ norm_weight, float eps,
+                          float* __restrict__ inverse, float* scores, float* __restrict__ probs, float* __restrict__ gate_w, int* __restrict__ expert_idx,
+                          int* __restrict__ dest_row, int* row_source, int* __restrict__ counts, int* __restrict__ offsets,
+                          int* __restrict__ tile_expert, int* __restrict__ meta, float* __restrict__ util, float* __restrict__ aux,
+                          float* __restrict__ block_colsum, int T, int E, int k, long long rows_bound) {
+    chain_begin();
+    const int i = threadIdx.x >> 5;
+    if (i < T * E) {
+        const int t = i / E, e = i - t * E;
+        float inv = 0.f;
+        const float logit = small_logit<X, NORM>(x + t * d, w + e * d, d, norm_weight, eps, inv);
+        if ((threadIdx.x & 31) == 0) {
+            scores[i] = logit;
+            if (NORM && e == 0) inverse[t] = inv;
+        }
+    }
+    __syncthreads();        // the block reads its own logits
+    route_small<1>(scores, probs, gate_w, expert_idx, dest_row, row_source, counts, offsets, tile_expert, meta, util, aux, block_colsum, T, E, k, rows_bound);
 }
 
 __global__ void route_export_kernel(const int* __restrict__ expert_idx, const int* __restrict__ dest_row,
@@ -493,6 +527,25 @@ extern "C" int qmoe_route(const qmoe_route_t* r, uint64_t scores, uint64_t strea
                                                         (const int*)r->offsets, (int*)r->dest_row,
                                                         (int*)r->row_source, T, E, k);
     QMOE_LAUNCH_CHECK("route_pack_kernel");
+    return 0;
+}
+
+bool qmoe::router_route_ok(const qmoe_route_t* r) { return r->tokens <= kSmallRouteTokens && r->experts <= 32 && r->tokens * r->experts <= kRouterRouteLogits; }
+
+int qmoe::router_route_small(const qmoe_route_t* r, uint64_t x, int32_t x_dtype, uint64_t w_router, uint64_t norm_weight, double eps, uint64_t inverse,
+                             uint64_t scores, int64_t width, uint64_t stream_) {
+    if (int rc = check_route(r, true)) return rc;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    TimedScope timed(KC_ROUTE, stream);
+#define LAUNCH(X, NORM)                                                                                                                    \
+    chained(router_route_small_kernel<X, NORM>, 1, kWarps * 32, 0, stream, (const X*)x, (const float*)w_router, (long long)width,          \
+            (const float*)norm_weight, (float)eps, (float*)inverse, (float*)scores, (float*)r->probs, (float*)r->gate_weights,             \
+            (int*)r->expert_index, (int*)r->dest_row, (int*)r->row_source, (int*)r->counts, (int*)r->offsets, (int*)r->tile_expert,        \
+            (int*)r->meta, (float*)r->utilization, (float*)r->aux, (float*)r->block_colsum, (int)r->tokens, r->experts, r->top_k, (long long)r->rows_bound)
+    if (x_dtype == QMOE_BF16) { if (norm_weight) LAUNCH(__nv_bfloat16, true); else LAUNCH(__nv_bfloat16, false); }
+    else { if (norm_weight) LAUNCH(float, true); else LAUNCH(float, false); }
+#undef LAUNCH
+    QMOE_LAUNCH_CHECK("router_route_small_kernel");
     return 0;
 }
 
