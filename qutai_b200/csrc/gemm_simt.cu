@@ -112,7 +112,7 @@ simt_gemm_kernel(SimtGemmArgs g) {
     }
 }
 
-// ---- fp32 operands, many rows: 128 x 128 tiles ------------------------------------------------------
+// ---- fp32 operands, many rows: 128 x 128 tiles, or 128 x 256 ------------------------------------------------------
 // The same sums in the same order (one fp32 FMA chain per output, k ascending) as the kernel above, bit for bit; what
 // differs is how the operands reach the FMAs.  That kernel fetches two shared-memory words for every four FMAs and
 // stalls on each tile's loads (19 .. 25 TFLOP/s from 128 tiles on); here (30 .. 46) a thread owns 8 x 8 outputs (two 4-row and two 4-column pieces, so that
@@ -120,19 +120,20 @@ simt_gemm_kernel(SimtGemmArgs g) {
 // 16-deep tile travels from global memory through registers into the other shared buffer meanwhile.
 // A_KFAST / B_KFAST: the operand is contiguous along k (rows of 4 k per load, transposed on the way into shared memory),
 // else along its own rows / columns.
-constexpr int TILE = 128, TILE_K = 16, TILE_PITCH = TILE + 4;
+constexpr int TILE = 128, TILE_K = 16, WIDE = 256;
 
-template <bool KFAST>
-struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice of one operand
+template <bool KFAST, int ROWS>
+struct TileLoader {          // this thread's ROWS / 16 values of a TILE_K x ROWS slice of one operand
     const float* base;       // element (row 0 of the tile, k = 0)
     long long pitch;         // elements between rows (KFAST) or between k (not KFAST)
     int rows_left;           // rows of the tile inside the matrix
-    float v[8];
+    static constexpr int PIECES = ROWS / 64;
+    float v[4 * PIECES];
     __device__ __forceinline__ void fetch(long long k0, long long k_end) {
 #pragma unroll
-        for (int l = 0; l < 2; ++l) {
+        for (int l = 0; l < PIECES; ++l) {
             const int i = threadIdx.x + l * 256;
-            const int row = KFAST ? i / 4 : i % (TILE / 4) * 4, k = KFAST ? i % 4 * 4 : i / (TILE / 4);
+            const int row = KFAST ? i / 4 : i % (ROWS / 4) * 4, k = KFAST ? i % 4 * 4 : i / (ROWS / 4);
             float* dst = v + 4 * l;
             const float* src = base + (KFAST ? row * pitch + (k0 + k) : (k0 + k) * pitch + row);
             const int along = KFAST ? (int)(k_end - (k0 + k) < 4 ? k_end - (k0 + k) : 4) : rows_left - row;   // values of the 4 that exist
@@ -146,15 +147,15 @@ struct TileLoader {          // this thread's 8 values of a TILE_K x TILE slice 
             }
         }
     }
-    __device__ __forceinline__ void store(float (*tile)[TILE_PITCH]) const {
+    __device__ __forceinline__ void store(float (*tile)[ROWS + 4]) const {
 #pragma unroll
-        for (int l = 0; l < 2; ++l) {
+        for (int l = 0; l < PIECES; ++l) {
             const int i = threadIdx.x + l * 256;
             if (KFAST) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) tile[i % 4 * 4 + e][i / 4] = v[4 * l + e];
             } else {
-                *reinterpret_cast<float4*>(&tile[i / (TILE / 4)][i % (TILE / 4) * 4]) = make_float4(v[4 * l], v[4 * l + 1], v[4 * l + 2], v[4 * l + 3]);
+                *reinterpret_cast<float4*>(&tile[i / (ROWS / 4)][i % (ROWS / 4) * 4]) = make_float4(v[4 * l], v[4 * l + 1], v[4 * l + 2], v[4 * l + 3]);
             }
         }
     }
@@ -175,25 +176,31 @@ __device__ __forceinline__ int product_index(const SimtTileArgs& args) {
 }
 __device__ __forceinline__ const SimtGemmArgs& product_at(const SimtGemmArgs& args, int) { return args; }
 __device__ __forceinline__ const SimtGemmArgs& product_at(const SimtTileArgs& args, int which) { return args.product[which]; }
+template <int TN>
 __device__ __forceinline__ void tile_at(const SimtGemmArgs&, int, long long& m0, long long& n0) {
     m0 = (long long)blockIdx.y * TILE;
-    n0 = (long long)blockIdx.x * TILE;
+    n0 = (long long)blockIdx.x * TN;
 }
+template <int TN>
 __device__ __forceinline__ void tile_at(const SimtTileArgs& args, int which, long long& m0, long long& n0) {
     const int local = (int)blockIdx.x - (which ? args.end[which - 1] : 0);
     m0 = (long long)(local / args.columns[which]) * TILE;
-    n0 = (long long)(local % args.columns[which]) * TILE;
+    n0 = (long long)(local % args.columns[which]) * TN;
 }
 
-template <bool A_KFAST, bool B_KFAST, bool ALONE>
-__global__ void __launch_bounds__(256, 2)
+template <bool A_KFAST, bool B_KFAST, bool ALONE, int TN, int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
 simt_tile_kernel(const __grid_constant__ TileArgs<ALONE> args) {
     const int which = product_index(args);
     const SimtGemmArgs& g = product_at(args, which);
-    __shared__ __align__(16) float As[2][TILE_K][TILE_PITCH];
-    __shared__ __align__(16) float Bs[2][TILE_K][TILE_PITCH];
+    __shared__ __align__(16) float a_fixed[TN == TILE ? 2 : 1][TILE_K][TILE + 4];
+    __shared__ __align__(16) float b_fixed[TN == TILE ? 2 : 1][TILE_K][TILE + 4];
+    extern __shared__ __align__(16) float launch_memory[];         // the wide tiles' 50 KiB
+    float (*const As)[TILE_K][TILE + 4] = TN == TILE ? a_fixed : reinterpret_cast<float (*)[TILE_K][TILE + 4]>(launch_memory);
+    float (*const Bs)[TILE_K][TN + 4] = reinterpret_cast<float (*)[TILE_K][TN + 4]>(TN == TILE ? &b_fixed[0][0][0] : launch_memory + 2 * TILE_K * (TILE + 4));
+    constexpr int GROUPS = TN / 64;       // four columns of every 64 are this thread's
     long long m0, n0;
-    tile_at(args, which, m0, n0);
+    tile_at<TN>(args, which, m0, n0);
     long long M = g.M, k_begin = 0, k_end = g.K, b_offset = 0;
     float* C = (float*)g.C;
     if (g.mode == SG_ROWS) {
@@ -208,17 +215,17 @@ simt_tile_kernel(const __grid_constant__ TileArgs<ALONE> args) {
         C += (long long)e * g.c_slab;
     }
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    uint64_t acc[8][4];
+    uint64_t acc[8][2 * GROUPS];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < 2 * GROUPS; ++j) acc[i][j] = 0ull;
     for (int seg = 0; seg < 2; ++seg) {
         const float* Ap = (const float*)(seg ? g.A2 : g.A);
         if (!Ap) break;
         const float* Bp = (const float*)(seg ? g.B2 : g.B) + b_offset;
-        TileLoader<A_KFAST> a{Ap + m0 * g.a_rs, A_KFAST ? g.a_rs : g.a_cs, (int)(M - m0 < TILE ? M - m0 : TILE)};
-        TileLoader<B_KFAST> b{Bp + n0 * g.b_cs, B_KFAST ? g.b_cs : g.b_rs, (int)(g.N - n0 < TILE ? g.N - n0 : TILE)};
+        TileLoader<A_KFAST, TILE> a{Ap + m0 * g.a_rs, A_KFAST ? g.a_rs : g.a_cs, (int)(M - m0 < TILE ? M - m0 : TILE)};
+        TileLoader<B_KFAST, TN> b{Bp + n0 * g.b_cs, B_KFAST ? g.b_cs : g.b_rs, (int)(g.N - n0 < TN ? g.N - n0 : TN)};
         a.fetch(k_begin, k_end);
         b.fetch(k_begin, k_end);
         __syncthreads();               // the segment before has been read out of the buffers
@@ -235,14 +242,19 @@ simt_tile_kernel(const __grid_constant__ TileArgs<ALONE> args) {
 #pragma unroll
             for (int kk = 0; kk < TILE_K; ++kk) {
                 const float4 a0 = *reinterpret_cast<const float4*>(&As[buffer][kk][ty * 4]), a1 = *reinterpret_cast<const float4*>(&As[buffer][kk][64 + ty * 4]);
-                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[buffer][kk][tx * 4]), b1 = *reinterpret_cast<const ulonglong2*>(&Bs[buffer][kk][64 + tx * 4]);
                 const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const uint64_t bv[4] = {b0.x, b0.y, b1.x, b1.y};
+                uint64_t bv[2 * GROUPS];
+#pragma unroll
+                for (int q = 0; q < GROUPS; ++q) {
+                    const ulonglong2 two = *reinterpret_cast<const ulonglong2*>(&Bs[buffer][kk][q * 64 + tx * 4]);
+                    bv[2 * q] = two.x;
+                    bv[2 * q + 1] = two.y;
+                }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const uint64_t twice = pair2(av[i], av[i]);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fma2(twice, bv[j], acc[i][j]);
+                    for (int j = 0; j < 2 * GROUPS; ++j) acc[i][j] = fma2(twice, bv[j], acc[i][j]);
                 }
             }
             if (more) {
@@ -258,7 +270,7 @@ simt_tile_kernel(const __grid_constant__ TileArgs<ALONE> args) {
         const long long m = m0 + (i / 4) * 64 + ty * 4 + i % 4;
         if (m >= M) continue;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int half = 0; half < GROUPS; ++half) {
             const long long n = n0 + half * 64 + tx * 4;
             float v[4];
             unpair2(acc[i][2 * half], v[0], v[1]);
@@ -293,13 +305,62 @@ bool tile_kernel_ok(const SimtGemmArgs& g, long long m_extent, int groups) {
     return (long long)ceil_div(g.N, TILE) * ceil_div(m_extent, TILE) * groups * 2 >= sm_count();
 }
 
+template <bool A_KFAST, bool B_KFAST, bool ALONE, int TN, int CTAS>
+int launch_tile_kernel(const TileArgs<ALONE>& args, dim3 grid, cudaStream_t stream) {
+    static bool configured[64] = {};          // per device
+    constexpr int SMEM_BYTES = TN == TILE ? 0 : 2 * TILE_K * (TILE + 4 + TN + 4) * (int)sizeof(float);
+    int dev = 0;
+    QMOE_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail_arg("device ordinal beyond 63");
+    if (SMEM_BYTES && !configured[dev]) {
+        QMOE_CUDA(cudaFuncSetAttribute(simt_tile_kernel<A_KFAST, B_KFAST, ALONE, TN, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        configured[dev] = true;
+    }
+    // Ordinary launches, as for the general kernel: in a chain the CTAs are handed out while those of the kernel before leave, two
+    // to some SMs and none to others, which costs kernels that are as long as their slowest SM more than the gap (2048
+    // rows, 512 x 1024, 8 experts, forward and backward: 1038 us, in a chain 1113; 700 rows, 320 x 300, 4 experts, on the general kernel: 346 and 445).
+    simt_tile_kernel<A_KFAST, B_KFAST, ALONE, TN, CTAS><<<grid, 256, SMEM_BYTES, stream>>>(args);
+    QMOE_LAUNCH_CHECK("simt_tile_kernel");
+    return 0;
+}
+// The forms of the kernel: tiles of 128 x 128, two to an SM (at 128 registers, which spills a little in some); one to an SM; tiles of 128 x 256.
+enum { TILES_TWO, TILES_ONE, TILES_WIDE };
+template <bool A_KFAST, bool B_KFAST, bool ALONE>
+int launch_tile_form(int form, const TileArgs<ALONE>& args, dim3 grid, cudaStream_t stream) {
+    if constexpr (!(A_KFAST && B_KFAST)) {
+        if (form == TILES_WIDE) return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, WIDE, 1>(args, grid, stream);
+        if (form == TILES_ONE) return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, TILE, 1>(args, grid, stream);
+    }
+    return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, TILE, 2>(args, grid, stream);
+}
+
+// Which form: the one that is through first, by the rounds it takes and what a round costs, in units of 128 x 128 tiles at the full rate of an SM's
+// FMA units (they reach two thirds of it in every form): 3.05 for two tiles on an SM (1.8 where the last round leaves one), 1.64 for
+// one alone, 2.5 for a wide one.  us as two to an SM, one and wide: g W 4096 x 1024 x 1024 200, 208 and 189; 1024 x 4096 x 2048 427, 405 and 728; 640 x 640 x
+// 2560 72, 68 and 120; weight gradients of 1024 rows, 4096 x 1024 194, 205 and 185; of 1500, 2048 x 776, 163, 155 and 271.  x W^T does not spill, and two to an
+// SM serve it best or nearly (4096 x 1024 x 1024 193, 209 and 191; 1024 x 4096 x 2048 409, 411 and 741).  The same bits in every form.  Forward and
+// backward, 2048 rows, 8 experts, 512 x 1024, all as two to an SM and by this rule: 1016 and 988 us (dX 225 and 203, a tile for each SM).
+int tile_form(const SimtGemmArgs* products, int count, long long m_extent, int groups) {
+    if (products[0].a_cs == 1 && products[0].b_rs == 1) return TILES_TWO;
+    long long narrow = 0, wide = 0;
+    for (int i = 0; i < count; ++i) {
+        const long long m = products[i].expected_rows ? products[i].expected_rows : m_extent > 0 ? m_extent : products[i].M;
+        narrow += (long long)ceil_div(m, TILE) * ceil_div(products[i].N, TILE) * groups;
+        wide += (long long)ceil_div(m, TILE) * ceil_div(products[i].N, WIDE) * groups;
+    }
+    const long long sms = sm_count(), left = narrow % (2 * sms);
+    const double two = 3.05 * (double)(narrow / (2 * sms)) + (left > sms ? 3.05 : left ? 1.8 : 0.0), one = 1.64 * ceil_div(narrow, sms), as_wide = 2.5 * ceil_div(wide, sms);
+    return as_wide < two && as_wide < one ? TILES_WIDE : one < two ? TILES_ONE : TILES_TWO;
+}
+
 int launch_tiles_together(const SimtGemmArgs* products, int count, long long m_extent, int groups, cudaStream_t stream) {
+    const int form = tile_form(products, count, m_extent, groups);
     SimtTileArgs args = {};
     long long tiles = 0;
     for (int i = 0; i < kSimtProducts; ++i) {
         if (i < count) {
             args.product[i] = products[i];
-            args.columns[i] = ceil_div(products[i].N, TILE);
+            args.columns[i] = ceil_div(products[i].N, form == TILES_WIDE ? WIDE : TILE);
             tiles += (long long)args.columns[i] * ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE);
         }
         args.end[i] = (int)tiles;
@@ -307,16 +368,11 @@ int launch_tiles_together(const SimtGemmArgs* products, int count, long long m_e
     if (tiles >= (1ll << 31)) return fail_arg("gemm: too many tiles");
     const SimtGemmArgs& g = products[0];
     const dim3 grid((unsigned)tiles, 1, (unsigned)groups);
-    // Ordinary launches, as for the general kernel: in a chain the CTAs are handed out while those of the kernel before leave, two
-    // to some SMs and none to others, which costs kernels that are as long as their slowest SM more than the gap (2048
-    // rows, 512 x 1024, 8 experts, forward and backward: 1038 us, in a chain 1113; 700 rows, 320 x 300, 4 experts, on the general kernel: 346 and 445).
     const bool a_kfast = g.a_cs == 1, b_kfast = g.b_rs == 1;
-    if (a_kfast && b_kfast) simt_tile_kernel<true, true, false><<<grid, 256, 0, stream>>>(args);
-    else if (a_kfast) simt_tile_kernel<true, false, false><<<grid, 256, 0, stream>>>(args);
-    else if (b_kfast) simt_tile_kernel<false, true, false><<<grid, 256, 0, stream>>>(args);
-    else simt_tile_kernel<false, false, false><<<grid, 256, 0, stream>>>(args);
-    QMOE_LAUNCH_CHECK("simt_tile_kernel");
-    return 0;
+    if (a_kfast && b_kfast) return launch_tile_form<true, true, false>(form, args, grid, stream);
+    if (a_kfast) return launch_tile_form<true, false, false>(form, args, grid, stream);
+    if (b_kfast) return launch_tile_form<false, true, false>(form, args, grid, stream);
+    return launch_tile_form<false, false, false>(form, args, grid, stream);
 }
 
 constexpr int kMaxGridY = 65535;      // of a launch
@@ -335,11 +391,13 @@ int launch_tiles(const SimtGemmArgs* products, int count, long long m_extent, in
     for (int i = 0; i < count; ++i) alone = alone && ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE) <= kMaxGridY;
     if (!alone) return launch_tiles_together(products, count, m_extent, groups, stream);
     for (int i = 0; i < count; ++i) {
-        const dim3 grid(ceil_div(products[i].N, TILE), ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE), groups);
-        if (a_kfast) simt_tile_kernel<true, true, true><<<grid, 256, 0, stream>>>(products[i]);
-        else if (b_kfast) simt_tile_kernel<false, true, true><<<grid, 256, 0, stream>>>(products[i]);
-        else simt_tile_kernel<false, false, true><<<grid, 256, 0, stream>>>(products[i]);
-        QMOE_LAUNCH_CHECK("simt_tile_kernel");
+        const int form = tile_form(products + i, 1, m_extent, groups);
+        const dim3 grid(ceil_div(products[i].N, form == TILES_WIDE ? WIDE : TILE), ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE), groups);
+        int rc;
+        if (a_kfast) rc = launch_tile_form<true, true, true>(form, products[i], grid, stream);
+        else if (b_kfast) rc = launch_tile_form<false, true, true>(form, products[i], grid, stream);
+        else rc = launch_tile_form<false, false, true>(form, products[i], grid, stream);
+        if (rc) return rc;
     }
     return 0;
 }

@@ -36,6 +36,7 @@ SimtGemmArgs simt_rows_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint6
     g.ldc = N; g.mode = SG_ROWS;
     g.tile_expert = (const int*)r->tile_expert; g.meta = (const int*)r->meta;
     g.b_slab = K * N;
+    g.expected_rows = r->tokens * r->top_k + (long long)r->experts * (kRowPad / 2);
     return g;
 }
 int simt_rows(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c,
