@@ -1,5 +1,7 @@
 // Expert FFN forward/backward (engine selection between the tcgen05 kernels and the CUDA-core
 // kernels), the single-group GEMM of the host function table, and the whole-layer entry points.
+#include <math.h>
+
 #include "common.cuh"
 
 namespace qmoe {
@@ -26,6 +28,17 @@ int check_experts(const qmoe_route_t* r, const qmoe_experts_t* ex, int* engine) 
     return 0;
 }
 
+// How many 128-row tiles the experts' rows take: under uniform load (every expert's rows near the mean, normally distributed about it), and with
+// last tiles that are half full on average, as a skewed load leaves them
+void dispatched_tiles(const qmoe_route_t* r, long long tiles[2]) {
+    const double rows = (double)r->tokens * r->top_k, mean = rows / r->experts;
+    double per_expert = 0;
+    for (double from = 0.5; from < mean + 6 * sqrt(mean) + 1; from += kRowPad) per_expert += 0.5 * erfc((from - mean) / sqrt(2 * mean));
+    tiles[0] = (long long)(per_expert * r->experts + 0.5);
+    tiles[1] = (long long)(rows / kRowPad + 0.5 * r->experts + 0.5);
+    for (int i = 0; i < 2; ++i)
+        if (tiles[i] < 1) tiles[i] = 1;
+}
 // C[rows, N] = A[rows, K] . op(B_e) on CUDA cores; b_kfast: B_e is [N, K] ("x W^T"), else [K, N]
 SimtGemmArgs simt_rows_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c, long long K, long long N, bool b_kfast) {
     SimtGemmArgs g = {};
@@ -36,7 +49,7 @@ SimtGemmArgs simt_rows_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint6
     g.ldc = N; g.mode = SG_ROWS;
     g.tile_expert = (const int*)r->tile_expert; g.meta = (const int*)r->meta;
     g.b_slab = K * N;
-    g.expected_rows = r->tokens * r->top_k + (long long)r->experts * (kRowPad / 2);
+    dispatched_tiles(r, g.row_tiles);
     return g;
 }
 int simt_rows(const qmoe_route_t* r, const qmoe_experts_t* ex, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, uint64_t c,
@@ -52,6 +65,7 @@ SimtGemmArgs simt_wgrad_args(const qmoe_route_t* r, uint64_t a, uint64_t b, uint
     g.a_rs = 1; g.a_cs = M;
     g.b_rs = N; g.b_cs = 1;
     g.ldc = N; g.mode = SG_K;
+    g.mean_rows = r->tokens * r->top_k / r->experts;
     g.offsets = (const int*)r->offsets; g.counts = (const int*)r->counts;
     g.c_slab = M * N;
     return g;
