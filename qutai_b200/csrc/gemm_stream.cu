@@ -5,7 +5,7 @@
 // The kernel for many rows (gemm_tcgen05.cu) gives every expert tiles of 256 rows: an expert with six rows still costs
 // the tensor time of 256 and stages 128 rows of activations beside every 128 rows of weights.  Here both follow the
 // expert's own row count, and what bounds a product is HBM: 96 KiB of weight tiles in flight per SM (STREAM_NT), 128 KiB in
-// the other two.  64 rows over 64 experts, top 6, 2048 x 1408: SwiGLU 144 -> 113 us (738 MB: 6.5 TB/s), down product 72 -> 60.
+// the other two, more for few tokens (few_tokens).  64 rows over 64 experts, top 6, 2048 x 1408: SwiGLU 144 -> 113 us (738 MB: 6.5 TB/s), down product 72 -> 60.
 //
 // One persistent CTA per SM, 6 warps: warp 0 asks TMA for the tiles, warp 1 issues the MMAs, warps 2-5 convert the
 // accumulators (lane = output column, TMEM column = row of the expert) and store them; two accumulator sets, so a

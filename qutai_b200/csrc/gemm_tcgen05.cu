@@ -9,8 +9,8 @@
 //               tiles (4 stages of 48 KiB, or 6 stages of 32 KiB per CTA of a pair; two fewer in dSwiGLU, whose
 //               epilogue stages its own operands in shared memory)
 //   warp 1      MMA issuer (one lane, in a pair only the first CTA's): 4 x tcgen05.mma (K = 16 each) per
-//               stage, commits free the stage in both CTAs; also allocates / frees the 512 TMEM columns
-//               (two 128x256 fp32 accumulators per CTA)
+//               stage, commits free the stage in both CTAs; also allocates / frees the TMEM columns
+//               (two 128x256 fp32 accumulators per CTA: all 512; two 128x64: 128)
 //   warps 2-9   epilogue: two warps per 32-lane TMEM quadrant (= 32 tile rows), each taking half of
 //               the columns; they convert and store to HBM while the MMA warp already works on the
 //               next tile in the other accumulator
