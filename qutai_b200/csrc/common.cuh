@@ -273,7 +273,7 @@ struct SimtGemmArgs {
     long long b_slab;        // SG_ROWS: elements of B per expert
     long long c_slab;        // SG_K / SG_SPLITK: elements of C per expert / per split
     long long k_chunk;       // SG_SPLITK: K handled by one split
-    long long row_tiles[2];  // SG_ROWS: 128-row tiles in use, two guesses for the choice of a kernel (0: ceil(M / 128))
+    long long row_tiles[3];  // SG_ROWS: 128-row tiles in use, guesses for the choice of a kernel (0: ceil(M / 128))
     long long mean_rows;     // SG_K: rows of an expert, on average
 };
 // dtype codes QMOE_F32 / QMOE_BF16 for A, B, C; m_extent = rows the grid must cover

@@ -336,7 +336,7 @@ int launch_tile_form(int form, const TileArgs<ALONE>& args, dim3 grid, cudaStrea
 
 // Which form: two to an SM, unless another is through first, by the rounds it takes and what a round costs, in units of 128 x 128 tiles at the full rate of an SM's
 // FMA units (they reach two thirds of it in every form): 3.05 for two tiles on an SM (1.8 where the last round leaves one), 1.64 for
-// one alone, 2.5 for a wide one.  us as two to an SM, one and wide: g W 4096 x 1024 x 1024 200, 208 and 189; 1024 x 4096 x 2048 427, 405 and 728; 640 x 640 x
+// one alone, 2.92 for a wide one.  us as two to an SM, one and wide: g W 4096 x 1024 x 1024 200, 208 and 189; 1024 x 4096 x 2048 427, 405 and 728; 640 x 640 x
 // 2560 72, 68 and 120; weight gradients of 1024 rows, 4096 x 1024 194, 205 and 185; of 1500, 2048 x 776, 163, 155 and 271.  x W^T does not spill, and two to an
 // SM serve it best or nearly (4096 x 1024 x 1024 193, 209 and 191; 1024 x 4096 x 2048 409, 411 and 741).  The same bits in every form.  With a short
 // inner size the results' way to memory is the work, which more and smaller tiles do better (weight gradients of 5 rows per expert, 64 x 3 x 1600 x 320, in a
@@ -347,8 +347,8 @@ int tile_form(const SimtGemmArgs* products, int count, long long m_extent, int g
     if (products[0].a_cs == 1 && products[0].b_rs == 1) return TILES_TWO;
     if ((products[0].mode == SG_K ? products[0].mean_rows : products[0].K) < kFormDepth) return TILES_TWO;
     const long long sms = sm_count();
-    bool one_better = true, wide_better = true, wide_over_one = true;      // by both guesses of the rows
-    for (int guess = 0; guess < 2; ++guess) {
+    bool one_better = true, wide_better = true, wide_over_one = true;      // by every guess of the rows
+    for (int guess = 0; guess < 3; ++guess) {
         long long narrow = 0, wide = 0;
         for (int i = 0; i < count; ++i) {
             const long long rows = products[i].row_tiles[guess] ? products[i].row_tiles[guess] : ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE);
@@ -356,7 +356,7 @@ int tile_form(const SimtGemmArgs* products, int count, long long m_extent, int g
             wide += rows * ceil_div(products[i].N, WIDE) * groups;
         }
         const long long left = narrow % (2 * sms);
-        const double two = 3.05 * (double)(narrow / (2 * sms)) + (left > sms ? 3.05 : left ? 1.8 : 0.0), one = 1.64 * ceil_div(narrow, sms), as_wide = 2.5 * ceil_div(wide, sms);
+        const double two = 3.05 * (double)(narrow / (2 * sms)) + (left > sms ? 3.05 : left ? 1.8 : 0.0), one = 1.64 * ceil_div(narrow, sms), as_wide = 2.92 * ceil_div(wide, sms);
         one_better = one_better && one < two;
         wide_better = wide_better && as_wide < two;
         wide_over_one = wide_over_one && as_wide < one;

@@ -29,14 +29,15 @@ int check_experts(const qmoe_route_t* r, const qmoe_experts_t* ex, int* engine) 
 }
 
 // How many 128-row tiles the experts' rows take: under uniform load (every expert's rows near the mean, normally distributed about it), and with
-// last tiles that are half full on average, as a skewed load leaves them
-void dispatched_tiles(const qmoe_route_t* r, long long tiles[2]) {
+// last tiles that are half full on average, as a skewed load leaves them, and as many as that by one standard deviation
+void dispatched_tiles(const qmoe_route_t* r, long long tiles[3]) {
     const double rows = (double)r->tokens * r->top_k, mean = rows / r->experts;
     double per_expert = 0;
     for (double from = 0.5; from < mean + 6 * sqrt(mean) + 1; from += kRowPad) per_expert += 0.5 * erfc((from - mean) / sqrt(2 * mean));
     tiles[0] = (long long)(per_expert * r->experts + 0.5);
     tiles[1] = (long long)(rows / kRowPad + 0.5 * r->experts + 0.5);
-    for (int i = 0; i < 2; ++i)
+    tiles[2] = (long long)(rows / kRowPad + 0.5 * r->experts + 0.5 * sqrt((double)r->experts));
+    for (int i = 0; i < 3; ++i)
         if (tiles[i] < 1) tiles[i] = 1;
 }
 // C[rows, N] = A[rows, K] . op(B_e) on CUDA cores; b_kfast: B_e is [N, K] ("x W^T"), else [K, N]
