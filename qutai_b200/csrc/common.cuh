@@ -57,7 +57,8 @@ struct TimedScope {  // records a pair of events around the launches made while 
 // else be able to take the columns first and wait, holding them, for this one.  Without chain_next a kernel lets the next one
 // start as its CTAs leave: so do the backward of the combine, the permutation unless a product for few rows follows (permute.cu), and those products unless
 // the down product follows for few tokens (gemm_stream.cu).  The CUDA-core products are launched in the ordinary way (see there).
-// One kernel reads before its wait: a product for few rows fetches tables and weights that nothing within the last launch wrote (gemm_stream.cu).
+// One kernel reads before its wait: a product for few rows fetches tables (load_l2) and weights (TMA, which reads the L2) that nothing within the
+// last launch wrote (gemm_stream.cu).
 // 3001 rows, 16 experts, forward and backward (27 launches): 472 us in ordinary launches, 440 like this; 64 rows over 64 experts, replayed, L2
 // flushed: 220 and 215.
 // The wait is a volatile statement that clobbers memory, and griddepcontrol.wait is what orders the kernel's loads behind the writes of the
@@ -66,6 +67,13 @@ struct TimedScope {  // records a pair of events around the launches made while 
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() { chain_wait(); chain_next(); }
+// A value that a completed kernel wrote, for a grid that has not waited itself: what a wait makes visible is promised to the grid that waited, and
+// an ordinary load may meet a line that the SM kept from an earlier kernel.  The L2 has the write.
+__device__ __forceinline__ int load_l2(const int* p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 inline cudaLaunchAttribute chain_attribute() {
     cudaLaunchAttribute attribute = {};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -121,9 +121,9 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     // The tables in one round trip to L2: a thread per expert loads, a warp sums up (every thread adding up the counts before its
     // expert is a chain of L2 latencies: 64 rows over 64 experts, replayed, L2 flushed before every call, 217 us and 215 like this).
     for (int e = threadIdx.x; e < p.experts; e += STREAM_THREADS) {
-        const int count = p.counts[e];
+        const int count = load_l2(p.counts + e);
         s_rows[e] = count;
-        s_row0[e] = p.offsets[e];
+        s_row0[e] = load_l2(p.offsets + e);
         s_first[e + 1] = (count + kRowPad - 1) / kRowPad * p.m_tiles;
     }
     __syncthreads();

@@ -86,3 +86,14 @@ def test_no_load_is_declared_free_of_order():
             text = re.sub(r"//[^\n]*", "", file.read())
         assert "__ldg" not in text, name
         assert re.findall(r'asm\s*\(\s*"ld\.', text) == [], name      # loads in inline PTX are volatile: they keep their place behind the wait
+
+
+def test_what_is_read_ahead_of_a_wait_comes_from_the_l2():
+    """A kernel that may read before it waits: what griddepcontrol.wait makes visible is promised to the grid that waited, and a line that
+    an SM kept from an earlier kernel is none of it.  Such reads name the L2, where the writes of a completed kernel are."""
+    found, _ = kernels()
+    early = [(name, body[:body.rfind("chain_wait();")]) for name, body in found if re.search(r"if \([^;{}]*\)\s*chain_wait\(\);", body)]
+    assert [name for name, _ in early] == ["stream_gemm_kernel"]
+    for name, before in early:
+        assert "load_l2(p.counts + " in before and "load_l2(p.offsets + " in before, name
+        assert re.findall(r"\bp\.\w+\[", before) == [], name
