@@ -34,7 +34,7 @@ enum { STATUS_STREAM_PRODUCER = 111, STATUS_STREAM_MMA = 112, STATUS_STREAM_EPIL
 // FEW: at most X_BOX rows per expert, one box of activations per stage, and the room for more stages
 template <int MODE, bool FEW> struct StreamCfg {
     static constexpr int W_TILES = MODE == STREAM_NT ? 1 : 2;
-    static constexpr int MOST_ROWS = FEW ? X_BOX : kRowPad;                       // of an expert in a tile
+    static constexpr int MOST_ROWS = FEW ? X_BOX : kRowPad;                       // of an expert in a tile; more rows are more tiles
     static constexpr int STAGE_BYTES = W_TILES * W_BYTES + (FEW ? X_BOX_BYTES : X_BYTES);
     static constexpr int STAGES = MODE == STREAM_NT ? (FEW ? 11 : 6) : FEW ? 6 : 4;
     static constexpr int COLUMNS = MODE == STREAM_NT2 ? 2 * SM_ROWS : SM_ROWS;    // output columns of a tile
@@ -56,9 +56,10 @@ struct alignas(64) StreamParams {
     int pad_rows;                  // zero every pad row; else those from `columns` on are left as they are
 };
 
-struct StreamTile { int expert, n0, row0, columns; };   // `columns`: rows of the expert in this tile, rounded up to 16
+// `columns`: rows of the expert in this tile, rounded up to 16; `end`: with the pad rows that are this tile's to fill
+struct StreamTile { int expert, n0, row0, columns, end; };
 
-// tiles of expert e: m_tiles weight tiles x its 128-row chunks, the chunks of one weight tile side by side (the second
+// tiles of expert e: m_tiles weight tiles x its chunks of most_rows rows, the chunks of one weight tile side by side (the second
 // finds the weights in L2)
 // (first, row0, rows: each expert's first tile, first dispatched row and rows, in shared memory; most_rows: what a stage has room for)
 __device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const int* first, const int* row0, const int* rows, int t, int columns, int most_rows) {
@@ -71,9 +72,10 @@ __device__ __forceinline__ StreamTile stream_tile(const StreamParams& p, const i
     StreamTile tile;
     tile.expert = lo;
     tile.n0 = local / chunks * columns;
-    tile.row0 = row0[lo] + chunk * kRowPad;
-    const int left = rows[lo] - chunk * kRowPad;
+    tile.row0 = row0[lo] + chunk * most_rows;
+    const int left = rows[lo] - chunk * most_rows;
     tile.columns = left >= most_rows ? most_rows : (left + kStreamPad - 1) / kStreamPad * kStreamPad;
+    tile.end = left > most_rows ? most_rows : kRowPad - chunk * most_rows % kRowPad;      // the last chunk fills up to the next 128
     return tile;
 }
 
@@ -124,7 +126,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
         const int count = load_l2(p.counts + e);
         s_rows[e] = count;
         s_row0[e] = load_l2(p.offsets + e);
-        s_first[e + 1] = (count + kRowPad - 1) / kRowPad * p.m_tiles;
+        s_first[e + 1] = (count + Config::MOST_ROWS - 1) / Config::MOST_ROWS * p.m_tiles;
     }
     __syncthreads();
     if (warp == 0) {
@@ -274,7 +276,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
             if (lane == 0) mbar_arrive(tempty_bar(a));
             if (p.pad_rows && n < p.N) {
                 const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
-                for (int c = tile.columns; c < kRowPad; ++c) {
+                for (int c = tile.columns; c < tile.end; ++c) {
                     const long long to = at + (long long)c * p.N;
                     p.out0[to] = zero;
                     if (MODE == STREAM_SWIGLU) { p.out1[to] = zero; p.out2[to] = zero; }
@@ -314,8 +316,8 @@ int stream_launch(const StreamParams& p, cudaStream_t stream) {
     return 0;
 }
 
-// The form with more stages: up to X_BOX tokens (a token goes to an expert once, so no expert has more rows than there are tokens), and with the
-// experts that uniform load reaches on average at most two tiles per SM.  There a tile's time is what one SM has on its way; with more tiles
+// The form with more stages: up to X_BOX tokens (a routing sends a token to an expert once, so that no expert has more rows; tables that a caller
+// filled may, which takes tiles of X_BOX rows each), and with the experts that uniform load reaches on average at most two tiles per SM.  There a tile's time is what one SM has on its way; with more tiles
 // HBM is the limit, and the more is asked for at once the less it gives.  us a call, 128 KiB of weights in flight per SM and 192: 8 experts,
 // 1024 x 2816, 4 rows 40.9 and 40.6, 32 rows 52.2 and 51.4, 1 row of 4096 x 2816 67.9 and 62.8, 64 experts, 2048 x 1408, 1 row 46.9 and 45.1, but
 // 16 rows 169.9 and 172.8, 32 rows 196.6 and 203.2.
