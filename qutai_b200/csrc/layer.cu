@@ -32,8 +32,10 @@ int check_experts(const qmoe_route_t* r, const qmoe_experts_t* ex, int* engine) 
 // last tiles that are half full on average, as a skewed load leaves them, and as many as that by one standard deviation
 void dispatched_tiles(const qmoe_route_t* r, long long tiles[3]) {
     const double rows = (double)r->tokens * r->top_k, mean = rows / r->experts;
-    double per_expert = 0;
-    for (double from = 0.5; from < mean + 6 * sqrt(mean) + 1; from += kRowPad) per_expert += 0.5 * erfc((from - mean) / sqrt(2 * mean));
+    // an expert has a tile's first row for certain (to 1e-9) below six standard deviations under the mean: what is left to add up grows with their number only
+    const double reach = 6 * sqrt(mean) + 1, certain = mean > reach ? floor((mean - reach) / kRowPad) : 0;
+    double per_expert = certain;
+    for (double from = certain * kRowPad + 0.5; from < mean + reach; from += kRowPad) per_expert += 0.5 * erfc((from - mean) / sqrt(2 * mean));
     tiles[0] = (long long)(per_expert * r->experts + 0.5);
     tiles[1] = (long long)(rows / kRowPad + 0.5 * r->experts + 0.5);
     tiles[2] = (long long)(rows / kRowPad + 0.5 * r->experts + 0.5 * sqrt((double)r->experts));
