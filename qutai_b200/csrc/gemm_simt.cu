@@ -341,8 +341,13 @@ int launch_tile_form(int form, const TileArgs<ALONE>& args, dim3 grid, cudaStrea
 // SM serve it best or nearly (4096 x 1024 x 1024 193, 209 and 191; 1024 x 4096 x 2048 409, 411 and 741).  The same bits in every form.  With a short
 // inner size the results' way to memory is the work, which more and smaller tiles do better (weight gradients of 5 rows per expert, 64 x 3 x 1600 x 320, in a
 // call of 1672 us: 1806 wide).  Forward and
-// backward, 2048 rows, 8 experts, 512 x 1024, all as two to an SM and by this rule: 1016 and 988 us (dX 225 and 203, a tile for each SM).
+// backward, 2048 rows, 8 experts, 512 x 1024, all as two to an SM and by this rule: 1021 and 998 us (dX 225 and 203, a tile for each SM).
+// The rounds are an estimate: two CTAs to an SM follow one another freely, and which experts' tiles there are is a guess.  So another form has to be
+// 6 % cheaper by it, except for a plain product that two to an SM do in one round, whose rounds are certain.  330 layers of 64 .. 4096 rows, 4 .. 64 experts,
+// forward and backward, against all as two to an SM: without the 6 % 0.99 on average but up to 1.09 (4096 rows, 1984 x 448, 16 experts, top 1:
+// 1851 us and 2020), like this 0.993 and at most 1.006; 468 plain products 0.97 on average, at most 1.008 (without it 1.022).
 constexpr long long kFormDepth = 128;
+constexpr double kFormMargin = 1.06;
 int tile_form(const SimtGemmArgs* products, int count, long long m_extent, int groups) {
     if (products[0].a_cs == 1 && products[0].b_rs == 1) return TILES_TWO;
     if ((products[0].mode == SG_K ? products[0].mean_rows : products[0].K) < kFormDepth) return TILES_TWO;
@@ -357,8 +362,9 @@ int tile_form(const SimtGemmArgs* products, int count, long long m_extent, int g
         }
         const long long left = narrow % (2 * sms);
         const double two = 3.05 * (double)(narrow / (2 * sms)) + (left > sms ? 3.05 : left ? 1.8 : 0.0), one = 1.64 * ceil_div(narrow, sms), as_wide = 2.92 * ceil_div(wide, sms);
-        one_better = one_better && one < two;
-        wide_better = wide_better && as_wide < two;
+        const double margin = products[0].mode == SG_PLAIN && narrow <= 2 * sms ? 1.0 : kFormMargin;
+        one_better = one_better && one * margin < two;
+        wide_better = wide_better && as_wide * margin < two;
         wide_over_one = wide_over_one && as_wide < one;
     }
     return wide_better && (wide_over_one || !one_better) ? TILES_WIDE : one_better ? TILES_ONE : TILES_TWO;
