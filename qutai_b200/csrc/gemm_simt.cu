@@ -323,51 +323,49 @@ int launch_tile_kernel(const TileArgs<ALONE>& args, dim3 grid, cudaStream_t stre
     QMOE_LAUNCH_CHECK("simt_tile_kernel");
     return 0;
 }
-// The forms of the kernel: tiles of 128 x 128, two to an SM (at 128 registers, which spills a little in some); one to an SM; tiles of 128 x 256.
+// The forms of the kernel: tiles of 128 x 128, two to an SM (at 128 registers, which spills a little in some); one to an SM; tiles of 128 x 256
+// (for a product by itself, see tile_form: A transposed comes by itself without the index, A as it is with it).
 enum { TILES_TWO, TILES_ONE, TILES_WIDE };
 template <bool A_KFAST, bool B_KFAST, bool ALONE>
 int launch_tile_form(int form, const TileArgs<ALONE>& args, dim3 grid, cudaStream_t stream) {
     if constexpr (!(A_KFAST && B_KFAST)) {
-        if (form == TILES_WIDE) return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, WIDE, 1>(args, grid, stream);
+        if constexpr (A_KFAST != ALONE)
+            if (form == TILES_WIDE) return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, WIDE, 1>(args, grid, stream);
         if (form == TILES_ONE) return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, TILE, 1>(args, grid, stream);
     }
     return launch_tile_kernel<A_KFAST, B_KFAST, ALONE, TILE, 2>(args, grid, stream);
 }
 
-// Which form: two to an SM, unless another is through first, by the rounds it takes and what a round costs, in units of 128 x 128 tiles at the full rate of an SM's
-// FMA units (they reach two thirds of it in every form): 3.05 for two tiles on an SM (1.8 where the last round leaves one), 1.64 for
-// one alone, 2.92 for a wide one.  us as two to an SM, one and wide: g W 4096 x 1024 x 1024 200, 208 and 189; 1024 x 4096 x 2048 427, 405 and 728; 640 x 640 x
-// 2560 72, 68 and 120; weight gradients of 1024 rows, 4096 x 1024 194, 205 and 185; of 1500, 2048 x 776, 163, 155 and 271.  x W^T does not spill, and two to an
+// Which form: two to an SM, except where the tiles of another are a single round.  An SM takes 3.05 units (128 x 128 tiles at the full rate of its
+// FMA units, of which every form reaches two thirds) for two tiles, 1.8 for the one of two that a last round leaves it, 1.64 for one
+// alone, 2.92 for a wide one: up to a tile for every SM one alone is through first, and up to two a wide one, if the wide ones are no more than SMs.  In more
+// rounds the 4 % of the wide ones is less than what two CTAs gain that follow one another freely, or than a guess of the experts' tiles is
+// off, so wide tiles are for plain products alone.  us as two to an SM, one and wide: g W 4096 x 1024 x 1024 200, 208 and 189; 1024 x 4096 x 2048 427, 405
+// and 728; 640 x 640 x 2560 72, 68 and 120; weight gradients of 1024 rows, 4096 x 1024 194, 205 and 185; of 1500, 2048 x 776, 163, 155 and 271; A
+// transposed, 6684 x 140 x 4020 169, and 172 wide.  x W^T does not spill, and two to an
 // SM serve it best or nearly (4096 x 1024 x 1024 193, 209 and 191; 1024 x 4096 x 2048 409, 411 and 741).  The same bits in every form.  With a short
 // inner size the results' way to memory is the work, which more and smaller tiles do better (weight gradients of 5 rows per expert, 64 x 3 x 1600 x 320, in a
-// call of 1672 us: 1806 wide).  Forward and
-// backward, 2048 rows, 8 experts, 512 x 1024, all as two to an SM and by this rule: 1021 and 998 us (dX 225 and 203, a tile for each SM).
-// The rounds are an estimate: two CTAs to an SM follow one another freely, and which experts' tiles there are is a guess.  So another form has to be
-// 6 % cheaper by it, except for a plain product that two to an SM do in one round, whose rounds are certain.  330 layers of 64 .. 4096 rows, 4 .. 64 experts,
-// forward and backward, against all as two to an SM: without the 6 % 0.99 on average but up to 1.09 (4096 rows, 1984 x 448, 16 experts, top 1:
-// 1851 us and 2020), like this 0.993 and at most 1.006; 468 plain products 0.97 on average, at most 1.008 (without it 1.022).
+// call of 1672 us: 1806 wide).
+// Against all as two to an SM: 468 plain products 0.97 on average, at most 1.008; 330 layers of 64 .. 4096 rows, 4 .. 64 experts, forward and
+// backward, 0.993 and at most 1.006 (with wide tiles in every number of rounds 0.991, but up to 1.09: 4096 rows, 1984 x 448, 16 experts, top 1, 1851 us and
+// 2020).  2048 rows, 512 x 1024, 8 experts: 1021 and 998 us (dX 225 and 203, a tile for each SM).
 constexpr long long kFormDepth = 128;
-constexpr double kFormMargin = 1.06;
 int tile_form(const SimtGemmArgs* products, int count, long long m_extent, int groups) {
     if (products[0].a_cs == 1 && products[0].b_rs == 1) return TILES_TWO;
     if ((products[0].mode == SG_K ? products[0].mean_rows : products[0].K) < kFormDepth) return TILES_TWO;
     const long long sms = sm_count();
-    bool one_better = true, wide_better = true, wide_over_one = true;      // by every guess of the rows
+    long long narrow = 0, wide = 0;      // by the largest guess of the rows
     for (int guess = 0; guess < 3; ++guess) {
-        long long narrow = 0, wide = 0;
+        long long tiles = 0, tiles_wide = 0;
         for (int i = 0; i < count; ++i) {
             const long long rows = products[i].row_tiles[guess] ? products[i].row_tiles[guess] : ceil_div(m_extent > 0 ? m_extent : products[i].M, TILE);
-            narrow += rows * ceil_div(products[i].N, TILE) * groups;
-            wide += rows * ceil_div(products[i].N, WIDE) * groups;
+            tiles += rows * ceil_div(products[i].N, TILE) * groups;
+            tiles_wide += rows * ceil_div(products[i].N, WIDE) * groups;
         }
-        const long long left = narrow % (2 * sms);
-        const double two = 3.05 * (double)(narrow / (2 * sms)) + (left > sms ? 3.05 : left ? 1.8 : 0.0), one = 1.64 * ceil_div(narrow, sms), as_wide = 2.92 * ceil_div(wide, sms);
-        const double margin = products[0].mode == SG_PLAIN && narrow <= 2 * sms ? 1.0 : kFormMargin;
-        one_better = one_better && one * margin < two;
-        wide_better = wide_better && as_wide * margin < two;
-        wide_over_one = wide_over_one && as_wide < one;
+        if (tiles > narrow) { narrow = tiles; wide = tiles_wide; }
     }
-    return wide_better && (wide_over_one || !one_better) ? TILES_WIDE : one_better ? TILES_ONE : TILES_TWO;
+    if (narrow <= sms) return TILES_ONE;
+    return products[0].mode == SG_PLAIN && count == 1 && narrow <= 2 * sms && wide <= sms ? TILES_WIDE : TILES_TWO;
 }
 
 int launch_tiles_together(const SimtGemmArgs* products, int count, long long m_extent, int groups, cudaStream_t stream) {
