@@ -1,12 +1,12 @@
-"""Which form of the float32 tile kernel a product takes (``tile_form`` in csrc/gemm_simt.cu), for products of which both sides were measured.
-No GPU: compiles the file and calls the function."""
+"""Which form of the float32 tile kernel a product takes (``tile_form`` in csrc/gemm_simt.cu): the rule that the GPU test of the forms restates,
+and products of which both sides were measured.  No GPU: compiles the file and calls the function."""
+import random
 import subprocess
 
 import pytest
 
 from qutai_b200 import build
-
-SMS, (TWO, ONE, WIDE), (ROWS, SPLIT_ROWS) = 148, range(3), (1, 2)
+from test_gpu_float32_tile_forms import ONE, ROWS, SMS, SPLIT_ROWS, TWO, WIDE, tile_form
 
 PROGRAM = """
 #include <stdio.h>
@@ -70,3 +70,21 @@ def test_products_that_were_measured_in_every_form(forms):
         ([(5120, 1024, 512)], dict(mode=ROWS, row_tiles=(36, 36, 37)), ONE),             # dX of 2048 x 512 x 1024, 2 of 8: 225, one 203
     ]
     assert forms([(shapes, kwargs) for shapes, kwargs, _ in questions]) == [want for _, _, want in questions]
+
+
+def test_the_rule_restated_for_the_gpu_test_is_the_rule(forms):
+    rng = random.Random(3)
+    questions = []
+    for _ in range(3000):
+        mode, count = rng.choice((0, ROWS, SPLIT_ROWS)), rng.choice((1, 1, 2, 3))
+        m = rng.randint(1, 9000)
+        shapes = [(m if mode == ROWS else rng.randint(1, 9000), rng.randint(16, 1000), rng.randint(65, 5000)) for _ in range(count if mode else 1)]
+        kwargs = dict(mode=mode, a_kfast=rng.random() < 0.5, b_kfast=rng.random() < 0.5)
+        if mode == ROWS:
+            kwargs["row_tiles"] = tuple(rng.randint(1, 80) for _ in range(3)) if rng.random() < 0.5 else (rng.randint(1, 80),) * 3
+        if mode == SPLIT_ROWS:
+            kwargs.update(groups=rng.randint(1, 64), mean_rows=rng.choice((16, 127, 128, 500)))
+        questions.append((shapes, kwargs))
+    got = forms(questions)
+    assert {form: got.count(form) > 50 for form in (TWO, ONE, WIDE)} == {TWO: True, ONE: True, WIDE: True}
+    assert got == [tile_form(shapes, **kwargs) for shapes, kwargs in questions]
