@@ -7,7 +7,7 @@
 // expert's own row count, and what bounds a product is HBM: 96 KiB of weight tiles in flight per SM (STREAM_NT), 128 KiB in
 // the other two, more for few tokens (few_tokens).  64 rows over 64 experts, top 6, 2048 x 1408: SwiGLU 144 -> 113 us (738 MB: 6.5 TB/s), down product 72 -> 60.
 //
-// One persistent CTA per SM, 6 warps: warp 0 asks TMA for the tiles, warp 1 issues the MMAs, warps 2-5 convert the
+// One persistent CTA per SM, or per tile where those are fewer, 6 warps: warp 0 asks TMA for the tiles, warp 1 issues the MMAs, warps 2-5 convert the
 // accumulators (lane = output column, TMEM column = row of the expert) and store them; two accumulator sets, so a
 // tile's epilogue runs beside the next tile's main loop.
 //   STREAM_SWIGLU   G, U, H from X: a stage holds 64 columns of a gate tile and of the up tile beside it
@@ -116,9 +116,11 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
     // `early`: the kernel before is this call's own (the permutation, or the product that forms H), writes neither tables nor weights and lets
     // this one start behind its own wait, so whatever wrote those lies at least two launches back and is complete.  The tables and the first
     // stages' weights are then fetched beside the kernel before; what that one writes (the activations), and whatever this one writes, waits.
-    // us a call without it and with it: 4 rows, 8 experts, 1024 x 2816, 45.9 and 43.4 (46.0 of 47.2 with the up product alone), 16 rows, 4 experts,
-    // 512 x 264, 24.1 and 21.2.  64 rows over 64 experts, replayed on one stream 200 and 195, but on several at a time 158.6 and 160.6: CTAs that
-    // wait for the tail of the up product keep other streams' kernels from those SMs.  So the down product starts early for few tokens alone.
+    // us a replay with neither product early, the up product, and both, on one stream, then of two at a time, then of four: 4 rows, 8 experts,
+    // 1024 x 2816, 38.4 35.8 33.0, 45.7 45.3 46.1, 70.1 67.5 67.5; 16 rows, 4 experts, 512 x 264, 24.7 24.7 20.6, 24.7 24.7 22.6, 27.9 26.6 24.4; 1 row,
+    // 32 experts, 2048 x 1408, 45.0 41.9 41.1, 55.3 54.2 59.2, 86.4 84.2 84.3.  CTAs that wait for the tail of the up product keep other streams'
+    // kernels from their SMs, which two streams of short tails feel most; 64 rows over 64 experts, on several streams 158.6 without the down product and
+    // 160.6 with it.  So the down product starts early for few tokens alone.
     if (!p.early) chain_wait();
     // The tables in one round trip to L2: a thread per expert loads, a warp sums up (every thread adding up the counts before its
     // expert is a chain of L2 latencies: 64 rows over 64 experts, replayed, L2 flushed before every call, 217 us and 215 like this).
@@ -299,7 +301,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams p) {
 }
 
 template <int MODE, bool FEW = false>
-int stream_launch(const StreamParams& p, cudaStream_t stream) {
+int stream_launch(const StreamParams& p, const qmoe_route_t* r, cudaStream_t stream) {
     static bool configured[64] = {};      // per device, like the kernels of gemm_tcgen05.cu
     constexpr int SMEM_BYTES = StreamCfg<MODE, FEW>::SMEM_BYTES;
     static_assert(SMEM_BYTES + 3 * 4 * (kMaxExperts + 1) + 16 <= 227 * 1024, "the stages and the tables exceed the shared memory of a block");
@@ -310,7 +312,11 @@ int stream_launch(const StreamParams& p, cudaStream_t stream) {
         QMOE_CUDA(cudaFuncSetAttribute(stream_gemm_kernel<MODE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         configured[dev] = true;
     }
-    chained(stream_gemm_kernel<MODE, FEW>, sm_count(), STREAM_THREADS, SMEM_BYTES, stream, p);
+    // No more CTAs than there can be tiles (a caller's own tables may hold more: a CTA walks them in steps of the grid).  One that finds none would
+    // hold its SM until the kernel before is done: 16 rows, 4 experts, 512 x 264, replayed on four streams 30.6 us with a CTA for every SM and
+    // 24.4 like this, 1 row, 32 experts, 2048 x 1408, 90.1 and 84.3, on one stream even.
+    const long long rows = r->tokens * r->top_k, most = ((rows < p.experts ? rows : p.experts) + rows / StreamCfg<MODE, FEW>::MOST_ROWS) * p.m_tiles;
+    chained(stream_gemm_kernel<MODE, FEW>, most < sm_count() ? (int)most : sm_count(), STREAM_THREADS, SMEM_BYTES, stream, p);
     count_tensor_core_launch();
     QMOE_LAUNCH_CHECK("stream_gemm_kernel");
     return 0;
@@ -361,7 +367,7 @@ int stream_swiglu_forward(const qmoe_route_t* r, const qmoe_experts_t* ex, uint6
     p.out0 = (__nv_bfloat16*)g; p.out1 = (__nv_bfloat16*)u; p.out2 = (__nv_bfloat16*)h;
     p.experts = ex->experts; p.m_tiles = ceil_div((long long)hd, SM_ROWS); p.N = (int)hd; p.K = (int)d;
     p.pad_rows = pad_rows; p.early = early; p.let_next = let_next;
-    return few_tokens(r, ex->experts, p.m_tiles) ? stream_launch<STREAM_SWIGLU, true>(p, stream) : stream_launch<STREAM_SWIGLU>(p, stream);
+    return few_tokens(r, ex->experts, p.m_tiles) ? stream_launch<STREAM_SWIGLU, true>(p, r, stream) : stream_launch<STREAM_SWIGLU>(p, r, stream);
 }
 
 int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, uint64_t c, long long K, long long N, bool pad_rows, bool early,
@@ -378,10 +384,10 @@ int stream_rows_nt(const qmoe_route_t* r, int experts, uint64_t a, uint64_t b, u
     // 2048 -> 1024 columns (64 tiles of 256): 27 with one, 32 with two.
     if (r->tokens * r->top_k > (long long)X_BOX * experts && (long long)ceil_div(N, 2 * SM_ROWS) * experts >= sm_count()) {
         p.m_tiles = ceil_div(N, 2 * SM_ROWS);
-        return stream_launch<STREAM_NT2>(p, stream);
+        return stream_launch<STREAM_NT2>(p, r, stream);
     }
     p.m_tiles = ceil_div(N, SM_ROWS);
-    return few_tokens(r, experts, p.m_tiles) ? stream_launch<STREAM_NT, true>(p, stream) : stream_launch<STREAM_NT>(p, stream);
+    return few_tokens(r, experts, p.m_tiles) ? stream_launch<STREAM_NT, true>(p, r, stream) : stream_launch<STREAM_NT>(p, r, stream);
 }
 
 }  // namespace qmoe
