@@ -7,6 +7,8 @@
 // upstream's does, so every result is the same on every run.
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace qmoe {
@@ -150,42 +152,45 @@ rms_norm_dx_kernel(const TG* __restrict__ gradient, const TX* __restrict__ x, co
     }
 }
 
-// partial[b, c] = sum over the rows of slab b of g[r, c] x[r, c] inverse[r]   (lm_rms_dw, one slab of rows per block)
-template <typename TG, typename TX, bool VEC>
+// partial[b, c] = sum over the rows of slab b of g[r, c] x[r, c] inverse[r]   (lm_rms_dw, one slab of rows per block).  VEC: a thread owns COLS
+// neighbouring columns, and the rows are added in order, FLIGHT of them in flight (launch_dw_partial).
+template <typename TG, typename TX, bool VEC, int COLS, int FLIGHT>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_dw_partial_kernel(const TG* __restrict__ gradient, const TX* __restrict__ x, const float* __restrict__ inverse,
                            float* __restrict__ partial, long long rows, long long width) {
     chain_begin();
     const long long first = (long long)blockIdx.x * kSlabRows;
     const long long last = first + kSlabRows < rows ? first + kSlabRows : rows;
-    // A thread owns four neighbouring columns; the rows are added in order, sixteen (8 of fp32) of them in flight.  A slab is a chain of round
-    // trips to memory: with four rows in flight and eight columns per thread, 602 x 512 13.4 us and 8192 x 1024 19, like this 4.5 and 12.9.
     if (VEC) {
-        constexpr int kFlight = sizeof(TG) + sizeof(TX) == 4 ? 16 : 8;
-        for (long long c = (long long)threadIdx.x * 4; c < width; c += 4ll * kThreads) {
-            float total[4] = {0.f, 0.f, 0.f, 0.f};
-            for (long long r0 = first; r0 < last; r0 += kFlight) {
-                Raw4<TG> g[kFlight];
-                Raw4<TX> v[kFlight];
-                float inv[kFlight];
+        for (long long c = (long long)threadIdx.x * COLS; c < width; c += (long long)COLS * kThreads) {
+            float total[COLS] = {};
+            for (long long r0 = first; r0 < last; r0 += FLIGHT) {
+                std::conditional_t<COLS == 8, Raw8<TG>, Raw4<TG>> g[FLIGHT];
+                std::conditional_t<COLS == 8, Raw8<TX>, Raw4<TX>> v[FLIGHT];
+                float inv[FLIGHT];
 #pragma unroll
-                for (int u = 0; u < kFlight; ++u)
-                    if (r0 + u < last) {
-                        g[u].load(gradient + (r0 + u) * width + c);
-                        v[u].load(x + (r0 + u) * width + c);
-                        inv[u] = inverse[r0 + u];
-                    }
+                for (int u = 0; u < FLIGHT; ++u) {
+                    // past the slab's end: of four rows the last one again, left out of the sum below, so that no load waits for a test (fp32, 16384 x
+                    // 2048, 161 us with one and 154); of more, nothing
+                    const long long r = FLIGHT > 4 || r0 + u < last ? r0 + u : last - 1;
+                    if (FLIGHT > 4 && r >= last) continue;
+                    g[u].load(gradient + r * width + c);
+                    v[u].load(x + r * width + c);
+                    inv[u] = inverse[r];
+                }
 #pragma unroll
-                for (int u = 0; u < kFlight; ++u)
+                for (int u = 0; u < FLIGHT; ++u)
                     if (r0 + u < last) {
-                        float a[4], b[4];
+                        float a[COLS], b[COLS];
                         g[u].unpack(a);
                         v[u].unpack(b);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) total[j] = fmaf(a[j] * b[j], inv[u], total[j]);
+                        for (int j = 0; j < COLS; ++j) total[j] = fmaf(a[j] * b[j], inv[u], total[j]);
                     }
             }
-            *reinterpret_cast<float4*>(partial + (long long)blockIdx.x * width + c) = make_float4(total[0], total[1], total[2], total[3]);
+#pragma unroll
+            for (int j = 0; j < COLS; j += 4)
+                *reinterpret_cast<float4*>(partial + (long long)blockIdx.x * width + c + j) = make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]);
         }
         return;
     }
@@ -397,6 +402,25 @@ extern "C" int qmoe_rms_norm(uint64_t x, int32_t x_dtype, uint64_t weight, uint6
     return 0;
 }
 
+// A slab of 32 rows is a chain of round trips to memory: the fewer slabs there are, the more rows of a slab have to be in flight, and with more slabs
+// than SMs other blocks' loads are, and wide loads and few registers serve better.  Up to a slab for every SM: four columns per thread (twice the
+// threads with work) and sixteen rows (8 of fp32), but eight columns where four take a second walk (width above 1024) or few rows are
+// there to be had.  us for the whole backward with 4 columns x 16 rows, 8 x 8 and 8 x 4, bf16: 602 x 512 8.1, 8.3 and 9.7; 602 x 2048 13.6, 11.5 and 12.9; 4 x
+// 1024 6.2, 5.7 and 5.6; 4096 x 1024 13.4, 13.6 and 15.0; 8192 x 512 17.9, 18.2 and 17.5; 16384 x 1024 47.0, 45.7 and 41.1; 32768 x 2048 170, 158 and 152.  fp32 with
+// 4 x 8 and 8 x 4: 602 x 512 7.9 and 9.6; 8192 x 1024 34.2 and 36.3; 8192 x 2048 74.7 and 71.6.
+template <typename TG, typename TX>
+static void launch_dw_partial(bool vec, const TG* gradient, const TX* x, const float* inverse, float* partial, long long slabs, long long rows, long long width,
+                       cudaStream_t stream) {
+#define DW_PARTIAL(VEC, COLS, FLIGHT) chained(rms_norm_dw_partial_kernel<TG, TX, VEC, COLS, FLIGHT>, (unsigned)slabs, kThreads, 0, stream, gradient, x, inverse, partial, rows, width)
+    constexpr bool HALF = sizeof(TG) + sizeof(TX) == 4;
+    const bool many = slabs > sm_count();
+    if (!vec) DW_PARTIAL(false, 4, 1);
+    else if (HALF ? many : (many || rows <= 8) && width > 4 * kThreads) DW_PARTIAL(true, 8, 4);
+    else if (HALF && (width > 4 * kThreads || rows <= 8)) DW_PARTIAL(true, 8, 8);
+    else DW_PARTIAL(true, 4, (HALF ? 16 : 8));
+#undef DW_PARTIAL
+}
+
 extern "C" int64_t qmoe_rms_norm_partials(int64_t rows, int64_t width) {
     return rows > 0 && width > 0 ? ((rows + kSlabRows - 1) / kSlabRows) * width : 0;
 }
@@ -419,8 +443,7 @@ extern "C" int qmoe_rms_norm_backward(uint64_t gradient, int32_t g_dtype, uint64
     do {                                                                                                                       \
         if (vec) chained(rms_norm_dx_kernel<TG, TX, true>, grid, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, w, inv, (TX*)dx, rows, width);   \
         else chained(rms_norm_dx_kernel<TG, TX, false>, grid, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, w, inv, (TX*)dx, rows, width);      \
-        if (vec) chained(rms_norm_dw_partial_kernel<TG, TX, true>, (unsigned)slabs, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, inv, part, rows, width); \
-        else chained(rms_norm_dw_partial_kernel<TG, TX, false>, (unsigned)slabs, kThreads, 0, stream, (const TG*)gradient, (const TX*)x, inv, part, rows, width); \
+        launch_dw_partial(vec, (const TG*)gradient, (const TX*)x, inv, part, slabs, rows, width, stream);                                                 \
     } while (0)
     if (g_dtype == QMOE_BF16 && x_dtype == QMOE_BF16) QMOE_RMS_BACKWARD(__nv_bfloat16, __nv_bfloat16);
     else if (g_dtype == QMOE_BF16) QMOE_RMS_BACKWARD(__nv_bfloat16, float);

@@ -66,6 +66,25 @@ def test_rms_norm_bf16_rows_against_the_oracle(rows, width):
     assert np.array_equal(to_host(again), to_host(dw))   # fixed summation order
 
 
+# both sides of the rule that says how many columns a thread of the weight gradient owns and how many rows it has in flight: 8 rows, a slab of 32
+# rows for each of 148 SMs, 1024 columns; slabs that end after 1, 9 and 32 rows, and a second walk over the columns
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rows,width", [(8, 72), (9, 72), (41, 1032), (4736, 72), (4737, 264), (4737, 1032), (4800, 2056)])
+def test_norm_weight_gradient_in_every_form(rows, width, dtype):
+    from gpu_util import to_device, to_host
+    from qutai_b200 import cuda_lm
+
+    rng = np.random.default_rng(rows + width)
+    x, grad = (to_device(rng.standard_normal((rows, width)), dtype) for _ in range(2))
+    weight = to_device(1.0 + 0.1 * rng.standard_normal(width), "float32")
+    _, inverse = cuda_lm.rms_norm(x, weight, width, 1e-6)
+    _, dw = cuda_lm.rms_norm_backward(grad, x, weight, inverse, width)
+    g, v, inv = to_host(grad, (rows, width)), to_host(x, (rows, width)), to_host(inverse)[:, None]
+    # products rounded once and added in fp32: slabs of 32 in a chain, then at most 19 slabs in a chain and the eight chains
+    bound = 2.0 ** -24 * (2 + 32 + 19 + 8) * np.abs(g * v * inv).sum(0)
+    assert (np.abs(to_host(dw) - (g * v * inv).sum(0)) <= bound).all()
+
+
 def test_rope_matches_the_upstream_fixture_and_undoes_itself():
     from gpu_util import to_device, to_host
     from qutai_b200 import cuda_lm
