@@ -150,8 +150,9 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         rem -= turn * per_product;
         const int e = s_order[slot];
         tile.expert = e;
-        tile.row0 = (p.columns_first ? rem / p.n_tiles : rem % p.m_tiles) * (BM * CTAS) + cta_rank * BM;
-        tile.n0 = (p.columns_first ? rem % p.n_tiles : rem / p.m_tiles) * TN;
+        const int along = p.columns_first ? p.n_tiles : p.m_tiles, line = rem / along, at = rem - line * along;
+        tile.row0 = (p.columns_first ? line : at) * (BM * CTAS) + cta_rank * BM;
+        tile.n0 = (p.columns_first ? at : line) * TN;
         int count = s_pair[e];            // WGRAD keeps the row counts in this table
         tile.krow0 = s_start[e] * kRowPad;
         if (p.sum_rows > 0) {
@@ -174,12 +175,13 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams& p, const StartTabl
         const int e = lo;
         const int groups = first_of(e + 1) - first_of(e);
         const int local = t - (first_of(e) - first) * p.n_tiles;
-        const int m_tile = (p.columns_first ? local / p.n_tiles : local % groups) * CTAS + cta_rank;  // 128-row tile inside the expert
+        const int along = p.columns_first ? p.n_tiles : groups, line = local / along, at = local - line * along;
+        const int m_tile = (p.columns_first ? line : at) * CTAS + cta_rank;  // 128-row tile inside the expert
         const int start = s_start[e];
         tile.expert = e;
         tile.row0 = (start + m_tile) * BM;
         tile.rows_valid = m_tile < s_start[e + 1] - start;
-        tile.n0 = (p.columns_first ? local % p.n_tiles : local / groups) * (MODE == MODE_SWIGLU ? 128 : TN);
+        tile.n0 = (p.columns_first ? at : line) * (MODE == MODE_SWIGLU ? 128 : TN);
         tile.kblocks = ((p.K + BK - 1) / BK) * p.segments;
         tile.krow0 = 0;
     }
