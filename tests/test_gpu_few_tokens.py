@@ -11,14 +11,25 @@ from oracle import moe_oracle as oracle
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("counts,width,hidden", [
-    ((0, 1, 15, 16), 64, 128),               # 32 tokens; fewer k-blocks than stages
-    ((32,), 584, 136),                       # one expert with every row, widths that fill no tile
-    ((33,), 584, 136),                       # one token more: the form with 128 rows per stage
-    ((0, 17, 2, 0, 0, 13), 1032, 264),       # two steps of 16 rows; more k-blocks than stages
-    ((1,) * 30, 2048, 1408),                 # more than two tiles per SM: the form with 128 rows per stage
+def few_tokens(tokens, top_k, experts, tiles_per_expert, sms=148):
+    """The rule of ``few_tokens`` in csrc/gemm_stream.cu, restated: at most 32 tokens, and two tiles per SM for the experts that uniform load reaches."""
+    return tokens <= 32 and (1 - (1 - min(1, top_k / experts)) ** tokens) * experts * tiles_per_expert <= 2 * sms
+
+
+@pytest.mark.parametrize("counts,width,hidden,forms", [      # forms: whether gate and up, and down, are in the form for few tokens
+    ((0, 1, 15, 16), 64, 128, (True, True)),                 # 32 tokens; fewer k-blocks than stages
+    ((32,), 584, 136, (True, True)),                         # one expert with every row, widths that fill no tile
+    ((33,), 584, 136, (False, False)),                       # one token more
+    ((0, 17, 2, 0, 0, 13), 1032, 264, (True, True)),         # two steps of 16 rows; more k-blocks than stages
+    ((1,) * 30, 2048, 1408, (True, False)),                  # 211 tiles of the hidden width and 306 of the other, against two for every SM
+    ((1,) * 30, 1408, 2048, (False, True)),                  # the other way round: down by itself in the form for few tokens, which then does not start early
+    ((1,) * 30, 2048, 2048, (False, False)),
 ])
-def test_products_of_few_tokens(counts, width, hidden, kernel_variant):
+def test_products_of_few_tokens(counts, width, hidden, forms, kernel_variant):
+    from qutai_b200 import lib
+
+    assert lib.device_info()["sm_count"] == 148
+    assert forms == tuple(few_tokens(sum(counts), 1, len(counts), -(-columns // 128)) for columns in (hidden, width))
     few_rows.test_streamed_products_match_the_kernel_for_many_rows(counts, width, hidden, kernel_variant)
 
 
