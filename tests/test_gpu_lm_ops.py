@@ -105,6 +105,24 @@ def test_rope_matches_the_upstream_fixture_and_undoes_itself():
     assert oracle.elementwise_err(got, oracle.rope(big, 4, 10000.0), bf16=True) <= 0.012
 
 
+# heads in fours of a thread: one, part of one, a second one of two and of one, four of four; a width that the kernel for heads of any width takes
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,dim", [(1, 64), (3, 8), (6, 64), (10, 32), (9, 72), (16, 64), (6, 66)])
+def test_rope_of_any_number_of_heads(heads, dim, dtype):
+    from gpu_util import to_device, to_host
+    from qutai_b200 import cuda_lm
+
+    shape = (2, 301, heads * dim)
+    values = to_device(np.random.default_rng(heads + dim).standard_normal(shape), dtype)
+    got = to_host(cuda_lm.rope(values, 2, 301, heads, dim, 10000.0, 3), shape)
+    want = oracle.rope(to_host(values, shape), heads, 10000.0, 3)
+    if dtype == "float32":
+        # an angle of up to 304, its two factors and their product rounded to 2^-24 each, turns its pair by as much; the rest is rounding
+        assert np.abs(got - want).max() <= 2.0 ** -24 * (4 * 304 + 8) * np.abs(want).max()
+    else:
+        assert oracle.elementwise_err(got, want, bf16=True) <= 0.012
+
+
 def test_embedding_and_its_backward_match_the_upstream_fixture():
     from gpu_util import to_device, to_host
     from qutai_b200 import cuda_lm
