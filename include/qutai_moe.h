@@ -117,12 +117,12 @@ int qmoe_device_status_async(uint64_t stream, void* host_status);
  * parity tests run against the default form.  value 0 = default, 1 = comparison form.  Not for production
  * hosts: the defaults are the measured-faster forms. */
 enum {
-    QMOE_VARIANT_SINGLE_CTA_GEMM = 0,   /* expert GEMMs with one CTA per 128 x 256 tile instead of a CTA pair per 256 x 256 */
+    QMOE_VARIANT_SINGLE_CTA_GEMM = 0,   /* expert and plain GEMMs with one CTA per 128 x 256 tile instead of a CTA pair per 256 x 256, or of one CTA per 128 x 64 */
     QMOE_VARIANT_WGRAD_PER_PRODUCT = 1, /* one launch per weight-gradient product instead of one for all three */
     QMOE_VARIANT_NARROW_SCATTER = 2,    /* 64-byte instead of 256-byte row pieces in the peer-memory scatter epilogues */
     QMOE_VARIANT_PLAIN_GEMM_ON_CUDA_CORES = 3, /* qmoe_gemm never takes the tensor-core kernels */
     QMOE_VARIANT_NO_STREAM_GEMM = 4,    /* expert products of few rows on the kernel for many rows */
-    QMOE_VARIANT_NO_FLOAT32_TILES = 5,  /* float32 products on the general CUDA-core kernel, never on 128 x 128 tiles */
+    QMOE_VARIANT_NO_FLOAT32_TILES = 5,  /* float32 products on the general CUDA-core kernel, never on 128 x 128 or 128 x 256 tiles */
     QMOE_VARIANT_COUNT = 6
 };
 int qmoe_test_select_variant(int32_t which, int32_t value);

@@ -59,8 +59,8 @@ struct TimedScope {  // records a pair of events around the launches made while 
 // the down product follows for few tokens (gemm_stream.cu).  The CUDA-core products are launched in the ordinary way (see there).
 // One kernel reads before its wait: a product for few rows fetches tables (load_l2) and weights (TMA, which reads the L2) that nothing within the
 // last launch wrote (gemm_stream.cu).
-// 3001 rows, 16 experts, forward and backward (27 launches): 472 us in ordinary launches, 440 like this; 64 rows over 64 experts, replayed, L2
-// flushed: 220 and 215.
+// 3001 rows, 16 experts, forward and backward (27 launches when this was measured, 21 now): 472 us in ordinary launches, 440 like this; 64 rows over 64
+// experts, replayed, L2 flushed: 220 and 215.
 // The wait is a volatile statement that clobbers memory, and griddepcontrol.wait is what orders the kernel's loads behind the writes of the
 // one before; no load is declared free of order (no __ldg, loads in inline PTX are volatile), and parameters that are const __restrict__ are read
 // behind it in program order.

@@ -528,12 +528,11 @@ grouped_gemm_kernel(const __grid_constant__ GemmParams p) {
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        // One elected lane.  Inside a test of the lane number every tcgen05 and TMA instruction took its thread of the order of a
-        // hundred cycles (operands moved to uniform registers lane by lane), and 578 .. 606 cycles passed per k-block, whose tensor work is 512;
-        // like this 520 .. 530 where DRAM keeps up (8188 x 32000 x 1024).  Where the power limit sets the clock it is worth less: 16384 rows,
-        // 8 experts, 1024 x 2816, forward and backward 1827 -> 1791 us; 3001 rows, 16 experts, 1024 x 2048, 440 -> 434 (three weight gradients
-        // 97.6 -> 94.4, dX 60.8 -> 58.7).  The lane walks the k-blocks by itself: a warp that waits, votes and elects per k-block is as
-        // fast on 256 columns, but not on 128 x 64 tiles (weight gradient of 4096 rows, 1024 x 512, 21.5 us, like this 15.7).
+        // One elected lane.  Inside a test of the lane number 578 .. 606 cycles passed per k-block, whose tensor work is 512; with a lane elected
+        // for every k-block 520 .. 530 where DRAM keeps up (8188 x 32000 x 1024), three weight gradients of 3001 rows, 16 experts, 1024 x 2048,
+        // 97.6 -> 94.4 us, dX 60.8 -> 58.7 (the call 440 -> 434); where the power limit sets the clock (16384 rows, 8 experts) no more than runs differ by.  A lane
+        // that is elected once and walks the k-blocks by itself is as fast on 256 columns (the same call 428 .. 426 since) and faster
+        // on 128 x 64 tiles (weight gradient of 4096 rows, 1024 x 512, 21.5 us with a warp that waits, votes and elects, like this 15.7).
         if (cta_rank == 0 && elect_one()) {
             int stage = 0;
             uint32_t phase = 0;

@@ -203,8 +203,10 @@ qmoe_route_t one_group_route(long long rows) {
 // one long product grows with k, that of an FMA chain with its root (2-norm, from the exact product: 602 rows 5.7e-7 in one
 // product, 1.8e-7 in a chain; 8191 rows 9.1e-6 and 9.6e-7); an eighth of k, between 64 and 512 rows, keeps the sum below the chain's.
 constexpr long long kRaggedContraction = 128;
-// Ragged rows with an inner size of less than one k-block are the CUDA cores' too: a tensor-core launch takes 9 .. 11 us
-// (L2 flushed) before there is work, 4503 x 32 x 64 9 us there and 11 here, 60001 x 16 x 16 11 and 19; at 64 they are even (4503 x 64 x 64 11 and 11).
+// Ragged rows with an inner size of less than one k-block are the CUDA cores' too.  The line was drawn for tiles of 256 x 256, which were even with the CUDA
+// cores at 64 (4503 x 64 x 64 11 us on both, L2 flushed).  Since the tiles of 128 x 64 it lies high by time: CUDA cores and tensor
+// cores, us in a loop, 60001 x 16 x 16 8.3 and 14.4, 2001 x 16 x 1024 8.3 and 7.2, 4503 x 32 x 64 6.3 and 3.9 (L2 flushed 10.2 and 9.2), 9001 x 56 x 1024 56 and 10; but
+// the calls below it have the sums of an FMA chain, which tensor memory, dropping low bits, does not give.
 constexpr long long kRaggedInner = 64;
 int ragged_sum_rows(long long k) {
     const long long rows = (k / 8 + 63) / 64 * 64;
@@ -219,7 +221,7 @@ int ragged_sum_rows(long long k) {
 // kRaggedInner on, of the first two; K, from kRaggedContraction on, of the third) need be no multiple of anything: TMA fills the
 // last tile with zeros and its rows past the end are not stored.  What must be a multiple of 8 is what a row pitch is made of (16 bytes): K and N of the
 // first two, M and N of the third.
-// 602 rows, 512 x 512: 40 us on the CUDA cores (74 for the weight gradient), 10 .. 14 here (21).
+// 602 rows, 512 x 512, us in a loop: 41 on the CUDA cores (48 for the weight gradient), 5.3 here (8.0).
 extern "C" int qmoe_gemm(uint64_t a, int32_t a_dtype, uint64_t b, int32_t b_dtype, uint64_t c, int32_t c_dtype, int64_t m,
                          int64_t k, int64_t n, int32_t transpose_a, int32_t transpose_b, int32_t accumulate, uint64_t stream_) {
     if (!a || !b || !c) return fail_arg("gemm: null address");

@@ -151,12 +151,15 @@ router_reduce_dw_kernel(const float* __restrict__ partial, const float* __restri
 // Few tokens (decode): one block per token, a warp per expert in turn, fp32 dot products with the lanes
 // striding over the width and a fixed shuffle tree, so the logits are run-to-run identical.  A tile kernel
 // would put the whole product on one or two SMs and walk the width serially.
-// The warps of a token read every weight row again, from L2: up to 512 tokens that is the shorter way whatever the sizes (602
-// tokens, 8 experts, d 512, with the norm: 4 us in one launch, 15 in five).  Beyond them by an estimate of both ways, in us beyond
+// The warps of a token read every weight row again, from L2: up to 512 tokens that is the shorter way whatever the sizes (a call of 600
+// tokens, 32 experts, d 584, with the norm: 40 us, 43 with the logits on the tensor cores).  Beyond them by an estimate of both ways, in us beyond
 // what a launch takes, fitted to 600 .. 65536 tokens, 1 .. 128 experts, widths 64 .. 4096 with L2 flushed: this kernel takes a
 // block's issue per 8 logits (16384 x 16 x 64: 46 us) or the weight reads (32768 x 16 x 2048: 293); three times that when the
 // width is no multiple of 4, half as much again with the norm; the tile kernel a chain of `width` products per tile until its
 // tiles fill the machine (16 and 212); the tensor cores two launches and little else (bf16, 16384 x 16 x 64: 13, against 50 here).
+// With the norm the CUDA cores' other way has three launches more, 9 us.  The tensor cores' has none more (router_forward_scaled) and by time would
+// be worth 3: of what the 9 leave here, calls of 1000 x 64 x 256 take 45 us and 41 there, 2000 x 32 x 256 51 and 44, 4000 x 16 x 256 52 and 44, 8000 x 8 x 256 56 and 47.  They stay
+// for their precision: the logits' error here is 0.97e-7 of their norm, there 2.3e-7 (width 256; 4.7e-7 at 512).
 constexpr long long kSmallRouterTokens = 512, kSmallRouterProducts = 1ll << 24;
 bool small_router(long long tokens, int experts, long long width, int x_dtype, bool tensor_cores, bool norm) {
     if (tokens <= kSmallRouterTokens) return true;
@@ -165,7 +168,7 @@ bool small_router(long long tokens, int experts, long long width, int x_dtype, b
     const double blocks = T * (4.5e-4 * ((experts + 7) / 8) + 1e-4 * experts), reads = T * experts * (3e-5 + 2.7e-7 * d);
     const double here = (blocks > reads ? blocks : reads) * (width % 4 ? 3 : 1) * (norm ? 1.5 : 1);
     const double there = tensor_cores ? 6 + 5.6e-3 * d + 6e-7 * T * d : 7.5e-2 * d * (T > 30000 ? T / 30000 : 1);
-    return here <= there + (norm ? 9 : 0);     // with the norm: three launches more
+    return here <= there + (norm ? 9 : 0);
 }
 // grid (tokens, ceil(E / 8)): warp w of block (t, g) computes scores[t, 8 g + w]
 template <typename T, bool NORM>

@@ -376,8 +376,8 @@ route_small_kernel(const float* __restrict__ scores, float* __restrict__ probs, 
 }
 
 // The logits of a handful of tokens and their routing in one launch, a warp per logit.  us a call, in two launches and one: 4 rows, 8 experts,
-// 1024 x 2816, norm to residual, called step by step 45.2 and 42.7 (its launches bound the host), the device alone 38.9 and 39.1; 1 row of
-// 2048, 32 experts, 32.7 and 33.1.  A second logit per warp is a second round trip: 8 rows, 8 experts, 39.8 and 41.5, 2 rows, 32 experts, 41.9 and 45.0.
+// 1024 x 2816, norm to residual, called step by step 45.2 and 42.7 (its launches bound the host), the device alone 38.9 and 39.1; replayed without the
+// norm 33.1 and 33.0, 1 row, 32 experts, 2048 x 1408, 41.2 .. 42.0 and 41.1, 1 row, 8 experts, 512 x 264, 22.6 and 20.6.  A second logit per warp is a second round trip: 8 rows, 8 experts, 39.8 and 41.5, 2 rows, 32 experts, 41.9 and 45.0.
 constexpr int kRouterRouteLogits = kWarps;
 template <typename X, bool NORM>
 __global__ void __launch_bounds__(kWarps * 32, 1)
