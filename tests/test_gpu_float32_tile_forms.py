@@ -24,9 +24,10 @@ def tile_form(shapes, *, mode=0, a_kfast=True, b_kfast=False, groups=1, row_tile
 
 
 # (m, k, n) and the form: wide tiles with 4, 132, 252 and 256 columns in the last and 68, 128 and 4 rows; one tile to an SM, few and as many as
-# there are; two; inner sizes of whole slices, part of one, and below the rule's 128
-SHAPES = [(2500, 128, 1028, WIDE), (2560, 140, 1156, WIDE), (2564, 132, 1276, WIDE), (4096, 260, 1024, WIDE), (644, 300, 2500, ONE), (508, 144, 4732, ONE),
-          (4100, 132, 1280, TWO), (2500, 124, 1028, TWO)]
+# there are; two, many and, with inner sizes below the rule's 128, few; inner sizes of whole slices, one value more and one less
+SHAPES = [(2500, 128, 1028, WIDE), (2560, 143, 1156, WIDE), (2564, 129, 1276, WIDE), (4096, 260, 1024, WIDE), (644, 301, 2500, ONE), (508, 144, 4732, ONE),
+          (640, 640, 2560, ONE), (4100, 129, 1280, TWO), (2500, 124, 1028, TWO), (1024, 16, 1024, TWO), (2048, 33, 1028, TWO), (2044, 47, 1156, TWO),
+          (4096, 64, 1276, TWO), (4100, 48, 1000, TWO)]
 
 
 @pytest.mark.parametrize("form", ["nn", "tn", "tt"])
@@ -36,7 +37,7 @@ def test_tile_forms_give_the_bits_of_the_general_kernel(form, m, k, n, tiles_of,
     from qutai_b200 import lib
     from qutai_b200.storage import DeviceStorage
 
-    k += form == "tn" and tiles_of != TWO       # an odd inner size, where no row is as long
+    k = k if form == "tn" else -(-k // 4) * 4       # whole 16-byte pieces along what is contiguous
     assert tile_form([(m, k, n)], a_kfast=form[0] == "n", b_kfast=form[1] == "t") == tiles_of and lib.device_info()["sm_count"] == SMS
     rng = np.random.default_rng(m + k + n)
     a, b = (to_device(rng.standard_normal(size).astype(np.float32), "float32") for size in (m * k, k * n))
